@@ -124,11 +124,6 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
   }
 }
 
-// FP64 operator with its contractions in fixed point (ax_helm_fx.cu); returns
-// NTG_ERR_UNSUPPORTED where the plain FP64 kernel above is to run.
-int ax_fx_launch(ntg_plan* p, double* w, const double* u, const double* const* g, const double* h1, double h1c,
-                 const double* hB, Scalars* sc, cudaStream_t s);
-
 // TMA-pipelined FP32 kernel for lx = 8 (ax_helm_f32_tma.cu); returns
 // NTG_ERR_UNSUPPORTED when a pointer is not 16-byte aligned.
 int ax_f32_tma_launch(ntg_plan* p, float* w, const float* u, const float* const* g, const float* h1, float h1c,
@@ -178,17 +173,6 @@ static int ax_dispatch(ntg_plan* p, T* w, const T* u, const T* const* g, const T
     case 10: return launch_lx<T, 10>(p, w, u, g, h1, h1c, hB, sc, s);
     default: set_error("ax_helm: lx=%d not compiled", p->lx); return NTG_ERR_UNSUPPORTED;
   }
-}
-
-int ax_launch(ntg_plan* p, double* w, const double* u, Scalars* dot_scal, int, cudaStream_t s) {
-  const double* g[6] = {p->g[0], p->g[1], p->g[2], p->g[3], p->g[4], p->g[5]};
-  timer_start(TM_AX64, s);
-  const double* h1 = p->h1_const ? nullptr : p->h1;
-  const double* hB = p->ifh2 ? p->hB : nullptr;
-  int st = ax_fx_launch(p, w, u, g, h1, p->h1c, hB, dot_scal, s);
-  if (st == NTG_ERR_UNSUPPORTED) st = ax_dispatch<double>(p, w, u, g, h1, p->h1c, hB, dot_scal, s);
-  timer_stop(TM_AX64, s);
-  return st;
 }
 
 int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int, cudaStream_t s) {

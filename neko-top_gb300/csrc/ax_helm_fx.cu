@@ -9,18 +9,12 @@
 namespace ntg {
 
 template <int LX>
-struct FxMats {
-  fx::Mat<LX, LX> D, DT;           // D and scale * D^T
-  double d[LX * LX], dt[LX * LX];  // the same as FP64 numbers
-};
-
-template <int LX>
 struct FxAxShape {
   static constexpr int LX2 = LX * LX, LX3 = LX2 * LX;
   static constexpr int RS = LX | 1, TILE = LX2 * RS;  // odd row stride: rows and columns without bank conflicts
-  static constexpr int EPB = LX >= 7 ? 2 : LX >= 5 ? 4 : 8;
+  static constexpr int EPB = LX == 8 ? 1 : LX <= 3 ? 14 : LX == 4 ? 4 : LX == 6 ? 7 : LX <= 7 ? 5 : 3;
   static constexpr int NW = LX2 * EPB, NT = (NW + 31) / 32 * 32;
-  static constexpr int MINB = 896 / NT;
+  static constexpr int MINB = LX == 8 ? 16 : 896 / NT;
   static constexpr size_t SMEM = EPB * (3 * TILE * sizeof(double) + 2 * LX2 * sizeof(int));
 };
 
@@ -29,7 +23,7 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
     k_ax_fx(double* __restrict__ w, const double* __restrict__ u, const double* __restrict__ g11,
             const double* __restrict__ g12, const double* __restrict__ g13, const double* __restrict__ g22,
             const double* __restrict__ g23, const double* __restrict__ g33, const double* __restrict__ h1,
-            const double* __restrict__ hB, int64_t nelv, const __grid_constant__ FxMats<LX> P,
+            double h1s, const double* __restrict__ hB, int64_t nelv, const __grid_constant__ fx::Mats<LX> P,
             double* __restrict__ part, Scalars* sc) {
   using S = FxAxShape<LX>;
   constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB, RS = S::RS, TILE = S::TILE;
@@ -46,10 +40,6 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
   const int ro = (a + LX * b) * RS;  // row (j, k) = (a, b)
   const int so = LX * b * RS + a;    // column along j at (i, k) = (a, b)
   const int to = b * RS + a;         // column along k at (i, j) = (a, b)
-  auto sync = [&]() {
-    if constexpr (LX == 8) asm volatile("bar.sync %0, 64;" ::"r"(le + 1) : "memory");
-    else __syncthreads();
-  };
   double dot = 0.0;
   for (int64_t grp = blockIdx.x; grp * EPB < nelv; grp += gridDim.x) {
     const int64_t e = grp * EPB + le;
@@ -63,7 +53,7 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
         U[to + k * LX * RS] = wt[k];
       }
     }
-    sync();
+    __syncthreads();
     if (worker) {
       double x[LX];
 #pragma unroll
@@ -76,7 +66,7 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
       for (int l = 0; l < LX; ++l) x[l] = wt[l];
       fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) { wt[A] = y; });
     }
-    sync();
+    __syncthreads();
     if (act) {
 #pragma unroll
       for (int k = 0; k < LX; ++k) {
@@ -84,21 +74,22 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
         const int p = to + k * LX * RS;
         const double ur = R[p], us = V[p], ut = wt[k];
         const double a12 = g12[q], a13 = g13[q], a23 = g23[q];
-        double fr = g11[q] * ur + a12 * us + a13 * ut;
-        double fs = a12 * ur + g22[q] * us + a23 * ut;
-        double ft = a13 * ur + a23 * us + g33[q] * ut;
-        if (h1) {
-          const double hh = h1[q];
-          fr *= hh;
-          fs *= hh;
-          ft *= hh;
+        R[p] = g11[q] * ur + a12 * us + a13 * ut;
+        V[p] = a12 * ur + g22[q] * us + a23 * ut;
+        wt[k] = a13 * ur + a23 * us + g33[q] * ut;
+      }
+      if (h1 || h1s != 1.0) {  // its own loop: a predicated-off FP64 product takes the pipe all the same
+#pragma unroll
+        for (int k = 0; k < LX; ++k) {
+          const int p = to + k * LX * RS;
+          const double hh = h1 ? h1[base + k * LX2] : h1s;
+          R[p] *= hh;
+          V[p] *= hh;
+          wt[k] *= hh;
         }
-        R[p] = fr;
-        V[p] = fs;
-        wt[k] = ft;
       }
     }
-    sync();
+    __syncthreads();
     int64_t Y[LX];
     int kt = fx::kZero;
     if (worker) {
@@ -113,20 +104,23 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
                                           [&](int A, int64_t y) { V[so + A * RS] = __longlong_as_double(y); });
       kt = fx::line_int<LX, LX, true>(P.DT, P.dt, wt, [&](int A, int64_t y) { Y[A] = y; });
     }
-    sync();
+    __syncthreads();
     if (act) {
+      double acc[LX];
 #pragma unroll
       for (int k = 0; k < LX; ++k) {
-        const int64_t q = base + k * LX2;
         const int p = to + k * LX * RS;
-        double acc = fx::sum3(__double_as_longlong(R[p]), kr[b + LX * k], __double_as_longlong(V[p]), ks[a + LX * k],
-                              Y[k], kt);
-        if (DOT || hB) {
-          const double uk = U[p];
-          if (hB) acc = fma(hB[q], uk, acc);
-          if (DOT) dot = fma(uk, acc, dot);
-        }
-        w[q] = acc;
+        acc[k] = fx::sum3(__double_as_longlong(R[p]), kr[b + LX * k], __double_as_longlong(V[p]), ks[a + LX * k],
+                          Y[k], kt);
+      }
+      if (hB) {
+#pragma unroll
+        for (int k = 0; k < LX; ++k) acc[k] = fma(hB[base + k * LX2], U[to + k * LX * RS], acc[k]);
+      }
+#pragma unroll
+      for (int k = 0; k < LX; ++k) {
+        w[base + k * LX2] = acc[k];
+        if (DOT) dot = fma(U[to + k * LX * RS], acc[k], dot);
       }
     }
   }
@@ -140,44 +134,45 @@ template <int LX>
 static int launch_fx(ntg_plan* p, double* w, const double* u, const double* const* g, const double* h1, double h1c,
                      const double* hB, Scalars* sc, cudaStream_t s) {
   using S = FxAxShape<LX>;
-  FxMats<LX> P;
-  for (int i = 0; i < LX; ++i)
-    for (int j = 0; j < LX; ++j) {
-      P.d[i * LX + j] = p->D[i * LX + j];
-      P.dt[i * LX + j] = p->D[j * LX + i] * (h1 ? 1.0 : h1c);
-    }
-  double dt[LX * LX];
-  for (int i = 0; i < LX; ++i)
-    for (int j = 0; j < LX; ++j) dt[i * LX + j] = p->D[j * LX + i];
-  P.D = fx::make_mat<LX, LX>(p->D);
-  P.DT = fx::make_mat<LX, LX>(dt, h1 ? 1.0 : h1c);
+  const double fold = !h1 && fx::foldable(h1c) ? h1c : 1.0;  // a constant h1 goes into D^T
+  const double h1s = h1 || fold == h1c ? 1.0 : h1c;
+  const fx::Mats<LX> P = fx::plan_mats<LX>(p, fold);
   const int64_t ngroups = (p->nelv + S::EPB - 1) / S::EPB, cap = sc ? kRedSlots : (int64_t)1 << 30;
   const int grid = (int)(ngroups < cap ? ngroups : cap);
-  auto run = [&](auto kernel) -> int {
-    NTG_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
-    kernel<<<grid, S::NT, S::SMEM, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, hB, p->nelv, P, p->red_part, sc);
-    NTG_COUNT_LAUNCH();
-    return NTG_OK;
-  };
-  NTG_TRY(sc ? run(k_ax_fx<LX, true>) : run(k_ax_fx<LX, false>));
+  if (sc) {
+    NTG_TRY((fx::use_smem<k_ax_fx<LX, true>>(S::SMEM)));
+    k_ax_fx<LX, true><<<grid, S::NT, S::SMEM, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1s, hB, p->nelv, P,
+                                                   p->red_part, sc);
+  } else {
+    NTG_TRY((fx::use_smem<k_ax_fx<LX, false>>(S::SMEM)));
+    k_ax_fx<LX, false><<<grid, S::NT, S::SMEM, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1s, hB, p->nelv, P,
+                                                    p->red_part, sc);
+  }
+  NTG_COUNT_LAUNCH();
   NTG_CUDA_TRY(cudaGetLastError());
   return NTG_OK;
 }
 
-int ax_fx_launch(ntg_plan* p, double* w, const double* u, const double* const* g, const double* h1, double h1c,
-                 const double* hB, Scalars* sc, cudaStream_t s) {
-  // a constant h1 is folded into D^T, whose exponent offset must stay small
-  if (!h1 && h1c != 0.0 && !(std::fabs(h1c) > 1e-6 && std::fabs(h1c) < 1e6)) return NTG_ERR_UNSUPPORTED;
+int ax_launch(ntg_plan* p, double* w, const double* u, Scalars* dot_scal, int, cudaStream_t s) {
+  const double* g[6] = {p->g[0], p->g[1], p->g[2], p->g[3], p->g[4], p->g[5]};
+  const double* h1 = p->h1_const ? nullptr : p->h1;
+  const double* hB = p->ifh2 ? p->hB : nullptr;
+  timer_start(TM_AX64, s);
+  int st = NTG_OK;
   switch (p->lx) {
-    case 4: return launch_fx<4>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 5: return launch_fx<5>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 6: return launch_fx<6>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 7: return launch_fx<7>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 8: return launch_fx<8>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 9: return launch_fx<9>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 10: return launch_fx<10>(p, w, u, g, h1, h1c, hB, sc, s);
-    default: return NTG_ERR_UNSUPPORTED;
+    case 2: st = launch_fx<2>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 3: st = launch_fx<3>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 4: st = launch_fx<4>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 5: st = launch_fx<5>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 6: st = launch_fx<6>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 7: st = launch_fx<7>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 8: st = launch_fx<8>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 9: st = launch_fx<9>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    case 10: st = launch_fx<10>(p, w, u, g, h1, p->h1c, hB, dot_scal, s); break;
+    default: set_error("ax_helm: lx=%d not compiled", p->lx); st = NTG_ERR_UNSUPPORTED;
   }
+  timer_stop(TM_AX64, s);
+  return st;
 }
 
 }  // namespace ntg

@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -151,6 +153,17 @@ struct ntg_plan {
   double* binv = nullptr;
   double* dscr = nullptr;  // their scratch (plan_scratch)
   int64_t dscr_n = 0;
+  // fixed-point forms of D and D^T (fx.cuh), made on first use
+  struct FxCache {
+    std::mutex mu;
+    struct Entry {
+      double scale;
+      bool weighted;
+      std::shared_ptr<void> mats;
+    };
+    std::vector<Entry> mats;
+  };
+  std::unique_ptr<FxCache> fx{new FxCache};
 };
 
 namespace ntg {
@@ -177,6 +190,8 @@ int ax_launch(ntg_plan* p, double* w, const double* u, Scalars* dot_scal, int do
 int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int dot_slot, cudaStream_t s);
 int gs_launch(ntg_plan* p, double* u, int op, cudaStream_t s);
 int gs_launch_f32(ntg_plan* p, float* u, int op, cudaStream_t s);
+int gs_launch3(ntg_plan* p, double* u0, double* u1, double* u2, cudaStream_t s);
+int gs_cls_launch3(ntg_plan* p, double* u0, double* u1, double* u2, cudaStream_t s);
 int mask_launch(ntg_plan* p, double* u, cudaStream_t s);
 int mask_launch_f32(ntg_plan* p, float* u, cudaStream_t s);
 // assembled masked operator w = mask(gs(A u)); optional fused (u, Au_local)

@@ -17,10 +17,11 @@
 //             half as many products as the full matrix has;
 //   from_fix  the 64-bit sum becomes an FP64 number, rounded to nearest.
 //
-// Error: products of the low limbs (2^-60 of the largest matrix entry times
-// the largest line entry) and the last bit of the sum (2^-57) are dropped,
-// which is below the rounding of the eight FP64 FMAs it replaces; each line
-// has its own exponent, so a small line beside a large one loses nothing.
+// Error: products of the low limbs and the last bit of the sum are dropped,
+// 2^-56 of the row's largest entry times the line's largest; the eight FP64
+// FMAs replaced round by more.  Each line has its own exponent and each row
+// of the matrix its own scale, so a small line beside a large one, or an
+// inner row beside an end row, loses nothing.
 //
 // Lines whose largest entry is outside [2^-913, 2^977] (NaN and infinity
 // included) take the plain FP64 sum instead (`ok` false): same results as
@@ -28,7 +29,10 @@
 #pragma once
 #include <stdint.h>
 #include <algorithm>
+#include <atomic>
 #include <cmath>
+#include <memory>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -47,39 +51,115 @@ struct Mat {
   // bits of the line integers: sums of HE products of both limbs stay inside 63 bits
   static constexpr int XB = HE <= 5 ? 60 : 59;
   int eh[RO][HE], el[RO][HE], oh[RO][HO], ol[RO][HO];
-  int k0;  // exponent offset of the result: y = Y 2^(E + k0 - 1023)
+  // every row is scaled to 60 bits by itself (the rows of a derivative matrix
+  // differ by a factor of ten): y_A = Y_A 2^(E + k[A] - 1023); the common
+  // scale of line_int is kc, Y_A 2^s[A] under it
+  int k[RO], s[RO], kc;
 };
 
-// host: M row-major (NOUT x NIN), centro-symmetric (+1) or -antisymmetric, times scale
-template <int NIN, int NOUT>
-Mat<NIN, NOUT> make_mat(const double* M, double scale = 1.0) {
+// host: M row-major (NOUT x NIN), centro-symmetric or -antisymmetric
+template <int NIN, int NOUT, typename T0>
+Mat<NIN, NOUT> make_mat(const T0* M) {
   using T = Mat<NIN, NOUT>;
   T r;
-  long double e[T::RO][T::HE], o[T::RO][T::HO], mx = 0;
+  long double e[T::RO][T::HE], o[T::RO][T::HO];
+  int ex[T::RO], top = -100000;
   for (int A = 0; A < T::RO; ++A) {
+    long double mx = 0;
     for (int a = 0; a < T::HE; ++a) {
       const int b = NIN - 1 - a;
-      const long double p = (long double)M[A * NIN + a] * scale, q = (long double)M[A * NIN + b] * scale;
+      const long double p = M[A * NIN + a], q = M[A * NIN + b];
       e[A][a] = a == b ? p : 0.5L * (p + q);
-      if (a < T::HO) o[A][a] = 0.5L * (p - q);
       mx = std::max(mx, std::fabs(e[A][a]));
-      if (a < T::HO) mx = std::max(mx, std::fabs(o[A][a]));
+      if (a < T::HO) {
+        o[A][a] = 0.5L * (p - q);
+        mx = std::max(mx, std::fabs(o[A][a]));
+      }
     }
+    ex[A] = -100000;
+    if (mx > 0) std::frexp(mx, &ex[A]);  // mx in [2^(ex-1), 2^ex)
+    top = std::max(top, ex[A]);
   }
-  int ex = 0;
-  if (mx > 0) std::frexp(mx, &ex);  // mx in [2^(ex-1), 2^ex)
-  const int sh = 60 - ex;
-  auto put = [&](long double v, int& h, int& l) {
-    const int64_t q = (int64_t)std::llrint(std::ldexp(v, sh));
-    l = (int32_t)(uint32_t)(q & 0xffffffffll);
-    h = (int32_t)((q - (int64_t)l) >> 32);
-  };
+  if (top == -100000) top = 0;
+  // a row's result under the common scale, and the sum of three of them, stay
+  // inside 63 bits: |Y_A| <= 2^(XB - 4) sum |M_Aa| / 2^ex, and sum |M_Aa| < 8 2^ex here
+  constexpr int LEFT = 63 - 2 - 3 - (T::XB - 4);
+  static_assert(LEFT >= 2, "bits");
   for (int A = 0; A < T::RO; ++A) {
+    ex[A] = std::max(ex[A], top - LEFT);
+    const int sh = 60 - ex[A];
+    auto put = [&](long double v, int& h, int& l) {
+      const int64_t q = (int64_t)std::llrint(std::ldexp(v, sh));
+      l = (int32_t)(uint32_t)(q & 0xffffffffll);
+      h = (int32_t)((q - (int64_t)l) >> 32);
+    };
     for (int a = 0; a < T::HE; ++a) put(e[A][a], r.eh[A][a], r.el[A][a]);
     for (int a = 0; a < T::HO; ++a) put(o[A][a], r.oh[A][a], r.ol[A][a]);
+    r.k[A] = 64 - sh - T::XB + 1;
   }
-  r.k0 = 64 - sh - T::XB + 1;
+  r.kc = 64 - (60 - top) - T::XB + 1 - LEFT;
+  for (int A = 0; A < T::RO; ++A) r.s[A] = r.k[A] - r.kc;
   return r;
+}
+
+// the derivative matrix of the GLL points, its transpose times `scale`, and
+// both as FP64 numbers
+template <int LX>
+struct Mats {
+  Mat<LX, LX> D, DT;
+  double d[LX * LX], dt[LX * LX];
+};
+
+// w: null, or weights for the form of D^T that acts before them:
+// DT = W^-1 D^T W, so that D^T (W f) = W (DT f)
+template <int LX>
+Mats<LX> make_mats(const double* D, const double* w, double scale) {
+  Mats<LX> P;
+  long double t[LX * LX];
+  for (int i = 0; i < LX; ++i)
+    for (int j = 0; j < LX; ++j) {
+      t[i * LX + j] = (long double)D[j * LX + i] * scale;
+      if (w) t[i * LX + j] = t[i * LX + j] * w[j] / w[i];
+      P.d[i * LX + j] = D[i * LX + j];
+      P.dt[i * LX + j] = (double)t[i * LX + j];
+    }
+  P.D = make_mat<LX, LX>(D);
+  P.DT = make_mat<LX, LX>(t);
+  return P;
+}
+
+// The plan's matrices, made once per plan and scale (a constant h1 or mu).
+// The few scales in use at a time stay; a copy goes to the caller, so plans
+// may be used from several threads.
+// `weighted`: the D^T that acts before the GLL weights (make_mats).
+template <int LX>
+Mats<LX> plan_mats(const ntg_plan* p, double scale, bool weighted = false) {
+  std::lock_guard<std::mutex> lk(p->fx->mu);
+  auto& c = p->fx->mats;
+  for (auto& e : c)
+    if (e.scale == scale && e.weighted == weighted) return *static_cast<const Mats<LX>*>(e.mats.get());
+  if (c.size() >= 6) c.erase(c.begin());
+  auto m = std::make_shared<Mats<LX>>(make_mats<LX>(p->D, weighted ? p->wq : nullptr, scale));
+  c.push_back({scale, weighted, m});
+  return *m;
+}
+
+// whether a constant factor may be folded into a matrix (its exponent offset must stay small)
+inline bool foldable(double c) { return c == 0.0 || (std::fabs(c) > 1e-6 && std::fabs(c) < 1e6); }
+
+// lets Kernel use `bytes` of dynamic shared memory and the largest carve-out; set once per device
+template <auto Kernel>
+int use_smem(size_t bytes) {
+  static std::atomic<uint64_t> set{0};
+  int dev = 0;
+  NTG_CUDA_TRY(cudaGetDevice(&dev));
+  const uint64_t bit = 1ull << (dev & 63);
+  if (set.load(std::memory_order_acquire) & bit) return NTG_OK;
+  NTG_CUDA_TRY(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  NTG_CUDA_TRY(cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                    cudaSharedmemCarveoutMaxShared));
+  set.fetch_or(bit, std::memory_order_release);
+  return NTG_OK;
 }
 
 __device__ __forceinline__ int64_t mk64(uint32_t lo, uint32_t hi) {
@@ -156,7 +236,8 @@ __device__ __forceinline__ int64_t dot_limbs(const int (&mh)[NT], const int (&ml
   return hh + (mid >> 32);
 }
 
-// Y = M X for a line of integers; out(A, Y_A) per output
+// Y = M X for a line of integers; out(A, row, Y_A) per output, row = the
+// one of the mirrored rows A, NOUT-1-A whose scale holds
 template <int NIN, int NOUT, bool ANTI, typename F>
 __device__ __forceinline__ void line(const Mat<NIN, NOUT>& M, const int64_t (&X)[NIN], F&& out) {
   using T = Mat<NIN, NOUT>;
@@ -178,11 +259,11 @@ __device__ __forceinline__ void line(const Mat<NIN, NOUT>& M, const int64_t (&X)
   for (int A = 0; A < T::RO; ++A) {
     const int B = NOUT - 1 - A;
     if (A == B) {
-      out(A, ANTI ? dot_limbs<T::HO>(M.oh[A], M.ol[A], oh, ol) : dot_limbs<T::HE>(M.eh[A], M.el[A], eh, el));
+      out(A, A, ANTI ? dot_limbs<T::HO>(M.oh[A], M.ol[A], oh, ol) : dot_limbs<T::HE>(M.eh[A], M.el[A], eh, el));
     } else {
       const int64_t p = dot_limbs<T::HE>(M.eh[A], M.el[A], eh, el), q = dot_limbs<T::HO>(M.oh[A], M.ol[A], oh, ol);
-      out(A, p + q);
-      out(B, ANTI ? q - p : p - q);
+      out(A, A, p + q);
+      out(B, A, ANTI ? q - p : p - q);
     }
   }
 }
@@ -198,8 +279,8 @@ __device__ __forceinline__ int line_int(const Mat<NIN, NOUT>& M, const double* M
     int64_t X[NIN];
 #pragma unroll
     for (int l = 0; l < NIN; ++l) X[l] = to_fix<Mat<NIN, NOUT>::XB>(x[l], E);
-    line<NIN, NOUT, ANTI>(M, X, out);
-    return E + M.k0;
+    line<NIN, NOUT, ANTI>(M, X, [&](int A, int row, int64_t Y) { out(A, shl(Y, M.s[row])); });
+    return E + M.kc;
   }
 #pragma unroll
   for (int A = 0; A < NOUT; ++A) {
@@ -221,8 +302,7 @@ __device__ __forceinline__ void line_dbl(const Mat<NIN, NOUT>& M, const double* 
     int64_t X[NIN];
 #pragma unroll
     for (int l = 0; l < NIN; ++l) X[l] = to_fix<Mat<NIN, NOUT>::XB>(x[l], E);
-    const int K = E + M.k0;
-    line<NIN, NOUT, ANTI>(M, X, [&](int A, int64_t Y) { out(A, from_fix(Y, K)); });
+    line<NIN, NOUT, ANTI>(M, X, [&](int A, int row, int64_t Y) { out(A, from_fix(Y, E + M.k[row])); });
     return;
   }
 #pragma unroll
@@ -244,6 +324,50 @@ __device__ __forceinline__ double sum3(int64_t a, int Ka, int64_t b, int Kb, int
   const double y = Kb == kSlow ? __longlong_as_double(b) : from_fix(b, Kb);
   const double z = Kc == kSlow ? __longlong_as_double(c) : from_fix(c, Kc);
   return x + y + z;
+}
+
+// A tile of L^3 FP64 numbers in shared memory with an odd row stride: the
+// lines of all three directions are read and written without bank conflicts.
+template <int L>
+struct Tile {
+  static constexpr int L2 = L * L, L3 = L2 * L, RS = L | 1, SIZE = L2 * RS;
+  static __device__ __forceinline__ int at(int node) { return node / L * RS + node % L; }
+  // first entry and stride of line q (0 .. L2-1) of direction d
+  static __device__ __forceinline__ int base(int d, int q) {
+    const int p = q % L, r = q / L;
+    return d == 0 ? (p + L * r) * RS : d == 1 ? L * r * RS + p : r * RS + p;
+  }
+  static __device__ __forceinline__ int stride(int d) { return d == 0 ? 1 : d == 1 ? RS : L * RS; }
+};
+
+// the derivative tile of direction d of `in`, line q, into `out` (which may be `in`)
+template <int L>
+__device__ __forceinline__ void deriv_line(const Mat<L, L>& D, const double* d_, const double* in, double* out, int d,
+                                           int q) {
+  const int b = Tile<L>::base(d, q), st = Tile<L>::stride(d);
+  double x[L];
+#pragma unroll
+  for (int l = 0; l < L; ++l) x[l] = in[b + l * st];
+  line_dbl<L, L, true>(D, d_, x, [&](int A, double y) { out[b + A * st] = y; });
+}
+
+// the transposed derivative of a flux tile in place, as integers; *k: their exponent
+template <int L>
+__device__ __forceinline__ void flux_line(const Mat<L, L>& DT, const double* dt_, double* f, int* k, int d, int q) {
+  const int b = Tile<L>::base(d, q), st = Tile<L>::stride(d);
+  double x[L];
+#pragma unroll
+  for (int l = 0; l < L; ++l) x[l] = f[b + l * st];
+  *k = line_int<L, L, true>(DT, dt_, x, [&](int A, int64_t y) { f[b + A * st] = __longlong_as_double(y); });
+}
+
+// the sum of the three transposed derivatives at a node: f[d], k[d] (k + d L2) of flux_line
+template <int L>
+__device__ __forceinline__ double flux_sum(const double* f0, const double* f1, const double* f2, const int* k, int node) {
+  constexpr int L2 = L * L;
+  const int i = node % L, j = node / L % L, kk = node / L2, p = Tile<L>::at(node);
+  return sum3(__double_as_longlong(f0[p]), k[j + L * kk], __double_as_longlong(f1[p]), k[L2 + i + L * kk],
+              __double_as_longlong(f2[p]), k[2 * L2 + i + L * j]);
 }
 
 }  // namespace fx
