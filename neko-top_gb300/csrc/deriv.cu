@@ -18,10 +18,9 @@
 //       f += scale curl(curl(u)), kept inside a zone (mask_exterior_const,
 //       sources/neko_ext/mask_ops.f90:55-82) when one is given
 //
-// Layout and mapping as ax_helm: one element per LX x LX thread group
-// (thread (i, j) owns the column k = 0..LX-1), element tiles in shared
-// memory, D from the kernel-parameter bank.  FP64 throughout (these feed the
-// adjoint right-hand sides and sensitivities).
+// Layout: element tiles in shared memory; contractions in fixed point
+// (fx.cuh), everything else FP64 (these feed the adjoint right-hand sides
+// and sensitivities).
 #include "deriv.cuh"
 
 namespace ntg {
@@ -67,182 +66,149 @@ __global__ void __launch_bounds__(Shape<LX, 3>::THREADS)
   }
 }
 
-// Gradient of u with the cofactors.  MODE 0: out_d = (strong) or w3 * (weak)
-// derivative, d in {0, 1, 2} selected by mask bits; MODE 1: f_d -= mul *
-// opgrad_d(u) for all d (the first term of the adjoint advection).
-template <int LX, int MODE, bool WEAK>
-__global__ void __launch_bounds__(Shape<LX, 1>::THREADS)
+// Gradient of u with the cofactors: out_d = (strong) or w3 * (weak)
+// derivative, for the non-null out_d.
+template <int LX, bool WEAK>
+__global__ void __launch_bounds__(FxShape<LX, 4>::NT, FxShape<LX, 4>::MINB)
     k_grad(double* __restrict__ o0, double* __restrict__ o1, double* __restrict__ o2, const double* __restrict__ u,
-           const double* __restrict__ mul, int64_t nelv, const __grid_constant__ DMat<LX> M,
+           int64_t nelv, const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P,
            const double* __restrict__ met, int64_t n) {
-  using S = Shape<LX, 1>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double su[EPB][LX3];
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k) su[le][k * LX2 + ij] = act ? u[e * LX3 + k * LX2 + ij] : 0.0;
+  NTG_FX_PROLOGUE(4)
+  if (WEAK) stage_w3<LX>(w3t, M, NT);
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    NTG_FX_NODES { NTG_FX_NODE T[p] = u[q]; }
     __syncthreads();
-    if (act) {
-      for (int k = 0; k < LX; ++k) {
-        double ur, us, ut;
-        rgrad<LX>(su[le], M, i, j, k, ur, us, ut);
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        const double sc = WEAK ? M.w[i] * M.w[j] * M.w[k] : met[9 * n + q];
-        double* outs[3] = {o0, o1, o2};
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          if (MODE == 0 && !outs[d]) continue;
-          const double v = sc * (met[d * n + q] * ur + met[(3 + d) * n + q] * us + met[(6 + d) * n + q] * ut);
-          if (MODE == 0) outs[d][q] = v;
-          else outs[d][q] -= mul[q] * v;
-        }
-      }
+    NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T, T + (1 + d) * TS, d, lq); }
+    __syncthreads();
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      const double ur = T[TS + p], us = T[2 * TS + p], ut = T[3 * TS + p];
+      const double sc = WEAK ? w3t[node] : met[9 * n + q];
+      if (o0) o0[q] = sc * (met[q] * ur + met[3 * n + q] * us + met[6 * n + q] * ut);
+      if (o1) o1[q] = sc * (met[n + q] * ur + met[4 * n + q] * us + met[7 * n + q] * ut);
+      if (o2) o2[q] = sc * (met[2 * n + q] * ur + met[5 * n + q] * us + met[8 * n + q] * ut);
     }
-    __syncthreads();
   }
 }
 
-// out (= or -=) sum_d cdtp_d(a_d), a_d = mul * in_d (mul null: 1; in_d null: 0)
-template <int LX, bool SUB>
-__global__ void __launch_bounds__(Shape<LX, 3>::THREADS)
-    k_cdtp(double* __restrict__ out, const double* __restrict__ in0, const double* __restrict__ in1,
-           const double* __restrict__ in2, const double* __restrict__ mul, int64_t nelv,
-           const __grid_constant__ DMat<LX> M, const double* __restrict__ met, int64_t n) {
-  using S = Shape<LX, 3>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double fr[EPB][LX3], fs[EPB][LX3], ft[EPB][LX3];
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k) {
-      const int64_t q = e * LX3 + k * LX2 + ij;
-      double a[3] = {0.0, 0.0, 0.0};
-      if (act) {
-        const double mq = mul ? mul[q] : 1.0;
-        if (in0) a[0] = mq * in0[q];
-        if (in1) a[1] = mq * in1[q];
-        if (in2) a[2] = mq * in2[q];
-      }
-      const double w3 = M.w[i] * M.w[j] * M.w[k];
-      double r = 0.0, s = 0.0, t = 0.0;
-      if (act) {
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          r = fma(met[d * n + q], a[d], r);
-          s = fma(met[(3 + d) * n + q], a[d], s);
-          t = fma(met[(6 + d) * n + q], a[d], t);
-        }
-      }
-      fr[le][k * LX2 + ij] = w3 * r;
-      fs[le][k * LX2 + ij] = w3 * s;
-      ft[le][k * LX2 + ij] = w3 * t;
-    }
-    __syncthreads();
-    if (act) {
-      for (int k = 0; k < LX; ++k) {
-        double acc = 0.0;
-#pragma unroll
-        for (int l = 0; l < LX; ++l) {
-          acc = fma(M.d[l * LX + i], fr[le][k * LX2 + j * LX + l], acc);
-          acc = fma(M.d[l * LX + j], fs[le][k * LX2 + l * LX + i], acc);
-          acc = fma(M.d[l * LX + k], ft[le][l * LX2 + j * LX + i], acc);
-        }
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        if (SUB) out[q] -= acc;
-        else out[q] = acc;
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// MODE 0: out = va . grad(a) (conv1, strong);  MODE 1: out -= B (va . grad a + vb . grad b)
-template <int LX, int MODE>
-__global__ void __launch_bounds__(Shape<LX, 2>::THREADS)
-    k_conv(double* __restrict__ out, const double* __restrict__ a, const double* __restrict__ va0,
-           const double* __restrict__ va1, const double* __restrict__ va2, const double* __restrict__ b,
-           const double* __restrict__ vb0, const double* __restrict__ vb1, const double* __restrict__ vb2,
-           int64_t nelv, const __grid_constant__ DMat<LX> M, const double* __restrict__ met, int64_t n) {
-  using S = Shape<LX, 2>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double sa[EPB][LX3], sb[EPB][LX3];
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k) {
-      const int64_t q = e * LX3 + k * LX2 + ij;
-      sa[le][k * LX2 + ij] = act ? a[q] : 0.0;
-      if (MODE == 1) sb[le][k * LX2 + ij] = act ? b[q] : 0.0;
-    }
-    __syncthreads();
-    if (act) {
-      for (int k = 0; k < LX; ++k) {
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        double ur, us, ut;
-        rgrad<LX>(sa[le], M, i, j, k, ur, us, ut);
-        const double* vv[3] = {va0, va1, va2};
-        double acc = 0.0;
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          acc = fma(vv[d][q], met[d * n + q] * ur + met[(3 + d) * n + q] * us + met[(6 + d) * n + q] * ut, acc);
-        if (MODE == 0) {
-          out[q] = acc * met[9 * n + q];
-        } else {
-          rgrad<LX>(sb[le], M, i, j, k, ur, us, ut);
-          const double* vw[3] = {vb0, vb1, vb2};
-#pragma unroll
-          for (int d = 0; d < 3; ++d)
-            acc = fma(vw[d][q], met[d * n + q] * ur + met[(3 + d) * n + q] * us + met[(6 + d) * n + q] * ut, acc);
-          out[q] -= M.w[i] * M.w[j] * M.w[k] * acc;  // B / jac = w3
-        }
-      }
-    }
-    __syncthreads();
-  }
-}
-
-// B curl(u) (strong curl times B = w3 * cofactor combinations)
+// out = cdtp of x with the cofactors of direction dir
 template <int LX>
-__global__ void __launch_bounds__(Shape<LX, 3>::THREADS)
-    k_curl(double* __restrict__ w0, double* __restrict__ w1, double* __restrict__ w2, const double* __restrict__ ux,
-           const double* __restrict__ uy, const double* __restrict__ uz, int64_t nelv,
-           const __grid_constant__ DMat<LX> M, const double* __restrict__ met, int64_t n) {
-  using S = Shape<LX, 3>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double sx[EPB][LX3], sy[EPB][LX3], sz[EPB][LX3];
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k) {
-      const int64_t q = e * LX3 + k * LX2 + ij;
-      sx[le][k * LX2 + ij] = act ? ux[q] : 0.0;
-      sy[le][k * LX2 + ij] = act ? uy[q] : 0.0;
-      sz[le][k * LX2 + ij] = act ? uz[q] : 0.0;
+__global__ void __launch_bounds__(FxShape<LX, 3>::NT, FxShape<LX, 3>::MINB)
+    k_cdtp(double* __restrict__ out, const double* __restrict__ x, int dir, int64_t nelv,
+           const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P,
+           const double* __restrict__ met, int64_t n) {
+  NTG_FX_PROLOGUE(3)
+  stage_w3<LX>(w3t, M, NT);
+  __syncthreads();
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      const double a = w3t[node] * x[q];
+      T[p] = met[dir * n + q] * a;
+      T[TS + p] = met[(3 + dir) * n + q] * a;
+      T[2 * TS + p] = met[(6 + dir) * n + q] * a;
     }
     __syncthreads();
-    if (act) {
-      for (int k = 0; k < LX; ++k) {
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        double g[3][3];  // g[f][r|s|t]: reference derivatives of field f
-        rgrad<LX>(sx[le], M, i, j, k, g[0][0], g[0][1], g[0][2]);
-        rgrad<LX>(sy[le], M, i, j, k, g[1][0], g[1][1], g[1][2]);
-        rgrad<LX>(sz[le], M, i, j, k, g[2][0], g[2][1], g[2][2]);
-        auto d = [&](int f, int dir) {
-          return met[dir * n + q] * g[f][0] + met[(3 + dir) * n + q] * g[f][1] + met[(6 + dir) * n + q] * g[f][2];
-        };
-        const double w3 = M.w[i] * M.w[j] * M.w[k];
-        w0[q] = w3 * (d(2, 1) - d(1, 2));
-        w1[q] = w3 * (d(0, 2) - d(2, 0));
-        w2[q] = w3 * (d(1, 0) - d(0, 1));
+    NTG_FX_LINES {
+      NTG_FX_LINE
+      fx::flux_line<LX>(P.DT, P.dt, T + d * TS, reinterpret_cast<int*>(T + 3 * TS) + r, d, lq);
+    }
+    __syncthreads();
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      out[q] = fx::flux_sum<LX>(T, T + TS, T + 2 * TS, reinterpret_cast<const int*>(T + 3 * TS), node);
+    }
+    __syncthreads();
+  }
+}
+
+// out = v . grad(a) (conv1, strong)
+template <int LX>
+__global__ void __launch_bounds__(FxShape<LX, 4>::NT, FxShape<LX, 4>::MINB)
+    k_conv(double* __restrict__ out, const double* __restrict__ a, const double* __restrict__ v0,
+           const double* __restrict__ v1, const double* __restrict__ v2, int64_t nelv,
+           const __grid_constant__ fx::Mats<LX> P, const double* __restrict__ met, int64_t n) {
+  NTG_FX_PROLOGUE(4)
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    NTG_FX_NODES { NTG_FX_NODE T[p] = a[q]; }
+    __syncthreads();
+    NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T, T + (1 + d) * TS, d, lq); }
+    __syncthreads();
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      const double x = v0[q], y = v1[q], z = v2[q];
+      double acc = 0.0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        acc = fma(met[3 * d * n + q] * x + met[(3 * d + 1) * n + q] * y + met[(3 * d + 2) * n + q] * z,
+                  T[(1 + d) * TS + p], acc);
+      out[q] = acc * met[9 * n + q];
+    }
+  }
+}
+
+// B curl(u) (strong curl times B = w3 * cofactor combinations); scale: null,
+// or a factor per node that multiplies u first
+template <int LX>
+__global__ void __launch_bounds__(FxShape<LX, 9>::NT, FxShape<LX, 9>::MINB)
+    k_curl(double* __restrict__ w0, double* __restrict__ w1, double* __restrict__ w2, const double* __restrict__ ux,
+           const double* __restrict__ uy, const double* __restrict__ uz, const double* __restrict__ scale,
+           int64_t nelv, const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P,
+           const double* __restrict__ met, int64_t n) {
+  NTG_FX_PROLOGUE(9)
+  stage_w3<LX>(w3t, M, NT);
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    if (scale) {
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        const double b = scale[q];
+        T[p] = ux[q] * b;
+        T[TS + p] = uy[q] * b;
+        T[2 * TS + p] = uz[q] * b;
+      }
+    } else {
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        T[p] = ux[q];
+        T[TS + p] = uy[q];
+        T[2 * TS + p] = uz[q];
+      }
+    }
+#pragma unroll 1
+    for (int dir = 0; dir < 3; ++dir) {
+      __syncthreads();
+      NTG_FX_LINES {
+        NTG_FX_LINE  // d: the field here
+        fx::deriv_line<LX>(P.D, P.d, T + d * TS, T + (3 + d) * TS, dir, lq);
+      }
+      __syncthreads();
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        const double gx = T[3 * TS + p], gy = T[4 * TS + p], gz = T[5 * TS + p];
+        const double c0 = met[3 * dir * n + q], c1 = met[(3 * dir + 1) * n + q], c2 = met[(3 * dir + 2) * n + q];
+        double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+        if (dir > 0) {
+          a0 = T[6 * TS + p];
+          a1 = T[7 * TS + p];
+          a2 = T[8 * TS + p];
+        }
+        a0 = fma(c1, gz, fma(-c2, gy, a0));
+        a1 = fma(c2, gx, fma(-c0, gz, a1));
+        a2 = fma(c0, gy, fma(-c1, gx, a2));
+        if (dir < 2) {
+          T[6 * TS + p] = a0;
+          T[7 * TS + p] = a1;
+          T[8 * TS + p] = a2;
+        } else {
+          const double w3 = w3t[node];
+          w0[q] = w3 * a0;
+          w1[q] = w3 * a1;
+          w2[q] = w3 * a2;
+        }
       }
     }
     __syncthreads();
@@ -251,90 +217,78 @@ __global__ void __launch_bounds__(Shape<LX, 3>::THREADS)
 
 // The adjoint advection without dealiasing in one element pass:
 //   f_i -= sum_j u_j opgrad_i(Ub_j) + sum_d cdtp_d(u_i Ub_d).
-// The cdtp fluxes of all three components share the contravariant fluxes
-// V_r = w3 (drdx . Ub), V_s = w3 (dsdx . Ub), V_t = w3 (dtdx . Ub):
-// component i's fluxes are u_i V_r, u_i V_s, u_i V_t.  Phase 1 takes the
-// reference gradients of Ub from its tiles, subtracts the opgrad part and
-// stores V; then per component the Ub tiles hold u_i V and D^T is applied.
-// Inputs and the cofactors are read once per node instead of by six
-// separate kernels; the FP64 operation count is the separate kernels' less
-// the repeated flux sums (198 instead of 216 per node).
+// With a_d = sum_j u_j dUb_j/dr_d the first sum is w3 sum_d c_di a_d (18
+// products per node where mixing each gradient first takes 36); the second
+// shares the contravariant velocity V_d = sum_c c_dc Ub_c between the three
+// components, and the weights come out of D^T: D_d^T (w3 f) = w3 (DT_d f)
+// with DT = W^-1 D^T W.  42 FP64 operations per node (198 with the
+// contractions on the FP64 pipe).
 template <int LX>
-__global__ void __launch_bounds__(Shape<LX, 6>::THREADS)
+__global__ void __launch_bounds__(FxShape<LX, 9>::NT, FxShape<LX, 9>::MINB)
     k_adv_adj_nd(double* __restrict__ f0, double* __restrict__ f1, double* __restrict__ f2,
                  const double* __restrict__ u0, const double* __restrict__ u1, const double* __restrict__ u2,
                  const double* __restrict__ b0, const double* __restrict__ b1, const double* __restrict__ b2,
-                 int64_t nelv, const __grid_constant__ DMat<LX> M, const double* __restrict__ met, int64_t n) {
-  using S = Shape<LX, 6>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double sA[EPB][3][LX3];  // Ub, then u_i V_r, u_i V_s, u_i V_t
-  __shared__ double sV[EPB][3][LX3];  // V_r, V_s, V_t
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  const double* ub[3] = {b0, b1, b2};
-  const double* uu[3] = {u0, u1, u2};
-  double* ff[3] = {f0, f1, f2};
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) sA[le][c][k * LX2 + ij] = act ? ub[c][e * LX3 + k * LX2 + ij] : 0.0;
-    __syncthreads();
-    if (act) {
+                 int64_t nelv, const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P,
+                 const double* __restrict__ met, int64_t n) {
+  NTG_FX_PROLOGUE(9)
+  stage_w3<LX>(w3t, M, NT);
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    // tiles 0-2: Ub, then V; 3-5: derivatives, then fluxes; 6-8: a_d, then the opgrad part
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      T[p] = b0[q];
+      T[TS + p] = b1[q];
+      T[2 * TS + p] = b2[q];
+    }
 #pragma unroll 1
-      for (int k = 0; k < LX; ++k) {
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        const int p = k * LX2 + ij;
-        double gr[3][3];
+    for (int dir = 0; dir < 3; ++dir) {
+      __syncthreads();
+      NTG_FX_LINES {
+        NTG_FX_LINE  // d: the field here
+        fx::deriv_line<LX>(P.D, P.d, T + d * TS, T + (3 + d) * TS, dir, lq);
+      }
+      __syncthreads();
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        T[(6 + dir) * TS + p] = u0[q] * T[3 * TS + p] + u1[q] * T[4 * TS + p] + u2[q] * T[5 * TS + p];
+      }
+    }
+    NTG_FX_NODES {  // the node's own thread wrote its a_d
+      NTG_FX_NODE
+      double m[9];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) rgrad<LX>(sA[le][c], M, i, j, k, gr[c][0], gr[c][1], gr[c][2]);
-        double m[9];
+      for (int c = 0; c < 9; ++c) m[c] = met[c * n + q];
+      const double bx = T[p], by = T[TS + p], bz = T[2 * TS + p];
+      const double ar = T[6 * TS + p], as = T[7 * TS + p], at = T[8 * TS + p];
 #pragma unroll
-        for (int t = 0; t < 9; ++t) m[t] = met[t * n + q];
-        const double w3 = M.w[i] * M.w[j] * M.w[k];
-        const double uq[3] = {u0[q], u1[q], u2[q]};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          double acc = 0.0;
-#pragma unroll
-          for (int jj = 0; jj < 3; ++jj)
-            acc = fma(uq[jj], m[c] * gr[jj][0] + m[3 + c] * gr[jj][1] + m[6 + c] * gr[jj][2], acc);
-          ff[c][q] -= w3 * acc;
-        }
-        const double bq[3] = {sA[le][0][p], sA[le][1][p], sA[le][2][p]};
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-          sV[le][d][p] = w3 * (m[3 * d] * bq[0] + m[3 * d + 1] * bq[1] + m[3 * d + 2] * bq[2]);
+      for (int c = 0; c < 3; ++c) {
+        T[c * TS + p] = m[3 * c] * bx + m[3 * c + 1] * by + m[3 * c + 2] * bz;
+        T[(6 + c) * TS + p] = m[c] * ar + m[3 + c] * as + m[6 + c] * at;
       }
     }
 #pragma unroll 1
     for (int c = 0; c < 3; ++c) {
-      __syncthreads();
-      if (act) {
-        for (int k = 0; k < LX; ++k) {
-          const int p = k * LX2 + ij;
-          const double uc = uu[c][e * LX3 + p];
-#pragma unroll
-          for (int d = 0; d < 3; ++d) sA[le][d][p] = uc * sV[le][d][p];
-        }
+      const double* uc = c == 0 ? u0 : c == 1 ? u1 : u2;
+      double* fc = c == 0 ? f0 : c == 1 ? f1 : f2;
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        const double v = uc[q];
+        T[3 * TS + p] = v * T[p];
+        T[4 * TS + p] = v * T[TS + p];
+        T[5 * TS + p] = v * T[2 * TS + p];
       }
       __syncthreads();
-      if (act) {
-        const double* fr = sA[le][0];
-        const double* fs = sA[le][1];
-        const double* ft = sA[le][2];
-#pragma unroll 1
-        for (int k = 0; k < LX; ++k) {
-          double acc = 0.0;
-#pragma unroll
-          for (int l = 0; l < LX; ++l) {
-            acc = fma(M.d[l * LX + i], fr[k * LX2 + j * LX + l], acc);
-            acc = fma(M.d[l * LX + j], fs[k * LX2 + l * LX + i], acc);
-            acc = fma(M.d[l * LX + k], ft[l * LX2 + j * LX + i], acc);
-          }
-          ff[c][e * LX3 + k * LX2 + ij] -= acc;
-        }
+      NTG_FX_LINES {
+        NTG_FX_LINE
+        fx::flux_line<LX>(P.DT, P.dt, T + (3 + d) * TS, reinterpret_cast<int*>(T + 9 * TS) + r, d, lq);
+      }
+      __syncthreads();
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        const double s = fx::flux_sum<LX>(T + 3 * TS, T + 4 * TS, T + 5 * TS,
+                                          reinterpret_cast<const int*>(T + 9 * TS), node);
+        fc[q] = fma(-w3t[node], s + T[(6 + c) * TS + p], fc[q]);
       }
     }
     __syncthreads();
@@ -343,68 +297,60 @@ __global__ void __launch_bounds__(Shape<LX, 6>::THREADS)
 
 // The linearised advection without dealiasing in one element pass:
 //   f_i -= B conv1(u_i; Ub) + B conv1(Ub_i; u)
-//        = w3 sum_d (Ub_d (drdx_d . grad u_i) + u_d (drdx_d . grad Ub_i)),
-// with u and Ub in six tiles, the cofactors read once per node.
+//        = w3 sum_d (V_d(Ub) du_i/dr_d + V_d(u) dUb_i/dr_d),
+// V_d(x) = sum_c c_dc x_c: 39 FP64 operations per node (216 with the
+// contractions on the FP64 pipe).
 template <int LX>
-__global__ void __launch_bounds__(Shape<LX, 6>::THREADS)
+__global__ void __launch_bounds__(FxShape<LX, 10>::NT, FxShape<LX, 10>::MINB)
     k_adv_lin_nd(double* __restrict__ f0, double* __restrict__ f1, double* __restrict__ f2,
                  const double* __restrict__ u0, const double* __restrict__ u1, const double* __restrict__ u2,
                  const double* __restrict__ b0, const double* __restrict__ b1, const double* __restrict__ b2,
-                 int64_t nelv, const __grid_constant__ DMat<LX> M, const double* __restrict__ met, int64_t n) {
-  using S = Shape<LX, 6>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double sU[EPB][3][LX3], sB[EPB][3][LX3];
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  const double* ub[3] = {b0, b1, b2};
-  const double* uu[3] = {u0, u1, u2};
-  double* ff[3] = {f0, f1, f2};
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k)
+                 int64_t nelv, const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P,
+                 const double* __restrict__ met, int64_t n) {
+  NTG_FX_PROLOGUE(10)
+  stage_w3<LX>(w3t, M, NT);
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    // tile 0: the field differentiated; 1-3: its derivatives; 4-6: V_d of the other velocity; 7-9: sums
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {
+      const double* x0 = pass ? b0 : u0;
+      const double* x1 = pass ? b1 : u1;
+      const double* x2 = pass ? b2 : u2;
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        const double x = x0[q], y = x1[q], z = x2[q];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        sU[le][c][k * LX2 + ij] = act ? uu[c][e * LX3 + k * LX2 + ij] : 0.0;
-        sB[le][c][k * LX2 + ij] = act ? ub[c][e * LX3 + k * LX2 + ij] : 0.0;
+        for (int c = 0; c < 3; ++c)
+          T[(4 + c) * TS + p] = met[3 * c * n + q] * x + met[(3 * c + 1) * n + q] * y + met[(3 * c + 2) * n + q] * z;
       }
-    __syncthreads();
-    if (act) {
 #pragma unroll 1
-      for (int k = 0; k < LX; ++k) {
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        const int p = k * LX2 + ij;
-        double m[9];
-#pragma unroll
-        for (int t = 0; t < 9; ++t) m[t] = met[t * n + q];
-        const double w3 = M.w[i] * M.w[j] * M.w[k];
-        const double uq[3] = {sU[le][0][p], sU[le][1][p], sU[le][2][p]};
-        const double bq[3] = {sB[le][0][p], sB[le][1][p], sB[le][2][p]};
-#pragma unroll 1
-        for (int c = 0; c < 3; ++c) {
-          double gu[3], gb[3];
-          rgrad<LX>(sU[le][c], M, i, j, k, gu[0], gu[1], gu[2]);
-          rgrad<LX>(sB[le][c], M, i, j, k, gb[0], gb[1], gb[2]);
-          double acc = 0.0;
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            acc = fma(bq[d], m[d] * gu[0] + m[3 + d] * gu[1] + m[6 + d] * gu[2], acc);
-            acc = fma(uq[d], m[d] * gb[0] + m[3 + d] * gb[1] + m[6 + d] * gb[2], acc);
-          }
-          ff[c][q] -= w3 * acc;
+      for (int c = 0; c < 3; ++c) {
+        const double* a = pass ? (c == 0 ? u0 : c == 1 ? u1 : u2) : (c == 0 ? b0 : c == 1 ? b1 : b2);
+        double* fc = c == 0 ? f0 : c == 1 ? f1 : f2;
+        NTG_FX_NODES { NTG_FX_NODE T[p] = a[q]; }
+        __syncthreads();
+        NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T, T + (1 + d) * TS, d, lq); }
+        __syncthreads();
+        NTG_FX_NODES {
+          NTG_FX_NODE
+          const double g = T[TS + p] * T[4 * TS + p] + T[2 * TS + p] * T[5 * TS + p] + T[3 * TS + p] * T[6 * TS + p];
+          if (pass) fc[q] = fma(-w3t[node], g + T[(7 + c) * TS + p], fc[q]);
+          else T[(7 + c) * TS + p] = g;
         }
       }
     }
-    __syncthreads();
   }
 }
 
+// a, b, c *= s
 __global__ void k_mul3(double* __restrict__ a, double* __restrict__ b, double* __restrict__ c,
                        const double* __restrict__ s, int64_t n) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
-    a[q] *= s[q];
-    b[q] *= s[q];
-    c[q] *= s[q];
+    const double f = s[q];
+    a[q] *= f;
+    b[q] *= f;
+    c[q] *= f;
   }
 }
 
@@ -413,18 +359,19 @@ __global__ void k_inv(double* __restrict__ a, int64_t n) {
     a[q] = 1.0 / a[q];
 }
 
-// f_c += scale w_c on all nodes (zone null) or on the zone's nodes only
+// f_c += scale binv w_c on all nodes (zone null) or on the zone's nodes only
 __global__ void k_add_zone(double* __restrict__ f0, double* __restrict__ f1, double* __restrict__ f2,
                            const double* __restrict__ w0, const double* __restrict__ w1,
-                           const double* __restrict__ w2, double scale, const int32_t* __restrict__ zone,
-                           int64_t nzone, int base, int64_t n) {
+                           const double* __restrict__ w2, const double* __restrict__ binv, double scale,
+                           const int32_t* __restrict__ zone, int64_t nzone, int base, int64_t n) {
   const int64_t cnt = zone ? nzone : n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < cnt; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t q = zone ? (int64_t)zone[t] - base : t;
     if (q < 0 || q >= n) continue;
-    f0[q] += scale * w0[q];
-    f1[q] += scale * w1[q];
-    f2[q] += scale * w2[q];
+    const double b = binv[q];
+    f0[q] = fma(scale, w0[q] * b, f0[q]);
+    f1[q] = fma(scale, w1[q] * b, f1[q]);
+    f2[q] = fma(scale, w2[q] * b, f2[q]);
   }
 }
 
@@ -442,27 +389,30 @@ double* plan_scratch(ntg_plan* p, int64_t count) {
   return p->dscr;
 }
 
-// w = B curl u (unassembled)
-int bcurl(ntg_plan* p, double* w0, double* w1, double* w2, const double* ux, const double* uy, const double* uz) {
+// w = gs(B curl(scale u)); scale null: 1
+int curl_gs(ntg_plan* p, double* w0, double* w1, double* w2, const double* ux, const double* uy, const double* uz,
+            const double* scale) {
   cudaStream_t s = p->stream;
-  return dv::dispatch<3>(p->lx, [&](auto L) -> int {
+  NTG_TRY(dv::dispatch<9>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    dv::k_curl<LX><<<dv::grid_of<LX, 3>(p), dv::Shape<LX, 3>::THREADS, 0, s>>>(w0, w1, w2, ux, uy, uz, p->nelv,
-                                                                                 dv::dmat<LX>(p), p->met, p->n);
+    using S = dv::FxShape<LX, 9>;
+    NTG_TRY(fx::use_smem<dv::k_curl<LX>>(S::SMEM));
+    dv::k_curl<LX><<<dv::fx_grid<LX, 9>(p), S::NT, S::SMEM, s>>>(w0, w1, w2, ux, uy, uz, scale, p->nelv,
+                                                                 dv::dmat<LX>(p), fx::plan_mats<LX>(p, 1.0), p->met,
+                                                                 p->n);
     NTG_COUNT_LAUNCH();
     return NTG_OK;
-  });
+  }));
+  NTG_TRY(gs_launch3(p, w0, w1, w2, s));
+  NTG_CUDA_TRY(cudaGetLastError());
+  return NTG_OK;
 }
 
 // w = Binv gs(B curl u)
-int curl_avg(ntg_plan* p, double* w0, double* w1, double* w2, const double* ux, const double* uy,
-             const double* uz) {
-  cudaStream_t s = p->stream;
-  NTG_TRY(bcurl(p, w0, w1, w2, ux, uy, uz));
-  NTG_TRY(gs_launch(p, w0, NTG_GS_ADD, s));
-  NTG_TRY(gs_launch(p, w1, NTG_GS_ADD, s));
-  NTG_TRY(gs_launch(p, w2, NTG_GS_ADD, s));
-  { dv::k_mul3<<<grid_for(p->n, 256), 256, 0, s>>>(w0, w1, w2, p->binv, p->n); NTG_COUNT_LAUNCH(); }
+static int curl_avg(ntg_plan* p, double* w0, double* w1, double* w2, const double* ux, const double* uy,
+                    const double* uz) {
+  NTG_TRY(curl_gs(p, w0, w1, w2, ux, uy, uz, nullptr));
+  { dv::k_mul3<<<grid_for(p->n, 256), 256, 0, p->stream>>>(w0, w1, w2, p->binv, p->n); NTG_COUNT_LAUNCH(); }
   NTG_CUDA_TRY(cudaGetLastError());
   return NTG_OK;
 }
@@ -501,8 +451,10 @@ int ntg_dudxyz(ntg_plan* p, double* du_d, const double* u_d, int dir) {
   o[dir] = du_d;
   return dv::dispatch<1>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    dv::k_grad<LX, 0, false><<<dv::grid_of<LX, 1>(p), dv::Shape<LX, 1>::THREADS, 0, p->stream>>>(
-        o[0], o[1], o[2], u_d, nullptr, p->nelv, dv::dmat<LX>(p), p->met, p->n);
+    using S = dv::FxShape<LX, 4>;
+    NTG_TRY((fx::use_smem<dv::k_grad<LX, false>>(S::SMEM)));
+    dv::k_grad<LX, false><<<dv::fx_grid<LX, 4>(p), S::NT, S::SMEM, p->stream>>>(
+        o[0], o[1], o[2], u_d, p->nelv, dv::dmat<LX>(p), fx::plan_mats<LX>(p, 1.0), p->met, p->n);
     NTG_COUNT_LAUNCH();
     NTG_CUDA_TRY(cudaGetLastError());
     return NTG_OK;
@@ -515,8 +467,10 @@ int ntg_opgrad(ntg_plan* p, double* ux_d, double* uy_d, double* uz_d, const doub
   NTG_TRY(need_metrics(p));
   return dv::dispatch<1>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    dv::k_grad<LX, 0, true><<<dv::grid_of<LX, 1>(p), dv::Shape<LX, 1>::THREADS, 0, p->stream>>>(
-        ux_d, uy_d, uz_d, u_d, nullptr, p->nelv, dv::dmat<LX>(p), p->met, p->n);
+    using S = dv::FxShape<LX, 4>;
+    NTG_TRY((fx::use_smem<dv::k_grad<LX, true>>(S::SMEM)));
+    dv::k_grad<LX, true><<<dv::fx_grid<LX, 4>(p), S::NT, S::SMEM, p->stream>>>(
+        ux_d, uy_d, uz_d, u_d, p->nelv, dv::dmat<LX>(p), fx::plan_mats<LX>(p, 1.0), p->met, p->n);
     NTG_COUNT_LAUNCH();
     NTG_CUDA_TRY(cudaGetLastError());
     return NTG_OK;
@@ -527,12 +481,12 @@ int ntg_cdtp(ntg_plan* p, double* dtx_d, const double* x_d, int dir) {
   clear_error();
   NTG_CHECK_ARG(p && dtx_d && x_d && dir >= 0 && dir <= 2, "ntg_cdtp: bad argument");
   NTG_TRY(need_metrics(p));
-  const double* in[3] = {nullptr, nullptr, nullptr};
-  in[dir] = x_d;
   return dv::dispatch<3>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    dv::k_cdtp<LX, false><<<dv::grid_of<LX, 3>(p), dv::Shape<LX, 3>::THREADS, 0, p->stream>>>(
-        dtx_d, in[0], in[1], in[2], nullptr, p->nelv, dv::dmat<LX>(p), p->met, p->n);
+    using S = dv::FxShape<LX, 3>;
+    NTG_TRY(fx::use_smem<dv::k_cdtp<LX>>(S::SMEM));
+    dv::k_cdtp<LX><<<dv::fx_grid<LX, 3>(p), S::NT, S::SMEM, p->stream>>>(
+        dtx_d, x_d, dir, p->nelv, dv::dmat<LX>(p), fx::plan_mats<LX>(p, 1.0), p->met, p->n);
     NTG_COUNT_LAUNCH();
     NTG_CUDA_TRY(cudaGetLastError());
     return NTG_OK;
@@ -546,8 +500,10 @@ int ntg_conv1(ntg_plan* p, double* du_d, const double* u_d, const double* vx_d, 
   NTG_TRY(need_metrics(p));
   return dv::dispatch<2>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    dv::k_conv<LX, 0><<<dv::grid_of<LX, 2>(p), dv::Shape<LX, 2>::THREADS, 0, p->stream>>>(
-        du_d, u_d, vx_d, vy_d, vz_d, nullptr, nullptr, nullptr, nullptr, p->nelv, dv::dmat<LX>(p), p->met, p->n);
+    using S = dv::FxShape<LX, 4>;
+    NTG_TRY(fx::use_smem<dv::k_conv<LX>>(S::SMEM));
+    dv::k_conv<LX><<<dv::fx_grid<LX, 4>(p), S::NT, S::SMEM, p->stream>>>(
+        du_d, u_d, vx_d, vy_d, vz_d, p->nelv, fx::plan_mats<LX>(p, 1.0), p->met, p->n);
     NTG_COUNT_LAUNCH();
     NTG_CUDA_TRY(cudaGetLastError());
     return NTG_OK;
@@ -576,8 +532,11 @@ int ntg_adjoint_advection_no_dealias(ntg_plan* p, double* fx, double* fy, double
   // f_i -= sum_j u_j opgrad_i(Ub_j) + sum_d cdtp_d(u_i Ub_d), one element pass
   NTG_TRY(dv::dispatch<6>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    dv::k_adv_adj_nd<LX><<<dv::grid_of<LX, 6>(p), dv::Shape<LX, 6>::THREADS, 0, s>>>(
-        f[0], f[1], f[2], u[0], u[1], u[2], ub[0], ub[1], ub[2], p->nelv, dv::dmat<LX>(p), p->met, p->n);
+    using S = dv::FxShape<LX, 9>;
+    NTG_TRY(fx::use_smem<dv::k_adv_adj_nd<LX>>(S::SMEM));
+    dv::k_adv_adj_nd<LX><<<dv::fx_grid<LX, 9>(p), S::NT, S::SMEM, s>>>(
+        f[0], f[1], f[2], u[0], u[1], u[2], ub[0], ub[1], ub[2], p->nelv, dv::dmat<LX>(p),
+        fx::plan_mats<LX>(p, 1.0, true), p->met, p->n);
     NTG_COUNT_LAUNCH();
     return NTG_OK;
   }));
@@ -598,8 +557,11 @@ int ntg_linear_advection_no_dealias(ntg_plan* p, double* fx, double* fy, double*
   // f_i -= B conv1(u_i; Ub) + B conv1(Ub_i; u), one element pass
   NTG_TRY(dv::dispatch<6>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    dv::k_adv_lin_nd<LX><<<dv::grid_of<LX, 6>(p), dv::Shape<LX, 6>::THREADS, 0, p->stream>>>(
-        f[0], f[1], f[2], u[0], u[1], u[2], ub[0], ub[1], ub[2], p->nelv, dv::dmat<LX>(p), p->met, p->n);
+    using S = dv::FxShape<LX, 10>;
+    NTG_TRY(fx::use_smem<dv::k_adv_lin_nd<LX>>(S::SMEM));
+    dv::k_adv_lin_nd<LX><<<dv::fx_grid<LX, 10>(p), S::NT, S::SMEM, p->stream>>>(
+        f[0], f[1], f[2], u[0], u[1], u[2], ub[0], ub[1], ub[2], p->nelv, dv::dmat<LX>(p),
+        fx::plan_mats<LX>(p, 1.0), p->met, p->n);
     NTG_COUNT_LAUNCH();
     return NTG_OK;
   }));
@@ -616,10 +578,11 @@ int ntg_adjoint_min_dissipation(ntg_plan* p, double* fx, double* fy, double* fz,
   const int64_t n = p->n;
   double* t = plan_scratch(p, 6 * n);
   if (!t) return NTG_ERR_ALLOC;
-  NTG_TRY(curl_avg(p, t, t + n, t + 2 * n, u, v, w));
-  NTG_TRY(curl_avg(p, t + 3 * n, t + 4 * n, t + 5 * n, t, t + n, t + 2 * n));
+  // the first curl's Binv is applied where the second reads it, the second's where it is added
+  NTG_TRY(curl_gs(p, t, t + n, t + 2 * n, u, v, w, nullptr));
+  NTG_TRY(curl_gs(p, t + 3 * n, t + 4 * n, t + 5 * n, t, t + n, t + 2 * n, p->binv));
   dv::k_add_zone<<<grid_for(nzone ? nzone : n, 256), 256, 0, p->stream>>>(
-      fx, fy, fz, t + 3 * n, t + 4 * n, t + 5 * n, scale, nzone ? zone_d : nullptr, nzone, base, n);
+      fx, fy, fz, t + 3 * n, t + 4 * n, t + 5 * n, p->binv, scale, nzone ? zone_d : nullptr, nzone, base, n);
   NTG_COUNT_LAUNCH();
   NTG_CUDA_TRY(cudaGetLastError());
   return NTG_OK;

@@ -6,6 +6,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "fx.cuh"
 
 namespace ntg {
 namespace dv {
@@ -24,6 +25,61 @@ struct Shape {
   static constexpr int EPB = EPB0 < EPBS ? EPB0 : EPBS;
   static constexpr int NW = EPB * LX2, THREADS = (NW + 31) / 32 * 32;
 };
+
+// Blocks of the kernels whose contractions run in fixed point (fx.cuh): EPB
+// elements and about one thread per line of a field's three directions.
+template <int LX, int TILES>
+struct FxShape {
+  static constexpr int L2 = LX * LX, L3 = L2 * LX, TS = fx::Tile<LX>::SIZE;
+  static constexpr int EPB = LX <= 2 ? 16 : LX == 3 ? 7 : LX == 4 ? 4 : LX == 5 ? 5 : LX == 6 ? 2 : 1;
+  static constexpr int NT = (EPB * 3 * L2 + 31) / 32 * 32;
+  // per element: tiles, the exponents of a flux's lines; once: the products of the GLL weights
+  static constexpr int EL = TILES * TS + (3 * L2 + 1) / 2;
+  static constexpr size_t SMEM = (size_t)(EPB * EL + L3) * sizeof(double);
+  static constexpr int FIT = (int)(230000 / (SMEM + 1024)), WANT = 1024 / NT;
+  static constexpr int MINB = FIT < 1 ? 1 : FIT < WANT ? FIT : WANT;
+};
+
+// the weights' products at the nodes, staged once per block
+template <int LX>
+__device__ __forceinline__ void stage_w3(double* w3, const DMat<LX>& M, int nt) {
+  for (int t = threadIdx.x; t < LX * LX * LX; t += nt) w3[t] = M.w[t % LX] * M.w[t / LX % LX] * M.w[t / (LX * LX)];
+}
+
+template <int LX, int TILES>
+int fx_grid(const ntg_plan* p) {
+  using S = FxShape<LX, TILES>;
+  const int64_t g = (p->nelv + S::EPB - 1) / S::EPB, cap = (int64_t)num_sms() * S::MINB;
+  return (int)(g < cap ? g : cap);
+}
+
+// The kernels with these walk elements in three kinds of passes: over nodes
+// (loads, metric products, results), over lines of one direction or of all
+// three (derivatives, fx::deriv_line / flux_line) and barriers between.
+// What bounds them is the FP64 pipe (2 operations per clock and SM), which
+// only the metric products still use; the contractions run beside them on
+// the integer pipes.  NODES / LINES number the work items of a block's ne
+// elements: item t -> element el of the block, node or line.
+#define NTG_FX_PROLOGUE(TILES)                                                                  \
+  using S = FxShape<LX, TILES>;                                                                 \
+  using TL = fx::Tile<LX>;                                                                      \
+  constexpr int L2 = S::L2, L3 = S::L3, TS = S::TS, EPB = S::EPB, NT = S::NT, EL = S::EL;       \
+  extern __shared__ double fxs[];                                                               \
+  double* w3t = fxs + EPB * EL;                                                                 \
+  (void)w3t;
+#define NTG_FX_ELEMENTS for (int64_t e0 = blockIdx.x * (int64_t)EPB; e0 < nelv; e0 += (int64_t)gridDim.x * EPB)
+#define NTG_FX_NE const int ne = nelv - e0 < EPB ? (int)(nelv - e0) : EPB
+#define NTG_FX_NODES for (int t = threadIdx.x; t < ne * L3; t += NT)
+#define NTG_FX_NODE                                                                             \
+  const int el = EPB == 1 ? 0 : t / L3, node = EPB == 1 ? t : t - el * L3, p = TL::at(node);    \
+  const int64_t q = e0 * L3 + t;                                                                \
+  double* T = fxs + el * EL;                                                                    \
+  (void)p; (void)T; (void)q;
+#define NTG_FX_LINES for (int t = threadIdx.x; t < ne * 3 * L2; t += NT)
+#define NTG_FX_LINE                                                                             \
+  const int el = EPB == 1 ? 0 : t / (3 * L2), r = EPB == 1 ? t : t - el * 3 * L2, d = r / L2;   \
+  const int lq = r - d * L2;                                                                    \
+  double* T = fxs + el * EL;
 
 // reference derivatives at (i, j, k) of the tile s (s[c * LX2 + b * LX + a])
 template <int LX>
@@ -80,10 +136,9 @@ inline int need_metrics(const ntg_plan* p) {
   return NTG_OK;
 }
 
-// w = B curl u, unassembled (deriv.cu)
-int bcurl(ntg_plan* p, double* w0, double* w1, double* w2, const double* ux, const double* uy, const double* uz);
-// w = Binv gs(B curl u) (deriv.cu)
-int curl_avg(ntg_plan* p, double* w0, double* w1, double* w2, const double* ux, const double* uy, const double* uz);
+// w = gs(B curl(scale u)), scale null: 1 (deriv.cu)
+int curl_gs(ntg_plan* p, double* w0, double* w1, double* w2, const double* ux, const double* uy, const double* uz,
+            const double* scale);
 
 // n-double device scratch owned by the plan (grown on demand, freed with it)
 double* plan_scratch(ntg_plan* p, int64_t count);

@@ -67,6 +67,19 @@ static int gs_any(ntg_plan* p, T* u, int op, cudaStream_t s, const Scalars* sc) 
 
 int gs_launch(ntg_plan* p, double* u, int op, cudaStream_t s) { return gs_any<double>(p, u, op, s, nullptr); }
 int gs_launch_f32(ntg_plan* p, float* u, int op, cudaStream_t s) { return gs_any<float>(p, u, op, s, nullptr); }
+// three distinct fields, one launch
+int gs_launch3(ntg_plan* p, double* u0, double* u1, double* u2, cudaStream_t s) {
+  if (p->nshared == 0) return NTG_OK;
+  if (p->gs_classes) {
+    timer_start(TM_GS64, s);
+    const int st = gs_cls_launch3(p, u0, u1, u2, s);
+    timer_stop(TM_GS64, s);
+    return st;
+  }
+  NTG_TRY(gs_launch(p, u0, NTG_GS_ADD, s));
+  NTG_TRY(gs_launch(p, u1, NTG_GS_ADD, s));
+  return gs_launch(p, u2, NTG_GS_ADD, s);
+}
 int gs_add_guarded(ntg_plan* p, double* u, cudaStream_t s, const Scalars* sc) {
   return gs_any<double>(p, u, NTG_GS_ADD, s, sc);
 }

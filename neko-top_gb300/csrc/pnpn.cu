@@ -26,19 +26,17 @@ namespace ntg {
 namespace pn {
 
 using dv::DMat;
-using dv::rgrad;
-using dv::Shape;
+using dv::FxShape;
 
 struct GPtr {
   const double* g[6];
 };
 
+// mu and rho: fields, or constants (ri: the constant's reciprocal)
 struct Coefs {
   const double* mu;
   const double* rho;
-  double muc, rhoc;
-  __device__ __forceinline__ double m(int64_t q) const { return mu ? mu[q] : muc; }
-  __device__ __forceinline__ double r(int64_t q) const { return rho ? rho[q] : rhoc; }
+  double muc, rhoc, ri;
 };
 
 // X_c holds gs(B curl t)_c; becomes f_c / rho - (mu / rho) B (Binv X_c)
@@ -46,132 +44,116 @@ __global__ void k_ta(double* __restrict__ x0, double* __restrict__ x1, double* _
                      const double* __restrict__ f0, const double* __restrict__ f1, const double* __restrict__ f2,
                      const double* __restrict__ B, const double* __restrict__ binv, Coefs c, int64_t n) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
-    const double rho = c.r(q), mr = c.m(q) / rho, bb = B[q], bi = binv[q];
-    x0[q] = f0[q] / rho - mr * bb * (bi * x0[q]);
-    x1[q] = f1[q] / rho - mr * bb * (bi * x1[q]);
-    x2[q] = f2[q] / rho - mr * bb * (bi * x2[q]);
+    const double ri = c.rho ? 1.0 / c.rho[q] : c.ri;
+    const double m = (c.mu ? c.mu[q] : c.muc) * ri * (B[q] * binv[q]);
+    x0[q] = fma(-m, x0[q], f0[q] * ri);
+    x1[q] = fma(-m, x1[q], f1[q] * ri);
+    x2[q] = fma(-m, x2[q], f2[q] * ri);
   }
 }
 
 // p_res = -D^T (h1 G D p) + sum_d cdtp_d(binv ta_d), h1 = 1 / rho
 template <int LX>
-__global__ void __launch_bounds__(Shape<LX, 4>::THREADS)
-    k_prs_core(double* __restrict__ pres, const double* __restrict__ p, const double* __restrict__ ta0,
+__global__ void __launch_bounds__(FxShape<LX, 4>::NT, FxShape<LX, 4>::MINB)
+    k_prs_core(double* __restrict__ pres, const double* __restrict__ pp, const double* __restrict__ ta0,
                const double* __restrict__ ta1, const double* __restrict__ ta2, const double* __restrict__ binv,
-               Coefs c, int64_t nelv, const __grid_constant__ DMat<LX> M, GPtr G, const double* __restrict__ met,
-               int64_t n) {
-  using S = Shape<LX, 4>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double sp[EPB][LX3], fr[EPB][LX3], fs[EPB][LX3], ft[EPB][LX3];
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k) sp[le][k * LX2 + ij] = act ? p[e * LX3 + k * LX2 + ij] : 0.0;
+               Coefs c, int64_t nelv, const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P,
+               GPtr G, const double* __restrict__ met, int64_t n) {
+  NTG_FX_PROLOGUE(4)
+  dv::stage_w3<LX>(w3t, M, NT);
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    NTG_FX_NODES { NTG_FX_NODE T[p] = pp[q]; }
     __syncthreads();
-    if (act) {
-      for (int k = 0; k < LX; ++k) {
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        double ur, us, ut;
-        rgrad<LX>(sp[le], M, i, j, k, ur, us, ut);
-        const double h1 = 1.0 / c.r(q), w3 = M.w[i] * M.w[j] * M.w[k], bi = binv[q];
-        const double a0 = bi * ta0[q], a1 = bi * ta1[q], a2 = bi * ta2[q];
-        const double g11 = G.g[0][q], g12 = G.g[1][q], g13 = G.g[2][q], g22 = G.g[3][q], g23 = G.g[4][q],
-                     g33 = G.g[5][q];
-        const double cr = met[0 * n + q] * a0 + met[1 * n + q] * a1 + met[2 * n + q] * a2;
-        const double cs = met[3 * n + q] * a0 + met[4 * n + q] * a1 + met[5 * n + q] * a2;
-        const double ct = met[6 * n + q] * a0 + met[7 * n + q] * a1 + met[8 * n + q] * a2;
-        fr[le][k * LX2 + ij] = w3 * cr - h1 * (g11 * ur + g12 * us + g13 * ut);
-        fs[le][k * LX2 + ij] = w3 * cs - h1 * (g12 * ur + g22 * us + g23 * ut);
-        ft[le][k * LX2 + ij] = w3 * ct - h1 * (g13 * ur + g23 * us + g33 * ut);
-      }
+    NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T, T + (1 + d) * TS, d, lq); }
+    __syncthreads();
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      const double ur = T[TS + p], us = T[2 * TS + p], ut = T[3 * TS + p];
+      const double h1 = c.rho ? 1.0 / c.rho[q] : c.ri, b = w3t[node] * binv[q];
+      const double a0 = b * ta0[q], a1 = b * ta1[q], a2 = b * ta2[q];
+      const double g12 = G.g[1][q], g13 = G.g[2][q], g23 = G.g[4][q];
+      const double er = G.g[0][q] * ur + g12 * us + g13 * ut, es = g12 * ur + G.g[3][q] * us + g23 * ut;
+      const double et = g13 * ur + g23 * us + G.g[5][q] * ut;
+      T[TS + p] = fma(-h1, er, met[0 * n + q] * a0 + met[1 * n + q] * a1 + met[2 * n + q] * a2);
+      T[2 * TS + p] = fma(-h1, es, met[3 * n + q] * a0 + met[4 * n + q] * a1 + met[5 * n + q] * a2);
+      T[3 * TS + p] = fma(-h1, et, met[6 * n + q] * a0 + met[7 * n + q] * a1 + met[8 * n + q] * a2);
     }
     __syncthreads();
-    if (act) {
-      for (int k = 0; k < LX; ++k) {
-        double acc = 0.0;
-#pragma unroll
-        for (int l = 0; l < LX; ++l) {
-          acc = fma(M.d[l * LX + i], fr[le][k * LX2 + j * LX + l], acc);
-          acc = fma(M.d[l * LX + j], fs[le][k * LX2 + l * LX + i], acc);
-          acc = fma(M.d[l * LX + k], ft[le][l * LX2 + j * LX + i], acc);
-        }
-        pres[e * LX3 + k * LX2 + ij] = acc;
-      }
+    NTG_FX_LINES {
+      NTG_FX_LINE
+      fx::flux_line<LX>(P.DT, P.dt, T + (1 + d) * TS, reinterpret_cast<int*>(T + 4 * TS) + r, d, lq);
     }
     __syncthreads();
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      pres[q] = fx::flux_sum<LX>(T + TS, T + 2 * TS, T + 3 * TS, reinterpret_cast<const int*>(T + 4 * TS), node);
+    }
   }
 }
 
-// res_c = f_c - D^T (mu G D u_c) - rho (bd/dt) B u_c - opgrad_c(p), c = 0..2
+// res_c = f_c - D^T (mu G D u_c) - rho (bd/dt) B u_c - opgrad_c(p), c = 0..2.
+// P.DT carries mus, a constant mu (1 when mu is a field, which then
+// multiplies the fluxes).
 template <int LX>
-__global__ void __launch_bounds__(Shape<LX, 5>::THREADS)
+__global__ void __launch_bounds__(FxShape<LX, 7>::NT, FxShape<LX, 7>::MINB)
     k_vel_res(double* __restrict__ r0, double* __restrict__ r1, double* __restrict__ r2,
               const double* __restrict__ u0, const double* __restrict__ u1, const double* __restrict__ u2,
-              const double* __restrict__ p, const double* __restrict__ f0, const double* __restrict__ f1,
-              const double* __restrict__ f2, Coefs c, double bddt, int64_t nelv,
-              const __grid_constant__ DMat<LX> M, GPtr G, const double* __restrict__ B,
-              const double* __restrict__ met, int64_t n) {
-  using S = Shape<LX, 5>;
-  constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
-  __shared__ double su[EPB][LX3], sp[EPB][LX3], fr[EPB][LX3], fs[EPB][LX3], ft[EPB][LX3];
-  const int tid = threadIdx.x, le = tid / LX2, ij = tid - le * LX2, i = ij % LX, j = ij / LX;
-  const bool worker = tid < S::NW;
-  for (int64_t g = blockIdx.x; g * EPB < nelv; g += gridDim.x) {
-    const int64_t e = g * EPB + le;
-    const bool act = worker && e < nelv;
-    for (int k = 0; k < LX && worker; ++k) sp[le][k * LX2 + ij] = act ? p[e * LX3 + k * LX2 + ij] : 0.0;
+              const double* __restrict__ pp, const double* __restrict__ f0, const double* __restrict__ f1,
+              const double* __restrict__ f2, Coefs c, double mus, double bddt, int64_t nelv,
+              const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P, GPtr G,
+              const double* __restrict__ B, const double* __restrict__ met, int64_t n) {
+  NTG_FX_PROLOGUE(7)
+  dv::stage_w3<LX>(w3t, M, NT);
+  NTG_FX_ELEMENTS {
+    NTG_FX_NE;
+    // tiles 0-2: the gradient of p; 3: a component; 4-6: its derivatives, then fluxes
+    NTG_FX_NODES { NTG_FX_NODE T[3 * TS + p] = pp[q]; }
     __syncthreads();
-    // res_c = f_c - opgrad_c(p) first (the pressure gradient once for all
-    // three components); the thread that writes a node updates it below
-    if (act) {
-      for (int k = 0; k < LX; ++k) {
-        const int64_t q = e * LX3 + k * LX2 + ij;
-        double pr, ps, pt;
-        rgrad<LX>(sp[le], M, i, j, k, pr, ps, pt);
-        const double w3 = M.w[i] * M.w[j] * M.w[k];
-        r0[q] = f0[q] - w3 * (met[0 * n + q] * pr + met[3 * n + q] * ps + met[6 * n + q] * pt);
-        r1[q] = f1[q] - w3 * (met[1 * n + q] * pr + met[4 * n + q] * ps + met[7 * n + q] * pt);
-        r2[q] = f2[q] - w3 * (met[2 * n + q] * pr + met[5 * n + q] * ps + met[8 * n + q] * pt);
-      }
-    }
+    NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T + 3 * TS, T + d * TS, d, lq); }
 #pragma unroll 1
     for (int cc = 0; cc < 3; ++cc) {
-      const double* u = cc == 0 ? u0 : (cc == 1 ? u1 : u2);
-      double* r = cc == 0 ? r0 : (cc == 1 ? r1 : r2);
-      for (int k = 0; k < LX && worker; ++k) su[le][k * LX2 + ij] = act ? u[e * LX3 + k * LX2 + ij] : 0.0;
+      const double* u = cc == 0 ? u0 : cc == 1 ? u1 : u2;
+      const double* f = cc == 0 ? f0 : cc == 1 ? f1 : f2;
+      double* res = cc == 0 ? r0 : cc == 1 ? r1 : r2;
       __syncthreads();
-      if (act) {
-        for (int k = 0; k < LX; ++k) {
-          const int64_t q = e * LX3 + k * LX2 + ij;
-          double ur, us, ut;
-          rgrad<LX>(su[le], M, i, j, k, ur, us, ut);
-          const double h1 = c.m(q);
-          const double g11 = G.g[0][q], g12 = G.g[1][q], g13 = G.g[2][q], g22 = G.g[3][q], g23 = G.g[4][q],
-                       g33 = G.g[5][q];
-          fr[le][k * LX2 + ij] = h1 * (g11 * ur + g12 * us + g13 * ut);
-          fs[le][k * LX2 + ij] = h1 * (g12 * ur + g22 * us + g23 * ut);
-          ft[le][k * LX2 + ij] = h1 * (g13 * ur + g23 * us + g33 * ut);
+      NTG_FX_NODES { NTG_FX_NODE T[3 * TS + p] = u[q]; }
+      __syncthreads();
+      NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T + 3 * TS, T + (4 + d) * TS, d, lq); }
+      __syncthreads();
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        const double ur = T[4 * TS + p], us = T[5 * TS + p], ut = T[6 * TS + p];
+        const double g12 = G.g[1][q], g13 = G.g[2][q], g23 = G.g[4][q];
+        T[4 * TS + p] = G.g[0][q] * ur + g12 * us + g13 * ut;
+        T[5 * TS + p] = g12 * ur + G.g[3][q] * us + g23 * ut;
+        T[6 * TS + p] = g13 * ur + g23 * us + G.g[5][q] * ut;
+      }
+      if (c.mu || mus != 1.0) {  // a field, or a constant too large or small for P.DT
+        NTG_FX_NODES {
+          NTG_FX_NODE
+          const double m = c.mu ? c.mu[q] : mus;
+          T[4 * TS + p] *= m;
+          T[5 * TS + p] *= m;
+          T[6 * TS + p] *= m;
         }
       }
       __syncthreads();
-      if (act) {
-        for (int k = 0; k < LX; ++k) {
-          const int64_t q = e * LX3 + k * LX2 + ij;
-          double acc = 0.0;
-#pragma unroll
-          for (int l = 0; l < LX; ++l) {
-            acc = fma(M.d[l * LX + i], fr[le][k * LX2 + j * LX + l], acc);
-            acc = fma(M.d[l * LX + j], fs[le][k * LX2 + l * LX + i], acc);
-            acc = fma(M.d[l * LX + k], ft[le][l * LX2 + j * LX + i], acc);
-          }
-          const double h2 = c.r(q) * bddt;
-          r[q] -= acc + h2 * B[q] * su[le][k * LX2 + ij];
-        }
+      NTG_FX_LINES {
+        NTG_FX_LINE
+        fx::flux_line<LX>(P.DT, P.dt, T + (4 + d) * TS, reinterpret_cast<int*>(T + 7 * TS) + r, d, lq);
       }
       __syncthreads();
+      NTG_FX_NODES {
+        NTG_FX_NODE
+        const double h2 = (c.rho ? c.rho[q] : c.rhoc) * bddt;
+        const double gp = met[cc * n + q] * T[p] + met[(3 + cc) * n + q] * T[TS + p] + met[(6 + cc) * n + q] * T[2 * TS + p];
+        const double s = fx::flux_sum<LX>(T + 4 * TS, T + 5 * TS, T + 6 * TS,
+                                          reinterpret_cast<const int*>(T + 7 * TS), node);
+        res[q] = fma(-w3t[node], gp, f[q]) - fma(h2 * B[q], T[3 * TS + p], s);
+      }
     }
+    __syncthreads();
   }
 }
 
@@ -217,22 +199,20 @@ int ntg_pnpn_prs_res(ntg_plan* p, double* p_res, const double* pr, const double*
   if (!t) return NTG_ERR_ALLOC;
   double *t0 = t, *t1 = t + n, *t2 = t + 2 * n, *x0 = t + 3 * n, *x1 = t + 4 * n, *x2 = t + 5 * n;
   cudaStream_t s = p->stream;
-  const pn::Coefs c{mu_d, rho_d, mu_c, rho_c};
-  // t = curl(u_e); X = gs(B curl t)
-  NTG_TRY(curl_avg(p, t0, t1, t2, ue, ve, we));
-  NTG_TRY(bcurl(p, x0, x1, x2, t0, t1, t2));
-  NTG_TRY(gs_launch(p, x0, NTG_GS_ADD, s));
-  NTG_TRY(gs_launch(p, x1, NTG_GS_ADD, s));
-  NTG_TRY(gs_launch(p, x2, NTG_GS_ADD, s));
+  const pn::Coefs c{mu_d, rho_d, mu_c, rho_c, rho_d ? 1.0 : 1.0 / rho_c};
+  // Binv t = curl(u_e), its Binv applied where t is read; X = gs(B curl(Binv t))
+  NTG_TRY(curl_gs(p, t0, t1, t2, ue, ve, we, nullptr));
+  NTG_TRY(curl_gs(p, x0, x1, x2, t0, t1, t2, p->binv));
   // ta = gs(f / rho - (mu / rho) B wa); its Binv is applied where ta is read
   { pn::k_ta<<<grid_for(n, 256), 256, 0, s>>>(x0, x1, x2, fx, fy, fz, p->B, p->binv, c, n); NTG_COUNT_LAUNCH(); }
-  NTG_TRY(gs_launch(p, x0, NTG_GS_ADD, s));
-  NTG_TRY(gs_launch(p, x1, NTG_GS_ADD, s));
-  NTG_TRY(gs_launch(p, x2, NTG_GS_ADD, s));
+  NTG_TRY(gs_launch3(p, x0, x1, x2, s));
   NTG_TRY(dv::dispatch<4>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    pn::k_prs_core<LX><<<dv::grid_of<LX, 4>(p), dv::Shape<LX, 4>::THREADS, 0, s>>>(
-        p_res, pr, x0, x1, x2, p->binv, c, p->nelv, dv::dmat<LX>(p), pn::gptr(p), p->met, n);
+    using S = dv::FxShape<LX, 4>;
+    NTG_TRY(fx::use_smem<pn::k_prs_core<LX>>(S::SMEM));
+    pn::k_prs_core<LX><<<dv::fx_grid<LX, 4>(p), S::NT, S::SMEM, s>>>(
+        p_res, pr, x0, x1, x2, p->binv, c, p->nelv, dv::dmat<LX>(p), fx::plan_mats<LX>(p, 1.0), pn::gptr(p), p->met,
+        n);
     NTG_COUNT_LAUNCH();
     return NTG_OK;
   }));
@@ -258,12 +238,16 @@ int ntg_pnpn_vel_res(ntg_plan* p, double* u_res, double* v_res, double* w_res, c
                 "ntg_pnpn_vel_res: null field argument");
   NTG_CHECK_ARG(dt > 0.0, "ntg_pnpn_vel_res: need dt > 0");
   NTG_TRY(need_metrics(p));
-  const pn::Coefs c{mu_d, rho_d, mu_c, rho_c};
-  return dv::dispatch<5>(p->lx, [&](auto L) -> int {
+  const pn::Coefs c{mu_d, rho_d, mu_c, rho_c, 0.0};
+  const double fold = !mu_d && fx::foldable(mu_c) ? mu_c : 1.0;  // a constant mu goes into D^T
+  const double mus = mu_d || fold == mu_c ? 1.0 : mu_c;
+  return dv::dispatch<7>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    pn::k_vel_res<LX><<<dv::grid_of<LX, 5>(p), dv::Shape<LX, 5>::THREADS, 0, p->stream>>>(
-        u_res, v_res, w_res, u, v, w, pr, fx, fy, fz, c, bd / dt, p->nelv, dv::dmat<LX>(p), pn::gptr(p), p->B,
-        p->met, p->n);
+    using S = dv::FxShape<LX, 7>;
+    NTG_TRY(fx::use_smem<pn::k_vel_res<LX>>(S::SMEM));
+    pn::k_vel_res<LX><<<dv::fx_grid<LX, 7>(p), S::NT, S::SMEM, p->stream>>>(
+        u_res, v_res, w_res, u, v, w, pr, fx, fy, fz, c, mus, bd / dt, p->nelv, dv::dmat<LX>(p),
+        fx::plan_mats<LX>(p, fold), pn::gptr(p), p->B, p->met, p->n);
     NTG_COUNT_LAUNCH();
     NTG_CUDA_TRY(cudaGetLastError());
     return NTG_OK;
