@@ -9,15 +9,12 @@
 //   adjoint  f_i -= J^T [ sum_j u_j opgrad_i(Ub_j) + sum_d cdtp_d(u_i Ub_d) ]
 //   linear   f_i -= J^T [ u . opgrad(Ub_i) + Ub . opgrad(u_i) ]
 //
-// One element per block, everything between the GLL loads and the GLL
-// update in shared memory (12 GL tiles + interpolation buffers: 185 KB at
-// LX = 8, LXD = 12), so the six interpolated fields, the 27 GL derivatives
-// and the fluxes never touch HBM; only the GL cofactors (9 doubles per GL
-// point, interpolated once at create) stream from memory.  The reference
-// round-trips each of those through device arrays (20 GL-sized scratch
-// fields).  The sums are rewritten with contravariant fluxes V_r =
-// sum_d drdx_d Ub_d (etc.), so the three cdtp of a component become one D^T
-// contraction of u_i V and the linear term needs no contraction at all.
+// The reference round-trips the interpolated fields, their derivatives and
+// the fluxes through device arrays (20 GL-sized scratch fields); here only
+// the GL cofactors (9 doubles per GL point, interpolated once at create)
+// stream from memory.  The sums are rewritten with contravariant velocities,
+// so the three cdtp of a component become one transposed derivative and the
+// linear term needs none.
 #include <cmath>
 
 #include "deriv.cuh"
@@ -32,6 +29,7 @@ struct ntg_dealias {
   double* met_gl = nullptr;  // 9 x ngl cofactors at the GL points
   int grid = 0;
   size_t smem = 0;
+  std::shared_ptr<void> mats;  // the fixed-point matrices of the advection kernels
 };
 
 namespace ntg {
@@ -49,7 +47,7 @@ struct GLMat {
 template <int LX, int LXD>
 struct Smem {
   static constexpr int N3 = LXD * LXD * LXD, TA = LXD * LX * LX, TB = LXD * LXD * LX, G3 = LX * LX * LX;
-  static constexpr int DOUBLES = 12 * N3 + TA + TB + G3 + LXD * LX + LXD * LXD + LXD;
+  static constexpr int DOUBLES = 2 * N3 + TA + TB + LXD * LX + LXD * LXD + LXD;
   static constexpr size_t BYTES = sizeof(double) * DOUBLES;
 };
 
@@ -113,24 +111,11 @@ __device__ __forceinline__ void to_gll(double* __restrict__ out, const double* s
   __syncthreads();
 }
 
-template <int LXD>
-__device__ __forceinline__ void glgrad(const double* s, const double* D, int A, int B, int C, double& r, double& q,
-                                       double& t) {
-  constexpr int L2 = LXD * LXD;
-  r = q = t = 0.0;
-#pragma unroll
-  for (int l = 0; l < LXD; ++l) {
-    r = fma(D[A * LXD + l], s[C * L2 + B * LXD + l], r);
-    q = fma(D[B * LXD + l], s[C * L2 + l * LXD + A], q);
-    t = fma(D[C * LXD + l], s[l * L2 + B * LXD + A], t);
-  }
-}
-
 template <int LX, int LXD>
 __device__ __forceinline__ double* stage_mats(double* sm, const GLMat<LX, LXD>& M, double*& J, double*& D,
                                               double*& w) {
   using S = Smem<LX, LXD>;
-  J = sm + 12 * S::N3 + S::TA + S::TB + S::G3;
+  J = sm + 2 * S::N3 + S::TA + S::TB;
   D = J + LXD * LX;
   w = D + LXD * LXD;
   for (int t = threadIdx.x; t < LXD * LX; t += NT) J[t] = M.J[t];
@@ -149,7 +134,7 @@ __global__ void __launch_bounds__(NT) k_map(double* __restrict__ out, const doub
   double *J, *D, *w;
   stage_mats<LX, LXD>(sm, M, J, D, w);
   double* tile = sm;
-  double* tA = sm + 12 * S::N3;
+  double* tA = sm + 2 * S::N3;
   double* tB = tA + S::TA;
   constexpr int NIN = DIR == 0 ? S::G3 : S::N3;
   constexpr int NOUT = DIR == 0 ? S::N3 : S::G3;
@@ -171,97 +156,241 @@ __global__ void __launch_bounds__(NT) k_map(double* __restrict__ out, const doub
   }
 }
 
+// ---------------------------------------------------------------------------
+// The advection terms.  Everything between the GLL loads and the GLL update
+// stays in shared memory (12 tiles of LXD^3 numbers); the contractions (nine
+// interpolations, the GL derivatives and their transposes) run in fixed
+// point on the integer pipes (fx.cuh), the products on the FP64 pipe.
+//
+// The GL weights never appear in a product: they are folded into the
+// interpolation back (JW = J^T W per direction), which leaves the transposed
+// derivative acting before them, DT = W^-1 D^T W.  With V_d = sum_c c_dc
+// Ub_c and a_d = sum_j u_j dUb_j/dr_d the adjoint term of component i is
+//   sum_d c_di a_d + sum_d DT_d (u_i V_d)
+// (39 FP64 operations per GL point where mixing each gradient first and
+// weighting each product takes 162 with the contractions), the linear one
+//   sum_d (V_d(u) dUb_i/dr_d + V_d(Ub) du_i/dr_d)     (36).
+// ---------------------------------------------------------------------------
+template <int LX, int LXD>
+struct AdvMats {
+  fx::Mat<LX, LXD> J;
+  fx::Mat<LXD, LX> JW;
+  fx::Mat<LXD, LXD> D, DT;
+  double j[LXD * LX], jw[LX * LXD], d[LXD * LXD], dt[LXD * LXD];
+};
+
+template <int LX, int LXD>
+struct AdvShape {
+  using TG = fx::Tile<LXD>;
+  static constexpr int G2 = LXD * LXD, G3 = G2 * LXD, L2 = LX * LX, L3 = L2 * LX, RS = TG::RS, TS = TG::SIZE;
+  static constexpr int EPB = LXD == 6 ? 4 : LXD == 7 ? 3 : 1;
+  static constexpr int NT = (EPB * 3 * G2 + 31) / 32 * 32;  // a thread per line of three fields or directions
+  static constexpr int EL = 12 * TS + (3 * G2 + 1) / 2;     // doubles per element: tiles, line exponents
+  static constexpr size_t SMEM = sizeof(double) * EPB * EL;
+  static constexpr int MINB = (int)(232448 / (SMEM + 1024));
+  static constexpr int NR = (EPB * G3 + NT - 1) / NT;  // nodes per thread
+  // the interpolations' intermediate forms fit the tiles they pass through
+  static_assert(L2 * (LX | 1) * 6 <= 6 * TS && L2 * RS * 6 <= 6 * TS && LX * LXD * RS * 6 <= 6 * TS, "tiles");
+};
+
+template <int NIN, int NOUT, bool ANTI>
+__device__ __forceinline__ void line_at(const fx::Mat<NIN, NOUT>& M, const double* Md, const double* in, int si,
+                                        double* out, int so) {
+  double x[NIN];
+#pragma unroll
+  for (int l = 0; l < NIN; ++l) x[l] = in[l * si];
+  fx::line_dbl<NIN, NOUT, ANTI>(M, Md, x, [&](int A, double y) { out[A * so] = y; });
+}
+
 // MODE 0: adjoint, MODE 1: linear
 template <int LX, int LXD, int MODE>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB)
     k_adv(double* __restrict__ f0, double* __restrict__ f1, double* __restrict__ f2, const double* __restrict__ u0,
           const double* __restrict__ u1, const double* __restrict__ u2, const double* __restrict__ b0,
           const double* __restrict__ b1, const double* __restrict__ b2, const double* __restrict__ met, int64_t ngl,
-          int64_t nelv, const __grid_constant__ GLMat<LX, LXD> M) {
-  using S = Smem<LX, LXD>;
-  constexpr int N3 = S::N3, G3 = S::G3;
+          int64_t nelv, const __grid_constant__ AdvMats<LX, LXD> P) {
+  using S = AdvShape<LX, LXD>;
+  using TG = fx::Tile<LXD>;
+  constexpr int G2 = S::G2, G3 = S::G3, L2 = S::L2, L3 = S::L3, RS = S::RS, TS = S::TS, EPB = S::EPB, NT = S::NT;
+  constexpr int LS = LX | 1;
   extern __shared__ double sm[];
-  double *J, *D, *w;
-  stage_mats<LX, LXD>(sm, M, J, D, w);
-  double* sU = sm;            // 3 x N3: u on GL
-  double* sB = sm + 3 * N3;   // 3 x N3: Ub on GL
-  double* sW = sm + 6 * N3;   // 3 x N3: w3 V_r, w3 V_s, w3 V_t (adjoint)
-  double* sT = sm + 9 * N3;   // 3 x N3: the GL result per component
-  double* tA = sm + 12 * N3;
-  double* tB = tA + S::TA;
-  double* sIn = tB + S::TB;
-  double* fo[3] = {f0, f1, f2};
-  const double* ui[6] = {u0, u1, u2, b0, b1, b2};
-  __syncthreads();
-  for (int64_t e = blockIdx.x; e < nelv; e += gridDim.x) {
-    for (int fld = 0; fld < 6; ++fld) {
-      const double* src = ui[fld] + e * G3;
-      for (int t = threadIdx.x; t < G3; t += NT) sIn[t] = src[t];
-      __syncthreads();
-      to_gl<LX, LXD>(fld < 3 ? sU + fld * N3 : sB + (fld - 3) * N3, sIn, tA, tB, J);
-    }
-    for (int t = threadIdx.x; t < N3; t += NT) {
-      const int A = t % LXD, B = (t / LXD) % LXD, C = t / (LXD * LXD);
-      const int64_t q = e * N3 + t;
-      double c[9];
-#pragma unroll
-      for (int m = 0; m < 9; ++m) c[m] = met[m * ngl + q];
-      const double w3 = w[A] * w[B] * w[C];
-      const double U[3] = {sU[t], sU[N3 + t], sU[2 * N3 + t]};
-      const double V[3] = {sB[t], sB[N3 + t], sB[2 * N3 + t]};
-      const double vr = c[0] * V[0] + c[1] * V[1] + c[2] * V[2];
-      const double vs = c[3] * V[0] + c[4] * V[1] + c[5] * V[2];
-      const double vt = c[6] * V[0] + c[7] * V[1] + c[8] * V[2];
-      if (MODE == 0) {
-        double acc[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          double r, s, tt;
-          glgrad<LXD>(sB + j * N3, D, A, B, C, r, s, tt);
-#pragma unroll
-          for (int i = 0; i < 3; ++i) acc[i] = fma(U[j], c[i] * r + c[3 + i] * s + c[6 + i] * tt, acc[i]);
-        }
-#pragma unroll
-        for (int i = 0; i < 3; ++i) sT[i * N3 + t] = w3 * acc[i];
-        sW[t] = w3 * vr;
-        sW[N3 + t] = w3 * vs;
-        sW[2 * N3 + t] = w3 * vt;
-      } else {
-        const double ur_ = c[0] * U[0] + c[1] * U[1] + c[2] * U[2];
-        const double us_ = c[3] * U[0] + c[4] * U[1] + c[5] * U[2];
-        const double ut_ = c[6] * U[0] + c[7] * U[1] + c[8] * U[2];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          double br, bs, bt, ar, as, at;
-          glgrad<LXD>(sB + i * N3, D, A, B, C, br, bs, bt);
-          glgrad<LXD>(sU + i * N3, D, A, B, C, ar, as, at);
-          sT[i * N3 + t] = w3 * (br * ur_ + bs * us_ + bt * ut_ + ar * vr + as * vs + at * vt);
-        }
+  for (int64_t e0 = blockIdx.x * (int64_t)EPB; e0 < nelv; e0 += (int64_t)gridDim.x * EPB) {
+    const int ne = nelv - e0 < EPB ? (int)(nelv - e0) : EPB;
+    // items t of `per` per element: element slot, index in it
+    auto items = [&](int per, auto&& fn) {
+      for (int t = threadIdx.x; t < ne * per; t += NT) {
+        const int el = EPB == 1 ? 0 : t / per;
+        fn(sm + el * S::EL, EPB == 1 ? t : t - el * per, e0 + el);
       }
-    }
+    };
+    // the fields (u, Ub), staged by rows of LS; J along r, s, t
+    items(6 * L3, [&](double* T, int i, int64_t e) {
+      const int f = i / L3, node = i - f * L3;
+      const double* src = f == 0 ? u0 : f == 1 ? u1 : f == 2 ? u2 : f == 3 ? b0 : f == 4 ? b1 : b2;
+      T[6 * TS + (f * L2 + node / LX) * LS + node % LX] = src[e * L3 + node];
+    });
     __syncthreads();
-    if (MODE == 0) {
-      constexpr int L2 = LXD * LXD;
-      for (int t = threadIdx.x; t < N3; t += NT) {
-        const int A = t % LXD, B = (t / LXD) % LXD, C = t / L2;
+    items(6 * L2, [&](double* T, int i, int64_t) {
+      line_at<LX, LXD, false>(P.J, P.j, T + 6 * TS + i * LS, 1, T + i * RS, 1);
+    });
+    __syncthreads();
+    items(6 * LX * LXD, [&](double* T, int i, int64_t) {  // (f, c), A
+      const int fc = i / LXD, A = i - fc * LXD;
+      line_at<LX, LXD, false>(P.J, P.j, T + fc * LX * RS + A, RS, T + 6 * TS + fc * LXD * RS + A, RS);
+    });
+    __syncthreads();
+    items(6 * G2, [&](double* T, int i, int64_t) {  // f, B, A
+      const int f = i / G2, r = i - f * G2, p = r / LXD * RS + r % LXD;
+      line_at<LX, LXD, false>(P.J, P.j, T + 6 * TS + f * LX * LXD * RS + p, LXD * RS, T + f * TS + p, LXD * RS);
+    });
+    __syncthreads();
+    // tiles 0-2: u, 3-5: Ub, 6-8: derivatives or fluxes, 9-11: a_d, then the result per component
+    if constexpr (MODE == 0) {
+#pragma unroll 1
+      for (int d = 0; d < 3; ++d) {
+        items(3 * G2, [&](double* T, int i, int64_t) {
+          const int f = i / G2;
+          fx::deriv_line<LXD>(P.D, P.d, T + (3 + f) * TS, T + (6 + f) * TS, d, i - f * G2);
+        });
+        __syncthreads();
+        items(G3, [&](double* T, int node, int64_t) {
+          const int p = TG::at(node);
+          T[(9 + d) * TS + p] = T[p] * T[6 * TS + p] + T[TS + p] * T[7 * TS + p] + T[2 * TS + p] * T[8 * TS + p];
+        });
+        __syncthreads();
+      }
+      items(G3, [&](double* T, int node, int64_t e) {
+        const int p = TG::at(node);
+        const int64_t q = e * G3 + node;
+        double c[9];
+#pragma unroll
+        for (int m = 0; m < 9; ++m) c[m] = met[m * ngl + q];
+        const double vx = T[3 * TS + p], vy = T[4 * TS + p], vz = T[5 * TS + p];
+        const double ar = T[9 * TS + p], as = T[10 * TS + p], at = T[11 * TS + p];
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          T[(3 + m) * TS + p] = c[3 * m] * vx + c[3 * m + 1] * vy + c[3 * m + 2] * vz;
+          T[(9 + m) * TS + p] = c[m] * ar + c[3 + m] * as + c[6 + m] * at;
+        }
+      });
+      __syncthreads();
+#pragma unroll 1
+      for (int i = 0; i < 3; ++i) {
+        items(3 * G2, [&](double* T, int t, int64_t) {
+          const int d = t / G2, b = TG::base(d, t - d * G2), st = TG::stride(d);
+          const double *u = T + i * TS + b, *v = T + (3 + d) * TS + b;
+          double* o = T + (6 + d) * TS + b;
+          double x[LXD];
+#pragma unroll
+          for (int l = 0; l < LXD; ++l) x[l] = u[l * st] * v[l * st];
+          reinterpret_cast<int*>(T + 12 * TS)[t] = fx::line_int<LXD, LXD, true>(
+              P.DT, P.dt, x, [&](int A, int64_t y) { o[A * st] = __longlong_as_double(y); });
+        });
+        __syncthreads();
+        items(G3, [&](double* T, int node, int64_t) {
+          const int p = TG::at(node);
+          T[(9 + i) * TS + p] += fx::flux_sum<LXD>(T + 6 * TS, T + 7 * TS, T + 8 * TS,
+                                                   reinterpret_cast<const int*>(T + 12 * TS), node);
+        });
+        __syncthreads();
+      }
+    } else {
+      double acc[S::NR][3];
+#pragma unroll
+      for (int r = 0; r < S::NR; ++r) acc[r][0] = acc[r][1] = acc[r][2] = 0.0;
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass) {
+        items(G3, [&](double* T, int node, int64_t e) {
+          const int p = TG::at(node);
+          const int64_t q = e * G3 + node;
+          const double* X = T + (pass ? 3 : 0) * TS + p;
+          const double x = X[0], y = X[TS], z = X[2 * TS];
+#pragma unroll
+          for (int m = 0; m < 3; ++m)
+            T[(9 + m) * TS + p] = met[3 * m * ngl + q] * x + met[(3 * m + 1) * ngl + q] * y + met[(3 * m + 2) * ngl + q] * z;
+        });
 #pragma unroll 1
         for (int i = 0; i < 3; ++i) {
-          const double* su = sU + i * N3;
-          double acc = 0.0;
+          items(3 * G2, [&](double* T, int t, int64_t) {
+            const int d = t / G2;
+            fx::deriv_line<LXD>(P.D, P.d, T + ((pass ? 0 : 3) + i) * TS, T + (6 + d) * TS, d, t - d * G2);
+          });
+          __syncthreads();
 #pragma unroll
-          for (int l = 0; l < LXD; ++l) {
-            const int pr = C * L2 + B * LXD + l, ps = C * L2 + l * LXD + A, pt = l * L2 + B * LXD + A;
-            acc = fma(D[l * LXD + A], su[pr] * sW[pr], acc);
-            acc = fma(D[l * LXD + B], su[ps] * sW[N3 + ps], acc);
-            acc = fma(D[l * LXD + C], su[pt] * sW[2 * N3 + pt], acc);
+          for (int r = 0; r < S::NR; ++r) {
+            const int t = threadIdx.x + r * NT;
+            if (t < ne * G3) {
+              const int el = EPB == 1 ? 0 : t / G3;
+              const double* T = sm + el * S::EL + TG::at(EPB == 1 ? t : t - el * G3);
+              const double g = T[6 * TS] * T[9 * TS] + T[7 * TS] * T[10 * TS] + T[8 * TS] * T[11 * TS];
+              if (i == 0) acc[r][0] += g;
+              else if (i == 1) acc[r][1] += g;
+              else acc[r][2] += g;
+            }
           }
-          sT[i * N3 + t] += acc;
+          __syncthreads();
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < S::NR; ++r) {
+        const int t = threadIdx.x + r * NT;
+        if (t < ne * G3) {
+          const int el = EPB == 1 ? 0 : t / G3;
+          double* T = sm + el * S::EL + TG::at(EPB == 1 ? t : t - el * G3);
+          T[9 * TS] = acc[r][0];
+          T[10 * TS] = acc[r][1];
+          T[11 * TS] = acc[r][2];
         }
       }
       __syncthreads();
     }
-    for (int i = 0; i < 3; ++i) to_gll<LX, LXD>(fo[i] + e * G3, sT + i * N3, tA, tB, J, true);
+    // back: JW along t, s, r, then f -= the result
+    items(3 * G2, [&](double* T, int t, int64_t) {  // i, B, A
+      const int i = t / G2, r = t - i * G2, p = r / LXD * RS + r % LXD;
+      line_at<LXD, LX, false>(P.JW, P.jw, T + (9 + i) * TS + p, LXD * RS, T + i * LX * LXD * RS + p, LXD * RS);
+    });
+    __syncthreads();
+    items(3 * LX * LXD, [&](double* T, int t, int64_t) {  // (i, c), A
+      const int ic = t / LXD, A = t - ic * LXD;
+      line_at<LXD, LX, false>(P.JW, P.jw, T + ic * LXD * RS + A, RS, T + 6 * TS + ic * LX * RS + A, RS);
+    });
+    __syncthreads();
+    items(3 * L2, [&](double* T, int t, int64_t) {  // (i, c, b)
+      line_at<LXD, LX, false>(P.JW, P.jw, T + 6 * TS + t * RS, 1, T + t * LS, 1);
+    });
+    __syncthreads();
+    items(3 * L3, [&](double* T, int t, int64_t e) {
+      const int i = t / L3, node = t - i * L3;
+      double* f = (i == 0 ? f0 : i == 1 ? f1 : f2) + e * L3 + node;
+      *f -= T[(i * L2 + node / LX) * LS + node % LX];
+    });
+    // the next element's fields go to tiles 6 on, read last before the barrier above
   }
+}
+
+template <int LX, int LXD>
+AdvMats<LX, LXD> adv_mats(const ntg_dealias* d) {
+  AdvMats<LX, LXD> P;
+  long double dt[LXD * LXD];
+  for (int A = 0; A < LXD; ++A) {
+    for (int a = 0; a < LX; ++a) {
+      P.j[A * LX + a] = d->J[A * LX + a];
+      P.jw[a * LXD + A] = d->J[A * LX + a] * d->wg[A];
+    }
+    for (int l = 0; l < LXD; ++l) {
+      P.d[A * LXD + l] = d->Dg[A * LXD + l];
+      dt[A * LXD + l] = (long double)d->Dg[l * LXD + A] * d->wg[l] / d->wg[A];
+      P.dt[A * LXD + l] = (double)dt[A * LXD + l];
+    }
+  }
+  P.J = fx::make_mat<LX, LXD>(d->J);
+  long double jw[LX * LXD];
+  for (int a = 0; a < LX; ++a)
+    for (int A = 0; A < LXD; ++A) jw[a * LXD + A] = (long double)d->J[A * LX + a] * d->wg[A];
+  P.JW = fx::make_mat<LXD, LX>(jw);
+  P.D = fx::make_mat<LXD, LXD>(d->Dg);
+  P.DT = fx::make_mat<LXD, LXD>(dt);
+  return P;
 }
 
 template <int LX, int LXD>
@@ -367,16 +496,13 @@ int ntg_dealias_create(ntg_dealias** out, ntg_plan* p, int lxd) {
       constexpr int LX = decltype(L)::value, LXD = decltype(LD)::value;
       using S = dl::Smem<LX, LXD>;
       d->smem = S::BYTES;
+      d->mats = std::make_shared<dl::AdvMats<LX, LXD>>(dl::adv_mats<LX, LXD>(d));
       NTG_CUDA_TRY(cudaFuncSetAttribute(dl::k_map<LX, LXD, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)S::BYTES));
       NTG_CUDA_TRY(cudaFuncSetAttribute(dl::k_map<LX, LXD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)S::BYTES));
-      NTG_CUDA_TRY(cudaFuncSetAttribute(dl::k_adv<LX, LXD, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)S::BYTES));
-      NTG_CUDA_TRY(cudaFuncSetAttribute(dl::k_adv<LX, LXD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)S::BYTES));
       int occ = 0;
-      NTG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dl::k_adv<LX, LXD, 0>, dl::NT, S::BYTES));
+      NTG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, dl::k_map<LX, LXD, 0>, dl::NT, S::BYTES));
       if (occ < 1) occ = 1;
       const int64_t g = (int64_t)num_sms() * occ;
       d->grid = (int)(p->nelv < g ? p->nelv : g);
@@ -430,21 +556,26 @@ int ntg_dealias_map(ntg_dealias* d, double* out_d, const double* in_d, int to_gl
   });
 }
 
-static int adv_dealias(ntg_dealias* d, int mode, double* fx, double* fy, double* fz, const double* vx,
+static int adv_dealias(ntg_dealias* d, int mode, double* f0, double* f1, double* f2, const double* vx,
                        const double* vy, const double* vz, const double* vxb, const double* vyb, const double* vzb) {
   clear_error();
-  NTG_CHECK_ARG(d && fx && fy && fz && vx && vy && vz && vxb && vyb && vzb, "dealiased advection: null argument");
+  NTG_CHECK_ARG(d && f0 && f1 && f2 && vx && vy && vz && vxb && vyb && vzb, "dealiased advection: null argument");
   ntg_plan* p = d->p;
   return dl::dispatch(d->lx, d->lxd, [&](auto L, auto LD) -> int {
     constexpr int LX = decltype(L)::value, LXD = decltype(LD)::value;
-    if (mode == 0)
-      dl::k_adv<LX, LXD, 0><<<d->grid, dl::NT, d->smem, p->stream>>>(fx, fy, fz, vx, vy, vz, vxb, vyb, vzb,
-                                                                      d->met_gl, d->ngl, p->nelv,
-                                                                      dl::glmat<LX, LXD>(d));
-    else
-      dl::k_adv<LX, LXD, 1><<<d->grid, dl::NT, d->smem, p->stream>>>(fx, fy, fz, vx, vy, vz, vxb, vyb, vzb,
-                                                                      d->met_gl, d->ngl, p->nelv,
-                                                                      dl::glmat<LX, LXD>(d));
+    using S = dl::AdvShape<LX, LXD>;
+    const auto& P = *static_cast<const dl::AdvMats<LX, LXD>*>(d->mats.get());
+    const int64_t g = (p->nelv + S::EPB - 1) / S::EPB, cap = (int64_t)num_sms() * S::MINB;
+    const int grid = (int)(g < cap ? g : cap);
+    if (mode == 0) {
+      NTG_TRY((fx::use_smem<dl::k_adv<LX, LXD, 0>>(S::SMEM)));
+      dl::k_adv<LX, LXD, 0><<<grid, S::NT, S::SMEM, p->stream>>>(f0, f1, f2, vx, vy, vz, vxb, vyb, vzb, d->met_gl,
+                                                                 d->ngl, p->nelv, P);
+    } else {
+      NTG_TRY((fx::use_smem<dl::k_adv<LX, LXD, 1>>(S::SMEM)));
+      dl::k_adv<LX, LXD, 1><<<grid, S::NT, S::SMEM, p->stream>>>(f0, f1, f2, vx, vy, vz, vxb, vyb, vzb, d->met_gl,
+                                                                 d->ngl, p->nelv, P);
+    }
     NTG_COUNT_LAUNCH();
     NTG_CUDA_TRY(cudaGetLastError());
     return NTG_OK;
