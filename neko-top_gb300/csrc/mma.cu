@@ -8,8 +8,8 @@
 // origins) lives on the device; the m-sized dual quantities (y, z, lambda,
 // s, mu, zeta) and the (m+1) x (m+1) Newton system live on the host, as in
 // the reference, where they are scalars per rank.  Each Newton step is
-// three kernels with fused reductions (residual, assembly, direction) and
-// one per line-search trial; each reduction is deterministic (per-block
+// a direction kernel and one per line-search trial, which also assembles the
+// next Newton system; each reduction is deterministic (per-block
 // partials summed in block order by the last block) and its m + 2 .. m(m+5)/2
 // totals come back in one small copy, the GPU stand-in for the reference's
 // MPI_Allreduce calls.  m <= 4 constraints.
@@ -28,23 +28,27 @@ constexpr int LANES = 2 * MMAX + MMAX * (MMAX + 1) / 2 + 2;  // sums + 1 max
 // the reference's default-kind (single precision) literals
 constexpr double C001 = (double)0.01f, C01 = (double)0.1f, C09 = (double)0.9f, C101 = (double)1.01f;
 
-// 1/a and 1/b from one division (1/(ab) times the other factor): the FP64
-// pipe, not memory, bounds these kernels, and a division costs it about ten
-// FMAs.  Each result is within a few ulp of the quotient.
-__device__ __forceinline__ void rcp2(double a, double b, double& ra, double& rb) {
-  const double r = 1.0 / (a * b);
-  ra = b * r;
-  rb = a * r;
+// 1/x by the third-order iteration r (1 + e + e^2), e = 1 - x r (Householder),
+// from the hardware's approximation r0: e0 < 2^-19 leaves e0^3 < 2^-57, the
+// result within an ulp.  The FP64 pipe (2 operations per clock and SM) bounds
+// these kernels; this takes three of them, a division about ten.
+__device__ __forceinline__ double rcp(double x) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(fma(e, e, e), r, r);
 }
 
-// 1/a, 1/b, 1/c, 1/d from one division
-__device__ __forceinline__ void rcp4(double a, double b, double c, double d, double& ra, double& rb, double& rc,
-                                     double& rd) {
-  const double ab = a * b, cd = c * d, r = 1.0 / (ab * cd), rab = cd * r, rcd = ab * r;
-  ra = b * rab;
-  rb = a * rab;
-  rc = d * rcd;
-  rd = c * rcd;
+// the larger of a >= 0 and |v| (NaN ignored, as fmax does) on the integer
+// pipes: an FP64 comparison takes a slot of the FP64 pipe
+__device__ __forceinline__ double max_abs(double a, double v) {
+  const long long m = __double_as_longlong(v) & 0x7fffffffffffffffll;
+  return m > __double_as_longlong(a) && m <= 0x7ff0000000000000ll ? __longlong_as_double(m) : a;
+}
+// the larger of a >= 0 and v of either sign
+__device__ __forceinline__ double max_pos(double a, double v) {
+  const long long m = __double_as_longlong(v);
+  return m > __double_as_longlong(a) && m <= 0x7ff0000000000000ll ? v : a;
 }
 
 __device__ __forceinline__ double warp_max(double v) {
@@ -125,7 +129,10 @@ __device__ __forceinline__ void reduce_out(double (&v)[NS], double mx, double* _
 
 struct Vecs {
   double *low, *upp, *alpha, *beta, *p0, *q0, *P, *Q, *xmin, *xmax, *xold1, *xold2;
-  double *x, *xsi, *eta, *dx, *dxsi, *deta, *x0, *xsi0, *eta0, *tdx, *diagx;
+  double *x, *xsi, *eta;     // the interior-point iterate
+  double *xt, *xsit, *etat;  // a line-search trial (they change places when it is taken)
+  double *dx, *dxsi, *deta;  // its direction
+  double *ral, *rbe, *rdg, *delx, *gg;  // at the trial: 1/(x - alpha), 1/(beta - x), 1/diagx, delx, the m rows of GG
 };
 
 struct Red {
@@ -192,117 +199,90 @@ struct Dual {
   double epsi, steg;
 };
 
-// Residual of the perturbed KKT system at (x, xsi, eta; lambda): sums
-// g_i(x) = sum_j P_ij/(u-x) + Q_ij/(x-l), sum of rex^2 + rexsi^2 + reeta^2
-// and max |rex|, |rexsi|, |reeta|.  TRIAL: first step from the line-search
-// origin: x = x0 + steg dx (likewise xsi, eta).
+// One pass over the variables at a point of the interior-point method: the
+// residual of the perturbed KKT system and the assembly of the Newton system
+// that starts there (mma_cpu.f90:307-405).  TRIAL: the point is the trial
+// x + steg dx (likewise xsi, eta), written to the trial vectors; a trial that
+// is taken, nearly always the first, needs no second pass for its Newton
+// system, and both share the reciprocals 1/(u-x), 1/(x-l), 1/(x-alpha),
+// 1/(beta-x).  Sums: g_i = sum_j P_ij/(u-x) + Q_ij/(x-l); b_i = sum_j GG_ij
+// delx_j/diagx_j; A_ik = sum_j GG_ij GG_kj / diagx_j (upper triangle); rex^2
+// + rexsi^2 + reeta^2; and max |rex|, |rexsi|, |reeta|.  49 FP64 operations
+// per variable at m = 1 (residual and assembly apart: 95, with divisions).
 template <int M, bool TRIAL>
-__global__ void __launch_bounds__(NT) k_resid(Vecs V, Dual D, int64_t n, Red R) {
-  double acc[M + 1];
-#pragma unroll
-  for (int i = 0; i <= M; ++i) acc[i] = 0.0;
-  double mx = 0.0;
-  for (int64_t j = blockIdx.x * (int64_t)NT + threadIdx.x; j < n; j += (int64_t)gridDim.x * NT) {
-    double x, xsi, eta;
-    if (TRIAL) {
-      x = V.x0[j] + D.steg * V.dx[j];
-      xsi = V.xsi0[j] + D.steg * V.dxsi[j];
-      eta = V.eta0[j] + D.steg * V.deta[j];
-      V.x[j] = x;
-      V.xsi[j] = xsi;
-      V.eta[j] = eta;
-    } else {
-      x = V.x[j];
-      xsi = V.xsi[j];
-      eta = V.eta[j];
-    }
-    double rux, rxl;
-    rcp2(V.upp[j] - x, x - V.low[j], rux, rxl);
-    double pl = V.p0[j], ql = V.q0[j];
-#pragma unroll
-    for (int i = 0; i < M; ++i) {
-      const double p = V.P[i * n + j], q = V.Q[i * n + j];
-      pl += p * D.lam[i];
-      ql += q * D.lam[i];
-      acc[i] += p * rux + q * rxl;
-    }
-    const double rex = pl * (rux * rux) - ql * (rxl * rxl) - xsi + eta;
-    const double rexsi = xsi * (x - V.alpha[j]) - D.epsi;
-    const double reeta = eta * (V.beta[j] - x) - D.epsi;
-    acc[M] += rex * rex + rexsi * rexsi + reeta * reeta;
-    mx = fmax(mx, fmax(fabs(rex), fmax(fabs(rexsi), fabs(reeta))));
-  }
-  reduce_out<M + 1>(acc, mx, R.part, R.ticket, R.out);
-}
-
-// Newton assembly (mma_cpu.f90:307-405): delx, diagx per j (delx/diagx and
-// 1/diagx kept), and the sums g_i(x), b_i = sum_j GG_ij delx_j/diagx_j,
-// A_ik = sum_j GG_ij GG_kj / diagx_j (upper triangle).  FP64 division is
-// costly on this GPU's narrow FP64 pipe, so each kernel forms the few
-// reciprocals it needs (1/(u-x), 1/(x-l), 1/(x-alpha), 1/(beta-x),
-// 1/diagx) once and multiplies: the reference's quotients to within an ulp.
-template <int M>
-__global__ void __launch_bounds__(NT) k_newton(Vecs V, Dual D, int64_t n, Red R) {
-  constexpr int NS = 2 * M + M * (M + 1) / 2;
+__global__ void __launch_bounds__(NT, M == 1 ? 3 : M == 2 ? 2 : 1) k_point(Vecs V, Dual D, int64_t n, Red R) {
+  constexpr int NS = 2 * M + M * (M + 1) / 2 + 1;
   double acc[NS];
 #pragma unroll
   for (int q = 0; q < NS; ++q) acc[q] = 0.0;
+  double mx = 0.0;
   for (int64_t j = blockIdx.x * (int64_t)NT + threadIdx.x; j < n; j += (int64_t)gridDim.x * NT) {
-    const double x = V.x[j], al = V.alpha[j], be = V.beta[j];
-    double rux, rxl, ral, rbe;
-    rcp4(V.upp[j] - x, x - V.low[j], x - al, be - x, rux, rxl, ral, rbe);
+    double x = V.x[j], xsi = V.xsi[j], eta = V.eta[j];
+    if (TRIAL) {
+      x = fma(D.steg, V.dx[j], x);
+      xsi = fma(D.steg, V.dxsi[j], xsi);
+      eta = fma(D.steg, V.deta[j], eta);
+      V.xt[j] = x;
+      V.xsit[j] = xsi;
+      V.etat[j] = eta;
+    }
+    const double xa = x - V.alpha[j], bx = V.beta[j] - x;
+    const double rux = rcp(V.upp[j] - x), rxl = rcp(x - V.low[j]), ral = rcp(xa), rbe = rcp(bx);
     const double rux2 = rux * rux, rxl2 = rxl * rxl;
     double pl = V.p0[j], ql = V.q0[j], gg[M];
 #pragma unroll
     for (int i = 0; i < M; ++i) {
       const double p = V.P[i * n + j], q = V.Q[i * n + j];
-      pl += p * D.lam[i];
-      ql += q * D.lam[i];
-      acc[i] += p * rux + q * rxl;
+      pl = fma(p, D.lam[i], pl);
+      ql = fma(q, D.lam[i], ql);
+      acc[i] = fma(p, rux, fma(q, rxl, acc[i]));
       gg[i] = p * rux2 - q * rxl2;
+      V.gg[i * n + j] = gg[i];
     }
-    const double delx = pl * rux2 - ql * rxl2 - D.epsi * ral + D.epsi * rbe;
-    double diagx = pl * (rux2 * rux) + ql * (rxl2 * rxl);
-    diagx = 2.0 * diagx + V.xsi[j] * ral + V.eta[j] * rbe;
-    const double rdg = 1.0 / diagx, t = delx * rdg;
-    V.tdx[j] = t;
-    V.diagx[j] = rdg;  // kept as its reciprocal
+    const double a = pl * rux2, b = ql * rxl2, ab = a - b;
+    const double rex = ab - xsi + eta, rexsi = fma(xsi, xa, -D.epsi), reeta = fma(eta, bx, -D.epsi);
+    acc[NS - 1] = fma(rex, rex, fma(rexsi, rexsi, fma(reeta, reeta, acc[NS - 1])));
+    mx = max_abs(max_abs(max_abs(mx, rex), rexsi), reeta);
+    const double delx = fma(D.epsi, rbe - ral, ab);
+    const double rdg = rcp(fma(2.0, fma(a, rux, b * rxl), fma(xsi, ral, eta * rbe)));
+    V.ral[j] = ral;
+    V.rbe[j] = rbe;
+    V.rdg[j] = rdg;
+    V.delx[j] = delx;
     int q = 2 * M;
 #pragma unroll
     for (int i = 0; i < M; ++i) {
-      acc[M + i] += gg[i] * t;
+      const double w = gg[i] * rdg;
+      acc[M + i] = fma(w, delx, acc[M + i]);
 #pragma unroll
-      for (int k = i; k < M; ++k) acc[q++] += gg[i] * rdg * gg[k];
+      for (int k = i; k < M; ++k) {
+        acc[q] = fma(w, gg[k], acc[q]);
+        ++q;
+      }
     }
   }
-  reduce_out<NS>(acc, -INFINITY, R.part, R.ticket, R.out);
+  reduce_out<NS>(acc, mx, R.part, R.ticket, R.out);
 }
 
-// Directions (mma_cpu.f90:418-433) and the largest step ratio (:436-439);
-// the line-search origin is saved.
+// Directions (mma_cpu.f90:418-433) and the largest step ratio (:436-439, its
+// factor 1.01 applied by the host).  16 FP64 operations per variable at m = 1
+// (60 with the reciprocals formed again by divisions).
 template <int M>
 __global__ void __launch_bounds__(NT) k_dir(Vecs V, Dual D, int64_t n, Red R) {
   double none[1] = {0.0};
-  double mx = -INFINITY;
+  double mx = 0.0;
   for (int64_t j = blockIdx.x * (int64_t)NT + threadIdx.x; j < n; j += (int64_t)gridDim.x * NT) {
-    const double x = V.x[j], al = V.alpha[j], be = V.beta[j], xsi = V.xsi[j], eta = V.eta[j];
-    double rux, rxl, ral, rbe, rxs, ret;
-    rcp4(V.upp[j] - x, x - V.low[j], x - al, be - x, rux, rxl, ral, rbe);
-    rcp2(xsi, eta, rxs, ret);
-    const double rux2 = rux * rux, rxl2 = rxl * rxl, rdg = V.diagx[j];
-    double gl = 0.0;
+    const double xsi = V.xsi[j], eta = V.eta[j], ral = V.ral[j], rbe = V.rbe[j];
+    double g = V.delx[j];
 #pragma unroll
-    for (int i = 0; i < M; ++i) gl += (V.P[i * n + j] * rux2 - V.Q[i * n + j] * rxl2) * D.dlam[i];
-    const double dx = -V.tdx[j] - gl * rdg;
-    const double dxsi = -xsi + (D.epsi - dx * xsi) * ral;
-    const double deta = -eta + (D.epsi + dx * eta) * rbe;
+    for (int i = 0; i < M; ++i) g = fma(V.gg[i * n + j], D.dlam[i], g);
+    const double dx = -g * V.rdg[j];
+    const double dxsi = fma(fma(-dx, xsi, D.epsi), ral, -xsi), deta = fma(fma(dx, eta, D.epsi), rbe, -eta);
     V.dx[j] = dx;
     V.dxsi[j] = dxsi;
     V.deta[j] = deta;
-    V.x0[j] = x;
-    V.xsi0[j] = xsi;
-    V.eta0[j] = eta;
-    mx = fmax(mx, fmax(fmax(-C101 * dxsi * rxs, -C101 * deta * ret), fmax(-C101 * dx * ral, C101 * dx * rbe)));
+    mx = max_pos(max_pos(mx, -dx * ral), dx * rbe);
+    mx = max_pos(max_pos(mx, -dxsi * rcp(xsi)), -deta * rcp(eta));
   }
   reduce_out<1>(none, mx, R.part, R.ticket, R.out);
 }
@@ -421,13 +401,13 @@ mm::Dual dual(const ntg_mma* o, double epsi) {
   return D;
 }
 
-// residual of the full perturbed KKT system from the device partial sums
-// (out: m sums g_i, the x-part sum of squares, the x-part max)
+// residual of the full perturbed KKT system from the sums of k_point (g_i
+// first, then b_i and A_ik, the x-part sum of squares and max last)
 void combine(const ntg_mma* o, const double* out, const std::vector<double>& y, double z,
              const std::vector<double>& lam, const std::vector<double>& s, const std::vector<double>& mu, double zeta,
              double epsi, double& norm, double& mx) {
-  const int m = o->m;
-  double sq = out[m], big = out[m + 1];
+  const int m = o->m, ns = 2 * m + m * (m + 1) / 2 + 1;
+  double sq = out[ns - 1], big = out[ns];
   double rez = o->a0 - zeta, rezeta = zeta * z - epsi;
   for (int i = 0; i < m; ++i) rez -= lam[i] * o->a[i];
   sq += rez * rez + rezeta * rezeta;
@@ -457,20 +437,16 @@ int subsolve(ntg_mma* o, double* designx) {
   while (epsi > mm::C09 * o->epsimin) {
     ++o->levels;
     o->lam = lam;
-    mm::k_resid<M, false><<<g, mm::NT, 0, st>>>(o->V, dual(o, epsi), n, red(o));
+    constexpr int NS = 2 * M + M * (M + 1) / 2 + 1;
+    mm::k_point<M, false><<<g, mm::NT, 0, st>>>(o->V, dual(o, epsi), n, red(o));
     NTG_COUNT_LAUNCH();
-    NTG_TRY(fetch(o, m + 2));
+    NTG_TRY(fetch(o, NS + 1));
     double residunorm, residumax;
     combine(o, o->out_h, y, z, lam, s, mu, zeta, epsi, residunorm, residumax);
     for (int it = 0; it < o->max_iter; ++it) {
       if (residumax < epsi) break;
       ++o->newton_steps;
-      o->lam = lam;
-      mm::k_newton<M><<<g, mm::NT, 0, st>>>(o->V, dual(o, epsi), n, red(o));
-      NTG_COUNT_LAUNCH();
-      constexpr int NS = 2 * M + M * (M + 1) / 2;
-      NTG_TRY(fetch(o, NS));
-      const double* out = o->out_h;
+      const double* out = o->out_h;  // of the pass over the current point
       std::vector<double> dely(m), dellam(m), bb(m + 1), AA((m + 1) * (m + 1));
       double delz = o->a0 - epsi / z;
       for (int i = 0; i < m; ++i) delz -= lam[i] * o->a[i];
@@ -510,7 +486,7 @@ int subsolve(ntg_mma* o, double* designx) {
       mm::k_dir<M><<<g, mm::NT, 0, st>>>(o->V, D, n, red(o));
       NTG_COUNT_LAUNCH();
       NTG_TRY(fetch(o, 2));
-      double steg = std::max(1.0, o->out_h[1]);
+      double steg = std::max(1.0, mm::C101 * o->out_h[1]);
       auto ratio = [&](double dv, double v) { steg = std::max(steg, -mm::C101 * dv / v); };
       for (int i = 0; i < m; ++i) {
         ratio(dy[i], y[i]);
@@ -539,13 +515,16 @@ int subsolve(ntg_mma* o, double* designx) {
         o->lam = lam;
         mm::Dual Dt = dual(o, epsi);
         Dt.steg = steg;
-        mm::k_resid<M, true><<<g, mm::NT, 0, st>>>(o->V, Dt, n, red(o));
+        mm::k_point<M, true><<<g, mm::NT, 0, st>>>(o->V, Dt, n, red(o));
         NTG_COUNT_LAUNCH();
-        NTG_TRY(fetch(o, m + 2));
+        NTG_TRY(fetch(o, NS + 1));
         combine(o, o->out_h, y, z, lam, s, mu, zeta, epsi, newres, residumax);
         steg = steg / 2.0;
       }
       residunorm = newres;
+      std::swap(o->V.x, o->V.xt);
+      std::swap(o->V.xsi, o->V.xsit);
+      std::swap(o->V.eta, o->V.etat);
     }
     epsi = 0.1 * epsi;
   }
@@ -566,8 +545,8 @@ int subsolve(ntg_mma* o, double* designx) {
 void mma_free(ntg_mma* o) {
   double** all[] = {&o->V.low, &o->V.upp, &o->V.alpha, &o->V.beta, &o->V.p0, &o->V.q0, &o->V.P, &o->V.Q,
                     &o->V.xmin, &o->V.xmax, &o->V.xold1, &o->V.xold2, &o->V.x, &o->V.xsi, &o->V.eta, &o->V.dx,
-                    &o->V.dxsi, &o->V.deta, &o->V.x0, &o->V.xsi0, &o->V.eta0, &o->V.tdx, &o->V.diagx,
-                    &o->part, &o->out_d};
+                    &o->V.dxsi, &o->V.deta, &o->V.xt, &o->V.xsit, &o->V.etat, &o->V.ral, &o->V.rbe, &o->V.rdg,
+                    &o->V.delx, &o->V.gg, &o->part, &o->out_d};
   for (double** p : all) dev_free(*p);
   dev_free(o->ticket);
   if (o->out_h) cudaFreeHost(o->out_h);
@@ -610,11 +589,12 @@ int ntg_mma_create(ntg_mma** out, int64_t n, int m, const double* x_d, double a0
   int st = NTG_OK;
   double** vecs[] = {&o->V.low, &o->V.upp, &o->V.alpha, &o->V.beta, &o->V.p0, &o->V.q0, &o->V.xmin, &o->V.xmax,
                      &o->V.xold1, &o->V.xold2, &o->V.x, &o->V.xsi, &o->V.eta, &o->V.dx, &o->V.dxsi, &o->V.deta,
-                     &o->V.x0, &o->V.xsi0, &o->V.eta0, &o->V.tdx, &o->V.diagx};
+                     &o->V.xt, &o->V.xsit, &o->V.etat, &o->V.ral, &o->V.rbe, &o->V.rdg, &o->V.delx};
   for (double** p : vecs)
     if (!st) st = dev_alloc(p, (size_t)n);
   if (!st) st = dev_alloc(&o->V.P, (size_t)(m * n));
   if (!st) st = dev_alloc(&o->V.Q, (size_t)(m * n));
+  if (!st) st = dev_alloc(&o->V.gg, (size_t)(m * n));
   if (!st) st = dev_alloc(&o->part, (size_t)mm::LANES * kRedSlots);
   if (!st) st = dev_alloc(&o->out_d, (size_t)mm::LANES);
   if (!st) st = dev_alloc(&o->ticket, 1);
@@ -641,8 +621,8 @@ int ntg_mma_create(ntg_mma** out, int64_t n, int m, const double* x_d, double a0
     st = fetch(o, 2);
     const double xmax = o->out_h[1];
     if (!st) {
-      mm::k_neg<<<o->grid, mm::NT, 0, o->stream>>>(o->V.x0, x_d, n);
-      mm::k_max<<<o->grid, mm::NT, 0, o->stream>>>(o->V.x0, n, red(o));
+      mm::k_neg<<<o->grid, mm::NT, 0, o->stream>>>(o->V.xt, x_d, n);
+      mm::k_max<<<o->grid, mm::NT, 0, o->stream>>>(o->V.xt, n, red(o));
       NTG_COUNT_LAUNCH();
       NTG_COUNT_LAUNCH();
       st = fetch(o, 2);
