@@ -26,8 +26,10 @@
 // its Schwarz part on the GLL grid and its coarse-grid part.
 //
 // Kernels per application: k_fdm (gather, six 1D transforms, coarse
-// restriction), k_crs_restrict + six k_crs_mode directions (coarse solve), k_pull
-// (prolongation of both levels, optional (r, z)), then the Dirichlet mask.
+// restriction), k_crs_fwd, k_crs_z and k_crs_back (coarse solve; on vertex
+// grids too large for them k_crs_restrict and six k_crs_mode directions),
+// k_pull (prolongation of both levels, optional (r, z)), then the Dirichlet
+// mask.
 //
 // Determinism: the prolongation is a pull -- every local node sums, in a fixed
 // order, the extended results of the elements whose extended box covers it --
@@ -41,6 +43,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fx.cuh"
 #include "reduce.cuh"
 #include "schwarz.cuh"
 
@@ -100,21 +103,23 @@ __global__ void k_coef_means(const double* __restrict__ h1, double h1c, const do
 // memory; an element brings only its six scalars.
 //
 // A thread owns two 1D lines of an element's extended box, (u, v) and
-// (u, v + LE/2).  Each direction pass loads a line from the shared tile,
-// applies S^ (or its transpose) two outputs at a time with packed FP32 FMAs
-// (__ffma2_rn: rows f, f+1 of S^ against the duplicated line value) and
-// writes the line back in place, so a pass needs one buffer and one barrier.
+// (u, v + LE/2), in registers.  The gather delivers lines along t, so the
+// order is t, r, s forward, the scaling, s, r, t back: t forward runs before
+// the tile is first written, s forward, scaling and s back are one pass, and
+// t back goes from registers to HBM, so the tile is written and read four
+// times.  The load / store pipe bounds it (664 wavefronts per element, of
+// them 469 shared): 101 us at 32^3 elements, lx = 8, where six passes with
+// the operator in shared memory (848 shared wavefronts) took 160.
 //   per element: scalars (sx, sy, sz, c, h1, h2) = (4/hx^2, 4/hy^2, 4/hz^2,
 //                8/(hx hy hz), h1, h2); tile A[a + RS b + PS c]
 // Tile strides: lines of a warp are consecutive (u fastest).  (RS, PS) make
-// the r and s passes (two each) free of bank conflicts and the tile stride
-// TPER keeps warps that span two elements free as well; the single t pass
-// takes two-way conflicts (no stride choice avoids all three passes).
-// the reference interval's extended 1D eigenvectors, as output pairs
+// the r and s passes free of bank conflicts and the tile stride TPER keeps
+// warps that span two elements free as well; the t columns take two-way
+// conflicts (no stride choice avoids all three).
+// the reference interval's extended 1D eigenvectors S[p][f] and eigenvalues
 template <int LE>
-struct FdmRef {
-  float P[LE / 2][LE][2];  // forward:  P[f/2][p][f&1] = S^[p][f]
-  float Q[LE / 2][LE][2];  // backward: Q[a/2][f][a&1] = S^[a][f]
+struct alignas(16) FdmRef {
+  float S[LE][LE];
   float lam[LE];
 };
 
@@ -125,15 +130,13 @@ struct FdmCfg {
   static constexpr int PS = LX == 8 ? 170 : LX == 6 ? 72 : 43;
   static constexpr int SPAN = (LE - 1) * (1 + RS + PS) + 1;
   static constexpr int TPER = LX == 8 ? 1714 : LX == 6 ? 576 : 257;
-  static constexpr int NSC = 8;  // per-element scalars (six used)
-  static constexpr int EPB = LX == 4 ? 16 : LX == 8 ? 4 : 8, THREADS = EPB * TPE, MINB = 4;
-  static constexpr int MINB_EO = LX == 8 ? 4 : 3;  // the even-odd form keeps the folded lines in registers
-  // (lx = 8: four elements per block measured 4% faster at 64^3 than eight, 1.14 vs 1.19 ms)
+  static constexpr int EPB = LX == 4 ? 16 : LX == 8 ? 4 : 8, THREADS = EPB * TPE;
+  static constexpr int MINB = 1024 / THREADS;
   // coarse restriction partials (8 per thread): in the tile rows' padding
   // (a in [LE, RS), two rows per thread) when it is wide enough, else after the tiles
   static constexpr bool HOLES = 2 * (RS - LE) >= 8;
   static constexpr int RED = HOLES ? 0 : EPB * TPE * 8;
-  static constexpr size_t SMEM = ((size_t)EPB * (NSC + TPER) + RED) * sizeof(float);
+  static constexpr size_t SMEM = ((size_t)EPB * TPER + RED) * sizeof(float);
   static_assert(LE % 2 == 0 && TPER >= SPAN && THREADS <= 1024, "layout");
 };
 
@@ -151,343 +154,260 @@ __device__ __forceinline__ float* crs_slot(float* A, float* red, int el, int tl,
   }
 }
 
-template <int LE>
-__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
-
-// out(line1, line2)[f * ST] = sum_p M[f][p] in2[p] for both lines of the
-// thread; M as interleaved output pairs in shared memory (row pair fp:
-// M[fp*2LE + 2p + k] = M[2fp + k][p]), read as float4 broadcasts
-template <int LE, int ST>
-__device__ __forceinline__ void fdm_pair(const float* __restrict__ M, const float2 (&in)[LE], float* d1, float* d2) {
-#pragma unroll
-  for (int fp = 0; fp < LE / 2; ++fp) {
-    const float* row = M + fp * 2 * LE;
-    float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int p = 0; p < LE; p += 2) {
-      const float4 m4 = *reinterpret_cast<const float4*>(row + 2 * p);
-      a0 = __ffma2_rn(dup<LE>(m4.x), in[p], a0);
-      a1 = __ffma2_rn(dup<LE>(m4.y), in[p], a1);
-      a0 = __ffma2_rn(dup<LE>(m4.z), in[p + 1], a0);
-      a1 = __ffma2_rn(dup<LE>(m4.w), in[p + 1], a1);
-    }
-    d1[(2 * fp) * ST] = a0.x;
-    d2[(2 * fp) * ST] = a0.y;
-    d1[(2 * fp + 1) * ST] = a1.x;
-    d2[(2 * fp + 1) * ST] = a1.y;
-  }
-}
-
-// the same into registers
-template <int LE>
-__device__ __forceinline__ void fdm_pair_reg(const float* __restrict__ M, const float2 (&in)[LE], float2 (&out)[LE]) {
-#pragma unroll
-  for (int fp = 0; fp < LE / 2; ++fp) {
-    const float* row = M + fp * 2 * LE;
-    float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int p = 0; p < LE; p += 2) {
-      const float4 m4 = *reinterpret_cast<const float4*>(row + 2 * p);
-      a0 = __ffma2_rn(dup<LE>(m4.x), in[p], a0);
-      a1 = __ffma2_rn(dup<LE>(m4.y), in[p], a1);
-      a0 = __ffma2_rn(dup<LE>(m4.z), in[p + 1], a0);
-      a1 = __ffma2_rn(dup<LE>(m4.w), in[p + 1], a1);
-    }
-    out[2 * fp] = a0;
-    out[2 * fp + 1] = a1;
-  }
-}
-
-// Even-odd forms of the same transforms.  The reference extended interval
-// is symmetric about its centre, so its eigenvectors alternate between
-// symmetric (f even) and antisymmetric (f odd): S[LE-1-p][f] = (-1)^f S[p][f]
-// (checked on the host before this path is chosen).  Then
+// y = S^T x (FWD) or S x of a line in registers, in place.  EO: the even-odd
+// form.  The reference extended interval is symmetric about its centre, so
+// its eigenvectors alternate between symmetric (f even) and antisymmetric (f
+// odd): S[LE-1-p][f] = (-1)^f S[p][f] (checked on the host before this form
+// is chosen).  Then
 //   forward  y_f = sum_{p<H} S[p][f] (x_p + (-1)^f x_{LE-1-p}),
 //   backward x_p = E_p + O_p, x_{LE-1-p} = E_p - O_p with
 //            E_p = sum_{f even} S[p][f] z_f, O_p = sum_{f odd} S[p][f] z_f,
-// half the FMAs of the full LE x LE products.  Both read the forward pair
-// table M = P (M[fp*2LE + 2p + k] = S[p][2fp + k]) at p < H only.
-template <int LE>
-__device__ __forceinline__ void eo_fold(float2 (&in)[LE]) {  // in[p] <- x_p + x_q, in[q] <- x_p - x_q (q = LE-1-p)
-#pragma unroll
-  for (int p = 0; p < LE / 2; ++p) {
-    const float2 a = in[p], b = in[LE - 1 - p];
-    in[p] = make_float2(a.x + b.x, a.y + b.y);
-    in[LE - 1 - p] = make_float2(a.x - b.x, a.y - b.y);
-  }
-}
-template <int LE, int ST>
-__device__ __forceinline__ void fdm_fwd_eo(const float* __restrict__ M, float2 (&in)[LE], float* d1, float* d2) {
+// half the FMAs of the full products, and both run on packed FMAs with the
+// even part in one half and the odd part in the other: the operand pairs
+// (S[p][2k], S[p][2k+1]) and (x_p + x_q, x_p - x_q) or (z_2k, z_2k+1) need
+// no duplication.  M: the pairs M[p * H + k] = (S[p][2k], S[p][2k+1]), in the
+// kernel parameters at compile-time indices: no shared memory is read for them.
+template <int LE, bool EO, bool FWD>
+__device__ __forceinline__ void fdm_line(const float2* M, float (&x)[LE]) {
   constexpr int H = LE / 2;
-  eo_fold<LE>(in);
+  if constexpr (!EO) {
+    float y[LE];
+    if constexpr (FWD) {
 #pragma unroll
-  for (int fp = 0; fp < H; ++fp) {
-    const float* row = M + fp * 2 * LE;
-    float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
+      for (int k = 0; k < H; ++k) {
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int p = 0; p < LE; ++p) acc = __ffma2_rn(M[p * H + k], make_float2(x[p], x[p]), acc);
+        y[2 * k] = acc.x;
+        y[2 * k + 1] = acc.y;
+      }
+    } else {
+#pragma unroll
+      for (int p = 0; p < LE; ++p) {
+        float2 acc = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < H; ++k) acc = __ffma2_rn(M[p * H + k], make_float2(x[2 * k], x[2 * k + 1]), acc);
+        y[p] = acc.x + acc.y;
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < LE; ++f) x[f] = y[f];
+  } else if constexpr (FWD) {
+    float2 d[H];
+#pragma unroll
+    for (int p = 0; p < H; ++p) d[p] = make_float2(x[p] + x[LE - 1 - p], x[p] - x[LE - 1 - p]);
+#pragma unroll
+    for (int k = 0; k < H; ++k) {
+      float2 acc = __fmul2_rn(M[k], d[0]);
+#pragma unroll
+      for (int p = 1; p < H; ++p) acc = __ffma2_rn(M[p * H + k], d[p], acc);
+      x[2 * k] = acc.x;
+      x[2 * k + 1] = acc.y;
+    }
+  } else {
+    float2 d[H];
+#pragma unroll
+    for (int k = 0; k < H; ++k) d[k] = make_float2(x[2 * k], x[2 * k + 1]);
 #pragma unroll
     for (int p = 0; p < H; ++p) {
-      const float2 m2 = *reinterpret_cast<const float2*>(row + 2 * p);
-      a0 = __ffma2_rn(dup<LE>(m2.x), in[p], a0);
-      a1 = __ffma2_rn(dup<LE>(m2.y), in[LE - 1 - p], a1);
+      float2 acc = __fmul2_rn(M[p * H], d[0]);
+#pragma unroll
+      for (int k = 1; k < H; ++k) acc = __ffma2_rn(M[p * H + k], d[k], acc);
+      x[p] = acc.x + acc.y;
+      x[LE - 1 - p] = acc.x - acc.y;
     }
-    d1[(2 * fp) * ST] = a0.x;
-    d2[(2 * fp) * ST] = a0.y;
-    d1[(2 * fp + 1) * ST] = a1.x;
-    d2[(2 * fp + 1) * ST] = a1.y;
   }
+}
+
+template <int LE>
+__device__ __forceinline__ void fdm_load(const float* l, int st, float (&x)[LE]) {
+#pragma unroll
+  for (int p = 0; p < LE; ++p) x[p] = l[p * st];
 }
 template <int LE>
-__device__ __forceinline__ void fdm_fwd_eo_reg(const float* __restrict__ M, float2 (&in)[LE], float2 (&out)[LE]) {
-  constexpr int H = LE / 2;
-  eo_fold<LE>(in);
+__device__ __forceinline__ void fdm_store(float* l, int st, const float (&x)[LE]) {
 #pragma unroll
-  for (int fp = 0; fp < H; ++fp) {
-    const float* row = M + fp * 2 * LE;
-    float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int p = 0; p < H; ++p) {
-      const float2 m2 = *reinterpret_cast<const float2*>(row + 2 * p);
-      a0 = __ffma2_rn(dup<LE>(m2.x), in[p], a0);
-      a1 = __ffma2_rn(dup<LE>(m2.y), in[LE - 1 - p], a1);
-    }
-    out[2 * fp] = a0;
-    out[2 * fp + 1] = a1;
-  }
-}
-template <int LE, int ST>
-__device__ __forceinline__ void fdm_bwd_eo(const float* __restrict__ M, const float2 (&in)[LE], float* d1, float* d2) {
-  constexpr int H = LE / 2;
-#pragma unroll
-  for (int p = 0; p < H; ++p) {
-    float2 e = make_float2(0.f, 0.f), o = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int fp = 0; fp < H; ++fp) {
-      const float2 m2 = *reinterpret_cast<const float2*>(M + fp * 2 * LE + 2 * p);
-      e = __ffma2_rn(dup<LE>(m2.x), in[2 * fp], e);
-      o = __ffma2_rn(dup<LE>(m2.y), in[2 * fp + 1], o);
-    }
-    d1[p * ST] = e.x + o.x;
-    d2[p * ST] = e.y + o.y;
-    d1[(LE - 1 - p) * ST] = e.x - o.x;
-    d2[(LE - 1 - p) * ST] = e.y - o.y;
-  }
+  for (int p = 0; p < LE; ++p) l[p * st] = x[p];
 }
 
 // GEN: a general mesh (Ex = nelv, Ey = Ez = 1): the ghost layers come from
 // the face-neighbour table (edge and corner positions stay zero) and the
 // coarse restriction weighs nodes by minv = 1 / multiplicity.
 template <int LX, bool EO, bool GEN>
-__global__ void __launch_bounds__(FdmCfg<LX>::THREADS, EO ? FdmCfg<LX>::MINB_EO : FdmCfg<LX>::MINB)
+__global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
     k_fdm(const float* __restrict__ r, float* __restrict__ ze, const float* __restrict__ esc, int Ex, int Ey,
           int Ez, const Scalars* sc, float* __restrict__ corner, CoarsePhi ph,
           const int32_t* __restrict__ ghost, const float* __restrict__ minv,
           const __grid_constant__ FdmRef<LX + 2> R) {
   using C = FdmCfg<LX>;
   constexpr int LE = C::LE, LE2 = C::LE2, LE3 = C::LE3, N = LX - 1, RS = C::RS, PS = C::PS, TPE = C::TPE;
-  constexpr int EPB = C::EPB, NSC = C::NSC, LX2 = LX * LX, LX3 = LX2 * LX, H = LE / 2;
+  constexpr int EPB = C::EPB, LX2 = LX * LX, LX3 = LX2 * LX, H = LE / 2;
   if (sc && sc->done) return;
   extern __shared__ __align__(16) float smem[];
   const int nelv = Ex * Ey * Ez;
   const int tid = threadIdx.x, el = tid / TPE, tl = tid - el * TPE;
   const int u = tl % LE, v1 = tl / LE, v2 = v1 + H;  // lines (u, v1) and (u, v2); tl + TPE = u + LE v2
-  float* es = smem + el * NSC;
-  float* A = smem + EPB * NSC + el * C::TPER;
-  float* red = smem + EPB * (NSC + C::TPER);
+  float* A = smem + el * C::TPER;
+  float* red = smem + EPB * C::TPER;
   __shared__ float sp[2][LX];  // Q1 basis at the GLL nodes
-  __shared__ __align__(16) float sP[LE2], sQ[LE2];  // reference pairs (forward, backward)
-  __shared__ float slam[LE];                        // reference eigenvalues
+  __shared__ float slam[LE];   // reference eigenvalues
   if (tid == 0) {
 #pragma unroll
     for (int t = 0; t < 2 * LX; ++t) sp[t / LX][t % LX] = ph.p[t / LX][t % LX];  // constant indices
+#pragma unroll
+    for (int t = 0; t < LE; ++t) slam[t] = R.lam[t];
   }
-  for (int t = tid; t < LE2; t += blockDim.x) {
-    sP[t] = (&R.P[0][0][0])[t];
-    sQ[t] = (&R.Q[0][0][0])[t];
-  }
-  if (tid < LE) slam[tid] = R.lam[tid];
-  __syncthreads();
-  float2 in[LE];
-  for (int e0 = blockIdx.x * EPB; e0 < nelv; e0 += gridDim.x * EPB) {
-    const int e = e0 + el;
-    const bool live = e < nelv;
-    if (tl < NSC) es[tl] = live ? esc[(int64_t)e * NSC + tl] : 1.f;
-    // gather R_e r: columns (a, b) = (u, v1), (u, v2) over c
-    if (GEN && live) {
-      const int64_t eb = (int64_t)e * LX3;
-      const int32_t* gh = ghost + eb / LX * 6;  // (e * 6) * LX2
-      const bool ia = u >= 1 && u <= LX;
-      float part[8];
+  const int e = blockIdx.x * EPB + el;
+  const bool live = e < nelv;
+  float x[2][LE];
+  // gather R_e r: columns (a, b) = (u, v1), (u, v2) over c, into registers
 #pragma unroll
-      for (int v = 0; v < 8; ++v) part[v] = 0.f;
+  for (int q = 0; q < 2; ++q)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int vb = q ? v2 : v1;
-        const bool ib = vb >= 1 && vb <= LX;
-        float* Ac = A + u + RS * vb;
-        if (ia && ib) {
-          // own column with the t-face ghosts at its ends
-          const int i = u - 1, j = vb - 1;
-          const int32_t g0 = gh[4 * LX2 + i + LX * j], g1 = gh[5 * LX2 + i + LX * j];
-          Ac[0] = g0 >= 0 ? r[g0] : 0.f;
-          Ac[PS * (LE - 1)] = g1 >= 0 ? r[g1] : 0.f;
-          const float* rc = r + eb + i + LX * j;
-          const float* mc = minv + eb + i + LX * j;
-          float s0 = 0.f, s1 = 0.f;
+    for (int c = 0; c < LE; ++c) x[q][c] = 0.f;
+  float part[2][2];  // own-element columns: sum_k phi_vz(k) r / multiplicity
+  part[0][0] = part[0][1] = part[1][0] = part[1][1] = 0.f;
+  if (GEN && live) {
+    const int64_t eb = (int64_t)e * LX3;
+    const int32_t* gh = ghost + eb / LX * 6;  // (e * 6) * LX2
+    const bool ia = u >= 1 && u <= LX;
 #pragma unroll
-          for (int c = 1; c < LE - 1; ++c) {
-            const float val = rc[(c - 1) * LX2];
-            Ac[PS * c] = val;
-            if (corner) {
-              const float wv = val * mc[(c - 1) * LX2];
-              s0 = fmaf(sp[0][c - 1], wv, s0);
-              s1 = fmaf(sp[1][c - 1], wv, s1);
-            }
-          }
-          if (corner) {
+    for (int q = 0; q < 2; ++q) {
+      const int vb = q ? v2 : v1;
+      const bool ib = vb >= 1 && vb <= LX;
+      if (ia && ib) {
+        // own column with the t-face ghosts at its ends
+        const int i = u - 1, j = vb - 1;
+        const int32_t g0 = gh[4 * LX2 + i + LX * j], g1 = gh[5 * LX2 + i + LX * j];
+        x[q][0] = g0 >= 0 ? r[g0] : 0.f;
+        x[q][LE - 1] = g1 >= 0 ? r[g1] : 0.f;
+        const float* rc = r + eb + i + LX * j;
 #pragma unroll
-            for (int v = 0; v < 8; ++v) part[v] = fmaf(sp[v & 1][i] * sp[(v >> 1) & 1][j], (v >> 2) ? s1 : s0, part[v]);
-          }
-        } else if (ia || ib) {
-          // an r-face (a at the border) or s-face (b at the border) ghost column
-          const int32_t* gf = ia ? gh + (vb == 0 ? 2 : 3) * LX2 + (u - 1) : gh + (u == 0 ? 0 : 1) * LX2 + (vb - 1);
-          Ac[0] = 0.f;
-          Ac[PS * (LE - 1)] = 0.f;
-#pragma unroll
-          for (int c = 1; c < LE - 1; ++c) {
-            const int32_t gi = gf[LX * (c - 1)];
-            Ac[PS * c] = gi >= 0 ? r[gi] : 0.f;
-          }
-        } else {
-#pragma unroll
-          for (int c = 0; c < LE; ++c) Ac[PS * c] = 0.f;
-        }
-      }
-      if (corner) {
-#pragma unroll
-        for (int v = 0; v < 8; ++v) *crs_slot<LX>(A, red, el, tl, v) = part[v];
-      }
-    }
-    if (!GEN && live) {
-      const int exy = e / Ex, ex = e - exy * Ex, ez = exy / Ey, ey = exy - ez * Ey;
-      int i = u - 1, dx = 0;
-      if (i < 0) { dx = -1; i = N - 1; } else if (i > N) { dx = 1; i = 1; }
-      const int nx = ex + dx;
-      const int64_t zs = (int64_t)Ex * Ey * LX3;
-      float part[8];
-#pragma unroll
-      for (int v = 0; v < 8; ++v) part[v] = 0.f;
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        const int vb = q ? v2 : v1;
-        int j = vb - 1, dy = 0;
-        if (j < 0) { dy = -1; j = N - 1; } else if (j > N) { dy = 1; j = 1; }
-        const int ny = ey + dy;
-        const bool okxy = nx >= 0 && nx < Ex && ny >= 0 && ny < Ey;
-        const float* rc = r + (int64_t)(nx + Ex * (ny + Ey * ez)) * LX3 + i + LX * j;
-        float* Ac = A + u + RS * vb;
-        Ac[0] = okxy && ez > 0 ? rc[(N - 1) * LX2 - zs] : 0.f;
-        // own-element columns also feed the coarse restriction:
-        // sum_k phi_vz(k) r / multiplicity, per column, then x / y weights
-        float s0 = 0.f, s1 = 0.f;
+        for (int c = 1; c < LE - 1; ++c) x[q][c] = rc[(c - 1) * LX2];
+      } else if (ia || ib) {
+        // an r-face (a at the border) or s-face (b at the border) ghost column
+        const int32_t* gf = ia ? gh + (vb == 0 ? 2 : 3) * LX2 + (u - 1) : gh + (u == 0 ? 0 : 1) * LX2 + (vb - 1);
 #pragma unroll
         for (int c = 1; c < LE - 1; ++c) {
-          const float val = okxy ? rc[(c - 1) * LX2] : 0.f;
-          Ac[PS * c] = val;
-          const int k = c - 1;
-          const float wz = ((k == 0 && ez > 0) || (k == N && ez < Ez - 1)) ? 0.5f : 1.f;
-          s0 = fmaf(sp[0][k] * wz, val, s0);
-          s1 = fmaf(sp[1][k] * wz, val, s1);
-        }
-        Ac[PS * (LE - 1)] = okxy && ez < Ez - 1 ? rc[LX2 + zs] : 0.f;
-        if (corner && dx == 0 && dy == 0) {
-          const float wx = ((i == 0 && ex > 0) || (i == N && ex < Ex - 1)) ? 0.5f : 1.f;
-          const float wy = ((j == 0 && ey > 0) || (j == N && ey < Ey - 1)) ? 0.5f : 1.f;
-#pragma unroll
-          for (int v = 0; v < 8; ++v)
-            part[v] = fmaf(sp[v & 1][i] * wx * (sp[(v >> 1) & 1][j] * wy), (v >> 2) ? s1 : s0, part[v]);
+          const int32_t gi = gf[LX * (c - 1)];
+          x[q][c] = gi >= 0 ? r[gi] : 0.f;
         }
       }
-      if (corner) {
+    }
+  }
+  int ex = 0, ey = 0, ez = 0;
+  if (!GEN && live) {
+    const int exy = e / Ex;
+    ex = e - exy * Ex;
+    ez = exy / Ey;
+    ey = exy - ez * Ey;
+    int i = u - 1, dx = 0;
+    if (i < 0) { dx = -1; i = N - 1; } else if (i > N) { dx = 1; i = 1; }
+    const int nx = ex + dx;
+    const int64_t zs = (int64_t)Ex * Ey * LX3;
 #pragma unroll
-        for (int v = 0; v < 8; ++v) *crs_slot<LX>(A, red, el, tl, v) = part[v];
+    for (int q = 0; q < 2; ++q) {
+      const int vb = q ? v2 : v1;
+      int j = vb - 1, dy = 0;
+      if (j < 0) { dy = -1; j = N - 1; } else if (j > N) { dy = 1; j = 1; }
+      const int ny = ey + dy;
+      if (nx >= 0 && nx < Ex && ny >= 0 && ny < Ey) {
+        const float* rc = r + (int64_t)(nx + Ex * (ny + Ey * ez)) * LX3 + i + LX * j;
+        if (ez > 0) x[q][0] = rc[(N - 1) * LX2 - zs];
+#pragma unroll
+        for (int c = 1; c < LE - 1; ++c) x[q][c] = rc[(c - 1) * LX2];
+        if (ez < Ez - 1) x[q][LE - 1] = rc[LX2 + zs];
       }
     }
-    __syncthreads();
-    // r forward: lines (b, c) = (u, v) along a
-    {
-      float* l1 = A + RS * u + PS * v1;
-      float* l2 = A + RS * u + PS * v2;
+  }
+  float es[6] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+  if (live) {
+    const float4 s4 = *reinterpret_cast<const float4*>(esc + (int64_t)e * 8);
+    const float2 s2 = *reinterpret_cast<const float2*>(esc + (int64_t)e * 8 + 4);
+    es[0] = s4.x; es[1] = s4.y; es[2] = s4.z; es[3] = s4.w; es[4] = s2.x; es[5] = s2.y;
+  }
+  __syncthreads();  // sp, slam
+  if (corner) {
+    // coarse restriction: own-element columns, z weights first, then x / y
+    float pt[8];
 #pragma unroll
-      for (int p = 0; p < LE; ++p) in[p] = make_float2(l1[p], l2[p]);
-      if constexpr (EO) fdm_fwd_eo<LE, 1>(sP, in, l1, l2);
-      else fdm_pair<LE, 1>(sP, in, l1, l2);
-    }
-    __syncthreads();
-    // s forward: lines (a, c) = (u, v) along b
-    {
-      float* l1 = A + u + PS * v1;
-      float* l2 = A + u + PS * v2;
+    for (int v = 0; v < 8; ++v) pt[v] = 0.f;
 #pragma unroll
-      for (int p = 0; p < LE; ++p) in[p] = make_float2(l1[RS * p], l2[RS * p]);
-      if constexpr (EO) fdm_fwd_eo<LE, RS>(sP, in, l1, l2);
-      else fdm_pair<LE, RS>(sP, in, l1, l2);
-    }
-    __syncthreads();
-    // t forward, scale (c_e / D_e), t back: lines (a, b) = (u, v) along c
-    {
-      float* l1 = A + u + RS * v1;
-      float* l2 = A + u + RS * v2;
-      const float sx = es[0], sy = es[1], sz = es[2], ce = es[3], h1 = es[4], h2 = es[5];
-      const float la1 = h1 * (sx * slam[u] + sy * slam[v1]) + h2, la2 = h1 * (sx * slam[u] + sy * slam[v2]) + h2;
+    for (int q = 0; q < 2; ++q) {
+      const int vb = q ? v2 : v1;
+      if (!(live && u >= 1 && u <= LX && vb >= 1 && vb <= LX)) continue;
+      const int i = u - 1, j = vb - 1;
+      float s0 = 0.f, s1 = 0.f, wxy = 1.f;
 #pragma unroll
-      for (int p = 0; p < LE; ++p) in[p] = make_float2(l1[PS * p], l2[PS * p]);
-      float2 t[LE];
-      if constexpr (EO) fdm_fwd_eo_reg<LE>(sP, in, t);
-      else fdm_pair_reg<LE>(sP, in, t);
-#pragma unroll
-      for (int f = 0; f < LE; ++f) {
-        const float lf = h1 * sz * slam[f];
-        in[f] = make_float2(__fdividef(ce * t[f].x, la1 + lf), __fdividef(ce * t[f].y, la2 + lf));
+      for (int k = 0; k < LX; ++k) {
+        float wv = x[q][k + 1];
+        if (GEN) wv *= minv[(int64_t)e * LX3 + i + LX * j + k * LX2];
+        else wv *= ((k == 0 && ez > 0) || (k == N && ez < Ez - 1)) ? 0.5f : 1.f;
+        s0 = fmaf(sp[0][k], wv, s0);
+        s1 = fmaf(sp[1][k], wv, s1);
       }
-      if constexpr (EO) fdm_bwd_eo<LE, PS>(sP, in, l1, l2);
-      else fdm_pair<LE, PS>(sQ, in, l1, l2);
-    }
-    __syncthreads();
-    // s back
-    {
-      float* l1 = A + u + PS * v1;
-      float* l2 = A + u + PS * v2;
-#pragma unroll
-      for (int p = 0; p < LE; ++p) in[p] = make_float2(l1[RS * p], l2[RS * p]);
-      if constexpr (EO) fdm_bwd_eo<LE, RS>(sP, in, l1, l2);
-      else fdm_pair<LE, RS>(sQ, in, l1, l2);
-    }
-    __syncthreads();
-    // r back
-    {
-      float* l1 = A + RS * u + PS * v1;
-      float* l2 = A + RS * u + PS * v2;
-#pragma unroll
-      for (int p = 0; p < LE; ++p) in[p] = make_float2(l1[p], l2[p]);
-      if constexpr (EO) fdm_bwd_eo<LE, 1>(sP, in, l1, l2);
-      else fdm_pair<LE, 1>(sQ, in, l1, l2);
-    }
-    __syncthreads();
-    // coarse restriction of the element: 8 threads sum the partials in order
-    if (corner && live && tl < 8) {
-      float acc = 0.f;
-      for (int t = 0; t < TPE; ++t) acc += *crs_slot<LX>(A, red, el, t, tl);
-      corner[(int64_t)e * 8 + tl] = acc;
-    }
-    // copy-out: columns (a, b) of ze[e][a + LE b + LE2 c] (consecutive lines -> consecutive addresses)
-    if (live) {
-#pragma unroll
-      for (int c = 0; c < LE; ++c) {
-        ze[(int64_t)e * LE3 + tl + LE2 * c] = A[u + RS * v1 + PS * c];
-        ze[(int64_t)e * LE3 + tl + TPE + LE2 * c] = A[u + RS * v2 + PS * c];
+      if (!GEN) {
+        if ((i == 0 && ex > 0) || (i == N && ex < Ex - 1)) wxy *= 0.5f;
+        if ((j == 0 && ey > 0) || (j == N && ey < Ey - 1)) wxy *= 0.5f;
       }
+#pragma unroll
+      for (int v = 0; v < 8; ++v) pt[v] = fmaf(sp[v & 1][i] * sp[(v >> 1) & 1][j] * wxy, (v >> 2) ? s1 : s0, pt[v]);
     }
-    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) *crs_slot<LX>(A, red, el, tl, v) = pt[v];
+  }
+  const float2* M = reinterpret_cast<const float2*>(&R.S[0][0]);
+  // t forward in registers: lines (a, b) = (u, v) along c
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    fdm_line<LE, EO, true>(M, x[q]);
+    fdm_store<LE>(A + u + RS * (q ? v2 : v1), PS, x[q]);
+  }
+  __syncthreads();
+  // r forward: lines (b, c) = (u, v) along a
+#pragma unroll
+  for (int q = 0; q < 2; ++q) fdm_load<LE>(A + RS * u + PS * (q ? v2 : v1), 1, x[q]);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    fdm_line<LE, EO, true>(M, x[q]);
+    fdm_store<LE>(A + RS * u + PS * (q ? v2 : v1), 1, x[q]);
+  }
+  __syncthreads();
+  // s forward, scale (c_e / D_e), s back: lines (a, c) = (u, v) along b
+#pragma unroll
+  for (int q = 0; q < 2; ++q) fdm_load<LE>(A + u + PS * (q ? v2 : v1), RS, x[q]);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const float la = es[4] * (es[0] * slam[u] + es[2] * slam[q ? v2 : v1]) + es[5], hs = es[4] * es[1];
+    fdm_line<LE, EO, true>(M, x[q]);
+#pragma unroll
+    for (int f = 0; f < LE; ++f) x[q][f] = __fdividef(es[3] * x[q][f], fmaf(hs, R.lam[f], la));
+    fdm_line<LE, EO, false>(M, x[q]);
+    fdm_store<LE>(A + u + PS * (q ? v2 : v1), RS, x[q]);
+  }
+  __syncthreads();
+  // r back
+#pragma unroll
+  for (int q = 0; q < 2; ++q) fdm_load<LE>(A + RS * u + PS * (q ? v2 : v1), 1, x[q]);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    fdm_line<LE, EO, false>(M, x[q]);
+    fdm_store<LE>(A + RS * u + PS * (q ? v2 : v1), 1, x[q]);
+  }
+  __syncthreads();
+  // coarse restriction of the element: 8 threads sum the partials in order
+  if (corner && live && tl < 8) {
+    float acc = 0.f;
+    for (int t = 0; t < TPE; ++t) acc += *crs_slot<LX>(A, red, el, t, tl);
+    corner[(int64_t)e * 8 + tl] = acc;
+  }
+  // t back and out: columns (a, b) of ze[e][a + LE b + LE2 c] (consecutive lines -> consecutive addresses)
+#pragma unroll
+  for (int q = 0; q < 2; ++q) fdm_load<LE>(A + u + RS * (q ? v2 : v1), PS, x[q]);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    fdm_line<LE, EO, false>(M, x[q]);
+    if (live) fdm_store<LE>(ze + (int64_t)e * LE3 + tl + q * TPE, LE2, x[q]);
   }
 }
 
@@ -589,6 +509,175 @@ __global__ void __launch_bounds__(256)
     } else {
       out[q] = acc;
     }
+  }
+}
+
+// The same solve in three kernels, a plane or a batch of columns of the vertex
+// grid in shared memory per block, for grids whose planes fit (up to about
+// 100 vertices a side): restriction with x and y forward per z plane; z
+// forward, scaling and z back per batch of columns; y and x back per z plane.
+// What bounds it is latency (the whole grid is a few MB at most): seven
+// dependent launches of L2 reads take 45 us at 33^3 vertices.
+// Rows are padded to multiples of four with zeros; a work item is four lines
+// times one output, so a matrix row read serves four FMAs.
+struct CrsPad {
+  int p0, p1, p2;  // padded row lengths
+  __host__ __device__ explicit CrsPad(const CoarseDims& d)
+      : p0((d.m[0] + 3) & ~3), p1((d.m[1] + 3) & ~3), p2((d.m[2] + 3) & ~3) {}
+  // two planes of p1 rows, the x and y matrices
+  size_t plane() const { return sizeof(float) * ((size_t)2 * p1 * p0 + (size_t)p0 * p0 + (size_t)p1 * p1); }
+  size_t column() const;
+};
+constexpr int kCrsCols = 16;    // columns per block of the z kernel
+constexpr int kCrsThreads = 512;
+inline size_t CrsPad::column() const { return sizeof(float) * ((size_t)2 * p2 * p2 + (size_t)2 * p2 * kCrsCols); }
+constexpr size_t kCrsSmem = 200 * 1024;
+
+// an m x m row-major matrix into rows of p (p x p, zero padded)
+__device__ __forceinline__ void crs_stage(float* dst, const float* __restrict__ src, int m, int p) {
+  for (int t = threadIdx.x; t < p * p; t += kCrsThreads) {
+    const int r = t / p, c = t - r * p;
+    dst[t] = r < m && c < m ? src[r * m + c] : 0.f;
+  }
+}
+
+// out[r][f] = sum_x M[x][f] in[r][x] for r < rows; rows of p floats
+__device__ __forceinline__ void crs_rows(const float* in, const float* M, int rows, int m, int p, float* out) {
+  for (int t = threadIdx.x; t < ((rows + 3) >> 2) * m; t += kCrsThreads) {
+    const int g = t / m, f = t - g * m;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* a = in + 4 * g * p;
+    for (int x = 0; x < p; x += 4) {
+      const float m0 = M[x * p + f], m1 = M[(x + 1) * p + f], m2 = M[(x + 2) * p + f], m3 = M[(x + 3) * p + f];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float4 v = *reinterpret_cast<const float4*>(a + k * p + x);
+        acc[k] = fmaf(v.x, m0, fmaf(v.y, m1, fmaf(v.z, m2, fmaf(v.w, m3, acc[k]))));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) out[(4 * g + k) * p + f] = acc[k];
+  }
+}
+
+// fn(g, c, sum_y M[y][g] in[y * w + c]) for g < m, c < cols; M rows of p
+template <typename F>
+__device__ __forceinline__ void crs_cols(const float* in, const float* M, int m, int p, int cols, int w, F&& fn) {
+  for (int t = threadIdx.x; t < ((m + 3) >> 2) * cols; t += kCrsThreads) {
+    const int g = t / cols, c = t - g * cols;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    const float* a = in + c;
+#pragma unroll 4
+    for (int y = 0; y < m; ++y) {
+      const float v = a[y * w];
+      const float4 q = *reinterpret_cast<const float4*>(M + y * p + 4 * g);
+      acc[0] = fmaf(q.x, v, acc[0]);
+      acc[1] = fmaf(q.y, v, acc[1]);
+      acc[2] = fmaf(q.z, v, acc[2]);
+      acc[3] = fmaf(q.w, v, acc[3]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (4 * g + k < m) fn(4 * g + k, c, acc[k]);
+  }
+}
+
+// the restricted residual at an active vertex: the corner sums of its
+// adjacent elements, in ascending element order
+__device__ __forceinline__ float crs_vertex(const float* __restrict__ corner, const CoarseDims& d, int x, int y, int z) {
+  const int gx = d.lo[0] + x, gy = d.lo[1] + y, gz = d.lo[2] + z;
+  float acc = 0.f;
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const int ez = gz - 1 + (v >> 2), ey = gy - 1 + ((v >> 1) & 1), ex = gx - 1 + (v & 1);
+    if (ez >= 0 && ez < d.Ez && ey >= 0 && ey < d.Ey && ex >= 0 && ex < d.Ex)
+      acc += corner[(ex + (int64_t)d.Ex * (ey + (int64_t)d.Ey * ez)) * 8 + (7 - v)];
+  }
+  return acc;
+}
+
+// blockIdx.x: z plane.  out: the plane's x and y forward transform
+__global__ void __launch_bounds__(kCrsThreads)
+    k_crs_fwd(const float* __restrict__ corner, float* __restrict__ out, const float* __restrict__ S0,
+              const float* __restrict__ S1, CoarseDims d, const Scalars* sc) {
+  if (sc && sc->done) return;
+  extern __shared__ __align__(16) float csm[];
+  const CrsPad q(d);
+  const int m0 = d.m[0], m1 = d.m[1];
+  float *A = csm, *B = A + q.p1 * q.p0, *X = B + q.p1 * q.p0, *Y = X + q.p0 * q.p0;
+  for (int t = threadIdx.x; t < q.p1 * q.p0; t += kCrsThreads) {
+    const int y = t / q.p0, x = t - y * q.p0;
+    A[t] = y < m1 && x < m0 ? crs_vertex(corner, d, x, y, blockIdx.x) : 0.f;
+  }
+  crs_stage(X, S0, m0, q.p0);
+  crs_stage(Y, S1, m1, q.p1);
+  __syncthreads();
+  crs_rows(A, X, m1, m0, q.p0, B);
+  __syncthreads();
+  float* o = out + (int64_t)blockIdx.x * m0 * m1;
+  crs_cols(B, Y, m1, q.p1, m0, q.p0, [&](int g, int c, float v) { o[g * m0 + c] = v; });
+}
+
+// blockIdx.x: batch of columns.  In place: z forward, divided by the
+// eigenvalue sum (the null mode dropped), z back
+__global__ void __launch_bounds__(kCrsThreads)
+    k_crs_z(float* __restrict__ io, const float* __restrict__ S2, const float* __restrict__ lam, CoarseDims d,
+            const Scalars* sc) {
+  if (sc && sc->done) return;
+  extern __shared__ __align__(16) float csm[];
+  const CrsPad q(d);
+  const int m0 = d.m[0], m1 = d.m[1], m2 = d.m[2], n = m0 * m1;
+  float *A = csm, *B = A + q.p2 * kCrsCols, *Z = B + q.p2 * kCrsCols, *ZT = Z + q.p2 * q.p2;
+  const int c0 = blockIdx.x * kCrsCols, cols = min(kCrsCols, n - c0);
+  for (int t = threadIdx.x; t < m2 * kCrsCols; t += kCrsThreads) {
+    const int z = t / kCrsCols, c = t - z * kCrsCols;
+    A[t] = c < cols ? io[(int64_t)z * n + c0 + c] : 0.f;
+  }
+  crs_stage(Z, S2, m2, q.p2);
+  crs_stage(ZT, S2 + (int64_t)m2 * m2, m2, q.p2);
+  __syncthreads();
+  crs_cols(A, Z, m2, q.p2, kCrsCols, kCrsCols, [&](int f, int c, float v) {
+    const int x = (c0 + c) % m0, y = (c0 + c) / m0;
+    float r = 0.f;
+    if (c < cols) {
+      const float D = d.h1 * (lam[x] + lam[m0 + y] + lam[m0 + m1 + f]) + d.h2;
+      r = D > d.dmin ? v / D : 0.f;
+    }
+    B[f * kCrsCols + c] = r;
+  });
+  __syncthreads();
+  crs_cols(B, ZT, m2, q.p2, kCrsCols, kCrsCols, [&](int z, int c, float v) {
+    if (c < cols) io[(int64_t)z * n + c0 + c] = v;
+  });
+}
+
+// blockIdx.x: z plane.  y and x back, into the full vertex grid
+__global__ void __launch_bounds__(kCrsThreads)
+    k_crs_back(const float* __restrict__ in, float* __restrict__ uc, const float* __restrict__ S0,
+               const float* __restrict__ S1, CoarseDims d, const Scalars* sc) {
+  if (sc && sc->done) return;
+  extern __shared__ __align__(16) float csm[];
+  const CrsPad q(d);
+  const int m0 = d.m[0], m1 = d.m[1];
+  float *A = csm, *B = A + q.p1 * q.p0, *X = B + q.p1 * q.p0, *Y = X + q.p0 * q.p0;
+  const float* src = in + (int64_t)blockIdx.x * m0 * m1;
+  for (int t = threadIdx.x; t < q.p1 * q.p0; t += kCrsThreads) {
+    const int y = t / q.p0, x = t - y * q.p0;
+    A[t] = y < m1 && x < m0 ? src[y * m0 + x] : 0.f;
+    B[t] = 0.f;
+  }
+  crs_stage(X, S0 + (int64_t)m0 * m0, m0, q.p0);
+  crs_stage(Y, S1 + (int64_t)m1 * m1, m1, q.p1);
+  __syncthreads();
+  crs_cols(A, Y, m1, q.p1, m0, q.p0, [&](int y, int c, float v) { B[y * q.p0 + c] = v; });
+  __syncthreads();
+  crs_rows(B, X, m1, m0, q.p0, A);
+  __syncthreads();
+  const int nx = d.Ex + 1, ny = d.Ey + 1;
+  float* o = uc + d.lo[0] + (int64_t)nx * (d.lo[1] + (int64_t)ny * (d.lo[2] + blockIdx.x));
+  for (int t = threadIdx.x; t < m1 * m0; t += kCrsThreads) {
+    const int y = t / m0, x = t - y * m0;
+    o[x + nx * y] = A[y * q.p0 + x];
   }
 }
 
@@ -788,7 +877,6 @@ struct ntg_schwarz {
   float* hc = nullptr;   // E x 2 (h1, h2 element means)
   std::vector<double> Sref, lamref;  // reference (h = 2) extended 1D eigenpairs
   float* ze = nullptr;   // E x LE^3 extended results
-  int fdm_grid = 0;      // persistent grid of the FDM kernel (blocks resident on all SMs)
   std::vector<double> hl;  // element lengths (host)
   // coarse level (Q1 on the vertex grid); the FDM kernel writes its restriction
   int coarse = 0, coarse_ready = 0;
@@ -1055,10 +1143,6 @@ namespace sw {
 // transforms rely on: S[LE-1-p][f] = (-1)^f S[p][f]
 inline int fdm_has_parity(const ntg_schwarz* w);
 
-// persistent grid of the selected FP32-core variant: blocks resident on all SMs
-template <int LX>
-int fdm_prepare_grid(ntg_schwarz* w);
-
 template <int LX>
 using FdmFn = void (*)(const float*, float*, const float*, int, int, int, const Scalars*, float*, CoarsePhi,
                        const int32_t*, const float*, const FdmRef<LX + 2>);
@@ -1074,10 +1158,13 @@ FdmFn<LX> fdm_kernel(const ntg_schwarz* w, bool eo) {
 template <int LX>
 int fdm_prepare(ntg_schwarz* w) {
   using C = FdmCfg<LX>;
-  for (int v = 0; v < 2; ++v)
+  for (int v = 0; v < 2; ++v) {
     NTG_CUDA_TRY(cudaFuncSetAttribute(fdm_kernel<LX>(w, v & 1), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)C::SMEM));
-  return fdm_prepare_grid<LX>(w);
+    NTG_CUDA_TRY(cudaFuncSetAttribute(fdm_kernel<LX>(w, v & 1), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      cudaSharedmemCarveoutMaxShared));
+  }
+  return NTG_OK;
 }
 
 inline int fdm_has_parity(const ntg_schwarz* w) {
@@ -1091,33 +1178,17 @@ inline int fdm_has_parity(const ntg_schwarz* w) {
 }
 
 template <int LX>
-int fdm_prepare_grid(ntg_schwarz* w) {
-  using C = FdmCfg<LX>;
-  int per_sm = 0;
-  NTG_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fdm_kernel<LX>(w, w->fdm_eo),
-                                                             C::THREADS, C::SMEM));
-  const int64_t batches = (w->plan->nelv + C::EPB - 1) / C::EPB;
-  const int64_t cap = (int64_t)num_sms() * (per_sm > 0 ? per_sm : 1);
-  w->fdm_grid = (int)(batches < cap ? batches : cap);
-  return NTG_OK;
-}
-
-template <int LX>
 int fdm_launch(ntg_schwarz* w, const float* r, cudaStream_t s, const Scalars* sc) {
   using C = FdmCfg<LX>;
   constexpr int LE = LX + 2;
   FdmRef<LE> R;
   for (int a = 0; a < LE; ++a) {
-    for (int f = 0; f < LE; ++f) {
-      const float v = (float)w->Sref[a * LE + f];
-      R.P[f >> 1][a][f & 1] = v;
-      R.Q[a >> 1][f][a & 1] = v;
-    }
+    for (int f = 0; f < LE; ++f) R.S[a][f] = (float)w->Sref[a * LE + f];
     R.lam[a] = (float)w->lamref[a];
   }
   float* corner = w->coarse_ready ? w->corner : nullptr;
   const bool g = w->gen != nullptr;
-  fdm_kernel<LX>(w, w->fdm_eo)<<<w->fdm_grid, C::THREADS, C::SMEM, s>>>(
+  fdm_kernel<LX>(w, w->fdm_eo)<<<(unsigned)((w->plan->nelv + C::EPB - 1) / C::EPB), C::THREADS, C::SMEM, s>>>(
       r, w->ze, w->esc, g ? (int)w->plan->nelv : w->Ex, g ? 1 : w->Ey, g ? 1 : w->Ez, sc, corner, w->ph,
       g ? w->gen->ghost : nullptr, g ? w->plan->multf : nullptr, R);
   NTG_COUNT_LAUNCH();
@@ -1151,6 +1222,19 @@ inline int coarse_launch(ntg_schwarz* w, cudaStream_t s, const Scalars* sc) {
   const int g = grid_for(total, 256);
   float* a = w->cwork;
   float* b = w->cwork + total;
+  const CrsPad q(d);
+  if (q.plane() <= kCrsSmem && q.column() <= kCrsSmem) {
+    NTG_TRY(fx::use_smem<k_crs_fwd>(kCrsSmem));
+    NTG_TRY(fx::use_smem<k_crs_z>(kCrsSmem));
+    NTG_TRY(fx::use_smem<k_crs_back>(kCrsSmem));
+    k_crs_fwd<<<d.m[2], kCrsThreads, q.plane(), s>>>(w->corner, a, w->cS[0], w->cS[1], d, sc);
+    NTG_COUNT_LAUNCH();
+    k_crs_z<<<(d.m[0] * d.m[1] + kCrsCols - 1) / kCrsCols, kCrsThreads, q.column(), s>>>(a, w->cS[2], w->clam, d, sc);
+    NTG_COUNT_LAUNCH();
+    k_crs_back<<<d.m[2], kCrsThreads, q.plane(), s>>>(a, w->uc, w->cS[0], w->cS[1], d, sc);
+    NTG_COUNT_LAUNCH();
+    return NTG_OK;
+  }
   k_crs_restrict<<<g, 256, 0, s>>>(w->corner, a, d, sc);
   NTG_COUNT_LAUNCH();
   k_crs_mode<0, false, false, false><<<g, 256, 0, s>>>(a, b, w->cS[0], w->clam, d, sc);
@@ -1412,8 +1496,6 @@ int ntg_schwarz_set_fdm_path(ntg_schwarz* s, int path) {
   s->fdm_tc = path == 1 ? 1 : 0;
   if (path != 1) {
     s->fdm_eo = path == 0 ? sw::fdm_has_parity(s) : 0;
-    const int lx = s->plan->lx;
-    NTG_TRY(lx == 4 ? sw::fdm_prepare_grid<4>(s) : lx == 6 ? sw::fdm_prepare_grid<6>(s) : sw::fdm_prepare_grid<8>(s));
   }
   return NTG_OK;
 }
