@@ -109,6 +109,8 @@ struct ntg_plan {
   double* B = nullptr;
   double* mult = nullptr;
   float* multf = nullptr;
+  double* multm = nullptr;      // mult, negative on Dirichlet nodes (plan_multm), and its FP32 copy
+  float* multmf = nullptr;
   // gather-scatter: full map (perm sorted by global id, offsets) and the
   // shared-node subset the hot kernels use
   int32_t* perm = nullptr;
@@ -209,6 +211,10 @@ int build_gs_classes(ntg_plan* p);
 template <typename T>
 int gs_cls_launch(ntg_plan* p, T* u, int op, cudaStream_t s, const Scalars* sc);
 int grid_for(int64_t work, int threads);
+int grid_red(int64_t work, int threads);
+// mult with the Dirichlet nodes' weights negative, built on first use after set_mask
+int plan_multm(ntg_plan* p, const double** out);
+int plan_multm(ntg_plan* p, const float** out);
 int jacobi_update(ntg_plan* p);
 int ensure_maskrow(ntg_plan* p);
 // the element counts of a Schwarz preconditioner built on a structured box

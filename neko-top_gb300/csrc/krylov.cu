@@ -7,8 +7,8 @@
 // sources/mapping_functions/PDE_filter_mapping.f90:180-184,246-262.
 //
 // Solver state lives on the device (Scalars); every iteration is a fixed
-// sequence of kernels (Ax with the fused (p, Ap) dot, gather-scatter, mask,
-// update with fused (r, z) and (r, r) dots, direction update), each of which
+// sequence of kernels (Ax with the fused (p, Ap) dot, gather-scatter,
+// update with the mask and fused (r, z) and (r, r) dots, direction update), each of which
 // returns at once after the device-side convergence flag is set.  The host
 // reads the flag every `check_every` iterations, so the iteration count is
 // exact and no per-iteration host round trip is needed.
@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "fx.cuh"
 #include "reduce.cuh"
 
 namespace ntg {
@@ -26,39 +27,90 @@ namespace ntg {
 //   sum_l D_li^2 G11(l,j,k) h1 + D_lj^2 G22(i,l,k) h1 + D_lk^2 G33(i,j,l) h1
 //   + 2 h1 (D_ii D_jj G12 + D_ii D_kk G13 + D_jj D_kk G23) + h2 B
 // ---------------------------------------------------------------------------
-struct DBig {
-  double d[NTG_LXMAX * NTG_LXMAX];
+// The sums are the transposed line operator with the squared entries of D
+// acting on G11 h1 along r, G22 h1 along s and G33 h1 along t: fixed point
+// on the integer pipes (fx.cuh), an element per block.  (As FP64 FMAs with a
+// thread per node it took 1.12 ms at 24^3 elements, lx = 8.)
+template <int LX>
+struct DiagMats {
+  fx::Mat<LX, LX> D2;
+  double d2[LX * LX];   // (D o D)^T
+  double dd[LX];        // diagonal of D
 };
 
-__global__ void k_helm_diag(int64_t nelv, int lx, const __grid_constant__ DBig D, const double* __restrict__ g11,
-                            const double* __restrict__ g12, const double* __restrict__ g13,
-                            const double* __restrict__ g22, const double* __restrict__ g23,
-                            const double* __restrict__ g33, const double* __restrict__ h1, double h1c,
-                            const double* __restrict__ hB, double* __restrict__ d) {
-  const int64_t lx3 = (int64_t)lx * lx * lx;
-  const int64_t n = nelv * lx3;
-  for (int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; m < n; m += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = m / lx3;
-    const int r = (int)(m - e * lx3);
-    const int i = r % lx, j = (r / lx) % lx, k = r / (lx * lx);
-    const int64_t base = e * lx3;
-    double acc = 0.0;
-    for (int l = 0; l < lx; ++l) {
-      int64_t qr = base + l + lx * (j + lx * k);
-      int64_t qs = base + i + lx * (l + lx * k);
-      int64_t qt = base + i + lx * (j + lx * l);
-      double hr = h1 ? h1[qr] : h1c, hs = h1 ? h1[qs] : h1c, ht = h1 ? h1[qt] : h1c;
-      double a = D.d[l * lx + i], b = D.d[l * lx + j], c = D.d[l * lx + k];
-      acc += a * a * g11[qr] * hr;
-      acc += b * b * g22[qs] * hs;
-      acc += c * c * g33[qt] * ht;
-    }
-    double hm = h1 ? h1[m] : h1c;
-    double di = D.d[i * lx + i], dj = D.d[j * lx + j], dk = D.d[k * lx + k];
-    acc += 2.0 * hm * (di * dj * g12[m] + di * dk * g13[m] + dj * dk * g23[m]);
-    if (hB) acc += hB[m];
-    d[m] = acc;
+template <int LX>
+struct DiagShape {
+  static constexpr int L2 = LX * LX, L3 = L2 * LX, TS = fx::Tile<LX>::SIZE;
+  static constexpr int EPB = LX <= 2 ? 16 : LX == 3 ? 7 : LX == 4 ? 4 : LX == 5 ? 5 : LX == 6 ? 2 : 1;
+  static constexpr int NT = (EPB * 3 * L2 + 31) / 32 * 32;
+  static constexpr size_t SMEM = sizeof(double) * EPB * 3 * TS;
+};
+
+template <int LX>
+__global__ void __launch_bounds__(DiagShape<LX>::NT)
+    k_helm_diag(int64_t nelv, const __grid_constant__ DiagMats<LX> P, const double* __restrict__ g11,
+                const double* __restrict__ g12, const double* __restrict__ g13, const double* __restrict__ g22,
+                const double* __restrict__ g23, const double* __restrict__ g33, const double* __restrict__ h1,
+                double h1c, const double* __restrict__ hB, double* __restrict__ d) {
+  using S = DiagShape<LX>;
+  using TL = fx::Tile<LX>;
+  constexpr int L2 = S::L2, L3 = S::L3, TS = S::TS, EPB = S::EPB, NT = S::NT;
+  extern __shared__ double dsm[];
+  const int64_t e0 = blockIdx.x * (int64_t)EPB;
+  const int ne = nelv - e0 < EPB ? (int)(nelv - e0) : EPB;
+  for (int t = threadIdx.x; t < ne * L3; t += NT) {
+    const int el = t / L3, p = TL::at(t - el * L3);
+    const int64_t q = e0 * L3 + t;
+    double* T = dsm + el * 3 * TS;
+    const double h = h1 ? h1[q] : h1c;
+    T[p] = g11[q] * h;
+    T[TS + p] = g22[q] * h;
+    T[2 * TS + p] = g33[q] * h;
   }
+  __syncthreads();
+  for (int t = threadIdx.x; t < ne * 3 * L2; t += NT) {
+    const int el = t / (3 * L2), r = t - el * 3 * L2, dir = r / L2;
+    double* l = dsm + (el * 3 + dir) * TS + TL::base(dir, r - dir * L2);
+    const int st = TL::stride(dir);
+    double x[LX];
+#pragma unroll
+    for (int a = 0; a < LX; ++a) x[a] = l[a * st];
+    fx::line_dbl<LX, LX, false>(P.D2, P.d2, x, [&](int A, double y) { l[A * st] = y; });
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < ne * L3; t += NT) {
+    const int el = t / L3, node = t - el * L3, p = TL::at(node);
+    const int64_t q = e0 * L3 + t;
+    const double* T = dsm + el * 3 * TS;
+    const double di = P.dd[node % LX], dj = P.dd[node / LX % LX], dk = P.dd[node / L2];
+    const double h = h1 ? h1[q] : h1c;
+    double acc = T[p] + T[TS + p] + T[2 * TS + p];
+    acc = fma(2.0 * h, di * dj * g12[q] + di * dk * g13[q] + dj * dk * g23[q], acc);
+    if (hB) acc += hB[q];
+    d[q] = acc;
+  }
+}
+
+template <int LX>
+int helm_diag(ntg_plan* p, cudaStream_t s) {
+  using S = DiagShape<LX>;
+  DiagMats<LX> P;
+  long double m[LX * LX];
+  for (int i = 0; i < LX; ++i) {
+    for (int l = 0; l < LX; ++l) {
+      const long double v = p->D[l * LX + i];
+      m[i * LX + l] = v * v;
+      P.d2[i * LX + l] = (double)(v * v);
+    }
+    P.dd[i] = p->D[i * LX + i];
+  }
+  P.D2 = fx::make_mat<LX, LX>(m);
+  NTG_TRY(fx::use_smem<k_helm_diag<LX>>(S::SMEM));
+  k_helm_diag<LX><<<(unsigned)((p->nelv + S::EPB - 1) / S::EPB), S::NT, S::SMEM, s>>>(
+      p->nelv, P, p->g[0], p->g[1], p->g[2], p->g[3], p->g[4], p->g[5], p->h1_const ? nullptr : p->h1, p->h1c,
+      p->ifh2 ? p->hB : nullptr, p->dinv);
+  NTG_COUNT_LAUNCH();
+  return NTG_OK;
 }
 
 __global__ void k_set_masked(double* __restrict__ u, const int32_t* __restrict__ mask, int64_t m, double v) {
@@ -81,11 +133,18 @@ int jacobi_update(ntg_plan* p) {
   cudaStream_t s = p->stream;
   if (!p->dinv) NTG_TRY(dev_alloc(&p->dinv, p->n));
   if (!p->dinvf) NTG_TRY(dev_alloc(&p->dinvf, p->n));
-  DBig D;
-  memcpy(D.d, p->D, sizeof(double) * p->lx * p->lx);
-  { k_helm_diag<<<grid_for(p->n, 256), 256, 0, s>>>(p->nelv, p->lx, D, p->g[0], p->g[1], p->g[2], p->g[3], p->g[4],
-                                                    p->g[5], p->h1_const ? nullptr : p->h1, p->h1c,
-                                                    p->ifh2 ? p->hB : nullptr, p->dinv); NTG_COUNT_LAUNCH(); }
+  switch (p->lx) {
+    case 2: NTG_TRY(helm_diag<2>(p, s)); break;
+    case 3: NTG_TRY(helm_diag<3>(p, s)); break;
+    case 4: NTG_TRY(helm_diag<4>(p, s)); break;
+    case 5: NTG_TRY(helm_diag<5>(p, s)); break;
+    case 6: NTG_TRY(helm_diag<6>(p, s)); break;
+    case 7: NTG_TRY(helm_diag<7>(p, s)); break;
+    case 8: NTG_TRY(helm_diag<8>(p, s)); break;
+    case 9: NTG_TRY(helm_diag<9>(p, s)); break;
+    case 10: NTG_TRY(helm_diag<10>(p, s)); break;
+    default: set_error("jacobi: lx=%d not compiled", p->lx); return NTG_ERR_UNSUPPORTED;
+  }
   NTG_CUDA_TRY(cudaGetLastError());
   NTG_TRY(gs_launch(p, p->dinv, NTG_GS_ADD, s));
   if (p->nmask) { k_set_masked<<<grid_for(p->nmask, 256), 256, 0, s>>>(p->dinv, p->mask, p->nmask, 1.0); NTG_COUNT_LAUNCH(); }
@@ -107,14 +166,14 @@ __global__ void k_wdot(const double* __restrict__ a, const double* __restrict__ 
                        int64_t n, double* __restrict__ part, Scalars* sc) {
   double s = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    s += c ? a[i] * b[i] * c[i] : a[i] * b[i];
+    s = c ? fma(a[i] * b[i], c[i], s) : fma(a[i], b[i], s);
   double v[1] = {s};
   grid_reduce<1>(v, part, sc, FinStore{0});
 }
 
 int wdot(ntg_plan* p, const double* a, const double* b, const double* c, int64_t n, double* host_out,
          cudaStream_t s) {
-  { k_wdot<<<grid_for(n, 256), 256, 0, s>>>(a, b, c, n, p->red_part, p->scal); NTG_COUNT_LAUNCH(); }
+  { k_wdot<<<grid_red(n, 256), 256, 0, s>>>(a, b, c, n, p->red_part, p->scal); NTG_COUNT_LAUNCH(); }
   NTG_CUDA_TRY(cudaGetLastError());
   NTG_CUDA_TRY(cudaMemcpyAsync(p->host_red, &p->scal->red[0], sizeof(double), cudaMemcpyDeviceToHost, s));
   NTG_CUDA_TRY(cudaStreamSynchronize(s));
@@ -211,7 +270,13 @@ struct FinUpd {
   }
 };
 
-// x += alpha p; r -= alpha w; sums (r, dinv r), (r, r)
+// the sign bit, without a slot of the FP64 pipe
+__device__ __forceinline__ bool is_neg(double m) { return __double2hiint(m) < 0; }
+__device__ __forceinline__ bool is_neg(float m) { return __float_as_int(m) < 0; }
+
+// x += alpha p; r -= alpha w; sums (r, dinv r), (r, r).  mult carries the
+// Dirichlet mask in its sign (plan_multm): w counts as zero there, so the
+// operator's image needs no masking pass of its own.
 template <typename T>
 __global__ void k_cg_update(T* __restrict__ x, const T* __restrict__ p, T* __restrict__ r, const T* __restrict__ w,
                             const T* __restrict__ dinv, const T* __restrict__ mult, int64_t n,
@@ -223,13 +288,15 @@ __global__ void k_cg_update(T* __restrict__ x, const T* __restrict__ p, T* __res
   // only the block/grid levels in FP64
   T rz = 0, rr = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const T ms = mult[i], m = fabs(ms);
     T xi = x[i] + alpha * p[i];
-    T ri = r[i] - alpha * w[i];
+    T ri = r[i];
+    if (!is_neg(ms)) ri -= alpha * w[i];
     x[i] = xi;
     r[i] = ri;
-    T mr = mult[i] * ri;
-    rz += mr * (dinv[i] * ri);
-    rr += mr * ri;
+    const T t = (m * ri) * ri;
+    rz += t * dinv[i];
+    rr += t;
   }
   double v[2] = {(double)rz, (double)rr};
   grid_reduce<2>(v, part, sc, FinUpd());
@@ -259,7 +326,9 @@ static int run_pcg(ntg_plan* pl, Scalars* sc, Scalars* hs_pinned, PcgVecs<T>& v,
                    int check_every, cudaStream_t s, int* fp_ax) {
   const int64_t n = pl->n;
   const int TPB = 256;
-  const int G = grid_for(n, TPB);
+  const int G = grid_for(n, TPB), GR = grid_red(n, TPB);
+  const T* multm = nullptr;
+  NTG_TRY(plan_multm(pl, &multm));
   // reset the scalar block
   memset(hs_pinned, 0, sizeof(Scalars));
   hs_pinned->rtol = rtol;
@@ -271,7 +340,7 @@ static int run_pcg(ntg_plan* pl, Scalars* sc, Scalars* hs_pinned, PcgVecs<T>& v,
     else NTG_TRY(op_apply_f32(pl, (float*)v.w, (const float*)x, s));
     if (fp_ax && sizeof(T) == 8) (*fp_ax)++;
   }
-  { k_cg_init<T><<<G, TPB, 0, s>>>(f, zero_guess ? nullptr : v.w, dinv, mult, v.r, v.p, n, pl->red_part, sc); NTG_COUNT_LAUNCH(); }
+  { k_cg_init<T><<<GR, TPB, 0, s>>>(f, zero_guess ? nullptr : v.w, dinv, mult, v.r, v.p, n, pl->red_part, sc); NTG_COUNT_LAUNCH(); }
   NTG_CUDA_TRY(cudaGetLastError());
   int launched = 0;
   for (;;) {
@@ -283,14 +352,12 @@ static int run_pcg(ntg_plan* pl, Scalars* sc, Scalars* hs_pinned, PcgVecs<T>& v,
       if (sizeof(T) == 8) {
         NTG_TRY(ax_launch(pl, (double*)v.w, (const double*)v.p, sc, 0, s));
         NTG_TRY(gs_add_guarded(pl, (double*)v.w, s, sc));
-        NTG_TRY(mask_guarded(pl, (double*)v.w, s, sc));
       } else {
         NTG_TRY(ax_launch_f32(pl, (float*)v.w, (const float*)v.p, sc, 0, s));
         NTG_TRY(gs_add_guarded_f32(pl, (float*)v.w, s, sc));
-        NTG_TRY(mask_guarded_f32(pl, (float*)v.w, s, sc));
       }
       timer_start(sizeof(T) == 8 ? TM_UPD64 : TM_UPD32, s);
-      { k_cg_update<T><<<G, TPB, 0, s>>>(x, v.p, v.r, v.w, dinv, mult, n, pl->red_part, sc); NTG_COUNT_LAUNCH(); }
+      { k_cg_update<T><<<GR, TPB, 0, s>>>(x, v.p, v.r, v.w, dinv, multm, n, pl->red_part, sc); NTG_COUNT_LAUNCH(); }
       timer_stop(sizeof(T) == 8 ? TM_UPD64 : TM_UPD32, s);
       timer_start(sizeof(T) == 8 ? TM_DIR64 : TM_DIR32, s);
       { k_cg_dir<T><<<G, TPB, 0, s>>>(v.p, v.r, dinv, n, sc); NTG_COUNT_LAUNCH(); }
@@ -690,10 +757,13 @@ __global__ void k_ru_init_pc(const double* __restrict__ f, const double* __restr
   grid_reduce<3>(v, part, sc, FinRUInit());
 }
 
-// r = f - w (FP64); r32 = (float) r; sums (r, r)_mult, (r32, dinv32 r32)_mult
+// r = f - w (FP64); r32 = (float) r; sums (r, r)_mult and, with RZ, (r32,
+// dinv32 r32)_mult.  The FP64 pipe bounds it (a conversion takes a slot like
+// an add): four operations per node without RZ, whose terms are FP32.
+template <bool RZ>
 __global__ void k_ru_resid(const double* __restrict__ f, const double* __restrict__ w, const float* __restrict__ dinv,
-                           const double* __restrict__ mult, double* __restrict__ r, float* __restrict__ r32, int64_t n,
-                           int mode, double* __restrict__ part, Scalars* sc) {
+                           const double* __restrict__ mult, const float* __restrict__ multf, double* __restrict__ r,
+                           float* __restrict__ r32, int64_t n, int mode, double* __restrict__ part, Scalars* sc) {
   double rr = 0;
   float rz = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -701,9 +771,8 @@ __global__ void k_ru_resid(const double* __restrict__ f, const double* __restric
     const float rf = (float)ri;
     r[i] = ri;
     r32[i] = rf;
-    const double m = mult[i];
-    rr += m * ri * ri;
-    rz += (float)m * rf * (dinv[i] * rf);
+    rr = fma(mult[i] * ri, ri, rr);
+    if (RZ) rz += multf[i] * rf * (dinv[i] * rf);
   }
   double v[2] = {rr, (double)rz};
   grid_reduce<2>(v, part, sc, FinRU{mode});
@@ -883,8 +952,10 @@ static int ksp_solve_mixed_ru(ntg_ksp* k, double* x, const double* f, ntg_monito
   cudaStream_t s = p->stream;
   const int64_t n = p->n;
   const int TPB = 256;
-  const int G = grid_for(n, TPB);
+  const int G = grid_for(n, TPB), GR = grid_red(n, TPB);
   NTG_TRY(ensure_fp32(p));
+  const float* multm = nullptr;
+  NTG_TRY(plan_multm(p, &multm));
   if (!p->jacobi_ready) NTG_TRY(jacobi_update(p));
   double xx = 0.0;
   NTG_TRY(wdot(p, x, x, nullptr, n, &xx, s));
@@ -902,7 +973,7 @@ static int ksp_solve_mixed_ru(ntg_ksp* k, double* x, const double* f, ntg_monito
     if (k->ax_ready != 2) fpax++;  // 2: the FP32 operator's image
   }
   float* y32 = k->din;
-  { k_ru_init<<<G, TPB, 0, s>>>(f, xx != 0.0 ? k->v64.w : nullptr, p->dinvf, p->mult, k->v64.r, k->v32.r, k->v32.p, y32, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+  { k_ru_init<<<GR, TPB, 0, s>>>(f, xx != 0.0 ? k->v64.w : nullptr, p->dinvf, p->mult, k->v64.r, k->v32.r, k->v32.p, y32, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
   NTG_CUDA_TRY(cudaGetLastError());
   auto poll = [&]() -> int {
     NTG_CUDA_TRY(cudaMemcpyAsync(hs, k->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
@@ -914,7 +985,7 @@ static int ksp_solve_mixed_ru(ntg_ksp* k, double* x, const double* f, ntg_monito
     NTG_TRY(op_apply(p, k->v64.w, x, s));
     fpax++;
     nru++;
-    { k_ru_resid<<<G, TPB, 0, s>>>(f, k->v64.w, p->dinvf, p->mult, k->v64.r, k->v32.r, n, mode, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+    { k_ru_resid<true><<<GR, TPB, 0, s>>>(f, k->v64.w, p->dinvf, p->mult, p->multf, k->v64.r, k->v32.r, n, mode, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
     NTG_CUDA_TRY(cudaGetLastError());
     return poll();
   };
@@ -944,9 +1015,8 @@ static int ksp_solve_mixed_ru(ntg_ksp* k, double* x, const double* f, ntg_monito
     for (int c = 0; c < k->check_every; ++c) {
       NTG_TRY(ax_launch_f32(p, k->v32.w, k->v32.p, k->sc, 0, s));
       NTG_TRY(gs_add_guarded_f32(p, k->v32.w, s, k->sc));
-      NTG_TRY(mask_guarded_f32(p, k->v32.w, s, k->sc));
       timer_start(TM_UPD32, s);
-      { k_cg_update<float><<<G, TPB, 0, s>>>(y32, k->v32.p, k->v32.r, k->v32.w, p->dinvf, p->multf, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+      { k_cg_update<float><<<GR, TPB, 0, s>>>(y32, k->v32.p, k->v32.r, k->v32.w, p->dinvf, multm, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
       timer_stop(TM_UPD32, s);
       timer_start(TM_DIR32, s);
       { k_cg_dir<float><<<G, TPB, 0, s>>>(k->v32.p, k->v32.r, p->dinvf, n, k->sc); NTG_COUNT_LAUNCH(); }
@@ -983,7 +1053,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   cudaStream_t s = p->stream;
   const int64_t n = p->n;
   const int TPB = 256;
-  const int G = grid_for(n, TPB);
+  const int G = grid_for(n, TPB), GR = grid_red(n, TPB);
   NTG_TRY(ensure_fp32(p));
   double xx = 0.0;
   NTG_TRY(wdot(p, x, x, nullptr, n, &xx, s));
@@ -1006,7 +1076,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   float* p32 = k->v32.p;
   float* w32 = k->v32.w;
   float* z32 = k->z32;
-  { k_ru_init_pc<<<G, TPB, 0, s>>>(f, xx != 0.0 ? k->v64.w : nullptr, p->mult, k->v64.r, r32, y32, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+  { k_ru_init_pc<<<GR, TPB, 0, s>>>(f, xx != 0.0 ? k->v64.w : nullptr, p->mult, k->v64.r, r32, y32, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
   auto poll = [&]() -> int {
     NTG_CUDA_TRY(cudaMemcpyAsync(hs, k->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
     NTG_CUDA_TRY(cudaStreamSynchronize(s));
@@ -1021,7 +1091,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
     NTG_TRY(op_apply(p, k->v64.w, x, s));
     fpax++;
     nru++;
-    { k_ru_resid<<<G, TPB, 0, s>>>(f, k->v64.w, p->dinvf ? p->dinvf : r32, p->mult, k->v64.r, r32, n, mode, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+    { k_ru_resid<false><<<GR, TPB, 0, s>>>(f, k->v64.w, nullptr, p->mult, p->multf, k->v64.r, r32, n, mode, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
     NTG_CUDA_TRY(cudaGetLastError());
     NTG_TRY(poll());
     if (hs->done) return NTG_OK;
@@ -1067,7 +1137,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
       timer_start(TM_UPD32, s);
       if (box_lx) {
         // gather-scatter, mask and update in one pass over the box
-        const int GB = grid_for(n / p->lx, TPB);
+        const int GB = grid_red(n / p->lx, TPB);
         if (box_lx == 8) k_update_box<8><<<GB, TPB, 0, s>>>(y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc);
         else if (box_lx == 6) k_update_box<6><<<GB, TPB, 0, s>>>(y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc);
         else k_update_box<4><<<GB, TPB, 0, s>>>(y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc);
@@ -1077,7 +1147,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
         NTG_TRY(gs_add_guarded_f32(p, w32, s, k->sc));
         NTG_TRY(mask_guarded_f32(p, w32, s, k->sc));
         timer_start(TM_UPD32, s);
-        { k_update_rr<<<G, TPB, 0, s>>>(y32, p32, r32, w32, p->multf, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+        { k_update_rr<<<GR, TPB, 0, s>>>(y32, p32, r32, w32, p->multf, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
       }
       timer_stop(TM_UPD32, s);
       timer_start(TM_PC32, s);
@@ -1097,7 +1167,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
     { k_ru_accum<<<G, TPB, 0, s>>>(x, y32, n); NTG_COUNT_LAUNCH(); }
     NTG_TRY(op_apply(p, k->v64.w, x, s));
     fpax++;
-    { k_resid<<<G, TPB, 0, s>>>(f, k->v64.w, p->mult, k->v64.r, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+    { k_resid<<<GR, TPB, 0, s>>>(f, k->v64.w, p->mult, k->v64.r, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
     NTG_TRY(poll());
     rr_final = hs->rr;
     hs->iter = iters;

@@ -18,21 +18,50 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // Block-wide sum of NL values; result valid in thread 0.  NT = blockDim.
+// An FP64 add of a warp holds the FP64 pipe for 16 clocks whatever the number
+// of useful lanes, so up to four sums of up to 256 threads go through shared
+// memory: warp q adds the block's values of sum q lane by lane, then its
+// lanes by shuffles (12 adds per sum at 256 threads; shuffles in every warp
+// take 45).
+constexpr int kSumThreads = 256;
 template <int NL>
-__device__ __forceinline__ void block_sum(double (&v)[NL], double (*sred)[32]) {
+struct BlockSum {
+  static constexpr bool STAGED = NL <= 4;
+  double v[STAGED ? NL : 1][STAGED ? kSumThreads : 1];
+  double warp[NL][32];
+};
+template <int NL>
+__device__ __forceinline__ void block_sum(double (&v)[NL], BlockSum<NL>& sm) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nwarps = (blockDim.x + 31) >> 5;
+  if constexpr (BlockSum<NL>::STAGED) {
+    if (blockDim.x <= kSumThreads) {
+#pragma unroll
+      for (int q = 0; q < NL; ++q) sm.v[q][threadIdx.x] = v[q];
+      __syncthreads();
+      for (int q = warp; q < NL; q += nwarps) {
+        double t = lane < (int)blockDim.x ? sm.v[q][lane] : 0.0;
+        for (int i = lane + 32; i < (int)blockDim.x; i += 32) t += sm.v[q][i];
+        t = warp_sum(t);
+        if (lane == 0) sm.warp[q][0] = t;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < NL; ++q) v[q] = sm.warp[q][0];
+      return;
+    }
+  }
 #pragma unroll
   for (int q = 0; q < NL; ++q) v[q] = warp_sum(v[q]);
   if (lane == 0) {
 #pragma unroll
-    for (int q = 0; q < NL; ++q) sred[q][warp] = v[q];
+    for (int q = 0; q < NL; ++q) sm.warp[q][warp] = v[q];
   }
   __syncthreads();
   if (warp == 0) {
 #pragma unroll
     for (int q = 0; q < NL; ++q) {
-      double t = lane < nwarps ? sred[q][lane] : 0.0;
+      double t = lane < nwarps ? sm.warp[q][lane] : 0.0;
       v[q] = warp_sum(t);
     }
   }
@@ -43,7 +72,7 @@ __device__ __forceinline__ void block_sum(double (&v)[NL], double (*sred)[32]) {
 // thread of every block (blockDim.x threads, 1-D thread index).
 template <int NL, typename Fin>
 __device__ __forceinline__ void grid_reduce(double (&v)[NL], double* __restrict__ part, Scalars* sc, Fin fin) {
-  __shared__ double sred[NL][32];
+  __shared__ BlockSum<NL> sred;
   __shared__ int s_last;
   block_sum<NL>(v, sred);
   if (threadIdx.x == 0) {
@@ -62,6 +91,7 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NL], double* __restrict_
     acc[q] = 0.0;
     for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) acc[q] += __ldcg(part + q * kRedSlots + b);
   }
+  __syncthreads();
   block_sum<NL>(acc, sred);
   if (threadIdx.x == 0) {
     fin(acc, sc);
