@@ -92,25 +92,36 @@ __global__ void k_transpose_bf16(const __nv_bfloat16* __restrict__ S, int64_t ro
 }
 
 // Activation gradient of a row-major [M x N] block: dZ = dH * (Hact > 0)
-// (no mask when Hact is null).  Writes any of: FP32 dZ, BF16 dZb (both
-// row-major), BF16 dZT (transposed, leading dimension ldt).  A block takes
-// 32 rows; the transposed write goes through shared memory.
+// (no mask when Hact is null).  Writes any of: BF16 dZb (row-major), BF16 dZT
+// (transposed, leading dimension ldt).  A block takes 32 rows; the transposed
+// write goes through shared memory.  The column sums of dZ (the bias
+// gradient) are taken on the way, in FP32: one row of part per block, summed
+// by k_colsum_part.
 template <int N>
 __global__ void __launch_bounds__(256) k_act_back(const float* __restrict__ dH, const __nv_bfloat16* __restrict__ Hact,
-                                                  int64_t M, float* __restrict__ dZ, __nv_bfloat16* __restrict__ dZb,
-                                                  __nv_bfloat16* __restrict__ dZT, int64_t ldt) {
+                                                  int64_t M, __nv_bfloat16* __restrict__ dZb,
+                                                  __nv_bfloat16* __restrict__ dZT, int64_t ldt,
+                                                  float* __restrict__ part) {
   __shared__ __nv_bfloat16 tile[32][N + 2];
+  __shared__ float red[256];
+  // a thread's columns: threadIdx.x % N, and the ones 256 further on
+  constexpr int W = N > 256 ? N / 256 : 1;
+  static_assert(N % 256 == 0 || 256 % N == 0, "columns per thread");
+  float acc[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) acc[w] = 0.f;
   for (int64_t r0 = (int64_t)blockIdx.x * 32; r0 < M; r0 += (int64_t)gridDim.x * 32) {
-    for (int q = threadIdx.x; q < 32 * N; q += blockDim.x) {
-      const int rr = q / N, c = q - rr * N;
+#pragma unroll
+    for (int it = 0; it < 32 * N / 256; ++it) {
+      const int q = threadIdx.x + 256 * it, rr = q / N, c = q - rr * N;
       const int64_t r = r0 + rr;
       float v = 0.f;
       if (r < M) {
         v = dH[r * N + c];
         if (Hact && !(__bfloat162float(Hact[r * N + c]) > 0.f)) v = 0.f;
-        if (dZ) dZ[r * N + c] = v;
         if (dZb) dZb[r * N + c] = __float2bfloat16(v);
       }
+      acc[it % W] += v;
       tile[rr][c] = __float2bfloat16(v);
     }
     __syncthreads();
@@ -123,24 +134,41 @@ __global__ void __launch_bounds__(256) k_act_back(const float* __restrict__ dH, 
     }
     __syncthreads();
   }
+  float* o = part + (int64_t)blockIdx.x * N;
+  if constexpr (N >= 256) {
+#pragma unroll
+    for (int w = 0; w < W; ++w) o[threadIdx.x + 256 * w] = acc[w];
+  } else {
+    red[threadIdx.x] = acc[0];
+    __syncthreads();
+    if (threadIdx.x < N) {
+      float t = 0.f;
+      for (int q = threadIdx.x; q < 256; q += N) t += red[q];
+      o[threadIdx.x] = t;
+    }
+  }
 }
 
-// column sums of a row-major [M x N] FP32 matrix, deterministic: a block per
-// 32 columns, fixed row partition, fixed tree
-__global__ void k_colsum(const float* __restrict__ a, int64_t M, int N, float* __restrict__ out) {
-  __shared__ float red[8][32];
-  const int col = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int rw = threadIdx.x >> 5;
+// out[c] = sum of part[r * N + c] over r < rows, deterministic: a block of
+// 1024 threads per 32 columns, 32 row groups and a fixed tree.  Latency
+// bounds it; the whole bias gradient took 250 us as column sums of the
+// FP32 gradient itself (16384 x 512) with eight rows in flight.
+__global__ void __launch_bounds__(1024) k_colsum_part(const float* __restrict__ part, int rows, int N,
+                                                      float* __restrict__ out) {
+  __shared__ float red[32][33];
+  const int cl = threadIdx.x & 31, rw = threadIdx.x >> 5, col = blockIdx.x * 32 + cl;
   float s = 0.f;
-  if (col < N)
-    for (int64_t r = rw; r < M; r += 8) s += a[r * N + col];
-  red[rw][threadIdx.x & 31] = s;
-  __syncthreads();
-  if (rw == 0 && col < N) {
-    float t = 0.f;
-    for (int q = 0; q < 8; ++q) t += red[q][threadIdx.x & 31];
-    out[col] = t;
+  if (col < N) {
+#pragma unroll 8
+    for (int r = rw; r < rows; r += 32) s += part[(int64_t)r * N + col];
   }
+  red[rw][cl] = s;
+  __syncthreads();
+  // the transposed tile: warp rw sums column rw
+  float t = red[cl][rw];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (cl == 0 && blockIdx.x * 32 + rw < N) out[blockIdx.x * 32 + rw] = t;
 }
 
 // dY = (Y - T) * g (MSE gradient), loss partials
@@ -275,7 +303,7 @@ struct ntg_guess {
   // activations (row-major [E x .]) and transposed copies ([. x ldt])
   __nv_bfloat16 *X = nullptr, *XT = nullptr, *H1b = nullptr, *H2b = nullptr, *H1T = nullptr, *H2T = nullptr;
   __nv_bfloat16 *dYb = nullptr, *dYT = nullptr, *dZb = nullptr, *dZT = nullptr;
-  float *Y = nullptr, *T = nullptr, *dY = nullptr, *dH = nullptr, *dZ = nullptr, *split = nullptr;
+  float *Y = nullptr, *T = nullptr, *dY = nullptr, *dH = nullptr, *split = nullptr;
   int64_t split_len = 0;
   float *D = nullptr, *AD = nullptr;  // energy loss: error and its element-local A image
   double tat = 1.0, tt = 1.0;         // (T, A T) and (T, T) of the current target
@@ -301,7 +329,7 @@ static void guess_free(ntg_guess* g) {
   dev_free(g->W1T); dev_free(g->W2T); dev_free(g->W3T); dev_free(g->W2b); dev_free(g->W3b);
   dev_free(g->X); dev_free(g->XT); dev_free(g->H1b); dev_free(g->H2b); dev_free(g->H1T); dev_free(g->H2T);
   dev_free(g->dYb); dev_free(g->dYT); dev_free(g->dZb); dev_free(g->dZT);
-  dev_free(g->Y); dev_free(g->T); dev_free(g->dY); dev_free(g->dH); dev_free(g->dZ); dev_free(g->split);
+  dev_free(g->Y); dev_free(g->T); dev_free(g->dY); dev_free(g->dH); dev_free(g->split);
   dev_free(g->D); dev_free(g->AD);
   for (int i = 0; i < 8; ++i) dev_free(g->hist[i]);
   dev_free(g->sc);
@@ -352,24 +380,24 @@ static int guess_backward(ntg_guess* g, int64_t E) {
   const int64_t F = g->F, H = g->H, O = g->O, ldt = g->ldt;
   const int ab = (int)std::min<int64_t>((E + 31) / 32, 4096);
   // dY -> BF16 row-major (A of dH2) and transposed (B of dW3)
-  { k_act_back<512><<<ab, 256, 0, s>>>(g->dY, nullptr, E, nullptr, g->dYb, g->dYT, ldt); NTG_COUNT_LAUNCH(); }
-  { k_colsum<<<(int)((O + 31) / 32), 256, 0, s>>>(g->dY, E, (int)O, g->G + g->ob3); NTG_COUNT_LAUNCH(); }
+  { k_act_back<512><<<ab, 256, 0, s>>>(g->dY, nullptr, E, g->dYb, g->dYT, ldt, g->split); NTG_COUNT_LAUNCH(); }
+  { k_colsum_part<<<(int)((O + 31) / 32), 1024, 0, s>>>(g->split, ab, (int)O, g->G + g->ob3); NTG_COUNT_LAUNCH(); }
   // dW3 [H x O] = H2^T dY
   NTG_TRY(tc_gemm_bf16(g->H2T, ldt, g->dYT, ldt, H, O, E, g->G + g->oW3, O, nullptr, 0, nullptr, 0, nullptr, 0,
                        wsplits(g, H, O), g->split, 0, err, s));
   // dH2 = dY W3^T ; dZ2 = dH2 * (H2 > 0)
   NTG_TRY(tc_gemm_bf16(g->dYb, O, g->W3b, O, E, H, O, g->dH, H, nullptr, 0, nullptr, 0, nullptr, 0, 1, nullptr, 0,
                        err, s));
-  { k_act_back<64><<<ab, 256, 0, s>>>(g->dH, g->H2b, E, g->dZ, g->dZb, g->dZT, ldt); NTG_COUNT_LAUNCH(); }
-  { k_colsum<<<(int)((H + 31) / 32), 256, 0, s>>>(g->dZ, E, (int)H, g->G + g->ob2); NTG_COUNT_LAUNCH(); }
+  { k_act_back<64><<<ab, 256, 0, s>>>(g->dH, g->H2b, E, g->dZb, g->dZT, ldt, g->split); NTG_COUNT_LAUNCH(); }
+  { k_colsum_part<<<(int)((H + 31) / 32), 1024, 0, s>>>(g->split, ab, (int)H, g->G + g->ob2); NTG_COUNT_LAUNCH(); }
   // dW2 [H x H] = H1^T dZ2
   NTG_TRY(tc_gemm_bf16(g->H1T, ldt, g->dZT, ldt, H, H, E, g->G + g->oW2, H, nullptr, 0, nullptr, 0, nullptr, 0,
                        wsplits(g, H, H), g->split, 0, err, s));
   // dH1 = dZ2 W2^T ; dZ1 = dH1 * (H1 > 0)
   NTG_TRY(tc_gemm_bf16(g->dZb, H, g->W2b, H, E, H, H, g->dH, H, nullptr, 0, nullptr, 0, nullptr, 0, 1, nullptr, 0,
                        err, s));
-  { k_act_back<64><<<ab, 256, 0, s>>>(g->dH, g->H1b, E, g->dZ, nullptr, g->dZT, ldt); NTG_COUNT_LAUNCH(); }
-  { k_colsum<<<(int)((H + 31) / 32), 256, 0, s>>>(g->dZ, E, (int)H, g->G + g->ob1); NTG_COUNT_LAUNCH(); }
+  { k_act_back<64><<<ab, 256, 0, s>>>(g->dH, g->H1b, E, nullptr, g->dZT, ldt, g->split); NTG_COUNT_LAUNCH(); }
+  { k_colsum_part<<<(int)((H + 31) / 32), 1024, 0, s>>>(g->split, ab, (int)H, g->G + g->ob1); NTG_COUNT_LAUNCH(); }
   // dW1 [F x H] = X^T dZ1
   NTG_TRY(tc_gemm_bf16(g->XT, ldt, g->dZT, ldt, F, H, E, g->G + g->oW1, H, nullptr, 0, nullptr, 0, nullptr, 0,
                        wsplits(g, F, H), g->split, 0, err, s));
@@ -500,7 +528,7 @@ int ntg_guess_create(ntg_plan* plan, int history, int hidden, uint64_t seed, ntg
       break;
     // Y, T, dY, D, AD hold nodal fields (E * lx^3 = n) or E * O raw values
     if ((st = dev_alloc(&g->Y, E * O)) || (st = dev_alloc(&g->T, std::max(g->n, E * O))) ||
-        (st = dev_alloc(&g->dY, E * O)) || (st = dev_alloc(&g->dH, E * H)) || (st = dev_alloc(&g->dZ, E * H)) ||
+        (st = dev_alloc(&g->dY, E * O)) || (st = dev_alloc(&g->dH, E * H)) ||
         (st = dev_alloc(&g->D, g->n)) || (st = dev_alloc(&g->AD, g->n)))
       break;
     g->split_len = (int64_t)1 << 24;  // 64 MB of split-K partials

@@ -211,16 +211,35 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // out = sum over z of S partial [M x N] slabs in order z = 0..S-1, then
 // bias / ReLU; FP32 row-major (ldc) or transposed ((m, n) at n * ldc + m)
-__global__ void k_splitk_sum(const float* __restrict__ part, int S, int64_t M, int64_t N, float* __restrict__ C,
-                             int64_t ldc, int transpose, const float* __restrict__ bias, int relu) {
+// The splits are shared out over 8 groups of a block and summed in a fixed
+// order: with one thread per output the few thousand outputs of a narrow
+// layer left 300 dependent loads per thread (30 us; latency bound).
+constexpr int kSumGroups = 8;
+__global__ void __launch_bounds__(32 * kSumGroups)
+    k_splitk_sum(const float* __restrict__ part, int S, int64_t M, int64_t N, float* __restrict__ C, int64_t ldc,
+                 int transpose, const float* __restrict__ bias, int relu) {
+  __shared__ float red[kSumGroups][32];
   const int64_t MN = M * N;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < MN; i += (int64_t)gridDim.x * blockDim.x) {
+  const int per = (S + kSumGroups - 1) / kSumGroups;
+  for (int64_t i0 = blockIdx.x * (int64_t)32; i0 < MN; i0 += (int64_t)gridDim.x * 32) {
+    const int64_t i = i0 + threadIdx.x;
+    const int z0 = threadIdx.y * per, z1 = min(S, z0 + per);
     float s = 0.f;
-    for (int z = 0; z < S; ++z) s += part[(int64_t)z * MN + i];
-    const int64_t m = i / N, n = i - m * N;
-    if (bias) s += bias[n];
-    if (relu) s = s > 0.f ? s : 0.f;
-    C[transpose ? n * ldc + m : m * ldc + n] = s;
+    if (i < MN) {
+#pragma unroll 8
+      for (int z = z0; z < z1; ++z) s += part[(int64_t)z * MN + i];
+    }
+    red[threadIdx.y][threadIdx.x] = s;
+    __syncthreads();
+    if (threadIdx.y == 0 && i < MN) {
+#pragma unroll
+      for (int g = 1; g < kSumGroups; ++g) s += red[g][threadIdx.x];
+      const int64_t m = i / N, n = i - m * N;
+      if (bias) s += bias[n];
+      if (relu) s = s > 0.f ? s : 0.f;
+      C[transpose ? n * ldc + m : m * ldc + n] = s;
+    }
+    __syncthreads();
   }
 }
 
@@ -341,7 +360,7 @@ int tc_gemm_bf16(const __nv_bfloat16* A, int64_t lda, const __nv_bfloat16* B, in
   else if (BN == 128) NTG_TRY((launch<128, 3>(ta, tb, ep, M, N, kb_total, kb_per_split, splits, err, s)));
   else NTG_TRY((launch<256, 2>(ta, tb, ep, M, N, kb_total, kb_per_split, splits, err, s)));
   if (splits > 1) {
-    { k_splitk_sum<<<grid_for(M * N, 256), 256, 0, s>>>(split_buf, splits, M, N, C, ldc, transpose_c, bias, relu); NTG_COUNT_LAUNCH(); }
+    { k_splitk_sum<<<grid_for(M * N, 32), dim3(32, kSumGroups), 0, s>>>(split_buf, splits, M, N, C, ldc, transpose_c, bias, relu); NTG_COUNT_LAUNCH(); }
     NTG_CUDA_TRY(cudaGetLastError());
   }
   return NTG_OK;
