@@ -14,6 +14,7 @@
 // exact and no per-iteration host round trip is needed.
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -659,23 +660,44 @@ __global__ void k_update_rr(float* __restrict__ y, const float* __restrict__ p, 
 // row) and y += alpha p, r -= alpha w; (r, r)_mult is summed over each
 // node's owning copy (no lower neighbour in any direction), which the
 // mult-weighted sum over copies equals, with no multiplicity stream.
+// HBM and the bytes in flight bound it (80 us at 32^3 elements, lx = 8,
+// 24 B per node): a whole row per thread, its loads first; half a row per
+// thread, with contiguous lanes, took 84.
 template <int LX>
 __global__ void __launch_bounds__(256)
     k_update_box(float* __restrict__ y, const float* __restrict__ p, float* __restrict__ r,
                  const float* __restrict__ w, const uint8_t* __restrict__ maskrow, int Ex,
                  int Ey, int Ez, double* __restrict__ part, Scalars* sc) {
   constexpr int N = LX - 1, LX2 = LX * LX, LX3 = LX2 * LX;
+  using V = std::conditional_t<LX % 4 == 0, float4, float2>;
+  constexpr int NV = LX * 4 / (int)sizeof(V);
   if (sc->done) return;
   const float alpha = (float)sc->alpha;
   const int64_t nrow = (int64_t)Ex * Ey * Ez * LX2;
   const int64_t sy = (int64_t)Ex * LX3, sz = (int64_t)Ex * Ey * LX3;
   float rr = 0.f;
+  union Row {
+    V v[NV];
+    float f[LX];
+  };
+  auto load = [](const float* a, Row& v) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v.v[q] = reinterpret_cast<const V*>(a)[q];
+  };
+  auto store = [](float* a, const Row& v) {
+#pragma unroll
+    for (int q = 0; q < NV; ++q) reinterpret_cast<V*>(a)[q] = v.v[q];
+  };
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nrow; t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = t / LX2;
-    const int m = (int)(t - e * LX2), j = m % LX, k = m / LX;
-    const int64_t o = e * LX3 + (int64_t)m * LX;
-    const int64_t exy = e / Ex;
-    const int cx = (int)(e - exy * Ex), cz = (int)(exy / Ey), cy = (int)(exy - (int64_t)cz * Ey);
+    const int e = (int)(t / LX2);
+    const int m = (int)(t - (int64_t)e * LX2), j = m % LX, k = m / LX;
+    const int64_t o = t * LX;
+    Row pv, yv, rv;
+    load(p + o, pv);
+    load(y + o, yv);
+    load(r + o, rv);
+    const unsigned mb = maskrow[t];
+    const int exy = e / Ex, cx = e - exy * Ex, cz = exy / Ey, cy = exy - cz * Ey;
     // covering rows, lower element first: offsets from the own row
     int64_t zo[2] = {0, 0}, yo[2] = {0, 0};
     int nz = 1, ny = 1;
@@ -693,34 +715,26 @@ __global__ void __launch_bounds__(256)
 #pragma unroll
       for (int vy = 0; vy < 2; ++vy) {
         if (vy >= ny) break;
-        const float* row = w + o + (nz == 2 ? zo[vz] : 0) + (ny == 2 ? yo[vy] : 0);
-        if (xl) acc[0] += row[N - LX3];
+        const float* q = w + o + (nz == 2 ? zo[vz] : 0) + (ny == 2 ? yo[vy] : 0);
+        Row wv;
+        load(q, wv);
+        if (xl) acc[0] += q[N - LX3];
 #pragma unroll
-        for (int i = 0; i < LX; i += 2) {
-          const float2 v = *reinterpret_cast<const float2*>(row + i);
-          acc[i] += v.x;
-          acc[i + 1] += v.y;
-        }
-        if (xh) acc[N] += row[LX3];
+        for (int i = 0; i < LX; ++i) acc[i] += wv.f[i];
+        if (xh) acc[N] += q[LX3];
       }
     }
-    const unsigned mb = maskrow[t];
-    const bool own_jk = (j > 0 || cy == 0) && (k > 0 || cz == 0);
 #pragma unroll
-    for (int i = 0; i < LX; i += 2) {
-      const float2 pp = *reinterpret_cast<const float2*>(p + o + i);
-      float2 yy = *reinterpret_cast<const float2*>(y + o + i);
-      float2 rv = *reinterpret_cast<const float2*>(r + o + i);
-      yy.x += alpha * pp.x;
-      yy.y += alpha * pp.y;
-      rv.x -= alpha * (((mb >> i) & 1u) ? 0.f : acc[i]);
-      rv.y -= alpha * (((mb >> (i + 1)) & 1u) ? 0.f : acc[i + 1]);
-      *reinterpret_cast<float2*>(y + o + i) = yy;
-      *reinterpret_cast<float2*>(r + o + i) = rv;
-      if (own_jk) {
-        if (i > 0 || cx == 0) rr += rv.x * rv.x;
-        rr += rv.y * rv.y;  // node i + 1 > 0
-      }
+    for (int i = 0; i < LX; ++i) {
+      yv.f[i] += alpha * pv.f[i];
+      rv.f[i] -= alpha * (((mb >> i) & 1u) ? 0.f : acc[i]);
+    }
+    store(y + o, yv);
+    store(r + o, rv);
+    if ((j > 0 || cy == 0) && (k > 0 || cz == 0)) {
+#pragma unroll
+      for (int i = 0; i < LX; ++i)
+        if (i > 0 || cx == 0) rr += rv.f[i] * rv.f[i];
     }
   }
   double v[2] = {0.0, (double)rr};

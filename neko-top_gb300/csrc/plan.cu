@@ -396,22 +396,28 @@ int plan_multm(ntg_plan* p, const float** out) {
   return NTG_OK;
 }
 
+__global__ void k_mask_rows(uint32_t* __restrict__ rows, const int32_t* __restrict__ mask, int64_t m, int lx) {
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t l = mask[q], b = l / lx;
+    atomicOr(rows + b / 4, 1u << (l % lx + 8 * (b & 3)));
+  }
+}
+
 int ensure_maskrow(ntg_plan* p) {
   if (p->maskrow) return NTG_OK;
   if (p->lx > 8) {
     set_error("mask rows: lx=%d above 8", p->lx);
     return NTG_ERR_UNSUPPORTED;
   }
-  const int64_t rows = p->n / p->lx;
-  std::vector<uint8_t> bits((size_t)rows, 0);
-  if (p->nmask > 0) {
-    std::vector<int32_t> mk((size_t)p->nmask);
-    NTG_CUDA_TRY(cudaMemcpyAsync(mk.data(), p->mask, sizeof(int32_t) * mk.size(), cudaMemcpyDeviceToHost, p->stream));
-    NTG_CUDA_TRY(cudaStreamSynchronize(p->stream));
-    for (int32_t l : mk) bits[l / p->lx] |= (uint8_t)(1u << (l % p->lx));
+  const size_t bytes = ((size_t)(p->n / p->lx) + 3) / 4 * 4;
+  NTG_TRY(dev_alloc(&p->maskrow, bytes));
+  NTG_CUDA_TRY(cudaMemsetAsync(p->maskrow, 0, bytes, p->stream));
+  if (p->nmask) {
+    k_mask_rows<<<grid_for(p->nmask, 256), 256, 0, p->stream>>>(reinterpret_cast<uint32_t*>(p->maskrow), p->mask,
+                                                                p->nmask, p->lx);
+    NTG_COUNT_LAUNCH();
+    NTG_CUDA_TRY(cudaGetLastError());
   }
-  NTG_TRY(dev_alloc(&p->maskrow, (size_t)rows));
-  NTG_CUDA_TRY(cudaMemcpy(p->maskrow, bits.data(), (size_t)rows, cudaMemcpyHostToDevice));
   return NTG_OK;
 }
 

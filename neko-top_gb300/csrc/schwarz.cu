@@ -28,8 +28,7 @@
 // Kernels per application: k_fdm (gather, six 1D transforms, coarse
 // restriction), k_crs_fwd, k_crs_z and k_crs_back (coarse solve; on vertex
 // grids too large for them k_crs_restrict and six k_crs_mode directions),
-// k_pull (prolongation of both levels, optional (r, z)), then the Dirichlet
-// mask.
+// k_pull (prolongation of both levels, Dirichlet mask, optional (r, z)).
 //
 // Determinism: the prolongation is a pull -- every local node sums, in a fixed
 // order, the extended results of the elements whose extended box covers it --
@@ -707,17 +706,20 @@ __global__ void k_mass_term(const double* __restrict__ hBa, const double* __rest
 // 2x2x2 combinations are summed z-major, y, x (= ascending element index).
 // A thread handles one row (j, k) of an element: per covering (y, z) choice
 // it reads the covering element's extended row (LE values, float2 pairs) and
-// the adjacent pair of each x neighbour.  DOT: also (r, z)_mult, summed over
-// each node's owning copy (no multiplicity stream), reduced deterministically
-// and finalised by FinRz (the mask applied afterwards does not change it: r
-// vanishes on masked nodes); the mult argument only selects this variant.
-// cv.uc: plus the trilinear prolongation of the coarse correction.
+// the adjacent pair of each x neighbour.  HBM and the bytes in flight bound
+// it; half a row per thread, with contiguous lanes, was slower (73 against
+// 62 us at 32^3 elements, lx = 8).
+// DOT: also (r, z)_mult, summed over each node's owning copy (no multiplicity
+// stream), reduced deterministically and finalised by FinRz (the mask does
+// not change it: r vanishes on masked nodes).  cv.uc: plus the trilinear
+// prolongation of the coarse correction.  maskrow: null, or a Dirichlet bit
+// per node, one byte per row.
 template <int LX, bool DOT>
 __global__ void __launch_bounds__(256, 4)
     k_pull(const float* __restrict__ ze, float* __restrict__ z, int Ex, int Ey, int Ez,
-           const float* __restrict__ r, const float* __restrict__ mult, int mode,
+           const float* __restrict__ r, const uint8_t* __restrict__ maskrow, int mode,
            double* __restrict__ part, Scalars* sc, CoarseView cv) {
-  constexpr int N = LX - 1, LE = LX + 2, LE2 = LE * LE, LE3 = LE2 * LE, LX2 = LX * LX, LX3 = LX2 * LX;
+  constexpr int N = LX - 1, LE = LX + 2, LE2 = LE * LE, LE3 = LE2 * LE, LX2 = LX * LX;
   static_assert(N >= 3 && LE % 2 == 0, "one neighbour per direction; rows of float2 pairs");
   if (sc && sc->done) return;
   __shared__ float sp[2][LX];
@@ -732,7 +734,7 @@ __global__ void __launch_bounds__(256, 4)
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < nrow; t += (int64_t)gridDim.x * blockDim.x) {
     const int e = (int)(t / LX2);
     const int m = (int)(t - (int64_t)e * LX2), j = m % LX, k = m / LX;
-    const int64_t o = (int64_t)e * LX3 + (int64_t)m * LX;  // first node of the row in z / r / mult
+    const int64_t o = t * LX;
     float rv[LX];
     if (DOT || cv.dw) {
 #pragma unroll
@@ -741,6 +743,7 @@ __global__ void __launch_bounds__(256, 4)
         rv[q] = r2.x; rv[q + 1] = r2.y;
       }
     }
+    const unsigned mb = maskrow ? maskrow[t] : 0u;
     const int exy = e / Ex, cx = e - exy * Ex, cz = exy / Ey, cy = exy - cz * Ey;
     const bool ly = j <= 1 && cy > 0, hy = j >= N - 1 && cy < Ey - 1;
     const bool lz = k <= 1 && cz > 0, hz = k >= N - 1 && cz < Ez - 1;
@@ -759,48 +762,41 @@ __global__ void __launch_bounds__(256, 4)
 #pragma unroll
       for (int vy = 0; vy < 2; ++vy) {
         if (vy >= ny) break;
-        // the covering row of element (cx, ., .) and its x neighbours' adjacent pairs
-        const float* row = ze + (vz ? z1 : z0) + (vy ? y1 : y0) + (int64_t)cx * LE3;
+        // the covering row of element (cx, ., .): its LE entries
+        const float* q = ze + (vz ? z1 : z0) + (vy ? y1 : y0) + (int64_t)cx * LE3;
         float w[LE];
 #pragma unroll
         for (int a = 0; a < LE; a += 2) {
-          const float2 p2 = *reinterpret_cast<const float2*>(row + a);
+          const float2 p2 = *reinterpret_cast<const float2*>(q + a);
           w[a] = p2.x; w[a + 1] = p2.y;
         }
-        const float2 lo = xl ? *reinterpret_cast<const float2*>(row - LE3 + (LE - 2)) : make_float2(0.f, 0.f);
-        const float2 hi = xh ? *reinterpret_cast<const float2*>(row + LE3) : make_float2(0.f, 0.f);
+        float2 lo = make_float2(0.f, 0.f), hi = lo;
+        if (xl) lo = *reinterpret_cast<const float2*>(q - LE3 + (LE - 2));
+        if (xh) hi = *reinterpret_cast<const float2*>(q + LE3);
         // per node: lower neighbour, own, upper neighbour (ascending element order)
         if (xl) { acc[0] += lo.x; acc[1] += lo.y; }
 #pragma unroll
         for (int i = 0; i < LX; ++i) acc[i] += w[i + 1];
-        if (xh) { acc[N - 1] += hi.x; acc[N] += hi.y; }
+        if (xh) { acc[LX - 2] += hi.x; acc[LX - 1] += hi.y; }
       }
     }
     if (cv.uc) {
-      // + P u_c: trilinear in the element's eight vertices (z-, y-, x-major);
-      // on a shared face the other element's vertices have weight exactly 0,
-      // so every copy of a node sums the same terms in the same order
+      // + P u_c: linear along z, y, x in turn; on a shared face the other
+      // element's vertices have weight exactly 0, so every copy of a node
+      // gets the same sum
       const int nx = Ex + 1, nyv = Ey + 1;
       const float* u0 = cv.uc + cx + (int64_t)nx * (cy + (int64_t)nyv * cz);
-      float cvz[2][2][2];
+      const float pj[2] = {sp[0][j], sp[1][j]}, pk[2] = {sp[0][k], sp[1][k]};
+      float c[2] = {0.f, 0.f};
 #pragma unroll
       for (int vz = 0; vz < 2; ++vz)
 #pragma unroll
         for (int vy = 0; vy < 2; ++vy)
 #pragma unroll
-          for (int vx = 0; vx < 2; ++vx) cvz[vz][vy][vx] = u0[vx + (int64_t)nx * (vy + (int64_t)nyv * vz)];
-      const float pj[2] = {sp[0][j], sp[1][j]}, pk[2] = {sp[0][k], sp[1][k]};
+          for (int vx = 0; vx < 2; ++vx)
+            c[vx] += (pj[vy] * pk[vz]) * u0[vx + (int64_t)nx * (vy + (int64_t)nyv * vz)];
 #pragma unroll
-      for (int i = 0; i < LX; ++i) {
-        float c = 0.f;
-#pragma unroll
-        for (int vz = 0; vz < 2; ++vz)
-#pragma unroll
-          for (int vy = 0; vy < 2; ++vy)
-#pragma unroll
-            for (int vx = 0; vx < 2; ++vx) c += (sp[vx][i] * pj[vy] * pk[vz]) * cvz[vz][vy][vx];
-        acc[i] += c;
-      }
+      for (int i = 0; i < LX; ++i) acc[i] += sp[0][i] * c[0] + sp[1][i] * c[1];
     }
     if (cv.dw) {
 #pragma unroll
@@ -810,6 +806,10 @@ __global__ void __launch_bounds__(256, 4)
         acc[q + 1] += d2.y * rv[q + 1];
       }
     }
+#pragma unroll
+    for (int i = 0; i < LX; ++i)
+      if ((mb >> i) & 1u) acc[i] = 0.f;
+    // pairs: z may be a caller's field of any 8-byte alignment
 #pragma unroll
     for (int q = 0; q < LX; q += 2) *reinterpret_cast<float2*>(z + o + q) = make_float2(acc[q], acc[q + 1]);
     if constexpr (DOT) {
@@ -1202,14 +1202,17 @@ namespace ntg {
 namespace sw {
 
 template <int LX>
-int pull_launch(ntg_schwarz* w, float* z, const float* r, cudaStream_t s, Scalars* sc, const float* mult,
-                double* part, int mode) {
-  const int g = grid_for(w->plan->n / LX, 256);
+int pull_launch(ntg_schwarz* w, float* z, const float* r, cudaStream_t s, Scalars* sc, bool dot, double* part,
+                int mode) {
+  ntg_plan* p = w->plan;
+  if (p->nmask) NTG_TRY(ensure_maskrow(p));
+  const uint8_t* mask = p->nmask ? p->maskrow : nullptr;
+  const int64_t rows = p->n / LX;
   const CoarseView cv{w->coarse_ready ? w->uc : nullptr, w->ph, w->dw};
-  if (mult)
-    k_pull<LX, true><<<g, 256, 0, s>>>(w->ze, z, w->Ex, w->Ey, w->Ez, r, mult, mode, part, sc, cv);
+  if (dot)
+    k_pull<LX, true><<<grid_red(rows, 256), 256, 0, s>>>(w->ze, z, w->Ex, w->Ey, w->Ez, r, mask, mode, part, sc, cv);
   else
-    k_pull<LX, false><<<g, 256, 0, s>>>(w->ze, z, w->Ex, w->Ey, w->Ez, r, nullptr, 0, nullptr, sc, cv);
+    k_pull<LX, false><<<grid_for(rows, 256), 256, 0, s>>>(w->ze, z, w->Ex, w->Ey, w->Ez, r, mask, 0, nullptr, sc, cv);
   NTG_COUNT_LAUNCH();
   return NTG_OK;
 }
@@ -1315,7 +1318,7 @@ int ntg::schwarz_apply(ntg_schwarz* w, float* z, const float* r, cudaStream_t s,
         timer_stop(TM_CRS, s);
       }
       timer_start(TM_PULL, s);
-      NTG_TRY(sw::pull_launch<4>(w, z, r, s, sc, mult, part, rz_mode));
+      NTG_TRY(sw::pull_launch<4>(w, z, r, s, sc, mult != nullptr, part, rz_mode));
       timer_stop(TM_PULL, s);
       break;
     case 6:
@@ -1328,7 +1331,7 @@ int ntg::schwarz_apply(ntg_schwarz* w, float* z, const float* r, cudaStream_t s,
         timer_stop(TM_CRS, s);
       }
       timer_start(TM_PULL, s);
-      NTG_TRY(sw::pull_launch<6>(w, z, r, s, sc, mult, part, rz_mode));
+      NTG_TRY(sw::pull_launch<6>(w, z, r, s, sc, mult != nullptr, part, rz_mode));
       timer_stop(TM_PULL, s);
       break;
     case 8:
@@ -1345,7 +1348,7 @@ int ntg::schwarz_apply(ntg_schwarz* w, float* z, const float* r, cudaStream_t s,
         timer_stop(TM_CRS, s);
       }
       timer_start(TM_PULL, s);
-      NTG_TRY(sw::pull_launch<8>(w, z, r, s, sc, mult, part, rz_mode));
+      NTG_TRY(sw::pull_launch<8>(w, z, r, s, sc, mult != nullptr, part, rz_mode));
       timer_stop(TM_PULL, s);
       break;
     default:
@@ -1353,8 +1356,8 @@ int ntg::schwarz_apply(ntg_schwarz* w, float* z, const float* r, cudaStream_t s,
       return NTG_ERR_UNSUPPORTED;
   }
   NTG_CUDA_TRY(cudaGetLastError());
-  // the pull assembles (identical sums on every copy): only the mask remains
-  return mask_guarded_f32(p, z, s, sc);
+  // the pull assembles (identical sums on every copy) and masks
+  return NTG_OK;
 }
 
 extern "C" {
