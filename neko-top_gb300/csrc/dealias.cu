@@ -188,7 +188,6 @@ struct AdvShape {
   static constexpr int EL = 12 * TS + (3 * G2 + 1) / 2;     // doubles per element: tiles, line exponents
   static constexpr size_t SMEM = sizeof(double) * EPB * EL;
   static constexpr int MINB = (int)(232448 / (SMEM + 1024));
-  static constexpr int NR = (EPB * G3 + NT - 1) / NT;  // nodes per thread
   // the interpolations' intermediate forms fit the tiles they pass through
   static_assert(L2 * (LX | 1) * 6 <= 6 * TS && L2 * RS * 6 <= 6 * TS && LX * LXD * RS * 6 <= 6 * TS, "tiles");
 };
@@ -212,7 +211,7 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
   using S = AdvShape<LX, LXD>;
   using TG = fx::Tile<LXD>;
   constexpr int G2 = S::G2, G3 = S::G3, L2 = S::L2, L3 = S::L3, RS = S::RS, TS = S::TS, EPB = S::EPB, NT = S::NT;
-  constexpr int LS = LX | 1;
+  constexpr int LS = LX | 1, RES = MODE == 0 ? 9 : 6;  // first tile of the results
   extern __shared__ double sm[];
   for (int64_t e0 = blockIdx.x * (int64_t)EPB; e0 < nelv; e0 += (int64_t)gridDim.x * EPB) {
     const int ne = nelv - e0 < EPB ? (int)(nelv - e0) : EPB;
@@ -244,21 +243,29 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
       line_at<LX, LXD, false>(P.J, P.j, T + 6 * TS + f * LX * LXD * RS + p, LXD * RS, T + f * TS + p, LXD * RS);
     });
     __syncthreads();
-    // tiles 0-2: u, 3-5: Ub, 6-8: derivatives or fluxes, 9-11: a_d, then the result per component
+    // tiles 0-2: u, 3-5: Ub; adjoint: 6-8 fluxes, 9-11 a_d, then the result per
+    // component; linear: 6-8 the result, 9-11 V_d of the undifferentiated field
     if constexpr (MODE == 0) {
+// a_d along its lines: the three fields' derivatives of one line each
+      // are weighted by u and summed in registers
+      items(3 * G2, [&](double* T, int t, int64_t) {
+        const int d = t / G2, b = TG::base(d, t - d * G2), st = TG::stride(d);
+        double a[LXD];
+#pragma unroll
+        for (int l = 0; l < LXD; ++l) a[l] = 0.0;
 #pragma unroll 1
-      for (int d = 0; d < 3; ++d) {
-        items(3 * G2, [&](double* T, int i, int64_t) {
-          const int f = i / G2;
-          fx::deriv_line<LXD>(P.D, P.d, T + (3 + f) * TS, T + (6 + f) * TS, d, i - f * G2);
-        });
-        __syncthreads();
-        items(G3, [&](double* T, int node, int64_t) {
-          const int p = TG::at(node);
-          T[(9 + d) * TS + p] = T[p] * T[6 * TS + p] + T[TS + p] * T[7 * TS + p] + T[2 * TS + p] * T[8 * TS + p];
-        });
-        __syncthreads();
-      }
+        for (int f = 0; f < 3; ++f) {
+          const double *u = T + f * TS + b, *v = T + (3 + f) * TS + b;
+          double x[LXD];
+#pragma unroll
+          for (int l = 0; l < LXD; ++l) x[l] = v[l * st];
+          fx::line_dbl<LXD, LXD, true>(P.D, P.d, x, [&](int A, double y) { a[A] = fma(y, u[A * st], a[A]); });
+        }
+        double* o = T + (9 + d) * TS + b;
+#pragma unroll
+        for (int l = 0; l < LXD; ++l) o[l * st] = a[l];
+      });
+      __syncthreads();
       items(G3, [&](double* T, int node, int64_t e) {
         const int p = TG::at(node);
         const int64_t q = e * G3 + node;
@@ -295,9 +302,6 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
         __syncthreads();
       }
     } else {
-      double acc[S::NR][3];
-#pragma unroll
-      for (int r = 0; r < S::NR; ++r) acc[r][0] = acc[r][1] = acc[r][2] = 0.0;
 #pragma unroll 1
       for (int pass = 0; pass < 2; ++pass) {
         items(G3, [&](double* T, int node, int64_t e) {
@@ -305,49 +309,34 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
           const int64_t q = e * G3 + node;
           const double* X = T + (pass ? 3 : 0) * TS + p;
           const double x = X[0], y = X[TS], z = X[2 * TS];
+          if (pass == 0) T[6 * TS + p] = T[7 * TS + p] = T[8 * TS + p] = 0.0;
 #pragma unroll
           for (int m = 0; m < 3; ++m)
             T[(9 + m) * TS + p] = met[3 * m * ngl + q] * x + met[(3 * m + 1) * ngl + q] * y + met[(3 * m + 2) * ngl + q] * z;
         });
+        __syncthreads();
+        // the sums of tiles 6-8 line by line, one direction at a time
 #pragma unroll 1
-        for (int i = 0; i < 3; ++i) {
+        for (int d = 0; d < 3; ++d) {
           items(3 * G2, [&](double* T, int t, int64_t) {
-            const int d = t / G2;
-            fx::deriv_line<LXD>(P.D, P.d, T + ((pass ? 0 : 3) + i) * TS, T + (6 + d) * TS, d, t - d * G2);
+            const int i = t / G2, b = TG::base(d, t - i * G2), st = TG::stride(d);
+            const double *in = T + ((pass ? 0 : 3) + i) * TS + b, *v = T + (9 + d) * TS + b;
+            double* o = T + (6 + i) * TS + b;
+            double x[LXD];
+#pragma unroll
+            for (int l = 0; l < LXD; ++l) x[l] = in[l * st];
+            fx::line_dbl<LXD, LXD, true>(P.D, P.d, x, [&](int A, double y) {
+              o[A * st] = fma(y, v[A * st], o[A * st]);
+            });
           });
           __syncthreads();
-#pragma unroll
-          for (int r = 0; r < S::NR; ++r) {
-            const int t = threadIdx.x + r * NT;
-            if (t < ne * G3) {
-              const int el = EPB == 1 ? 0 : t / G3;
-              const double* T = sm + el * S::EL + TG::at(EPB == 1 ? t : t - el * G3);
-              const double g = T[6 * TS] * T[9 * TS] + T[7 * TS] * T[10 * TS] + T[8 * TS] * T[11 * TS];
-              if (i == 0) acc[r][0] += g;
-              else if (i == 1) acc[r][1] += g;
-              else acc[r][2] += g;
-            }
-          }
-          __syncthreads();
         }
       }
-#pragma unroll
-      for (int r = 0; r < S::NR; ++r) {
-        const int t = threadIdx.x + r * NT;
-        if (t < ne * G3) {
-          const int el = EPB == 1 ? 0 : t / G3;
-          double* T = sm + el * S::EL + TG::at(EPB == 1 ? t : t - el * G3);
-          T[9 * TS] = acc[r][0];
-          T[10 * TS] = acc[r][1];
-          T[11 * TS] = acc[r][2];
-        }
-      }
-      __syncthreads();
     }
     // back: JW along t, s, r, then f -= the result
     items(3 * G2, [&](double* T, int t, int64_t) {  // i, B, A
       const int i = t / G2, r = t - i * G2, p = r / LXD * RS + r % LXD;
-      line_at<LXD, LX, false>(P.JW, P.jw, T + (9 + i) * TS + p, LXD * RS, T + i * LX * LXD * RS + p, LXD * RS);
+      line_at<LXD, LX, false>(P.JW, P.jw, T + (RES + i) * TS + p, LXD * RS, T + i * LX * LXD * RS + p, LXD * RS);
     });
     __syncthreads();
     items(3 * LX * LXD, [&](double* T, int t, int64_t) {  // (i, c), A

@@ -234,27 +234,38 @@ __global__ void __launch_bounds__(FxShape<LX, 9>::NT, FxShape<LX, 9>::MINB)
   stage_w3<LX>(w3t, M, NT);
   NTG_FX_ELEMENTS {
     NTG_FX_NE;
-    // tiles 0-2: Ub, then V; 3-5: derivatives, then fluxes; 6-8: a_d, then the opgrad part
+    // tiles 0-2: Ub, then V; 3-5: u, then fluxes; 6-8: a_d, then the opgrad part
     NTG_FX_NODES {
       NTG_FX_NODE
       T[p] = b0[q];
       T[TS + p] = b1[q];
       T[2 * TS + p] = b2[q];
+      T[3 * TS + p] = u0[q];
+      T[4 * TS + p] = u1[q];
+      T[5 * TS + p] = u2[q];
     }
+    __syncthreads();
+    // a_d along its lines: the three fields' derivatives of one line each are
+    // weighted by u and summed in registers
+    NTG_FX_LINES {
+      NTG_FX_LINE
+      const int b = TL::base(d, lq), st = TL::stride(d);
+      double a[LX];
+#pragma unroll
+      for (int l = 0; l < LX; ++l) a[l] = 0.0;
 #pragma unroll 1
-    for (int dir = 0; dir < 3; ++dir) {
-      __syncthreads();
-      NTG_FX_LINES {
-        NTG_FX_LINE  // d: the field here
-        fx::deriv_line<LX>(P.D, P.d, T + d * TS, T + (3 + d) * TS, dir, lq);
+      for (int f = 0; f < 3; ++f) {
+        const double *v = T + f * TS + b, *u = T + (3 + f) * TS + b;
+        double x[LX];
+#pragma unroll
+        for (int l = 0; l < LX; ++l) x[l] = v[l * st];
+        fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) { a[A] = fma(y, u[A * st], a[A]); });
       }
-      __syncthreads();
-      NTG_FX_NODES {
-        NTG_FX_NODE
-        T[(6 + dir) * TS + p] = u0[q] * T[3 * TS + p] + u1[q] * T[4 * TS + p] + u2[q] * T[5 * TS + p];
-      }
+#pragma unroll
+      for (int l = 0; l < LX; ++l) T[(6 + d) * TS + b + l * st] = a[l];
     }
-    NTG_FX_NODES {  // the node's own thread wrote its a_d
+    __syncthreads();
+    NTG_FX_NODES {
       NTG_FX_NODE
       double m[9];
 #pragma unroll
@@ -301,45 +312,59 @@ __global__ void __launch_bounds__(FxShape<LX, 9>::NT, FxShape<LX, 9>::MINB)
 // V_d(x) = sum_c c_dc x_c: 39 FP64 operations per node (216 with the
 // contractions on the FP64 pipe).
 template <int LX>
-__global__ void __launch_bounds__(FxShape<LX, 10>::NT, FxShape<LX, 10>::MINB)
+__global__ void __launch_bounds__(FxShape<LX, 9>::NT, FxShape<LX, 9>::MINB)
     k_adv_lin_nd(double* __restrict__ f0, double* __restrict__ f1, double* __restrict__ f2,
                  const double* __restrict__ u0, const double* __restrict__ u1, const double* __restrict__ u2,
                  const double* __restrict__ b0, const double* __restrict__ b1, const double* __restrict__ b2,
                  int64_t nelv, const __grid_constant__ DMat<LX> M, const __grid_constant__ fx::Mats<LX> P,
                  const double* __restrict__ met, int64_t n) {
-  NTG_FX_PROLOGUE(10)
+  NTG_FX_PROLOGUE(9)
   stage_w3<LX>(w3t, M, NT);
   NTG_FX_ELEMENTS {
     NTG_FX_NE;
-    // tile 0: the field differentiated; 1-3: its derivatives; 4-6: V_d of the other velocity; 7-9: sums
+    // tiles 0-2: the velocity differentiated; 3-5: V_d of the other; 6-8: sums
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
-      const double* x0 = pass ? b0 : u0;
-      const double* x1 = pass ? b1 : u1;
-      const double* x2 = pass ? b2 : u2;
+      const double *x0 = pass ? b0 : u0, *x1 = pass ? b1 : u1, *x2 = pass ? b2 : u2;
+      const double *y0 = pass ? u0 : b0, *y1 = pass ? u1 : b1, *y2 = pass ? u2 : b2;
       NTG_FX_NODES {
         NTG_FX_NODE
         const double x = x0[q], y = x1[q], z = x2[q];
+        T[p] = y0[q];
+        T[TS + p] = y1[q];
+        T[2 * TS + p] = y2[q];
+        if (pass == 0) T[6 * TS + p] = T[7 * TS + p] = T[8 * TS + p] = 0.0;
 #pragma unroll
         for (int c = 0; c < 3; ++c)
-          T[(4 + c) * TS + p] = met[3 * c * n + q] * x + met[(3 * c + 1) * n + q] * y + met[(3 * c + 2) * n + q] * z;
+          T[(3 + c) * TS + p] = met[3 * c * n + q] * x + met[(3 * c + 1) * n + q] * y + met[(3 * c + 2) * n + q] * z;
       }
+      __syncthreads();
 #pragma unroll 1
-      for (int c = 0; c < 3; ++c) {
-        const double* a = pass ? (c == 0 ? u0 : c == 1 ? u1 : u2) : (c == 0 ? b0 : c == 1 ? b1 : b2);
-        double* fc = c == 0 ? f0 : c == 1 ? f1 : f2;
-        NTG_FX_NODES { NTG_FX_NODE T[p] = a[q]; }
-        __syncthreads();
-        NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T, T + (1 + d) * TS, d, lq); }
-        __syncthreads();
-        NTG_FX_NODES {
-          NTG_FX_NODE
-          const double g = T[TS + p] * T[4 * TS + p] + T[2 * TS + p] * T[5 * TS + p] + T[3 * TS + p] * T[6 * TS + p];
-          if (pass) fc[q] = fma(-w3t[node], g + T[(7 + c) * TS + p], fc[q]);
-          else T[(7 + c) * TS + p] = g;
+      for (int dir = 0; dir < 3; ++dir) {
+        NTG_FX_LINES {
+          NTG_FX_LINE  // d: the field here
+          const int b = TL::base(dir, lq), st = TL::stride(dir);
+          const double *in = T + d * TS + b, *v = T + (3 + dir) * TS + b;
+          double* o = T + (6 + d) * TS + b;
+          double x[LX];
+#pragma unroll
+          for (int l = 0; l < LX; ++l) x[l] = in[l * st];
+          fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) {
+            o[A * st] = fma(y, v[A * st], o[A * st]);
+          });
         }
+        __syncthreads();
       }
     }
+    NTG_FX_NODES {
+      NTG_FX_NODE
+      const double w = -w3t[node];
+      f0[q] = fma(w, T[6 * TS + p], f0[q]);
+      f1[q] = fma(w, T[7 * TS + p], f1[q]);
+      f2[q] = fma(w, T[8 * TS + p], f2[q]);
+    }
+    // the next element's first nodes write tiles 0-5, read last before the
+    // barrier above, and each thread's own nodes of tiles 6-8
   }
 }
 
@@ -557,9 +582,9 @@ int ntg_linear_advection_no_dealias(ntg_plan* p, double* fx, double* fy, double*
   // f_i -= B conv1(u_i; Ub) + B conv1(Ub_i; u), one element pass
   NTG_TRY(dv::dispatch<6>(p->lx, [&](auto L) -> int {
     constexpr int LX = decltype(L)::value;
-    using S = dv::FxShape<LX, 10>;
+    using S = dv::FxShape<LX, 9>;
     NTG_TRY(fx::use_smem<dv::k_adv_lin_nd<LX>>(S::SMEM));
-    dv::k_adv_lin_nd<LX><<<dv::fx_grid<LX, 10>(p), S::NT, S::SMEM, p->stream>>>(
+    dv::k_adv_lin_nd<LX><<<dv::fx_grid<LX, 9>(p), S::NT, S::SMEM, p->stream>>>(
         f[0], f[1], f[2], u[0], u[1], u[2], ub[0], ub[1], ub[2], p->nelv, dv::dmat<LX>(p),
         fx::plan_mats<LX>(p, 1.0), p->met, p->n);
     NTG_COUNT_LAUNCH();
