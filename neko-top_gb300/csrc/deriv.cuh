@@ -32,11 +32,13 @@ template <int LX, int TILES>
 struct FxShape {
   static constexpr int L2 = LX * LX, L3 = L2 * LX, TS = fx::Tile<LX>::SIZE;
   static constexpr int EPB = LX <= 2 ? 16 : LX == 3 ? 7 : LX == 4 ? 4 : LX == 5 ? 5 : LX == 6 ? 2 : 1;
-  static constexpr int NT = (EPB * 3 * L2 + 31) / 32 * 32;
+  // lx = 7 and 8: two whole passes over the nodes (256 against 192 threads at lx = 8: 2.50 and 2.56 ms for the
+  // residuals at 24^3 elements)
+  static constexpr int NT = LX == 8 ? 256 : LX == 7 ? 192 : (EPB * 3 * L2 + 31) / 32 * 32;
   // per element: tiles, the exponents of a flux's lines; once: the products of the GLL weights
   static constexpr int EL = TILES * TS + (3 * L2 + 1) / 2;
   static constexpr size_t SMEM = (size_t)(EPB * EL + L3) * sizeof(double);
-  static constexpr int FIT = (int)(230000 / (SMEM + 1024)), WANT = 1024 / NT;
+  static constexpr int FIT = (int)(230000 / (SMEM + 1024)), WANT = 1344 / NT;
   static constexpr int MINB = FIT < 1 ? 1 : FIT < WANT ? FIT : WANT;
 };
 
