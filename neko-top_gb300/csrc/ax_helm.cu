@@ -5,17 +5,16 @@
 // .false.) at sources/mapping_functions/PDE_filter_mapping.f90:177 and
 // sources/adjoint/adjoint_pnpn.f90:207,217; applied inside ksp%solve).
 //
-// Mapping: one element per 64-thread group (thread (i,j) owns the column
-// u(i,j,0..LX-1)); EPB elements per block.  The t-direction contraction runs
-// on the column held in registers with D taken from the kernel-parameter
-// (constant) bank at compile-time indices; the r- and s-direction
-// contractions read the element tile from shared memory, where a warp's
-// reads are broadcasts or 8 consecutive words (conflict-free).  Each thread
-// keeps its D rows/columns in registers.  The transposed contractions reuse
-// the same pattern on the metric-mixed fluxes.
-//
-// Bounds: FP64 is FP64-pipe bound on GB300 (about 1.2 TFLOP/s against ~116
-// flop per DOF); FP32 is HBM bound (32 B/DOF for Poisson).
+// The FP32 operator of the orders that have no bulk-copy pipeline (lx = 8:
+// ax_helm_f32_tma.cu; FP64: ax_helm_fx.cu).  One element per LX x LX thread
+// group (thread (i,j) owns the column u(i,j,0..LX-1)); EPB elements per
+// block.  The t-direction contraction runs on the column held in registers
+// with D taken from the kernel-parameter (constant) bank at compile-time
+// indices; the r- and s-direction contractions read the element tile from
+// shared memory, where a warp's reads are broadcasts or consecutive words.
+// Each thread keeps its D rows/columns in registers.  The transposed
+// contractions reuse the same pattern on the metric-mixed fluxes.  HBM bound
+// (32 B/DOF for Poisson).
 #include "common.cuh"
 #include "reduce.cuh"
 
@@ -67,12 +66,25 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
     const int64_t e = grp * EPB + le;
     const bool active = worker && e < nelv;
     const int64_t base = e * LX3 + ij;
-    T ureg[LX];
+    // every stream's loads first: the bytes in flight bound this kernel.  With
+    // the metric loads between the contractions the operator, gather-scatter and
+    // preconditioner of 4641 elements of lx = 6 took 89 us, so 81
+    T ureg[LX], G[6][LX], hh[LX];
 #pragma unroll
     for (int k = 0; k < LX; ++k) {
-      ureg[k] = active ? u[base + k * LX2] : T(0);
-      if (worker) s_u[le][ij + k * LX2] = ureg[k];
+      const int64_t q = base + k * LX2;
+      ureg[k] = active ? u[q] : T(0);
+      G[0][k] = active ? g11[q] : T(0);
+      G[1][k] = active ? g12[q] : T(0);
+      G[2][k] = active ? g13[q] : T(0);
+      G[3][k] = active ? g22[q] : T(0);
+      G[4][k] = active ? g23[q] : T(0);
+      G[5][k] = active ? g33[q] : T(0);
+      if (H1ARR) hh[k] = active ? h1[q] : T(0);
     }
+#pragma unroll
+    for (int k = 0; k < LX; ++k)
+      if (worker) s_u[le][ij + k * LX2] = ureg[k];
     __syncthreads();
     T wt[LX];
 #pragma unroll
@@ -84,20 +96,15 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
         us = fma(Dsj[l], s_u[le][k * LX2 + l * LX + i], us);
         ut = fma(Dp.d[k * LX + l], ureg[l], ut);
       }
-      T a11 = 0, a12 = 0, a13 = 0, a22 = 0, a23 = 0, a33 = 0, hh = h1c;
-      if (active) {
-        const int64_t q = base + k * LX2;
-        a11 = g11[q]; a12 = g12[q]; a13 = g13[q]; a22 = g22[q]; a23 = g23[q]; a33 = g33[q];
-        if (H1ARR) hh = h1[q];
-      }
-      T wr = a11 * ur + a12 * us + a13 * ut;
-      T ws = a12 * ur + a22 * us + a23 * ut;
-      T wtt = a13 * ur + a23 * us + a33 * ut;
+      const T h = H1ARR ? hh[k] : h1c;
+      const T wr = G[0][k] * ur + G[1][k] * us + G[2][k] * ut;
+      const T ws = G[1][k] * ur + G[3][k] * us + G[4][k] * ut;
+      const T wtt = G[2][k] * ur + G[4][k] * us + G[5][k] * ut;
       if (worker) {
-        s_r[le][ij + k * LX2] = hh * wr;
-        s_s[le][ij + k * LX2] = hh * ws;
+        s_r[le][ij + k * LX2] = h * wr;
+        s_s[le][ij + k * LX2] = h * ws;
       }
-      wt[k] = hh * wtt;
+      wt[k] = h * wtt;
     }
     __syncthreads();
 #pragma unroll
@@ -116,7 +123,8 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
         if (DOT) dot = fma(ureg[k], acc, dot);
       }
     }
-    __syncthreads();
+    // s_u is rewritten next, read last before the barrier above; s_r and s_s
+    // after the next one
   }
   if (DOT) {
     double v[1] = {(double)dot};
