@@ -43,6 +43,7 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
               const __grid_constant__ DParam<T, LX> Dp, double* __restrict__ part, Scalars* sc) {
   using S = AxShape<T, LX>;
   constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
+  dependent_start();
   if (DOT && sc->done) return;
   __shared__ T s_u[EPB][LX3];
   __shared__ T s_r[EPB][LX3];
@@ -150,8 +151,8 @@ static int launch_lx(ntg_plan* p, T* w, const T* u, const T* const* g, const T* 
   const bool h1arr = h1 != nullptr, h2 = hB != nullptr;
 #define NTG_AX_CASE(H1A, HH2, DT)                                                                              \
   if (h1arr == H1A && h2 == HH2 && (sc != nullptr) == DT) {                                                 \
-    { k_ax_helm<T, LX, H1A, HH2, DT><<<grid, NT, 0, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1c, \
-                                                            hB, p->nelv, Dp, p->red_part, sc); NTG_COUNT_LAUNCH(); }              \
+    NTG_TRY((launch_dependent(p, k_ax_helm<T, LX, H1A, HH2, DT>, grid, NT, 0, s, w, u, g[0], g[1], g[2], g[3], \
+                              g[4], g[5], h1, h1c, hB, p->nelv, Dp, p->red_part, sc)));                    \
   }
   NTG_AX_CASE(false, false, false)
   NTG_AX_CASE(false, true, false)

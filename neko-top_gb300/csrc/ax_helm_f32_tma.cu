@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(NT, 1)
   constexpr int NARR = 7 + (H1ARR ? 1 : 0) + (H2 ? 1 : 0);
   using St = Stages<NARR>;
   constexpr int NSTAGE = St::NSTAGE;
+  dependent_start();
   if (DOT && sc->done) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float* stage_base = reinterpret_cast<float*>(smem_raw);
@@ -254,9 +255,8 @@ static int launch_variant(ntg_plan* p, float* w, const float* u, const float* co
   const int64_t ngroups = (p->nelv + EPB - 1) / EPB;
   int grid = num_sms();
   if (ngroups < grid) grid = (int)ngroups;
-  { kern<<<grid, NT, SMEM, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1c, hB, p->nelv, Dp, p->red_part, sc, p->dev_err); NTG_COUNT_LAUNCH(); }
-  NTG_CUDA_TRY(cudaGetLastError());
-  return NTG_OK;
+  return launch_dependent(p, kern, grid, NT, SMEM, s, w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1c, hB, p->nelv, Dp,
+                          p->red_part, sc, p->dev_err);
 }
 
 }  // namespace tma

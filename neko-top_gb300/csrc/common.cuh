@@ -187,6 +187,47 @@ int schwarz_apply(ntg_schwarz* sw, float* z, const float* r, cudaStream_t s, Sca
 void timer_start(int id, cudaStream_t s);
 void timer_stop(int id, cudaStream_t s);
 
+// Programmatic dependent launch for the kernels of the solver iterations: on
+// small meshes they take 3 to 20 us each, one after another, and most of that
+// is the launch and the last blocks of the kernel before.  A kernel that begins
+// with dependent_wait() may be launched by launch_dependent() while its
+// predecessor still runs: it waits for the predecessor's end (which waited for
+// everything before it) before it touches memory.  dependent_start() also lets
+// the successor be scheduled.  k_fdm leaves that out (0.4% of a solve at 43M
+// nodes for the instruction alone), and the FP64 operator takes no part: with
+// its successors waiting beside it an FP64 solve at 0.26M nodes went from 38.7
+// to 43.9 ms, without from 38.7 to 35.1.
+//
+// The waiting blocks take room from the kernel that runs, so from some size on
+// they cost more than the launches they hide.  Measured with and without, one
+// FP32 operator and preconditioner at lx = 8: 28.6 and 45.1 us at 0.26M nodes,
+// 58 and 70 us at 1M; a mixed Poisson solve: 7.6 and 9.5 ms at 2.1M, 12.0 and
+// 14.0 ms at 4.2M; the sequence of Brinkman solves at 8.4M: 43.0 and 41.8 ms;
+// operator and preconditioner at 33M: 696 and 639 us.
+constexpr int64_t kDependentNodes = 6000000;
+__device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void dependent_start() {
+  dependent_wait();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+int launch_dependent(const ntg_plan* p, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                     A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = p->n <= kDependentNodes ? 1 : 0;
+  NTG_CUDA_TRY(cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...));
+  NTG_COUNT_LAUNCH();
+  return NTG_OK;
+}
+
 // launch helpers implemented in the .cu files
 int ax_launch(ntg_plan* p, double* w, const double* u, Scalars* dot_scal, int dot_slot, cudaStream_t s);
 int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int dot_slot, cudaStream_t s);

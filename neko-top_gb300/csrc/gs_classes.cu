@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(kGsThreads)
     k_gs_cls(GsFields<T> F, const int2* __restrict__ g2, int64_t n2, const int4* __restrict__ g4, int64_t n4,
              const int4* __restrict__ g8, int64_t n8, const int32_t* __restrict__ xidx,
              const int32_t* __restrict__ xoff, int64_t nx, int b2, int b4, int b8, const Scalars* sc) {
+  dependent_start();
   if (sc && sc->done) return;
   T* __restrict__ u = F.u[blockIdx.y];
   int blk = blockIdx.x;
@@ -234,35 +235,32 @@ int build_gs_classes(ntg_plan* p) {
 }
 
 template <typename T, int OP>
-static void launch_cls(ntg_plan* p, GsFields<T> u, int nf, cudaStream_t s, const Scalars* sc) {
+static int launch_cls(ntg_plan* p, GsFields<T> u, int nf, cudaStream_t s, const Scalars* sc) {
   const int b2 = (int)((p->ncls[0] + kGsPerBlock - 1) / kGsPerBlock);
   const int b4 = (int)((p->ncls[1] + kGsPerBlock - 1) / kGsPerBlock);
   const int b8 = (int)((p->ncls[2] + kGsPerBlock - 1) / kGsPerBlock);
   int bx = (int)((p->ncls[3] + kGsThreads - 1) / kGsThreads);
   if (bx > num_sms() * 4) bx = num_sms() * 4;
   const int grid = b2 + b4 + b8 + bx;
-  if (grid == 0) return;
-  { k_gs_cls<T, OP><<<dim3(grid, nf), kGsThreads, 0, s>>>(u, p->gs2, p->ncls[0], p->gs4, p->ncls[1], p->gs8, p->ncls[2], p->gsx_idx, p->gsx_off, p->ncls[3], b2, b4, b8, sc); NTG_COUNT_LAUNCH(); }
+  if (grid == 0) return NTG_OK;
+  return launch_dependent(p, k_gs_cls<T, OP>, dim3(grid, nf), kGsThreads, 0, s, u, p->gs2, p->ncls[0], p->gs4,
+                          p->ncls[1], p->gs8, p->ncls[2], p->gsx_idx, p->gsx_off, p->ncls[3], b2, b4, b8, sc);
 }
 
 template <typename T>
 int gs_cls_launch(ntg_plan* p, T* u, int op, cudaStream_t s, const Scalars* sc) {
   const GsFields<T> f{{u, u, u}};
   switch (op) {
-    case NTG_GS_ADD: launch_cls<T, NTG_GS_ADD>(p, f, 1, s, sc); break;
-    case NTG_GS_MUL: launch_cls<T, NTG_GS_MUL>(p, f, 1, s, sc); break;
-    case NTG_GS_MIN: launch_cls<T, NTG_GS_MIN>(p, f, 1, s, sc); break;
-    case NTG_GS_MAX: launch_cls<T, NTG_GS_MAX>(p, f, 1, s, sc); break;
+    case NTG_GS_ADD: return launch_cls<T, NTG_GS_ADD>(p, f, 1, s, sc);
+    case NTG_GS_MUL: return launch_cls<T, NTG_GS_MUL>(p, f, 1, s, sc);
+    case NTG_GS_MIN: return launch_cls<T, NTG_GS_MIN>(p, f, 1, s, sc);
+    case NTG_GS_MAX: return launch_cls<T, NTG_GS_MAX>(p, f, 1, s, sc);
     default: set_error("gs_op: unknown op %d", op); return NTG_ERR_INVALID;
   }
-  NTG_CUDA_TRY(cudaGetLastError());
-  return NTG_OK;
 }
 
 int gs_cls_launch3(ntg_plan* p, double* u0, double* u1, double* u2, cudaStream_t s) {
-  launch_cls<double, NTG_GS_ADD>(p, GsFields<double>{{u0, u1, u2}}, 3, s, nullptr);
-  NTG_CUDA_TRY(cudaGetLastError());
-  return NTG_OK;
+  return launch_cls<double, NTG_GS_ADD>(p, GsFields<double>{{u0, u1, u2}}, 3, s, nullptr);
 }
 
 template int gs_cls_launch<double>(ntg_plan*, double*, int, cudaStream_t, const Scalars*);

@@ -282,6 +282,7 @@ template <typename T>
 __global__ void k_cg_update(T* __restrict__ x, const T* __restrict__ p, T* __restrict__ r, const T* __restrict__ w,
                             const T* __restrict__ dinv, const T* __restrict__ mult, int64_t n,
                             double* __restrict__ part, Scalars* sc) {
+  dependent_start();
   if (sc->done) return;
   const T alpha = (T)sc->alpha;
   // per-thread partials in T: FP64 arithmetic is 1/58 of FP32 on GB300, so
@@ -307,6 +308,7 @@ __global__ void k_cg_update(T* __restrict__ x, const T* __restrict__ p, T* __res
 template <typename T>
 __global__ void k_cg_dir(T* __restrict__ p, const T* __restrict__ r, const T* __restrict__ dinv, int64_t n,
                          const Scalars* sc) {
+  dependent_start();
   if (sc->done) return;
   const T beta = (T)sc->beta;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -358,10 +360,10 @@ static int run_pcg(ntg_plan* pl, Scalars* sc, Scalars* hs_pinned, PcgVecs<T>& v,
         NTG_TRY(gs_add_guarded_f32(pl, (float*)v.w, s, sc));
       }
       timer_start(sizeof(T) == 8 ? TM_UPD64 : TM_UPD32, s);
-      { k_cg_update<T><<<GR, TPB, 0, s>>>(x, v.p, v.r, v.w, dinv, multm, n, pl->red_part, sc); NTG_COUNT_LAUNCH(); }
+      NTG_TRY(launch_dependent(pl, k_cg_update<T>, GR, TPB, 0, s, x, v.p, v.r, v.w, dinv, multm, n, pl->red_part, sc));
       timer_stop(sizeof(T) == 8 ? TM_UPD64 : TM_UPD32, s);
       timer_start(sizeof(T) == 8 ? TM_DIR64 : TM_DIR32, s);
-      { k_cg_dir<T><<<G, TPB, 0, s>>>(v.p, v.r, dinv, n, sc); NTG_COUNT_LAUNCH(); }
+      NTG_TRY(launch_dependent(pl, k_cg_dir<T>, G, TPB, 0, s, v.p, v.r, dinv, n, sc));
       timer_stop(sizeof(T) == 8 ? TM_DIR64 : TM_DIR32, s);
       NTG_CUDA_TRY(cudaGetLastError());
       ++launched;
@@ -625,6 +627,7 @@ struct FinRU {
 __global__ void k_update_rr(float* __restrict__ y, const float* __restrict__ p, float* __restrict__ r,
                             const float* __restrict__ w, const float* __restrict__ mult, int64_t n,
                             double* __restrict__ part, Scalars* sc) {
+  dependent_start();
   if (sc->done) return;
   const float alpha = (float)sc->alpha;
   float rr = 0.f;
@@ -668,6 +671,7 @@ __global__ void __launch_bounds__(256)
     k_update_box(float* __restrict__ y, const float* __restrict__ p, float* __restrict__ r,
                  const float* __restrict__ w, const uint8_t* __restrict__ maskrow, int Ex,
                  int Ey, int Ez, double* __restrict__ part, Scalars* sc) {
+  dependent_start();
   constexpr int N = LX - 1, LX2 = LX * LX, LX3 = LX2 * LX;
   using V = std::conditional_t<LX % 4 == 0, float4, float2>;
   constexpr int NV = LX * 4 / (int)sizeof(V);
@@ -742,6 +746,7 @@ __global__ void __launch_bounds__(256)
 }
 
 __global__ void k_dir_z(float* __restrict__ p, const float* __restrict__ z, int64_t n, int init, const Scalars* sc) {
+  dependent_start();
   if (sc->done) return;
   const float beta = init ? 0.f : (float)sc->beta;
   const int64_t n4 = n >> 2, g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, gs = (int64_t)gridDim.x * blockDim.x;
@@ -1015,7 +1020,7 @@ static int ksp_solve_mixed_ru(ntg_ksp* k, double* x, const double* f, ntg_monito
         NTG_TRY(replace(2));
         y_dirty = false;
         if (hs->done) break;
-        { k_cg_dir<float><<<G, TPB, 0, s>>>(k->v32.p, k->v32.r, p->dinvf, n, k->sc); NTG_COUNT_LAUNCH(); }
+        NTG_TRY(launch_dependent(p, k_cg_dir<float>, G, TPB, 0, s, k->v32.p, k->v32.r, p->dinvf, n, k->sc));
         continue;
       }
       break;
@@ -1030,10 +1035,11 @@ static int ksp_solve_mixed_ru(ntg_ksp* k, double* x, const double* f, ntg_monito
       NTG_TRY(ax_launch_f32(p, k->v32.w, k->v32.p, k->sc, 0, s));
       NTG_TRY(gs_add_guarded_f32(p, k->v32.w, s, k->sc));
       timer_start(TM_UPD32, s);
-      { k_cg_update<float><<<GR, TPB, 0, s>>>(y32, k->v32.p, k->v32.r, k->v32.w, p->dinvf, multm, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+      NTG_TRY(launch_dependent(p, k_cg_update<float>, GR, TPB, 0, s, y32, k->v32.p, k->v32.r, k->v32.w, p->dinvf, multm,
+                               n, p->red_part, k->sc));
       timer_stop(TM_UPD32, s);
       timer_start(TM_DIR32, s);
-      { k_cg_dir<float><<<G, TPB, 0, s>>>(k->v32.p, k->v32.r, p->dinvf, n, k->sc); NTG_COUNT_LAUNCH(); }
+      NTG_TRY(launch_dependent(p, k_cg_dir<float>, G, TPB, 0, s, k->v32.p, k->v32.r, p->dinvf, n, k->sc));
       timer_stop(TM_DIR32, s);
     }
     y_dirty = true;
@@ -1110,7 +1116,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
     NTG_TRY(poll());
     if (hs->done) return NTG_OK;
     NTG_TRY(precondition(mode == 2 ? 0 : 1));
-    if (mode == 2) { k_dir_z<<<G, TPB, 0, s>>>(p32, z32, n, 0, k->sc); NTG_COUNT_LAUNCH(); }
+    if (mode == 2) NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, n, 0, k->sc));
     return poll();
   };
   // structured box (the Schwarz preconditioner's form): the gather-scatter of
@@ -1125,7 +1131,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   const double rr0 = hs->rr0, ff = hs->ff;
   if (!hs->done) {
     NTG_TRY(precondition(3));
-    { k_dir_z<<<G, TPB, 0, s>>>(p32, z32, n, 1, k->sc); NTG_COUNT_LAUNCH(); }
+    NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, n, 1, k->sc));
     NTG_TRY(poll());
   }
   bool y_dirty = false;
@@ -1152,23 +1158,22 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
       if (box_lx) {
         // gather-scatter, mask and update in one pass over the box
         const int GB = grid_red(n / p->lx, TPB);
-        if (box_lx == 8) k_update_box<8><<<GB, TPB, 0, s>>>(y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc);
-        else if (box_lx == 6) k_update_box<6><<<GB, TPB, 0, s>>>(y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc);
-        else k_update_box<4><<<GB, TPB, 0, s>>>(y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc);
-        NTG_COUNT_LAUNCH();
+        auto kern = box_lx == 8 ? k_update_box<8> : box_lx == 6 ? k_update_box<6> : k_update_box<4>;
+        NTG_TRY(launch_dependent(p, kern, GB, TPB, 0, s, y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part,
+                                 k->sc));
       } else {
         timer_stop(TM_UPD32, s);
         NTG_TRY(gs_add_guarded_f32(p, w32, s, k->sc));
         NTG_TRY(mask_guarded_f32(p, w32, s, k->sc));
         timer_start(TM_UPD32, s);
-        { k_update_rr<<<GR, TPB, 0, s>>>(y32, p32, r32, w32, p->multf, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+        NTG_TRY(launch_dependent(p, k_update_rr, GR, TPB, 0, s, y32, p32, r32, w32, p->multf, n, p->red_part, k->sc));
       }
       timer_stop(TM_UPD32, s);
       timer_start(TM_PC32, s);
       NTG_TRY(precondition(0));
       timer_stop(TM_PC32, s);
       timer_start(TM_DIR32, s);
-      { k_dir_z<<<G, TPB, 0, s>>>(p32, z32, n, 0, k->sc); NTG_COUNT_LAUNCH(); }
+      NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, n, 0, k->sc));
       timer_stop(TM_DIR32, s);
     }
     y_dirty = true;

@@ -241,6 +241,7 @@ __global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
   using C = FdmCfg<LX>;
   constexpr int LE = C::LE, LE2 = C::LE2, LE3 = C::LE3, N = LX - 1, RS = C::RS, PS = C::PS, TPE = C::TPE;
   constexpr int EPB = C::EPB, LX2 = LX * LX, LX3 = LX2 * LX, H = LE / 2;
+  dependent_wait();
   if (sc && sc->done) return;
   extern __shared__ __align__(16) float smem[];
   const int nelv = Ex * Ey * Ez;
@@ -599,17 +600,23 @@ __device__ __forceinline__ float crs_vertex(const float* __restrict__ corner, co
 __global__ void __launch_bounds__(kCrsThreads)
     k_crs_fwd(const float* __restrict__ corner, float* __restrict__ out, const float* __restrict__ S0,
               const float* __restrict__ S1, CoarseDims d, const Scalars* sc) {
-  if (sc && sc->done) return;
   extern __shared__ __align__(16) float csm[];
   const CrsPad q(d);
   const int m0 = d.m[0], m1 = d.m[1];
   float *A = csm, *B = A + q.p1 * q.p0, *X = B + q.p1 * q.p0, *Y = X + q.p0 * q.p0;
+  // the matrices are set up long before, and the kernels that set sc->done have
+  // ended before the one ahead of this began: both are read before the wait
+  const bool done = sc && sc->done;
+  if (!done) {
+    crs_stage(X, S0, m0, q.p0);
+    crs_stage(Y, S1, m1, q.p1);
+  }
+  dependent_start();
+  if (done) return;
   for (int t = threadIdx.x; t < q.p1 * q.p0; t += kCrsThreads) {
     const int y = t / q.p0, x = t - y * q.p0;
     A[t] = y < m1 && x < m0 ? crs_vertex(corner, d, x, y, blockIdx.x) : 0.f;
   }
-  crs_stage(X, S0, m0, q.p0);
-  crs_stage(Y, S1, m1, q.p1);
   __syncthreads();
   crs_rows(A, X, m1, m0, q.p0, B);
   __syncthreads();
@@ -622,18 +629,22 @@ __global__ void __launch_bounds__(kCrsThreads)
 __global__ void __launch_bounds__(kCrsThreads)
     k_crs_z(float* __restrict__ io, const float* __restrict__ S2, const float* __restrict__ lam, CoarseDims d,
             const Scalars* sc) {
-  if (sc && sc->done) return;
   extern __shared__ __align__(16) float csm[];
   const CrsPad q(d);
   const int m0 = d.m[0], m1 = d.m[1], m2 = d.m[2], n = m0 * m1;
   float *A = csm, *B = A + q.p2 * kCrsCols, *Z = B + q.p2 * kCrsCols, *ZT = Z + q.p2 * q.p2;
+  const bool done = sc && sc->done;
+  if (!done) {
+    crs_stage(Z, S2, m2, q.p2);
+    crs_stage(ZT, S2 + (int64_t)m2 * m2, m2, q.p2);
+  }
+  dependent_start();
+  if (done) return;
   const int c0 = blockIdx.x * kCrsCols, cols = min(kCrsCols, n - c0);
   for (int t = threadIdx.x; t < m2 * kCrsCols; t += kCrsThreads) {
     const int z = t / kCrsCols, c = t - z * kCrsCols;
     A[t] = c < cols ? io[(int64_t)z * n + c0 + c] : 0.f;
   }
-  crs_stage(Z, S2, m2, q.p2);
-  crs_stage(ZT, S2 + (int64_t)m2 * m2, m2, q.p2);
   __syncthreads();
   crs_cols(A, Z, m2, q.p2, kCrsCols, kCrsCols, [&](int f, int c, float v) {
     const int x = (c0 + c) % m0, y = (c0 + c) / m0;
@@ -654,19 +665,23 @@ __global__ void __launch_bounds__(kCrsThreads)
 __global__ void __launch_bounds__(kCrsThreads)
     k_crs_back(const float* __restrict__ in, float* __restrict__ uc, const float* __restrict__ S0,
                const float* __restrict__ S1, CoarseDims d, const Scalars* sc) {
-  if (sc && sc->done) return;
   extern __shared__ __align__(16) float csm[];
   const CrsPad q(d);
   const int m0 = d.m[0], m1 = d.m[1];
   float *A = csm, *B = A + q.p1 * q.p0, *X = B + q.p1 * q.p0, *Y = X + q.p0 * q.p0;
+  const bool done = sc && sc->done;
+  if (!done) {
+    crs_stage(X, S0 + (int64_t)m0 * m0, m0, q.p0);
+    crs_stage(Y, S1 + (int64_t)m1 * m1, m1, q.p1);
+  }
+  dependent_start();
+  if (done) return;
   const float* src = in + (int64_t)blockIdx.x * m0 * m1;
   for (int t = threadIdx.x; t < q.p1 * q.p0; t += kCrsThreads) {
     const int y = t / q.p0, x = t - y * q.p0;
     A[t] = y < m1 && x < m0 ? src[y * m0 + x] : 0.f;
     B[t] = 0.f;
   }
-  crs_stage(X, S0 + (int64_t)m0 * m0, m0, q.p0);
-  crs_stage(Y, S1 + (int64_t)m1 * m1, m1, q.p1);
   __syncthreads();
   crs_cols(A, Y, m1, q.p1, m0, q.p0, [&](int y, int c, float v) { B[y * q.p0 + c] = v; });
   __syncthreads();
@@ -721,6 +736,7 @@ __global__ void __launch_bounds__(256, 4)
            double* __restrict__ part, Scalars* sc, CoarseView cv) {
   constexpr int N = LX - 1, LE = LX + 2, LE2 = LE * LE, LE3 = LE2 * LE, LX2 = LX * LX;
   static_assert(N >= 3 && LE % 2 == 0, "one neighbour per direction; rows of float2 pairs");
+  dependent_start();
   if (sc && sc->done) return;
   __shared__ float sp[2][LX];
   if (threadIdx.x == 0) {
@@ -1188,11 +1204,9 @@ int fdm_launch(ntg_schwarz* w, const float* r, cudaStream_t s, const Scalars* sc
   }
   float* corner = w->coarse_ready ? w->corner : nullptr;
   const bool g = w->gen != nullptr;
-  fdm_kernel<LX>(w, w->fdm_eo)<<<(unsigned)((w->plan->nelv + C::EPB - 1) / C::EPB), C::THREADS, C::SMEM, s>>>(
-      r, w->ze, w->esc, g ? (int)w->plan->nelv : w->Ex, g ? 1 : w->Ey, g ? 1 : w->Ez, sc, corner, w->ph,
-      g ? w->gen->ghost : nullptr, g ? w->plan->multf : nullptr, R);
-  NTG_COUNT_LAUNCH();
-  return NTG_OK;
+  const unsigned grid = (unsigned)((w->plan->nelv + C::EPB - 1) / C::EPB);
+  return launch_dependent(w->plan, fdm_kernel<LX>(w, w->fdm_eo), grid, C::THREADS, C::SMEM, s, r, w->ze, w->esc, g ? (int)w->plan->nelv : w->Ex, g ? 1 : w->Ey, g ? 1 : w->Ez,
+                          sc, corner, w->ph, g ? w->gen->ghost : nullptr, g ? w->plan->multf : nullptr, R);
 }
 
 }  // namespace sw
@@ -1210,11 +1224,10 @@ int pull_launch(ntg_schwarz* w, float* z, const float* r, cudaStream_t s, Scalar
   const int64_t rows = p->n / LX;
   const CoarseView cv{w->coarse_ready ? w->uc : nullptr, w->ph, w->dw};
   if (dot)
-    k_pull<LX, true><<<grid_red(rows, 256), 256, 0, s>>>(w->ze, z, w->Ex, w->Ey, w->Ez, r, mask, mode, part, sc, cv);
-  else
-    k_pull<LX, false><<<grid_for(rows, 256), 256, 0, s>>>(w->ze, z, w->Ex, w->Ey, w->Ez, r, mask, 0, nullptr, sc, cv);
-  NTG_COUNT_LAUNCH();
-  return NTG_OK;
+    return launch_dependent(p, k_pull<LX, true>, grid_red(rows, 256), 256, 0, s, w->ze, z, w->Ex, w->Ey, w->Ez, r, mask,
+                            mode, part, sc, cv);
+  return launch_dependent(p, k_pull<LX, false>, grid_for(rows, 256), 256, 0, s, w->ze, z, w->Ex, w->Ey, w->Ez, r, mask, 0,
+                          nullptr, sc, cv);
 }
 
 // coarse solve (after the FDM kernel has written the corner sums): the
@@ -1230,12 +1243,10 @@ inline int coarse_launch(ntg_schwarz* w, cudaStream_t s, const Scalars* sc) {
     NTG_TRY(fx::use_smem<k_crs_fwd>(kCrsSmem));
     NTG_TRY(fx::use_smem<k_crs_z>(kCrsSmem));
     NTG_TRY(fx::use_smem<k_crs_back>(kCrsSmem));
-    k_crs_fwd<<<d.m[2], kCrsThreads, q.plane(), s>>>(w->corner, a, w->cS[0], w->cS[1], d, sc);
-    NTG_COUNT_LAUNCH();
-    k_crs_z<<<(d.m[0] * d.m[1] + kCrsCols - 1) / kCrsCols, kCrsThreads, q.column(), s>>>(a, w->cS[2], w->clam, d, sc);
-    NTG_COUNT_LAUNCH();
-    k_crs_back<<<d.m[2], kCrsThreads, q.plane(), s>>>(a, w->uc, w->cS[0], w->cS[1], d, sc);
-    NTG_COUNT_LAUNCH();
+    NTG_TRY(launch_dependent(w->plan, k_crs_fwd, d.m[2], kCrsThreads, q.plane(), s, w->corner, a, w->cS[0], w->cS[1], d, sc));
+    NTG_TRY(launch_dependent(w->plan, k_crs_z, (d.m[0] * d.m[1] + kCrsCols - 1) / kCrsCols, kCrsThreads, q.column(), s, a,
+                             w->cS[2], w->clam, d, sc));
+    NTG_TRY(launch_dependent(w->plan, k_crs_back, d.m[2], kCrsThreads, q.plane(), s, a, w->uc, w->cS[0], w->cS[1], d, sc));
     return NTG_OK;
   }
   k_crs_restrict<<<g, 256, 0, s>>>(w->corner, a, d, sc);
