@@ -84,7 +84,7 @@ struct Scalars {
   int ru_mode;     // 1 = FP32 iteration with FP64 reliable updates
   int need_ru;     // 1 = residual replacement due, 2 = FP32 residual converged (confirm in FP64)
   int ext_pc;      // 1 = preconditioner applied by separate kernels: (r, z) and beta come from k_rz
-  int pad2;
+  int y_due;       // the last update's y += alpha p is still to be done (k_dir_z or k_ru_accum)
   int iter;        // iterations performed
   int done;        // 1 = converged or stopped: later kernels are no-ops
   int status;      // NTG_OK / NTG_MAXITER / NTG_BREAKDOWN / NTG_NONFINITE

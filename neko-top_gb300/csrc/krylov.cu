@@ -236,6 +236,7 @@ struct FinUpd {
   __device__ void operator()(const double* acc, Scalars* sc) const {
     // acc: rz_new, rr
     sc->iter += 1;
+    sc->y_due = 1;
     sc->rr = acc[1];
     if (!isfinite(acc[0]) || !isfinite(acc[1])) {
       sc->status = NTG_NONFINITE;
@@ -579,10 +580,15 @@ __global__ void k_ru_init(const double* __restrict__ f, const double* __restrict
   grid_reduce<3>(v, part, sc, FinRUInit());
 }
 
-// x += (double) y; y = 0
-__global__ void k_ru_accum(double* __restrict__ x, float* __restrict__ y, int64_t n) {
+// x += (double) y; y = 0.  p: the last update's y += alpha p is still to be
+// done, and comes first; null: it is not.
+__global__ void k_ru_accum(double* __restrict__ x, float* __restrict__ y, const float* __restrict__ p, int64_t n,
+                           const Scalars* sc) {
+  const float alpha = p ? (float)sc->alpha : 0.f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    x[i] += (double)y[i];
+    float yi = y[i];
+    if (p) yi += alpha * p[i];
+    x[i] += (double)yi;
     y[i] = 0.f;
   }
 }
@@ -621,30 +627,26 @@ struct FinRU {
 // ---------------------------------------------------------------------------
 // Explicit-preconditioner variant of the FP32 iteration (Schwarz): the
 // update forms only (r, r); z = M r is applied by its own kernels, the last
-// of which also forms (r, z) and beta; k_dir_z sets p = z + beta p.
-// Both stream float4s (a scalar tail covers n % 4).
+// of which also forms (r, z) and beta; k_dir_z sets y += alpha p, p = z + beta p
+// (p is in registers there, so the update need not read it).  When the
+// iteration stops between the two, Scalars::y_due says so and k_ru_accum adds
+// the last alpha p.  All stream float4s (a scalar tail covers n % 4).
 // ---------------------------------------------------------------------------
-__global__ void k_update_rr(float* __restrict__ y, const float* __restrict__ p, float* __restrict__ r,
-                            const float* __restrict__ w, const float* __restrict__ mult, int64_t n,
-                            double* __restrict__ part, Scalars* sc) {
+__global__ void k_update_rr(float* __restrict__ r, const float* __restrict__ w, const float* __restrict__ mult,
+                            int64_t n, double* __restrict__ part, Scalars* sc) {
   dependent_start();
   if (sc->done) return;
   const float alpha = (float)sc->alpha;
   float rr = 0.f;
   const int64_t n4 = n >> 2, g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, gs = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = g0; i < n4; i += gs) {
-    float4 y4 = reinterpret_cast<float4*>(y)[i];
-    const float4 p4 = reinterpret_cast<const float4*>(p)[i], w4 = reinterpret_cast<const float4*>(w)[i];
-    const float4 m4 = reinterpret_cast<const float4*>(mult)[i];
+    const float4 w4 = reinterpret_cast<const float4*>(w)[i], m4 = reinterpret_cast<const float4*>(mult)[i];
     float4 r4 = reinterpret_cast<float4*>(r)[i];
-    y4.x += alpha * p4.x; y4.y += alpha * p4.y; y4.z += alpha * p4.z; y4.w += alpha * p4.w;
     r4.x -= alpha * w4.x; r4.y -= alpha * w4.y; r4.z -= alpha * w4.z; r4.w -= alpha * w4.w;
-    reinterpret_cast<float4*>(y)[i] = y4;
     reinterpret_cast<float4*>(r)[i] = r4;
     rr += m4.x * r4.x * r4.x + m4.y * r4.y * r4.y + m4.z * r4.z * r4.z + m4.w * r4.w * r4.w;
   }
   for (int64_t i = 4 * n4 + g0; i < n; i += gs) {
-    y[i] += alpha * p[i];
     const float ri = r[i] - alpha * w[i];
     r[i] = ri;
     rr += mult[i] * ri * ri;
@@ -660,16 +662,16 @@ __global__ void k_update_rr(float* __restrict__ y, const float* __restrict__ p, 
 // in y and z, and the x neighbours' end values -- in ascending element
 // order (z-major, y, x), the order of the gather-scatter's groups, so every
 // copy of a node receives the same sum.  Then w is masked (one mask byte per
-// row) and y += alpha p, r -= alpha w; (r, r)_mult is summed over each
-// node's owning copy (no lower neighbour in any direction), which the
-// mult-weighted sum over copies equals, with no multiplicity stream.
-// HBM and the bytes in flight bound it (80 us at 32^3 elements, lx = 8,
-// 24 B per node): a whole row per thread, its loads first; half a row per
-// thread, with contiguous lanes, took 84.
+// row) and r -= alpha w; (r, r)_mult is summed over each node's owning copy
+// (no lower neighbour in any direction), which the mult-weighted sum over
+// copies equals, with no multiplicity stream.
+// HBM and the bytes in flight bound it: a whole row per thread, its loads
+// first, four blocks per SM (six take spills: +6% of a solve).  Half a row per
+// thread, with contiguous lanes, was slower.  With y += alpha p in this pass
+// the two kernels read p twice: a solve at 43M nodes took 98.5 ms, now 95.2.
 template <int LX>
-__global__ void __launch_bounds__(256)
-    k_update_box(float* __restrict__ y, const float* __restrict__ p, float* __restrict__ r,
-                 const float* __restrict__ w, const uint8_t* __restrict__ maskrow, int Ex,
+__global__ void __launch_bounds__(256, 4)
+    k_update_box(float* __restrict__ r, const float* __restrict__ w, const uint8_t* __restrict__ maskrow, int Ex,
                  int Ey, int Ez, double* __restrict__ part, Scalars* sc) {
   dependent_start();
   constexpr int N = LX - 1, LX2 = LX * LX, LX3 = LX2 * LX;
@@ -696,9 +698,7 @@ __global__ void __launch_bounds__(256)
     const int e = (int)(t / LX2);
     const int m = (int)(t - (int64_t)e * LX2), j = m % LX, k = m / LX;
     const int64_t o = t * LX;
-    Row pv, yv, rv;
-    load(p + o, pv);
-    load(y + o, yv);
+    Row rv;
     load(r + o, rv);
     const unsigned mb = maskrow[t];
     const int exy = e / Ex, cx = e - exy * Ex, cz = exy / Ey, cy = exy - cz * Ey;
@@ -729,11 +729,7 @@ __global__ void __launch_bounds__(256)
       }
     }
 #pragma unroll
-    for (int i = 0; i < LX; ++i) {
-      yv.f[i] += alpha * pv.f[i];
-      rv.f[i] -= alpha * (((mb >> i) & 1u) ? 0.f : acc[i]);
-    }
-    store(y + o, yv);
+    for (int i = 0; i < LX; ++i) rv.f[i] -= alpha * (((mb >> i) & 1u) ? 0.f : acc[i]);
     store(r + o, rv);
     if ((j > 0 || cy == 0) && (k > 0 || cz == 0)) {
 #pragma unroll
@@ -745,19 +741,31 @@ __global__ void __launch_bounds__(256)
   grid_reduce<2>(v, part, sc, FinUpd());
 }
 
-__global__ void k_dir_z(float* __restrict__ p, const float* __restrict__ z, int64_t n, int init, const Scalars* sc) {
+// y += alpha p (y null: not due), p = z + beta p (init: p = z).  HBM bound:
+// 20 B per node.
+__global__ void k_dir_z(float* __restrict__ p, const float* __restrict__ z, float* __restrict__ y, int64_t n, int init,
+                        const Scalars* sc) {
   dependent_start();
   if (sc->done) return;
-  const float beta = init ? 0.f : (float)sc->beta;
+  const float beta = init ? 0.f : (float)sc->beta, alpha = y ? (float)sc->alpha : 0.f;
   const int64_t n4 = n >> 2, g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, gs = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = g0; i < n4; i += gs) {
     const float4 z4 = reinterpret_cast<const float4*>(z)[i];
     float4 p4 = init ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(p)[i];
+    if (y) {
+      float4 y4 = reinterpret_cast<float4*>(y)[i];
+      y4.x += alpha * p4.x; y4.y += alpha * p4.y; y4.z += alpha * p4.z; y4.w += alpha * p4.w;
+      reinterpret_cast<float4*>(y)[i] = y4;
+    }
     p4.x = z4.x + beta * p4.x; p4.y = z4.y + beta * p4.y; p4.z = z4.z + beta * p4.z; p4.w = z4.w + beta * p4.w;
     reinterpret_cast<float4*>(p)[i] = p4;
   }
-  for (int64_t i = 4 * n4 + g0; i < n; i += gs) p[i] = init ? z[i] : z[i] + beta * p[i];
+  for (int64_t i = 4 * n4 + g0; i < n; i += gs) {
+    if (y) y[i] += alpha * p[i];
+    p[i] = init ? z[i] : z[i] + beta * p[i];
+  }
 }
+
 // start: r = f - w (w null: f); r32 = (float) r; y = 0; sums ff, rr
 __global__ void k_ru_init_pc(const double* __restrict__ f, const double* __restrict__ w, const double* __restrict__ mult,
                              double* __restrict__ r, float* __restrict__ r32, float* __restrict__ y32, int64_t n,
@@ -1000,7 +1008,7 @@ static int ksp_solve_mixed_ru(ntg_ksp* k, double* x, const double* f, ntg_monito
     return NTG_OK;
   };
   auto replace = [&](int mode) -> int {
-    { k_ru_accum<<<G, TPB, 0, s>>>(x, y32, n); NTG_COUNT_LAUNCH(); }
+    { k_ru_accum<<<G, TPB, 0, s>>>(x, y32, nullptr, n, k->sc); NTG_COUNT_LAUNCH(); }
     NTG_TRY(op_apply(p, k->v64.w, x, s));
     fpax++;
     nru++;
@@ -1106,8 +1114,14 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   auto precondition = [&](int mode) -> int {
     return schwarz_apply(k->sw, z32, r32, s, k->sc, p->multf, p->red_part, mode);
   };
+  // x += y, after a poll: stopped (done) behind an update, its alpha p is still due
+  auto accumulate = [&]() -> int {
+    k_ru_accum<<<G, TPB, 0, s>>>(x, y32, hs->done && hs->y_due ? p32 : nullptr, n, k->sc);
+    NTG_COUNT_LAUNCH();
+    return NTG_OK;
+  };
   auto replace = [&](int mode) -> int {
-    { k_ru_accum<<<G, TPB, 0, s>>>(x, y32, n); NTG_COUNT_LAUNCH(); }
+    NTG_TRY(accumulate());
     NTG_TRY(op_apply(p, k->v64.w, x, s));
     fpax++;
     nru++;
@@ -1116,7 +1130,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
     NTG_TRY(poll());
     if (hs->done) return NTG_OK;
     NTG_TRY(precondition(mode == 2 ? 0 : 1));
-    if (mode == 2) NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, n, 0, k->sc));
+    if (mode == 2) NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, nullptr, n, 0, k->sc));
     return poll();
   };
   // structured box (the Schwarz preconditioner's form): the gather-scatter of
@@ -1131,7 +1145,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   const double rr0 = hs->rr0, ff = hs->ff;
   if (!hs->done) {
     NTG_TRY(precondition(3));
-    NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, n, 1, k->sc));
+    NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, nullptr, n, 1, k->sc));
     NTG_TRY(poll());
   }
   bool y_dirty = false;
@@ -1159,21 +1173,20 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
         // gather-scatter, mask and update in one pass over the box
         const int GB = grid_red(n / p->lx, TPB);
         auto kern = box_lx == 8 ? k_update_box<8> : box_lx == 6 ? k_update_box<6> : k_update_box<4>;
-        NTG_TRY(launch_dependent(p, kern, GB, TPB, 0, s, y32, p32, r32, w32, p->maskrow, bx, by, bz, p->red_part,
-                                 k->sc));
+        NTG_TRY(launch_dependent(p, kern, GB, TPB, 0, s, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc));
       } else {
         timer_stop(TM_UPD32, s);
         NTG_TRY(gs_add_guarded_f32(p, w32, s, k->sc));
         NTG_TRY(mask_guarded_f32(p, w32, s, k->sc));
         timer_start(TM_UPD32, s);
-        NTG_TRY(launch_dependent(p, k_update_rr, GR, TPB, 0, s, y32, p32, r32, w32, p->multf, n, p->red_part, k->sc));
+        NTG_TRY(launch_dependent(p, k_update_rr, GR, TPB, 0, s, r32, w32, p->multf, n, p->red_part, k->sc));
       }
       timer_stop(TM_UPD32, s);
       timer_start(TM_PC32, s);
       NTG_TRY(precondition(0));
       timer_stop(TM_PC32, s);
       timer_start(TM_DIR32, s);
-      NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, n, 0, k->sc));
+      NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, y32, n, 0, k->sc));
       timer_stop(TM_DIR32, s);
     }
     y_dirty = true;
@@ -1183,7 +1196,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   double rr_final = hs->rr;
   if (y_dirty) {
     const int iters = hs->iter;
-    { k_ru_accum<<<G, TPB, 0, s>>>(x, y32, n); NTG_COUNT_LAUNCH(); }
+    NTG_TRY(accumulate());
     NTG_TRY(op_apply(p, k->v64.w, x, s));
     fpax++;
     { k_resid<<<GR, TPB, 0, s>>>(f, k->v64.w, p->mult, k->v64.r, n, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
