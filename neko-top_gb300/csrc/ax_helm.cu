@@ -35,16 +35,17 @@ struct AxShape {
   static constexpr int NT = (NW + 31) / 32 * 32;   // launched threads
 };
 
-template <typename T, int LX, bool H1ARR, bool H2, bool DOT>
+template <typename T, int LX, bool H1ARR, bool H2, bool DOT, bool DIR = false>
 __global__ void __launch_bounds__(AxShape<T, LX>::NT)
     k_ax_helm(T* __restrict__ w, const T* __restrict__ u, const T* __restrict__ g11, const T* __restrict__ g12,
               const T* __restrict__ g13, const T* __restrict__ g22, const T* __restrict__ g23,
               const T* __restrict__ g33, const T* __restrict__ h1, T h1c, const T* __restrict__ hB, int64_t nelv,
-              const __grid_constant__ DParam<T, LX> Dp, double* __restrict__ part, Scalars* sc) {
+              const __grid_constant__ DParam<T, LX> Dp, double* __restrict__ part, Scalars* sc, AxDir dir) {
   using S = AxShape<T, LX>;
   constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
   dependent_start();
   if (DOT && sc->done) return;
+  const T alpha = DIR ? (T)sc->alpha : T(0), beta = DIR ? (T)sc->beta : T(0);
   __shared__ T s_u[EPB][LX3];
   __shared__ T s_r[EPB][LX3];
   __shared__ T s_s[EPB][LX3];
@@ -70,11 +71,17 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
     // every stream's loads first: the bytes in flight bound this kernel.  With
     // the metric loads between the contractions the operator, gather-scatter and
     // preconditioner of 4641 elements of lx = 6 took 89 us, so 81
-    T ureg[LX], G[6][LX], hh[LX];
+    T ureg[LX], G[6][LX], hh[LX], zv[LX], yv[LX];
 #pragma unroll
     for (int k = 0; k < LX; ++k) {
       const int64_t q = base + k * LX2;
-      ureg[k] = active ? u[q] : T(0);
+      if constexpr (DIR) {
+        ureg[k] = active && dir.mode != 1 ? dir.p[q] : T(0);
+        zv[k] = active ? dir.z[q] : T(0);
+        yv[k] = active && dir.mode == 0 ? dir.y[q] : T(0);
+      } else {
+        ureg[k] = active ? u[q] : T(0);
+      }
       G[0][k] = active ? g11[q] : T(0);
       G[1][k] = active ? g12[q] : T(0);
       G[2][k] = active ? g13[q] : T(0);
@@ -82,6 +89,15 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
       G[4][k] = active ? g23[q] : T(0);
       G[5][k] = active ? g33[q] : T(0);
       if (H1ARR) hh[k] = active ? h1[q] : T(0);
+    }
+    if constexpr (DIR) {
+#pragma unroll
+      for (int k = 0; k < LX; ++k) {
+        const int64_t q = base + k * LX2;
+        if (active && dir.mode == 0) dir.y[q] = yv[k] + alpha * ureg[k];
+        ureg[k] = zv[k] + beta * ureg[k];
+        if (active) dir.p[q] = ureg[k];
+      }
     }
 #pragma unroll
     for (int k = 0; k < LX; ++k)
@@ -136,11 +152,11 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
 // TMA-pipelined FP32 kernel for lx = 8 (ax_helm_f32_tma.cu); returns
 // NTG_ERR_UNSUPPORTED when a pointer is not 16-byte aligned.
 int ax_f32_tma_launch(ntg_plan* p, float* w, const float* u, const float* const* g, const float* h1, float h1c,
-                      const float* hB, Scalars* sc, cudaStream_t s);
+                      const float* hB, Scalars* sc, const AxDir* dir, cudaStream_t s);
 
 template <typename T, int LX>
 static int launch_lx(ntg_plan* p, T* w, const T* u, const T* const* g, const T* h1, T h1c, const T* hB,
-                     Scalars* sc, cudaStream_t s) {
+                     Scalars* sc, const AxDir* dir, cudaStream_t s) {
   constexpr int EPB = AxShape<T, LX>::EPB;
   constexpr int NT = AxShape<T, LX>::NT;
   DParam<T, LX> Dp;
@@ -149,19 +165,32 @@ static int launch_lx(ntg_plan* p, T* w, const T* u, const T* const* g, const T* 
   int64_t cap = sc ? kRedSlots : (int64_t)num_sms() * 32;
   int grid = (int)(ngroups < cap ? ngroups : cap);
   const bool h1arr = h1 != nullptr, h2 = hB != nullptr;
-#define NTG_AX_CASE(H1A, HH2, DT)                                                                              \
-  if (h1arr == H1A && h2 == HH2 && (sc != nullptr) == DT) {                                                 \
-    NTG_TRY((launch_dependent(p, k_ax_helm<T, LX, H1A, HH2, DT>, grid, NT, 0, s, w, u, g[0], g[1], g[2], g[3], \
-                              g[4], g[5], h1, h1c, hB, p->nelv, Dp, p->red_part, sc)));                    \
+  const AxDir d = dir ? *dir : AxDir{};
+#define NTG_AX_CASE(H1A, HH2, DT, DR)                                                                              \
+  if (h1arr == H1A && h2 == HH2 && (sc != nullptr) == DT) {                                                     \
+    NTG_TRY((launch_dependent(p, k_ax_helm<T, LX, H1A, HH2, DT, DR>, grid, NT, 0, s, w, u, g[0], g[1], g[2],    \
+                              g[3], g[4], g[5], h1, h1c, hB, p->nelv, Dp, p->red_part, sc, d)));               \
   }
-  NTG_AX_CASE(false, false, false)
-  NTG_AX_CASE(false, true, false)
-  NTG_AX_CASE(true, false, false)
-  NTG_AX_CASE(true, true, false)
-  NTG_AX_CASE(false, false, true)
-  NTG_AX_CASE(false, true, true)
-  NTG_AX_CASE(true, false, true)
-  NTG_AX_CASE(true, true, true)
+  if (dir) {
+    // the orders of the Schwarz preconditioner
+    if constexpr (LX == 4 || LX == 6 || LX == 8) {
+      NTG_AX_CASE(false, false, true, true)
+      NTG_AX_CASE(false, true, true, true)
+      NTG_AX_CASE(true, false, true, true)
+      NTG_AX_CASE(true, true, true, true)
+      return NTG_OK;
+    }
+    set_error("ax_helm: no direction update at lx=%d", LX);
+    return NTG_ERR_UNSUPPORTED;
+  }
+  NTG_AX_CASE(false, false, false, false)
+  NTG_AX_CASE(false, true, false, false)
+  NTG_AX_CASE(true, false, false, false)
+  NTG_AX_CASE(true, true, false, false)
+  NTG_AX_CASE(false, false, true, false)
+  NTG_AX_CASE(false, true, true, false)
+  NTG_AX_CASE(true, false, true, false)
+  NTG_AX_CASE(true, true, true, false)
 #undef NTG_AX_CASE
   NTG_CUDA_TRY(cudaGetLastError());
   return NTG_OK;
@@ -169,30 +198,30 @@ static int launch_lx(ntg_plan* p, T* w, const T* u, const T* const* g, const T* 
 
 template <typename T>
 static int ax_dispatch(ntg_plan* p, T* w, const T* u, const T* const* g, const T* h1, T h1c, const T* hB,
-                       Scalars* sc, cudaStream_t s) {
+                       Scalars* sc, const AxDir* dir, cudaStream_t s) {
   switch (p->lx) {
-    case 2: return launch_lx<T, 2>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 3: return launch_lx<T, 3>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 4: return launch_lx<T, 4>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 5: return launch_lx<T, 5>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 6: return launch_lx<T, 6>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 7: return launch_lx<T, 7>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 8: return launch_lx<T, 8>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 9: return launch_lx<T, 9>(p, w, u, g, h1, h1c, hB, sc, s);
-    case 10: return launch_lx<T, 10>(p, w, u, g, h1, h1c, hB, sc, s);
+    case 2: return launch_lx<T, 2>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 3: return launch_lx<T, 3>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 4: return launch_lx<T, 4>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 5: return launch_lx<T, 5>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 6: return launch_lx<T, 6>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 7: return launch_lx<T, 7>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 8: return launch_lx<T, 8>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 9: return launch_lx<T, 9>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 10: return launch_lx<T, 10>(p, w, u, g, h1, h1c, hB, sc, dir, s);
     default: set_error("ax_helm: lx=%d not compiled", p->lx); return NTG_ERR_UNSUPPORTED;
   }
 }
 
-int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int, cudaStream_t s) {
+int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int, cudaStream_t s, const AxDir* dir) {
   NTG_TRY(ensure_fp32(p));
   const float* g[6] = {p->gf[0], p->gf[1], p->gf[2], p->gf[3], p->gf[4], p->gf[5]};
   timer_start(TM_AX32, s);
   const float* h1 = p->h1_const ? nullptr : p->h1f;
   const float* hB = p->ifh2 ? p->hBf : nullptr;
   int st = NTG_ERR_UNSUPPORTED;
-  if (p->lx == 8 && p->use_tma) st = ax_f32_tma_launch(p, w, u, g, h1, (float)p->h1c, hB, dot_scal, s);
-  if (st == NTG_ERR_UNSUPPORTED) st = ax_dispatch<float>(p, w, u, g, h1, (float)p->h1c, hB, dot_scal, s);
+  if (p->lx == 8 && p->use_tma) st = ax_f32_tma_launch(p, w, u, g, h1, (float)p->h1c, hB, dot_scal, dir, s);
+  if (st == NTG_ERR_UNSUPPORTED) st = ax_dispatch<float>(p, w, u, g, h1, (float)p->h1c, hB, dot_scal, dir, s);
   timer_stop(TM_AX32, s);
   return st;
 }

@@ -84,7 +84,7 @@ struct Scalars {
   int ru_mode;     // 1 = FP32 iteration with FP64 reliable updates
   int need_ru;     // 1 = residual replacement due, 2 = FP32 residual converged (confirm in FP64)
   int ext_pc;      // 1 = preconditioner applied by separate kernels: (r, z) and beta come from k_rz
-  int y_due;       // the last update's y += alpha p is still to be done (k_dir_z or k_ru_accum)
+  int y_due;       // the last update's y += alpha p is still to be done (AxDir or k_ru_accum)
   int iter;        // iterations performed
   int done;        // 1 = converged or stopped: later kernels are no-ops
   int status;      // NTG_OK / NTG_MAXITER / NTG_BREAKDOWN / NTG_NONFINITE
@@ -230,7 +230,17 @@ int launch_dependent(const ntg_plan* p, void (*kernel)(P...), dim3 grid, dim3 bl
 
 // launch helpers implemented in the .cu files
 int ax_launch(ntg_plan* p, double* w, const double* u, Scalars* dot_scal, int dot_slot, cudaStream_t s);
-int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int dot_slot, cudaStream_t s);
+// The direction update of the Schwarz-preconditioned CG, done by the operator
+// that reads the direction: y += alpha p (the update that the iteration before
+// left), p = z + beta p, then w = A p.  lx 4, 6, 8 with a dot product.
+struct AxDir {
+  float* p;
+  const float* z;
+  float* y;
+  int mode;  // 0 the above; 1 start: p = z; 2 after a replacement: y is up to date
+};
+int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int dot_slot, cudaStream_t s,
+                  const AxDir* dir = nullptr);
 int gs_launch(ntg_plan* p, double* u, int op, cudaStream_t s);
 int gs_launch_f32(ntg_plan* p, float* u, int op, cudaStream_t s);
 int gs_launch3(ntg_plan* p, double* u0, double* u1, double* u2, cudaStream_t s);

@@ -627,10 +627,10 @@ struct FinRU {
 // ---------------------------------------------------------------------------
 // Explicit-preconditioner variant of the FP32 iteration (Schwarz): the
 // update forms only (r, r); z = M r is applied by its own kernels, the last
-// of which also forms (r, z) and beta; k_dir_z sets y += alpha p, p = z + beta p
-// (p is in registers there, so the update need not read it).  When the
-// iteration stops between the two, Scalars::y_due says so and k_ru_accum adds
-// the last alpha p.  All stream float4s (a scalar tail covers n % 4).
+// of which also forms (r, z) and beta.  The next product then sets
+// y += alpha p, p = z + beta p before it reads p (AxDir); when the iteration
+// stops ahead of that, Scalars::y_due says so and k_ru_accum adds the last
+// alpha p.  float4 streams (a scalar tail covers n % 4).
 // ---------------------------------------------------------------------------
 __global__ void k_update_rr(float* __restrict__ r, const float* __restrict__ w, const float* __restrict__ mult,
                             int64_t n, double* __restrict__ part, Scalars* sc) {
@@ -667,8 +667,9 @@ __global__ void k_update_rr(float* __restrict__ r, const float* __restrict__ w, 
 // copies equals, with no multiplicity stream.
 // HBM and the bytes in flight bound it: a whole row per thread, its loads
 // first, four blocks per SM (six take spills: +6% of a solve).  Half a row per
-// thread, with contiguous lanes, was slower.  With y += alpha p in this pass
-// the two kernels read p twice: a solve at 43M nodes took 98.5 ms, now 95.2.
+// thread, with contiguous lanes, was slower.  y += alpha p here and again
+// reading p for the next direction cost a solve at 43M nodes 98.5 ms against
+// 95.2 with y in the direction update (AxDir).
 template <int LX>
 __global__ void __launch_bounds__(256, 4)
     k_update_box(float* __restrict__ r, const float* __restrict__ w, const uint8_t* __restrict__ maskrow, int Ex,
@@ -739,31 +740,6 @@ __global__ void __launch_bounds__(256, 4)
   }
   double v[2] = {0.0, (double)rr};
   grid_reduce<2>(v, part, sc, FinUpd());
-}
-
-// y += alpha p (y null: not due), p = z + beta p (init: p = z).  HBM bound:
-// 20 B per node.
-__global__ void k_dir_z(float* __restrict__ p, const float* __restrict__ z, float* __restrict__ y, int64_t n, int init,
-                        const Scalars* sc) {
-  dependent_start();
-  if (sc->done) return;
-  const float beta = init ? 0.f : (float)sc->beta, alpha = y ? (float)sc->alpha : 0.f;
-  const int64_t n4 = n >> 2, g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, gs = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = g0; i < n4; i += gs) {
-    const float4 z4 = reinterpret_cast<const float4*>(z)[i];
-    float4 p4 = init ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(p)[i];
-    if (y) {
-      float4 y4 = reinterpret_cast<float4*>(y)[i];
-      y4.x += alpha * p4.x; y4.y += alpha * p4.y; y4.z += alpha * p4.z; y4.w += alpha * p4.w;
-      reinterpret_cast<float4*>(y)[i] = y4;
-    }
-    p4.x = z4.x + beta * p4.x; p4.y = z4.y + beta * p4.y; p4.z = z4.z + beta * p4.z; p4.w = z4.w + beta * p4.w;
-    reinterpret_cast<float4*>(p)[i] = p4;
-  }
-  for (int64_t i = 4 * n4 + g0; i < n; i += gs) {
-    if (y) y[i] += alpha * p[i];
-    p[i] = init ? z[i] : z[i] + beta * p[i];
-  }
 }
 
 // start: r = f - w (w null: f); r32 = (float) r; y = 0; sums ff, rr
@@ -1114,23 +1090,25 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   auto precondition = [&](int mode) -> int {
     return schwarz_apply(k->sw, z32, r32, s, k->sc, p->multf, p->red_part, mode);
   };
-  // x += y, after a poll: stopped (done) behind an update, its alpha p is still due
+  AxDir dir{p32, z32, y32, 1};  // the next product's direction update
+  // x += y, after a poll; behind an update its alpha p is still due
   auto accumulate = [&]() -> int {
-    k_ru_accum<<<G, TPB, 0, s>>>(x, y32, hs->done && hs->y_due ? p32 : nullptr, n, k->sc);
+    k_ru_accum<<<G, TPB, 0, s>>>(x, y32, hs->y_due ? p32 : nullptr, n, k->sc);
     NTG_COUNT_LAUNCH();
     return NTG_OK;
   };
-  auto replace = [&](int mode) -> int {
+  // the FP32 residual is small enough, or has dropped by delta: confirm it in FP64
+  auto replace = [&]() -> int {
     NTG_TRY(accumulate());
     NTG_TRY(op_apply(p, k->v64.w, x, s));
     fpax++;
     nru++;
-    { k_ru_resid<false><<<GR, TPB, 0, s>>>(f, k->v64.w, nullptr, p->mult, p->multf, k->v64.r, r32, n, mode, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
+    { k_ru_resid<false><<<GR, TPB, 0, s>>>(f, k->v64.w, nullptr, p->mult, p->multf, k->v64.r, r32, n, 2, p->red_part, k->sc); NTG_COUNT_LAUNCH(); }
     NTG_CUDA_TRY(cudaGetLastError());
     NTG_TRY(poll());
     if (hs->done) return NTG_OK;
-    NTG_TRY(precondition(mode == 2 ? 0 : 1));
-    if (mode == 2) NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, nullptr, n, 0, k->sc));
+    NTG_TRY(precondition(0));
+    dir.mode = 2;
     return poll();
   };
   // structured box (the Schwarz preconditioner's form): the gather-scatter of
@@ -1145,7 +1123,6 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   const double rr0 = hs->rr0, ff = hs->ff;
   if (!hs->done) {
     NTG_TRY(precondition(3));
-    NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, nullptr, n, 1, k->sc));
     NTG_TRY(poll());
   }
   bool y_dirty = false;
@@ -1153,21 +1130,17 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   for (;;) {
     if (hs->done) {
       if (hs->need_ru == 2) {
-        NTG_TRY(replace(2));
+        NTG_TRY(replace());
         y_dirty = false;
         if (hs->done) break;
         continue;
       }
       break;
     }
-    if (hs->need_ru == 1) {
-      NTG_TRY(replace(1));
-      y_dirty = false;
-      if (hs->done) break;
-    }
     if (++guard > k->max_iter / k->check_every + 64) break;  // defensive: the device cap ends the loop first
     for (int c = 0; c < k->check_every; ++c) {
-      NTG_TRY(ax_launch_f32(p, w32, p32, k->sc, 0, s));
+      NTG_TRY(ax_launch_f32(p, w32, p32, k->sc, 0, s, &dir));
+      dir.mode = 0;
       timer_start(TM_UPD32, s);
       if (box_lx) {
         // gather-scatter, mask and update in one pass over the box
@@ -1185,9 +1158,6 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
       timer_start(TM_PC32, s);
       NTG_TRY(precondition(0));
       timer_stop(TM_PC32, s);
-      timer_start(TM_DIR32, s);
-      NTG_TRY(launch_dependent(p, k_dir_z, G, TPB, 0, s, p32, z32, y32, n, 0, k->sc));
-      timer_stop(TM_DIR32, s);
     }
     y_dirty = true;
     NTG_TRY(poll());

@@ -105,7 +105,7 @@ struct FinPap {
   __device__ void operator()(const double* acc, Scalars* sc) const {
     double pap = acc[0];
     sc->pap = pap;
-    sc->y_due = 0;  // the direction update before this operator did it
+    sc->y_due = 0;  // done with the direction update, ahead of this product
     if (!(pap > 0.0) || !isfinite(pap)) {
       sc->status = isfinite(pap) ? NTG_BREAKDOWN : NTG_NONFINITE;
       sc->done = 1;
