@@ -106,9 +106,12 @@ __global__ void k_coef_means(const double* __restrict__ h1, double h1c, const do
 // order is t, r, s forward, the scaling, s, r, t back: t forward runs before
 // the tile is first written, s forward, scaling and s back are one pass, and
 // t back goes from registers to HBM, so the tile is written and read four
-// times.  The load / store pipe bounds it (664 wavefronts per element, of
-// them 469 shared): 101 us at 32^3 elements, lx = 8, where six passes with
-// the operator in shared memory (848 shared wavefronts) took 160.
+// times.  The load / store pipe bounds it, at 72% of its rate with half
+// the warps the SM can hold: 99 us at 32^3 elements, lx = 8, where six passes
+// with the operator in shared memory (848 shared wavefronts per element) took
+// 160.  The coarse restriction beside
+// it goes z, x, y: columns, then rows, then vertices, 2 + 4 partials a column
+// and row; eight partials per thread summed by eight threads cost a solve 1%.
 //   per element: scalars (sx, sy, sz, c, h1, h2) = (4/hx^2, 4/hy^2, 4/hz^2,
 //                8/(hx hy hz), h1, h2); tile A[a + RS b + PS c]
 // Tile strides: lines of a warp are consecutive (u fastest).  (RS, PS) make
@@ -131,26 +134,26 @@ struct FdmCfg {
   static constexpr int TPER = LX == 8 ? 1714 : LX == 6 ? 576 : 257;
   static constexpr int EPB = LX == 4 ? 16 : LX == 8 ? 4 : 8, THREADS = EPB * TPE;
   static constexpr int MINB = 1024 / THREADS;
-  // coarse restriction partials (8 per thread): in the tile rows' padding
-  // (a in [LE, RS), two rows per thread) when it is wide enough, else after the tiles
-  static constexpr bool HOLES = 2 * (RS - LE) >= 8;
-  static constexpr int RED = HOLES ? 0 : EPB * TPE * 8;
+  // coarse restriction partials, 2 per own column and 4 per row j: in the tile
+  // rows' padding (a in [LE, RS)) when it is wide enough, else after the tiles
+  static constexpr bool HOLES = RS - LE >= 4;
+  static constexpr int RPER = LX * LX * 2 + LX * 4, RED = HOLES ? 0 : EPB * RPER;
   static constexpr size_t SMEM = ((size_t)EPB * TPER + RED) * sizeof(float);
   static_assert(LE % 2 == 0 && TPER >= SPAN && THREADS <= 1024, "layout");
 };
 
-// slot v of thread tl's coarse partials (A: the element's tile, red: the
-// block's partial region, el: element slot)
+// slots of the coarse partials (A: the element's tile, red: its region behind
+// the tiles): column (i, j) for the lower / upper z vertex, and row j for the
+// z vertex vz and the x vertex vx
 template <int LX>
-__device__ __forceinline__ float* crs_slot(float* A, float* red, int el, int tl, int v) {
+__device__ __forceinline__ float* crs_col(float* A, float* red, int i, int j, int vz) {
   using C = FdmCfg<LX>;
-  if constexpr (C::HOLES) {
-    constexpr int W = C::RS - C::LE;
-    const int b = tl % C::LE, c = tl / C::LE + (v < W ? 0 : C::LE / 2);
-    return A + C::LE + (v < W ? v : v - W) + C::RS * b + C::PS * c;
-  } else {
-    return red + (el * C::TPE + tl) * 8 + v;
-  }
+  return C::HOLES ? A + C::LE + vz + C::RS * j + C::PS * i : red + (i + LX * j) * 2 + vz;
+}
+template <int LX>
+__device__ __forceinline__ float* crs_row(float* A, float* red, int j, int vz, int vx) {
+  using C = FdmCfg<LX>;
+  return C::HOLES ? A + C::LE + 2 + vx + C::RS * j + C::PS * vz : red + LX * LX * 2 + (j * 2 + vz) * 2 + vx;
 }
 
 // y = S^T x (FWD) or S x of a line in registers, in place.  EO: the even-odd
@@ -248,7 +251,7 @@ __global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
   const int tid = threadIdx.x, el = tid / TPE, tl = tid - el * TPE;
   const int u = tl % LE, v1 = tl / LE, v2 = v1 + H;  // lines (u, v1) and (u, v2); tl + TPE = u + LE v2
   float* A = smem + el * C::TPER;
-  float* red = smem + EPB * C::TPER;
+  float* red = smem + EPB * C::TPER + el * C::RPER;
   __shared__ float sp[2][LX];  // Q1 basis at the GLL nodes
   __shared__ float slam[LE];   // reference eigenvalues
   if (tid == 0) {
@@ -328,10 +331,7 @@ __global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
   }
   __syncthreads();  // sp, slam
   if (corner) {
-    // coarse restriction: own-element columns, z weights first, then x / y
-    float pt[8];
-#pragma unroll
-    for (int v = 0; v < 8; ++v) pt[v] = 0.f;
+    // coarse restriction, z first: each own column's sums for its two z vertices
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
       const int vb = q ? v2 : v1;
@@ -350,11 +350,9 @@ __global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
         if ((i == 0 && ex > 0) || (i == N && ex < Ex - 1)) wxy *= 0.5f;
         if ((j == 0 && ey > 0) || (j == N && ey < Ey - 1)) wxy *= 0.5f;
       }
-#pragma unroll
-      for (int v = 0; v < 8; ++v) pt[v] = fmaf(sp[v & 1][i] * sp[(v >> 1) & 1][j] * wxy, (v >> 2) ? s1 : s0, pt[v]);
+      *crs_col<LX>(A, red, i, j, 0) = s0 * wxy;
+      *crs_col<LX>(A, red, i, j, 1) = s1 * wxy;
     }
-#pragma unroll
-    for (int v = 0; v < 8; ++v) *crs_slot<LX>(A, red, el, tl, v) = pt[v];
   }
   const float2* M = reinterpret_cast<const float2*>(&R.S[0][0]);
   // t forward in registers: lines (a, b) = (u, v) along c
@@ -364,6 +362,18 @@ __global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
     fdm_store<LE>(A + u + RS * (q ? v2 : v1), PS, x[q]);
   }
   __syncthreads();
+  if (corner && live && tl < 2 * LX) {  // x next, one thread per row and z vertex
+    const int j = tl % LX, vz = tl / LX;
+    float a0 = 0.f, a1 = 0.f;
+#pragma unroll
+    for (int i = 0; i < LX; ++i) {
+      const float v = *crs_col<LX>(A, red, i, j, vz);
+      a0 = fmaf(sp[0][i], v, a0);
+      a1 = fmaf(sp[1][i], v, a1);
+    }
+    *crs_row<LX>(A, red, j, vz, 0) = a0;
+    *crs_row<LX>(A, red, j, vz, 1) = a1;
+  }
   // r forward: lines (b, c) = (u, v) along a
 #pragma unroll
   for (int q = 0; q < 2; ++q) fdm_load<LE>(A + RS * u + PS * (q ? v2 : v1), 1, x[q]);
@@ -373,6 +383,12 @@ __global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
     fdm_store<LE>(A + RS * u + PS * (q ? v2 : v1), 1, x[q]);
   }
   __syncthreads();
+  if (corner && live && tl < 8) {  // y last, one thread per vertex
+    float acc = 0.f;
+#pragma unroll
+    for (int j = 0; j < LX; ++j) acc = fmaf(sp[(tl >> 1) & 1][j], *crs_row<LX>(A, red, j, tl >> 2, tl & 1), acc);
+    corner[(int64_t)e * 8 + tl] = acc;
+  }
   // s forward, scale (c_e / D_e), s back: lines (a, c) = (u, v) along b
 #pragma unroll
   for (int q = 0; q < 2; ++q) fdm_load<LE>(A + u + PS * (q ? v2 : v1), RS, x[q]);
@@ -395,12 +411,6 @@ __global__ void __launch_bounds__(FdmCfg<LX>::THREADS, FdmCfg<LX>::MINB)
     fdm_store<LE>(A + RS * u + PS * (q ? v2 : v1), 1, x[q]);
   }
   __syncthreads();
-  // coarse restriction of the element: 8 threads sum the partials in order
-  if (corner && live && tl < 8) {
-    float acc = 0.f;
-    for (int t = 0; t < TPE; ++t) acc += *crs_slot<LX>(A, red, el, t, tl);
-    corner[(int64_t)e * 8 + tl] = acc;
-  }
   // t back and out: columns (a, b) of ze[e][a + LE b + LE2 c] (consecutive lines -> consecutive addresses)
 #pragma unroll
   for (int q = 0; q < 2; ++q) fdm_load<LE>(A + u + RS * (q ? v2 : v1), PS, x[q]);
@@ -1205,8 +1215,8 @@ int fdm_launch(ntg_schwarz* w, const float* r, cudaStream_t s, const Scalars* sc
   float* corner = w->coarse_ready ? w->corner : nullptr;
   const bool g = w->gen != nullptr;
   const unsigned grid = (unsigned)((w->plan->nelv + C::EPB - 1) / C::EPB);
-  return launch_dependent(w->plan, fdm_kernel<LX>(w, w->fdm_eo), grid, C::THREADS, C::SMEM, s, r, w->ze, w->esc, g ? (int)w->plan->nelv : w->Ex, g ? 1 : w->Ey, g ? 1 : w->Ez,
-                          sc, corner, w->ph, g ? w->gen->ghost : nullptr, g ? w->plan->multf : nullptr, R);
+  return launch_dependent(w->plan, fdm_kernel<LX>(w, w->fdm_eo), grid, C::THREADS, C::SMEM, s, r, w->ze, w->esc,
+                          g ? (int)w->plan->nelv : w->Ex, g ? 1 : w->Ey, g ? 1 : w->Ez, sc, corner, w->ph, g ? w->gen->ghost : nullptr, g ? w->plan->multf : nullptr, R);
 }
 
 }  // namespace sw
