@@ -535,14 +535,18 @@ def run_headline_sequence(args, ws, rank, local):
     ax32 = ktimes.get("ax_fp32")
     bpd = (2 + 6 + ncoef) * 4
     t_in = ax32["avg_us"] * 1e-6 if ax32 else ax["fp32_s"]
-    roof = {"kernel": "k_ax_helm_f32_tma (FP32 Ax inside the timed solves)", "bound": "hbm",
-            "achieved": round(bpd * n / t_in / 1e9, 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
-            "frac": round(bpd * n / t_in / 1e9 / pk["hbm_gbs"], 4), "peak_source": pk_kind,
-            "bytes_per_dof": bpd, "standalone_cold": {
-                "us": round(ax["fp32_s"] * 1e6, 1), "achieved": round(bpd * n / ax["fp32_s"] / 1e9, 1),
-                "frac": round(bpd * n / ax["fp32_s"] / 1e9 / pk["hbm_gbs"], 4)},
-            "traffic": args.traffic if args.traffic is not None else measured_traffic("k_ax_helm_f32_tma", n, ncoef)}
+    # inside the Schwarz-preconditioned solves it also updates the direction:
+    # z, y read, p, y written
     fdm = ktimes.get("schwarz_fdm")
+    bpd_in = bpd + 16 if ax32 and fdm else bpd
+    traffic = args.traffic if args.traffic is not None else measured_traffic("k_ax_helm_f32_tma", n, ncoef)
+    roof = {"kernel": "k_ax_helm_f32_tma (FP32 Ax with the direction update, inside the timed solves)", "bound": "hbm",
+            "achieved": round(bpd_in * n / t_in / 1e9, 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
+            "frac": round(bpd_in * n / t_in / 1e9 / pk["hbm_gbs"], 4), "peak_source": pk_kind,
+            "bytes_per_dof": bpd_in, "standalone_cold": {
+                "us": round(ax["fp32_s"] * 1e6, 1), "achieved": round(bpd * n / ax["fp32_s"] / 1e9, 1),
+                "frac": round(bpd * n / ax["fp32_s"] / 1e9 / pk["hbm_gbs"], 4), "traffic": traffic},
+            "traffic": traffic if bpd_in == bpd else None}
     roof_fdm = None
     if fdm:
         # algorithmic bytes per element: the extended box's values of r are
@@ -560,10 +564,7 @@ def run_headline_sequence(args, ws, rank, local):
                                         "written + 6 scalars per element"}
     ax64 = ktimes.get("ax_fp64")
     t_k64 = ax64["avg_us"] * 1e-6 if ax64 else ax["fp64_s"]
-    roof64 = {"kernel": "k_ax_helm<double,8> (FP64 Ax: residual replacements, projection)", "bound": "fp64",
-              "achieved": round(116.0 * n / t_k64 / 1e9, 1), "peak": FP64_TFLOPS * 1e3, "unit": "GFLOP/s",
-              "frac": round(116.0 * n / t_k64 / 1e9 / (FP64_TFLOPS * 1e3), 4),
-              "peak_source": "FP64 FMA-chain probe, bench.py --fp64-peak"}
+    roof64 = fp64_ax_roof("residual replacements, projection", n, ncoef, t_k64, pk, pk_kind)
 
     ev_its = its_eval
     out = {
@@ -849,7 +850,8 @@ def run_terms(args, local):
             if name in flops:
                 tf = flops[name] * n / (ms * 1e-3) / 1e12
                 rec["fp64_tflops"] = round(tf, 3)
-                rec["frac_of_fp64_roof"] = round(tf / FP64_TFLOPS, 3)
+                # the contractions run on the integer pipes: this may pass 1
+                rec["ratio_to_fp64_pipe_roof"] = round(tf / FP64_TFLOPS, 3)
             out[name] = rec
     cpu_threads = None
     if not args.no_cpu:
@@ -987,6 +989,16 @@ def run_mma(args, local):
             "cpu_baseline": cpu}
 
 
+def fp64_ax_roof(use, n, ncoef, t, pk, kind):
+    """The FP64 operator against HBM.  Its contractions run in fixed point on
+    the integer pipes, which bound it; on the FP64 pipe its 116 flop per local
+    DOF would take longer than it does."""
+    gbs = (2 + 6 + ncoef) * 8 * n / t / 1e9
+    return {"kernel": f"k_ax_fx<8> (FP64 Ax: {use})", "bound": "integer pipes", "achieved": round(gbs, 1),
+            "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": round(gbs / pk["hbm_gbs"], 4), "peak_source": kind,
+            "ratio_to_fp64_pipe_roof": round(116.0 * n / t / 1e12 / FP64_TFLOPS, 3)}
+
+
 def run_ours(args, ws, rank, local):
     import torch
     import __graft_entry__ as ge
@@ -1085,23 +1097,19 @@ def run_ours(args, ws, rank, local):
     pk, pk_kind = peaks()
     ax32 = ktimes.get("ax_fp32")
     bytes_per_dof = (2 + 6 + ncoef) * 4
+    if ax32 and ktimes.get("schwarz_fdm"):
+        bytes_per_dof += 16  # the direction update: z, y read, p, y written
     t_launch = ax32["avg_us"] * 1e-6 if ax32 else t_ax32
     achieved = bytes_per_dof * n / t_launch / 1e9
     roof = {"kernel": "k_ax_helm<float,8> (FP32 Ax inside the timed solve)", "bound": "hbm",
             "achieved": round(achieved, 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
             "frac": round(achieved / pk["hbm_gbs"], 4), "peak_source": pk_kind,
             "bytes_per_dof": bytes_per_dof, "traffic": args.traffic if args.traffic is not None
-            else measured_traffic("k_ax_helm_f32_tma", n, ncoef)}
+            else measured_traffic("k_ax_helm_f32_tma", n, ncoef) if bytes_per_dof == (8 + ncoef) * 4 else None}
 
-    # the FP64 operator against the FP64 compute roof: 116 flop per local DOF
-    # (six contractions of 2(N+1) flop each, plus the metric mix), the peak
-    # from an FMA-chain probe on GB300 (not in MEASURED_PEAKS.json)
     ax64 = ktimes.get("ax_fp64")
     t_k64 = ax64["avg_us"] * 1e-6 if ax64 else t_ax64  # one FP64 Ax launch
-    fp64_peak = FP64_TFLOPS * 1e3
-    roof64 = {"kernel": "k_ax_helm<double,8> (FP64 Ax, residual replacements)", "bound": "fp64",
-              "achieved": round(116.0 * n / t_k64 / 1e9, 1), "peak": fp64_peak, "unit": "GFLOP/s",
-              "frac": round(116.0 * n / t_k64 / 1e9 / fp64_peak, 4), "peak_source": "FP64 FMA-chain probe, bench.py --fp64-peak"}
+    roof64 = fp64_ax_roof("residual replacements", n, ncoef, t_k64, pk, pk_kind)
 
     # end to end through the public API: host RHS in, host solution out
     f_h = f.cpu().pin_memory()

@@ -1,5 +1,9 @@
 // The FP64 matrix-free Helmholtz operator with its contractions in fixed
-// point on the integer pipes (fx.cuh).
+// point on the integer pipes (fx.cuh).  With every product on the FP64 pipe it
+// took 28 clocks per node and SM, 1.9 ms at 16.8M nodes of lx = 8; here the
+// metric products and the conversions leave that pipe 5.5 and the integer pipes
+// bound it: 0.38 ms, against 0.18 for its 72 B per node.  One element per block
+// at lx = 8: sixteen blocks per SM keep the phases of different elements apart.
 #include <cmath>
 
 #include "common.cuh"

@@ -14,7 +14,11 @@
 // the GL cofactors (9 doubles per GL point, interpolated once at create)
 // stream from memory.  The sums are rewritten with contravariant velocities,
 // so the three cdtp of a component become one transposed derivative and the
-// linear term needs none.
+// linear term needs none.  The contractions run in fixed point (fx.cuh): the
+// adjoint term of 24^3 elements, lx = 8, takes 5.3 ms where FP64 sums took
+// 22.5, the linear one of 315 elements, lx = 6, 63 us where they took 201.  The
+// integer pipes bound it, at 1.3 instructions per clock with the 14 warps that
+// the tiles of LXD^3 64-bit values leave room for.
 #include <cmath>
 
 #include "deriv.cuh"

@@ -1241,7 +1241,12 @@ int pull_launch(ntg_schwarz* w, float* z, const float* r, cudaStream_t s, Scalar
 }
 
 // coarse solve (after the FDM kernel has written the corner sums): the
-// restriction onto the vertex grid, then x, y, z forward (scaled), z, y, x back into uc
+// restriction onto the vertex grid, then x, y, z forward (scaled), z, y, x back
+// into uc.  Three kernels (planes, columns, planes) where a plane with its two
+// matrices and a block's columns with theirs fit in shared memory, up to about
+// 220 vertices in x and y together and 150 in z: 27 us at 32^3 elements, 59 at
+// 64^3.  A larger grid takes one kernel per direction, which reads its lines
+// from L2: 45 us and 110.
 inline int coarse_launch(ntg_schwarz* w, cudaStream_t s, const Scalars* sc) {
   const CoarseDims& d = w->cd;
   const int64_t total = (int64_t)d.m[0] * d.m[1] * d.m[2];
