@@ -95,8 +95,18 @@ struct Scalars {
 
 }  // namespace ntg
 
-// The plan: mesh, coef_t, gs_t, Jacobi.
-struct ntg_plan {
+// The Dirichlet mask and what is derived from it.  One object, so that a mask
+// that is set aside for a while (ntg_filter_apply) takes all of it along.
+struct ntg_mask_state {
+  int32_t* mask = nullptr;      // 0-based node list
+  int64_t nmask = 0;
+  uint8_t* maskrow = nullptr;   // n / lx (lx <= 8): bit i of byte t set when node i of row t is masked (built on first use)
+  double* multm = nullptr;      // mult, negative on Dirichlet nodes (plan_multm), and its FP32 copy
+  float* multmf = nullptr;
+};
+
+// The plan: mesh, coef_t, gs_t, Jacobi, the Dirichlet mask.
+struct ntg_plan : ntg_mask_state {
   int lx = 0;
   int64_t nelv = 0, n = 0, nu = 0, nshared = 0, nshared_idx = 0;
   cudaStream_t stream = 0;
@@ -109,8 +119,6 @@ struct ntg_plan {
   double* B = nullptr;
   double* mult = nullptr;
   float* multf = nullptr;
-  double* multm = nullptr;      // mult, negative on Dirichlet nodes (plan_multm), and its FP32 copy
-  float* multmf = nullptr;
   // gather-scatter: full map (perm sorted by global id, offsets) and the
   // shared-node subset the hot kernels use
   int32_t* perm = nullptr;
@@ -134,10 +142,6 @@ struct ntg_plan {
   int ifh2 = 0;
   double* hB = nullptr;   // h2*B (when ifh2)
   float* hBf = nullptr;
-  // Dirichlet mask (0-based)
-  int32_t* mask = nullptr;
-  int64_t nmask = 0;
-  uint8_t* maskrow = nullptr;  // n / lx (lx <= 8): bit i of byte t set when node i of row t is masked (built on first use)
   // Jacobi
   double* dinv = nullptr;
   float* dinvf = nullptr;
@@ -268,6 +272,7 @@ int plan_multm(ntg_plan* p, const double** out);
 int plan_multm(ntg_plan* p, const float** out);
 int jacobi_update(ntg_plan* p);
 int ensure_maskrow(ntg_plan* p);
+void mask_free(ntg_mask_state* m);
 // the element counts of a Schwarz preconditioner built on a structured box
 // (1), or 0 for one built on a general mesh
 int schwarz_box(const ntg_schwarz* w, int* ex, int* ey, int* ez);

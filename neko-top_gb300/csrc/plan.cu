@@ -435,15 +435,23 @@ int ensure_fp32(ntg_plan* p) {
   return NTG_OK;
 }
 
+void mask_free(ntg_mask_state* m) {
+  dev_free(m->mask);
+  dev_free(m->maskrow);
+  dev_free(m->multm);
+  dev_free(m->multmf);
+  m->nmask = 0;
+}
+
 static void plan_free(ntg_plan* p) {
   for (int a = 0; a < 6; ++a) {
     dev_free(p->g[a]);
     dev_free(p->gf[a]);
   }
-  dev_free(p->B); dev_free(p->mult); dev_free(p->multf); dev_free(p->multm); dev_free(p->multmf);
+  dev_free(p->B); dev_free(p->mult); dev_free(p->multf);
   dev_free(p->perm); dev_free(p->offs); dev_free(p->sh_idx); dev_free(p->sh_off);
   dev_free(p->h1); dev_free(p->h1f); dev_free(p->hB); dev_free(p->hBf);
-  dev_free(p->mask); dev_free(p->maskrow); dev_free(p->dinv); dev_free(p->dinvf);
+  mask_free(p); dev_free(p->dinv); dev_free(p->dinvf);
   dev_free(p->red_part); dev_free(p->scal); dev_free(p->dev_err);
   dev_free(p->gs2); dev_free(p->gs4); dev_free(p->gs8); dev_free(p->gsx_idx); dev_free(p->gsx_off);
   dev_free(p->met); dev_free(p->binv); dev_free(p->dscr);
@@ -763,11 +771,7 @@ int ntg_plan_set_mask(ntg_plan* p, const int32_t* mask_d, int64_t nmask, int bas
   clear_error();
   NTG_CHECK_ARG(p, "ntg_plan_set_mask: null plan");
   NTG_CHECK_ARG(nmask >= 0 && (nmask == 0 || mask_d), "ntg_plan_set_mask: bad mask");
-  dev_free(p->mask);
-  dev_free(p->maskrow);
-  dev_free(p->multm);
-  dev_free(p->multmf);
-  p->nmask = 0;
+  mask_free(p);
   p->jacobi_ready = 0;
   if (nmask == 0) return NTG_OK;
   NTG_TRY(dev_alloc(&p->mask, nmask));

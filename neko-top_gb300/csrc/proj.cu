@@ -15,6 +15,7 @@
 // (sources/mapping_functions/PDE_filter_mapping.f90:212-363).
 #include <cmath>
 #include <cstring>
+#include <utility>
 
 #include "common.cuh"
 #include "reduce.cuh"
@@ -402,10 +403,9 @@ int ntg_filter_apply(ntg_plan* p, ntg_ksp* ksp, double* X_out_d, const double* X
   NTG_TRY(ntg_coef_set(p, nullptr, r * r, nullptr, 1.0, 1));
   double* rhs = nullptr;
   NTG_TRY(dev_alloc(&rhs, n));
-  int32_t* saved_mask = p->mask;
-  int64_t saved_nmask = p->nmask;
-  p->mask = nullptr;
-  p->nmask = 0;
+  // everything derived from the mask goes with it: the solver may build its own meanwhile
+  ntg_mask_state kept;
+  std::swap(kept, static_cast<ntg_mask_state&>(*p));
   int st = NTG_OK;
   do {
     { k_mulB<<<G, 256, 0, s>>>(rhs, X_in_d, p->B, n); NTG_COUNT_LAUNCH(); }
@@ -417,10 +417,10 @@ int ntg_filter_apply(ntg_plan* p, ntg_ksp* ksp, double* X_out_d, const double* X
     if ((st = jacobi_update(p))) break;
     st = ntg_ksp_solve(ksp, X_out_d, rhs, mon);
   } while (0);
-  p->mask = saved_mask;
-  p->nmask = saved_nmask;
-  p->jacobi_ready = 0;  // the next solve rebuilds the diagonal with its mask
   cudaStreamSynchronize(s);
+  std::swap(kept, static_cast<ntg_mask_state&>(*p));
+  mask_free(&kept);
+  p->jacobi_ready = 0;  // the next solve rebuilds the diagonal with its mask
   dev_free(rhs);
   return st;
 }
