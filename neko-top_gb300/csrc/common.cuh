@@ -100,7 +100,7 @@ struct Scalars {
 struct ntg_mask_state {
   int32_t* mask = nullptr;      // 0-based node list
   int64_t nmask = 0;
-  uint8_t* maskrow = nullptr;   // n / lx (lx <= 8): bit i of byte t set when node i of row t is masked (built on first use)
+  uint8_t* maskrow = nullptr;   // n / lx (lx <= 8): bit i of byte t set when node i of row t is masked; null: no mask
   double* multm = nullptr;      // mult, negative on Dirichlet nodes (plan_multm), and its FP32 copy
   float* multmf = nullptr;
 };
@@ -271,7 +271,6 @@ int grid_red(int64_t work, int threads);
 int plan_multm(ntg_plan* p, const double** out);
 int plan_multm(ntg_plan* p, const float** out);
 int jacobi_update(ntg_plan* p);
-int ensure_maskrow(ntg_plan* p);
 void mask_free(ntg_mask_state* m);
 // the element counts of a Schwarz preconditioner built on a structured box
 // (1), or 0 for one built on a general mesh

@@ -680,9 +680,9 @@ __global__ void k_update_rr(float* __restrict__ r, const float* __restrict__ w, 
 // in y and z, and the x neighbours' end values -- in ascending element
 // order (z-major, y, x), the order of the gather-scatter's groups, so every
 // copy of a node receives the same sum.  Then w is masked (one mask byte per
-// row; maskrow null: no mask) and r -= alpha w; (r, r)_mult is summed over each node's owning copy
-// (no lower neighbour in any direction), which the mult-weighted sum over
-// copies equals, with no multiplicity stream.
+// row; maskrow null: no mask) and r -= alpha w; (r, r)_mult is summed over
+// each node's owning copy (no lower neighbour in any direction), which the
+// mult-weighted sum over copies equals, with no multiplicity stream.
 // HBM and the bytes in flight bound it: a whole row per thread, its loads
 // first, four blocks per SM (six take spills: +6% of a solve).  Half a row per
 // thread, with contiguous lanes, was slower.  y += alpha p here and again
@@ -1134,7 +1134,6 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
   int bx = 0, by = 0, bz = 0, box_lx = 0;
   if (k->box_update && schwarz_box(k->sw, &bx, &by, &bz) && (p->lx == 4 || p->lx == 6 || p->lx == 8) &&
       (int64_t)bx * by * bz == p->nelv) {
-    if (p->nmask) NTG_TRY(ensure_maskrow(p));
     box_lx = p->lx;
   }
   NTG_TRY(poll());
@@ -1164,7 +1163,7 @@ static int ksp_solve_mixed_ru_pc(ntg_ksp* k, double* x, const double* f, ntg_mon
         // gather-scatter, mask and update in one pass over the box
         const int GB = grid_red(n / p->lx, TPB);
         auto kern = box_lx == 8 ? k_update_box<8> : box_lx == 6 ? k_update_box<6> : k_update_box<4>;
-        NTG_TRY(launch_dependent(p, kern, GB, TPB, 0, s, r32, w32, p->nmask ? p->maskrow : nullptr, bx, by, bz, p->red_part, k->sc));
+        NTG_TRY(launch_dependent(p, kern, GB, TPB, 0, s, r32, w32, p->maskrow, bx, by, bz, p->red_part, k->sc));
       } else {
         timer_stop(TM_UPD32, s);
         NTG_TRY(gs_add_guarded_f32(p, w32, s, k->sc));

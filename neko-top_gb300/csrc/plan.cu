@@ -352,9 +352,6 @@ static Basis make_basis(int lx) {
   return b;
 }
 
-// the Dirichlet mask as one bit per node, a byte per row of lx <= 8 nodes
-// (rows x fastest, n / lx bytes), for kernels that assemble and mask a row
-// in one pass; built on the host from the mask list
 __global__ void k_flip_sign(double* __restrict__ a, float* __restrict__ b, const int32_t* __restrict__ mask, int64_t m) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
     const int32_t i = mask[q];
@@ -403,21 +400,23 @@ __global__ void k_mask_rows(uint32_t* __restrict__ rows, const int32_t* __restri
   }
 }
 
-int ensure_maskrow(ntg_plan* p) {
-  if (p->maskrow) return NTG_OK;
-  if (p->lx > 8) {
-    set_error("mask rows: lx=%d above 8", p->lx);
-    return NTG_ERR_UNSUPPORTED;
-  }
+// The Dirichlet mask as one bit per node, a byte per row of lx <= 8 nodes (rows
+// x fastest, n / lx bytes), for the kernels that assemble and mask a row in one
+// pass.  Built with the mask, so that no later call has to allocate.
+static int build_maskrow(ntg_plan* p) {
+  if (p->lx > 8) return NTG_OK;  // no such kernel there
   const size_t bytes = ((size_t)(p->n / p->lx) + 3) / 4 * 4;
-  NTG_TRY(dev_alloc(&p->maskrow, bytes));
-  NTG_CUDA_TRY(cudaMemsetAsync(p->maskrow, 0, bytes, p->stream));
-  if (p->nmask) {
-    k_mask_rows<<<grid_for(p->nmask, 256), 256, 0, p->stream>>>(reinterpret_cast<uint32_t*>(p->maskrow), p->mask,
-                                                                p->nmask, p->lx);
-    NTG_COUNT_LAUNCH();
-    NTG_CUDA_TRY(cudaGetLastError());
+  uint8_t* rows = nullptr;
+  NTG_TRY(dev_alloc(&rows, bytes));
+  cudaError_t e = cudaMemsetAsync(rows, 0, bytes, p->stream);
+  { k_mask_rows<<<grid_for(p->nmask, 256), 256, 0, p->stream>>>(reinterpret_cast<uint32_t*>(rows), p->mask, p->nmask, p->lx); NTG_COUNT_LAUNCH(); }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+  if (e != cudaSuccess) {
+    dev_free(rows);
+    set_error("mask rows: %s", cudaGetErrorString(e));
+    return NTG_ERR_CUDA;
   }
+  p->maskrow = rows;
   return NTG_OK;
 }
 
@@ -793,7 +792,9 @@ int ntg_plan_set_mask(ntg_plan* p, const int32_t* mask_d, int64_t nmask, int bas
     return NTG_ERR_INVALID;
   }
   p->nmask = nmask;
-  return NTG_OK;
+  const int st = build_maskrow(p);
+  if (st) mask_free(p);
+  return st;
 }
 
 }  // extern "C"

@@ -1229,15 +1229,13 @@ template <int LX>
 int pull_launch(ntg_schwarz* w, float* z, const float* r, cudaStream_t s, Scalars* sc, bool dot, double* part,
                 int mode) {
   ntg_plan* p = w->plan;
-  if (p->nmask) NTG_TRY(ensure_maskrow(p));
-  const uint8_t* mask = p->nmask ? p->maskrow : nullptr;
   const int64_t rows = p->n / LX;
   const CoarseView cv{w->coarse_ready ? w->uc : nullptr, w->ph, w->dw};
   if (dot)
-    return launch_dependent(p, k_pull<LX, true>, grid_red(rows, 256), 256, 0, s, w->ze, z, w->Ex, w->Ey, w->Ez, r, mask,
-                            mode, part, sc, cv);
-  return launch_dependent(p, k_pull<LX, false>, grid_for(rows, 256), 256, 0, s, w->ze, z, w->Ex, w->Ey, w->Ez, r, mask, 0,
-                          nullptr, sc, cv);
+    return launch_dependent(p, k_pull<LX, true>, grid_red(rows, 256), 256, 0, s, w->ze, z, w->Ex, w->Ey, w->Ez, r,
+                            p->maskrow, mode, part, sc, cv);
+  return launch_dependent(p, k_pull<LX, false>, grid_for(rows, 256), 256, 0, s, w->ze, z, w->Ex, w->Ey, w->Ez, r,
+                          p->maskrow, 0, nullptr, sc, cv);
 }
 
 // coarse solve (after the FDM kernel has written the corner sums): the

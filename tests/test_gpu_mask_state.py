@@ -66,3 +66,44 @@ def test_filter_leaves_the_mask_as_it_was(pkg, orc, dev, lx, solved_before):
     assert not z[torch.from_numpy(orc.mask_face_xmax(*E, lx).astype(np.int64) - 1).to(dev)].any()
     assert torch.equal(precondition(c, sw, f), z)
     assert torch.equal(solve(pkg, c, sw, f), solve(pkg, c3, sw3, f))
+
+
+@pytest.mark.parametrize("lx", [4, 6, 8])
+def test_first_application_under_a_new_mask_is_captured(pkg, orc, dev, lx):
+    """The first application after a mask is set allocates nothing: it can be
+    recorded into a graph, with the operator and the gather-scatter before it,
+    and the replays give what the calls by themselves give."""
+    mask = T(orc.mask_face_xmax(*E, lx), dev, torch.int32)
+    f = T(np.random.default_rng(lx).standard_normal(24 * lx ** 3), dev, torch.float32)
+
+    def program():
+        c = pkg.coef_t.box(*E, lx, amp=0.05, seed=7, device=dev)
+        c.set_coefs(h1c=1.0, h2c=0.5, ifh2=True)
+        sw = pkg.schwarz_t(c, coarse=True)
+        w, z = torch.zeros_like(f), torch.zeros_like(f)
+
+        def run():
+            pkg.ax_helm_t().compute(w, f, c)
+            pkg.gs_t(c).op(w)
+            pkg.api.bc_list_apply_scalar(c, w)
+            sw.apply(z, w)
+
+        run()
+        c.set_mask(mask, base=1)
+        return run, w, z, (c, sw)
+
+    stream = torch.cuda.Stream(dev)
+    with torch.cuda.stream(stream):
+        run, w_ref, z_ref, keep = program()
+        run()
+        recorded, w, z, keep2 = program()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        recorded()
+    for _ in range(2):
+        w.fill_(float("nan"))
+        z.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(w, w_ref) and torch.equal(z, z_ref)
