@@ -101,8 +101,8 @@ struct ntg_mask_state {
   int32_t* mask = nullptr;      // 0-based node list
   int64_t nmask = 0;
   uint8_t* maskrow = nullptr;   // n / lx (lx <= 8): bit i of byte t set when node i of row t is masked; null: no mask
-  double* multm = nullptr;      // mult, negative on Dirichlet nodes (plan_multm), and its FP32 copy
-  float* multmf = nullptr;
+  double* multm = nullptr;      // mult, negative on Dirichlet nodes (plan_multm; null until used)
+  float* multmf = nullptr;      // multf, likewise
 };
 
 // The plan: mesh, coef_t, gs_t, Jacobi, the Dirichlet mask.
@@ -267,7 +267,7 @@ template <typename T>
 int gs_cls_launch(ntg_plan* p, T* u, int op, cudaStream_t s, const Scalars* sc);
 int grid_for(int64_t work, int threads);
 int grid_red(int64_t work, int threads);
-// mult with the Dirichlet nodes' weights negative, built on first use after set_mask
+// mult (multf: after ensure_fp32) with the Dirichlet nodes' weights negative, built on first use after set_mask
 int plan_multm(ntg_plan* p, const double** out);
 int plan_multm(ntg_plan* p, const float** out);
 int jacobi_update(ntg_plan* p);

@@ -352,46 +352,36 @@ static Basis make_basis(int lx) {
   return b;
 }
 
-__global__ void k_flip_sign(double* __restrict__ a, float* __restrict__ b, const int32_t* __restrict__ mask, int64_t m) {
+template <typename T>
+__global__ void k_flip_sign(T* __restrict__ a, const int32_t* __restrict__ mask, int64_t m) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {
     const int32_t i = mask[q];
-    const double v = -fabs(a[i]);  // a node may be listed twice
-    a[i] = v;
-    b[i] = (float)v;
+    a[i] = -fabs(a[i]);  // a node may be listed twice
   }
 }
 
-static int build_multm(ntg_plan* p) {
-  if (p->multm || p->nmask == 0) return NTG_OK;
-  double* d = nullptr;
-  float* f = nullptr;
-  int st = dev_alloc(&d, (size_t)p->n);
-  if (!st) st = dev_alloc(&f, (size_t)p->n);
-  if (!st && cudaMemcpyAsync(d, p->mult, sizeof(double) * p->n, cudaMemcpyDeviceToDevice, p->stream) != cudaSuccess) {
-    set_error("plan: copy of the multiplicities failed");
-    st = NTG_ERR_CUDA;
-  }
-  if (st) {
+// *out: the weights with the mask in their signs, made on first use, in the
+// precision that is asked for alone
+template <typename T>
+static int signed_weights(ntg_plan* p, const T* mult, T** kept, const T** out) {
+  *out = p->nmask ? *kept : mult;
+  if (*out) return NTG_OK;
+  T* d = nullptr;
+  NTG_TRY(dev_alloc(&d, (size_t)p->n));
+  cudaError_t e = cudaMemcpyAsync(d, mult, sizeof(T) * p->n, cudaMemcpyDeviceToDevice, p->stream);
+  { k_flip_sign<T><<<grid_for(p->nmask, 256), 256, 0, p->stream>>>(d, p->mask, p->nmask); NTG_COUNT_LAUNCH(); }
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    cudaStreamSynchronize(p->stream);
     dev_free(d);
-    dev_free(f);
-    return st;
+    set_error("plan: weights of the masked nodes: %s", cudaGetErrorString(e));
+    return NTG_ERR_CUDA;
   }
-  { k_d2f<<<grid_for(p->n, 256), 256, 0, p->stream>>>(d, f, p->n); NTG_COUNT_LAUNCH(); }
-  { k_flip_sign<<<grid_for(p->nmask, 256), 256, 0, p->stream>>>(d, f, p->mask, p->nmask); NTG_COUNT_LAUNCH(); }
-  p->multm = d;
-  p->multmf = f;
+  *out = *kept = d;
   return NTG_OK;
 }
-int plan_multm(ntg_plan* p, const double** out) {
-  NTG_TRY(build_multm(p));
-  *out = p->nmask ? p->multm : p->mult;
-  return NTG_OK;
-}
-int plan_multm(ntg_plan* p, const float** out) {
-  NTG_TRY(build_multm(p));
-  *out = p->nmask ? p->multmf : p->multf;
-  return NTG_OK;
-}
+int plan_multm(ntg_plan* p, const double** out) { return signed_weights(p, p->mult, &p->multm, out); }
+int plan_multm(ntg_plan* p, const float** out) { return signed_weights(p, p->multf, &p->multmf, out); }
 
 __global__ void k_mask_rows(uint32_t* __restrict__ rows, const int32_t* __restrict__ mask, int64_t m, int lx) {
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < m; q += (int64_t)gridDim.x * blockDim.x) {

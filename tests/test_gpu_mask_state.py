@@ -107,3 +107,27 @@ def test_first_application_under_a_new_mask_is_captured(pkg, orc, dev, lx):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(w, w_ref) and torch.equal(z, z_ref)
+
+
+@pytest.mark.parametrize("method,bytes_per_node", [("cg", 8), ("cg_mixed", 4)])
+def test_first_solve_keeps_weights_of_one_precision(pkg, orc, dev, method, bytes_per_node):
+    """What the first Jacobi-preconditioned solve under a mask allocates beyond
+    one without: the weights that carry the mask, in its own precision."""
+    box, lx = (16, 16, 8), 8
+
+    def allocated(masked):
+        c = pkg.coef_t.box(*box, lx, device=dev)
+        if masked:
+            c.set_mask(T(orc.mask_face_xmax(*box, lx), dev, torch.int32), base=1)
+        c.set_coefs(h1c=1.0, h2c=1.0, ifh2=True)
+        f = c.rhs_assemble(torch.ones(c.n, dtype=torch.float64, device=dev))
+        ksp, x = pkg.krylov_solver_factory(c, method, 3, 1e-14), torch.zeros_like(f)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        ksp.solve(x, f)
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0], c.n
+
+    (a, n), (b, _) = allocated(True), allocated(False)
+    # the driver hands memory out in pieces of 2 MiB
+    assert abs(a - b - bytes_per_node * n) <= 1 << 21
