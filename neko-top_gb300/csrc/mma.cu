@@ -448,10 +448,11 @@ int subsolve(ntg_mma* o, double* designx) {
     NTG_TRY(fetch(o, NS + 1));
     double residunorm, residumax;
     combine(o, o->out_h, y, z, lam, s, mu, zeta, epsi, residunorm, residumax);
+    // the sums of the pass over the current point (out_h serves the direction's maximum too)
+    std::vector<double> out(o->out_h, o->out_h + NS);
     for (int it = 0; it < o->max_iter; ++it) {
       if (residumax < epsi) break;
       ++o->newton_steps;
-      const double* out = o->out_h;  // of the pass over the current point
       std::vector<double> dely(m), dellam(m), bb(m + 1), AA((m + 1) * (m + 1));
       double delz = o->a0 - epsi / z;
       for (int i = 0; i < m; ++i) delz -= lam[i] * o->a[i];
@@ -527,6 +528,9 @@ int subsolve(ntg_mma* o, double* designx) {
         steg = steg / 2.0;
       }
       residunorm = newres;
+      // a residual that is infinite or NaN leaves no trial to take: the point stays
+      if (itto == 0) continue;
+      out.assign(o->out_h, o->out_h + NS);
       std::swap(o->V.x, o->V.xt);
       std::swap(o->V.xsi, o->V.xsit);
       std::swap(o->V.eta, o->V.etat);
