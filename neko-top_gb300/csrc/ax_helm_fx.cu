@@ -22,7 +22,9 @@ struct FxAxShape {
   static constexpr size_t SMEM = EPB * (3 * TILE * sizeof(double) + 2 * LX2 * sizeof(int));
 };
 
-template <int LX, bool DOT>
+// FIELD: h1 is a field (the fluxes' guard, fx::flux_line); null otherwise.  The
+// pointer is tested all the same: products by h1s alone would be predicated.
+template <int LX, bool FIELD, bool DOT>
 __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
     k_ax_fx(double* __restrict__ w, const double* __restrict__ u, const double* __restrict__ g11,
             const double* __restrict__ g12, const double* __restrict__ g13, const double* __restrict__ g22,
@@ -62,13 +64,13 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
       double x[LX];
 #pragma unroll
       for (int l = 0; l < LX; ++l) x[l] = U[ro + l];
-      fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) { R[ro + A] = y; });
+      fx::line_dbl<LX, LX, true>(P.D, P.d, x, false, [&](int A, double y) { R[ro + A] = y; });
 #pragma unroll
       for (int l = 0; l < LX; ++l) x[l] = U[so + l * RS];
-      fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) { V[so + A * RS] = y; });
+      fx::line_dbl<LX, LX, true>(P.D, P.d, x, false, [&](int A, double y) { V[so + A * RS] = y; });
 #pragma unroll
       for (int l = 0; l < LX; ++l) x[l] = wt[l];
-      fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) { wt[A] = y; });
+      fx::line_dbl<LX, LX, true>(P.D, P.d, x, false, [&](int A, double y) { wt[A] = y; });
     }
     __syncthreads();
     if (act) {
@@ -100,13 +102,12 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
       double x[LX];
 #pragma unroll
       for (int l = 0; l < LX; ++l) x[l] = R[ro + l];
-      kr[ab] = fx::line_int<LX, LX, true>(P.DT, P.dt, x,
-                                          [&](int A, int64_t y) { R[ro + A] = __longlong_as_double(y); });
+      kr[ab] = fx::line_int_to<LX, LX, true>(P.DT, P.dt, x, FIELD, R + ro, 1);
 #pragma unroll
       for (int l = 0; l < LX; ++l) x[l] = V[so + l * RS];
-      ks[ab] = fx::line_int<LX, LX, true>(P.DT, P.dt, x,
-                                          [&](int A, int64_t y) { V[so + A * RS] = __longlong_as_double(y); });
-      kt = fx::line_int<LX, LX, true>(P.DT, P.dt, wt, [&](int A, int64_t y) { Y[A] = y; });
+      ks[ab] = fx::line_int_to<LX, LX, true>(P.DT, P.dt, x, FIELD, V + so, RS);
+      kt = fx::line_int<LX, LX, true>(
+          P.DT, P.dt, wt, FIELD, [&](int A, int64_t y) { Y[A] = y; }, [&](int A) { return Y[A]; });
     }
     __syncthreads();
     if (act) {
@@ -134,27 +135,30 @@ __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
   }
 }
 
-template <int LX>
+template <int LX, bool FIELD, bool DOT>
 static int launch_fx(ntg_plan* p, double* w, const double* u, const double* const* g, const double* h1, double h1c,
                      const double* hB, Scalars* sc, cudaStream_t s) {
   using S = FxAxShape<LX>;
-  const double fold = !h1 && fx::foldable(h1c) ? h1c : 1.0;  // a constant h1 goes into D^T
-  const double h1s = h1 || fold == h1c ? 1.0 : h1c;
+  const double fold = !FIELD && fx::foldable(h1c) ? h1c : 1.0;  // a constant h1 goes into D^T
+  const double h1s = FIELD || fold == h1c ? 1.0 : h1c;
   const fx::Mats<LX> P = fx::plan_mats<LX>(p, fold);
-  const int64_t ngroups = (p->nelv + S::EPB - 1) / S::EPB, cap = sc ? kRedSlots : (int64_t)1 << 30;
+  const int64_t ngroups = (p->nelv + S::EPB - 1) / S::EPB, cap = DOT ? kRedSlots : (int64_t)1 << 30;
   const int grid = (int)(ngroups < cap ? ngroups : cap);
-  if (sc) {
-    NTG_TRY((fx::use_smem<k_ax_fx<LX, true>>(S::SMEM)));
-    k_ax_fx<LX, true><<<grid, S::NT, S::SMEM, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1s, hB, p->nelv, P,
-                                                   p->red_part, sc);
-  } else {
-    NTG_TRY((fx::use_smem<k_ax_fx<LX, false>>(S::SMEM)));
-    k_ax_fx<LX, false><<<grid, S::NT, S::SMEM, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1s, hB, p->nelv, P,
+  NTG_TRY((fx::use_smem<k_ax_fx<LX, FIELD, DOT>>(S::SMEM)));
+  k_ax_fx<LX, FIELD, DOT><<<grid, S::NT, S::SMEM, s>>>(w, u, g[0], g[1], g[2], g[3], g[4], g[5], h1, h1s, hB, p->nelv, P,
                                                     p->red_part, sc);
-  }
   NTG_COUNT_LAUNCH();
   NTG_CUDA_TRY(cudaGetLastError());
   return NTG_OK;
+}
+
+template <int LX>
+static int launch_fx(ntg_plan* p, double* w, const double* u, const double* const* g, const double* h1, double h1c,
+                     const double* hB, Scalars* sc, cudaStream_t s) {
+  if (h1) return sc ? launch_fx<LX, true, true>(p, w, u, g, h1, h1c, hB, sc, s)
+                    : launch_fx<LX, true, false>(p, w, u, g, h1, h1c, hB, sc, s);
+  return sc ? launch_fx<LX, false, true>(p, w, u, g, h1, h1c, hB, sc, s)
+            : launch_fx<LX, false, false>(p, w, u, g, h1, h1c, hB, sc, s);
 }
 
 int ax_launch(ntg_plan* p, double* w, const double* u, Scalars* dot_scal, int, cudaStream_t s) {

@@ -202,7 +202,7 @@ __device__ __forceinline__ void line_at(const fx::Mat<NIN, NOUT>& M, const doubl
   double x[NIN];
 #pragma unroll
   for (int l = 0; l < NIN; ++l) x[l] = in[l * si];
-  fx::line_dbl<NIN, NOUT, ANTI>(M, Md, x, [&](int A, double y) { out[A * so] = y; });
+  fx::line_dbl<NIN, NOUT, ANTI>(M, Md, x, false, [&](int A, double y) { out[A * so] = y; });
 }
 
 // MODE 0: adjoint, MODE 1: linear
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
           double x[LXD];
 #pragma unroll
           for (int l = 0; l < LXD; ++l) x[l] = v[l * st];
-          fx::line_dbl<LXD, LXD, true>(P.D, P.d, x, [&](int A, double y) { a[A] = fma(y, u[A * st], a[A]); });
+          fx::line_dbl<LXD, LXD, true>(P.D, P.d, x, false, [&](int A, double y) { a[A] = fma(y, u[A * st], a[A]); });
         }
         double* o = T + (9 + d) * TS + b;
 #pragma unroll
@@ -294,8 +294,7 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
           double x[LXD];
 #pragma unroll
           for (int l = 0; l < LXD; ++l) x[l] = u[l * st] * v[l * st];
-          reinterpret_cast<int*>(T + 12 * TS)[t] = fx::line_int<LXD, LXD, true>(
-              P.DT, P.dt, x, [&](int A, int64_t y) { o[A * st] = __longlong_as_double(y); });
+          reinterpret_cast<int*>(T + 12 * TS)[t] = fx::line_int_to<LXD, LXD, true>(P.DT, P.dt, x, false, o, st);
         });
         __syncthreads();
         items(G3, [&](double* T, int node, int64_t) {
@@ -329,7 +328,7 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
             double x[LXD];
 #pragma unroll
             for (int l = 0; l < LXD; ++l) x[l] = in[l * st];
-            fx::line_dbl<LXD, LXD, true>(P.D, P.d, x, [&](int A, double y) {
+            fx::line_dbl<LXD, LXD, true>(P.D, P.d, x, false, [&](int A, double y) {
               o[A * st] = fma(y, v[A * st], o[A * st]);
             });
           });

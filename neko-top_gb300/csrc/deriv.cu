@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(FxShape<LX, 9>::NT, FxShape<LX, 9>::MINB)
         double x[LX];
 #pragma unroll
         for (int l = 0; l < LX; ++l) x[l] = v[l * st];
-        fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) { a[A] = fma(y, u[A * st], a[A]); });
+        fx::line_dbl<LX, LX, true>(P.D, P.d, x, true, [&](int A, double y) { a[A] = fma(y, u[A * st], a[A]); });
       }
 #pragma unroll
       for (int l = 0; l < LX; ++l) T[(6 + d) * TS + b + l * st] = a[l];
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(FxShape<LX, 9>::NT, FxShape<LX, 9>::MINB)
           double x[LX];
 #pragma unroll
           for (int l = 0; l < LX; ++l) x[l] = in[l * st];
-          fx::line_dbl<LX, LX, true>(P.D, P.d, x, [&](int A, double y) {
+          fx::line_dbl<LX, LX, true>(P.D, P.d, x, true, [&](int A, double y) {
             o[A * st] = fma(y, v[A * st], o[A * st]);
           });
         }

@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(DiagShape<LX>::NT)
     double x[LX];
 #pragma unroll
     for (int a = 0; a < LX; ++a) x[a] = l[a * st];
-    fx::line_dbl<LX, LX, false>(P.D2, P.d2, x, [&](int A, double y) { l[A * st] = y; });
+    fx::line_dbl<LX, LX, false>(P.D2, P.d2, x, true, [&](int A, double y) { l[A * st] = y; });
   }
   __syncthreads();
   for (int t = threadIdx.x; t < ne * L3; t += NT) {

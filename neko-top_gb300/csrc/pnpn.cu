@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(FxShape<LX, 4>::NT, FxShape<LX, 4>::MINB)
     NTG_FX_NE;
     NTG_FX_NODES { NTG_FX_NODE T[p] = pp[q]; }
     __syncthreads();
-    NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T, T + (1 + d) * TS, d, lq); }
+    NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T, T + (1 + d) * TS, d, lq, false); }
     __syncthreads();
     NTG_FX_NODES {
       NTG_FX_NODE
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(FxShape<LX, 7>::NT, FxShape<LX, 7>::MINB)
       __syncthreads();
       NTG_FX_NODES { NTG_FX_NODE T[3 * TS + p] = u[q]; }
       __syncthreads();
-      NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T + 3 * TS, T + (4 + d) * TS, d, lq); }
+      NTG_FX_LINES { NTG_FX_LINE fx::deriv_line<LX>(P.D, P.d, T + 3 * TS, T + (4 + d) * TS, d, lq, false); }
       __syncthreads();
       NTG_FX_NODES {
         NTG_FX_NODE
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(FxShape<LX, 7>::NT, FxShape<LX, 7>::MINB)
       __syncthreads();
       NTG_FX_LINES {
         NTG_FX_LINE
-        fx::flux_line<LX>(P.DT, P.dt, T + (4 + d) * TS, reinterpret_cast<int*>(T + 7 * TS) + r, d, lq);
+        fx::flux_line<LX>(P.DT, P.dt, T + (4 + d) * TS, reinterpret_cast<int*>(T + 7 * TS) + r, d, lq, c.mu != nullptr);
       }
       __syncthreads();
       NTG_FX_NODES {
