@@ -29,9 +29,13 @@ namespace ntg {
 //   + 2 h1 (D_ii D_jj G12 + D_ii D_kk G13 + D_jj D_kk G23) + h2 B
 // ---------------------------------------------------------------------------
 // The sums are the transposed line operator with the squared entries of D
-// acting on G11 h1 along r, G22 h1 along s and G33 h1 along t: fixed point
-// on the integer pipes (fx.cuh), an element per block.  (As FP64 FMAs with a
-// thread per node it took 1.12 ms at 24^3 elements, lx = 8.)
+// acting on G11 h1 along r, G22 h1 along s and G33 h1 along t, a line per
+// thread.  With a constant h1 they run in fixed point on the integer pipes
+// (fx.cuh).  A field h1 may jump inside an element, and the squares of a row of
+// D range over a factor of 1e3 and more, so that a node's integer sum would have
+// some hundred times the error of FP64 sums: those are FP64 FMAs, which the
+// FP64 pipe bounds.  With the gather-scatter and the reciprocals at 24^3
+// elements, lx = 8: 314 us and 656 us (a thread per node and FP64: 1244 us).
 template <int LX>
 struct DiagMats {
   fx::Mat<LX, LX> D2;
@@ -47,7 +51,7 @@ struct DiagShape {
   static constexpr size_t SMEM = sizeof(double) * EPB * 3 * TS;
 };
 
-template <int LX>
+template <int LX, bool FIELD>
 __global__ void __launch_bounds__(DiagShape<LX>::NT)
     k_helm_diag(int64_t nelv, const __grid_constant__ DiagMats<LX> P, const double* __restrict__ g11,
                 const double* __restrict__ g12, const double* __restrict__ g13, const double* __restrict__ g22,
@@ -76,7 +80,17 @@ __global__ void __launch_bounds__(DiagShape<LX>::NT)
     double x[LX];
 #pragma unroll
     for (int a = 0; a < LX; ++a) x[a] = l[a * st];
-    fx::line_dbl<LX, LX, false>(P.D2, P.d2, x, true, [&](int A, double y) { l[A * st] = y; });
+    if constexpr (FIELD) {
+#pragma unroll
+      for (int A = 0; A < LX; ++A) {
+        double acc = 0.0;
+#pragma unroll
+        for (int a = 0; a < LX; ++a) acc = fma(P.d2[A * LX + a], x[a], acc);
+        l[A * st] = acc;
+      }
+    } else {
+      fx::line_dbl<LX, LX, false>(P.D2, P.d2, x, false, [&](int A, double y) { l[A * st] = y; });
+    }
   }
   __syncthreads();
   for (int t = threadIdx.x; t < ne * L3; t += NT) {
@@ -106,8 +120,14 @@ int helm_diag(ntg_plan* p, cudaStream_t s) {
     P.dd[i] = p->D[i * LX + i];
   }
   P.D2 = fx::make_mat<LX, LX>(m);
-  NTG_TRY(fx::use_smem<k_helm_diag<LX>>(S::SMEM));
-  k_helm_diag<LX><<<(unsigned)((p->nelv + S::EPB - 1) / S::EPB), S::NT, S::SMEM, s>>>(
+  auto kern = k_helm_diag<LX, false>;
+  if (p->h1_const) {
+    NTG_TRY((fx::use_smem<k_helm_diag<LX, false>>(S::SMEM)));
+  } else {
+    NTG_TRY((fx::use_smem<k_helm_diag<LX, true>>(S::SMEM)));
+    kern = k_helm_diag<LX, true>;
+  }
+  kern<<<(unsigned)((p->nelv + S::EPB - 1) / S::EPB), S::NT, S::SMEM, s>>>(
       p->nelv, P, p->g[0], p->g[1], p->g[2], p->g[3], p->g[4], p->g[5], p->h1_const ? nullptr : p->h1, p->h1c,
       p->ifh2 ? p->hB : nullptr, p->dinv);
   NTG_COUNT_LAUNCH();
