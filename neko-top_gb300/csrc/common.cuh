@@ -196,9 +196,7 @@ void timer_stop(int id, cudaStream_t s);
 // is the launch and the last blocks of the kernel before.  A kernel that begins
 // with dependent_wait() may be launched by launch_dependent() while its
 // predecessor still runs: it waits for the predecessor's end (which waited for
-// everything before it) before it touches memory.  Only what the host has seen
-// completed before it launched anything of the call may be read ahead of the
-// wait (the coarse solve's matrices).  dependent_start() also lets
+// everything before it) before it touches memory.  dependent_start() also lets
 // the successor be scheduled.  k_fdm leaves that out (0.4% of a solve at 43M
 // nodes for the instruction alone), and the FP64 operator takes no part: with
 // its successors waiting beside it an FP64 solve at 0.26M nodes went from 38.7

@@ -614,10 +614,15 @@ __global__ void __launch_bounds__(kCrsThreads)
   const CrsPad q(d);
   const int m0 = d.m[0], m1 = d.m[1];
   float *A = csm, *B = A + q.p1 * q.p0, *X = B + q.p1 * q.p0, *Y = X + q.p0 * q.p0;
-  crs_stage(X, S0, m0, q.p0);  // the matrices are complete before any launch: the one thing read ahead of the wait
-  crs_stage(Y, S1, m1, q.p1);
+  // the matrices are set up long before, and the kernels that set sc->done have
+  // ended before the one ahead of this began: both are read before the wait
+  const bool done = sc && sc->done;
+  if (!done) {
+    crs_stage(X, S0, m0, q.p0);
+    crs_stage(Y, S1, m1, q.p1);
+  }
   dependent_start();
-  if (sc && sc->done) return;
+  if (done) return;
   for (int t = threadIdx.x; t < q.p1 * q.p0; t += kCrsThreads) {
     const int y = t / q.p0, x = t - y * q.p0;
     A[t] = y < m1 && x < m0 ? crs_vertex(corner, d, x, y, blockIdx.x) : 0.f;
@@ -638,10 +643,13 @@ __global__ void __launch_bounds__(kCrsThreads)
   const CrsPad q(d);
   const int m0 = d.m[0], m1 = d.m[1], m2 = d.m[2], n = m0 * m1;
   float *A = csm, *B = A + q.p2 * kCrsCols, *Z = B + q.p2 * kCrsCols, *ZT = Z + q.p2 * q.p2;
-  crs_stage(Z, S2, m2, q.p2);
-  crs_stage(ZT, S2 + (int64_t)m2 * m2, m2, q.p2);
+  const bool done = sc && sc->done;
+  if (!done) {
+    crs_stage(Z, S2, m2, q.p2);
+    crs_stage(ZT, S2 + (int64_t)m2 * m2, m2, q.p2);
+  }
   dependent_start();
-  if (sc && sc->done) return;
+  if (done) return;
   const int c0 = blockIdx.x * kCrsCols, cols = min(kCrsCols, n - c0);
   for (int t = threadIdx.x; t < m2 * kCrsCols; t += kCrsThreads) {
     const int z = t / kCrsCols, c = t - z * kCrsCols;
@@ -671,10 +679,13 @@ __global__ void __launch_bounds__(kCrsThreads)
   const CrsPad q(d);
   const int m0 = d.m[0], m1 = d.m[1];
   float *A = csm, *B = A + q.p1 * q.p0, *X = B + q.p1 * q.p0, *Y = X + q.p0 * q.p0;
-  crs_stage(X, S0 + (int64_t)m0 * m0, m0, q.p0);
-  crs_stage(Y, S1 + (int64_t)m1 * m1, m1, q.p1);
+  const bool done = sc && sc->done;
+  if (!done) {
+    crs_stage(X, S0 + (int64_t)m0 * m0, m0, q.p0);
+    crs_stage(Y, S1 + (int64_t)m1 * m1, m1, q.p1);
+  }
   dependent_start();
-  if (sc && sc->done) return;
+  if (done) return;
   const float* src = in + (int64_t)blockIdx.x * m0 * m1;
   for (int t = threadIdx.x; t < q.p1 * q.p0; t += kCrsThreads) {
     const int y = t / q.p0, x = t - y * q.p0;
