@@ -196,9 +196,10 @@ void timer_stop(int id, cudaStream_t s);
 // is the launch and the last blocks of the kernel before.  A kernel that begins
 // with dependent_wait() may be launched by launch_dependent() while its
 // predecessor still runs: it waits for the predecessor's end (which waited for
-// everything before it) before it touches memory.  dependent_start() also lets
+// everything before it) before it touches memory.  (Exceptions, each with its
+// reason: the coarse solve's matrices and stop flag.)  dependent_start() also lets
 // the successor be scheduled.  k_fdm leaves that out (0.4% of a solve at 43M
-// nodes for the instruction alone), and the FP64 operator takes no part: with
+// nodes for the instruction alone; the coarse solve relies on it), and the FP64 operator takes no part: with
 // its successors waiting beside it an FP64 solve at 0.26M nodes went from 38.7
 // to 43.9 ms, without from 38.7 to 35.1.
 //
