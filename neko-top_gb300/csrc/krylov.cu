@@ -292,6 +292,24 @@ struct FinUpd {
   }
 };
 
+// A grid-stride loop for FP32 per-thread sums, two items' sums at a time: the
+// chains of additions are then as short as with grid_for's blocks, of which
+// grid_red launches half.  item(i, t) adds its terms to t.
+template <int NS, typename F>
+__device__ __forceinline__ void sum_pairs(int64_t n, float (&s)[NS], F&& item) {
+  const int64_t gs = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += 2 * gs) {
+    float t[NS] = {};
+#pragma unroll
+    for (int64_t i = i0; i < i0 + 2 * gs; i += gs) {
+      if (i >= n) break;
+      item(i, t);
+    }
+#pragma unroll
+    for (int q = 0; q < NS; ++q) s[q] += t[q];
+  }
+}
+
 // the sign bit, without a slot of the FP64 pipe
 __device__ __forceinline__ bool is_neg(double m) { return __double2hiint(m) < 0; }
 __device__ __forceinline__ bool is_neg(float m) { return __float_as_int(m) < 0; }
@@ -309,18 +327,23 @@ __global__ void k_cg_update(T* __restrict__ x, const T* __restrict__ p, T* __res
   // per-thread partials in T: FP64 arithmetic is 1/58 of FP32 on GB300, so
   // the FP32 iteration accumulates its short per-thread sums in FP32 and
   // only the block/grid levels in FP64
-  T rz = 0, rr = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  T s[2] = {0, 0};  // (r, z), (r, r)
+  auto item = [&](int64_t i, T(&a)[2]) {
     const T ms = mult[i], m = fabs(ms);
     if (X) x[i] += alpha * p[i];
     T ri = r[i];
     if (!is_neg(ms)) ri -= alpha * w[i];
     r[i] = ri;
     const T t = (m * ri) * ri;
-    rz += t * dinv[i];
-    rr += t;
+    a[0] += t * dinv[i];
+    a[1] += t;
+  };
+  if constexpr (sizeof(T) == 4) {
+    sum_pairs(n, s, item);
+  } else {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) item(i, s);
   }
-  double v[2] = {(double)rz, (double)rr};
+  double v[2] = {(double)s[0], (double)s[1]};
   grid_reduce<2>(v, part, sc, FinUpd());
 }
 
@@ -599,8 +622,8 @@ __global__ void k_ru_init(const double* __restrict__ f, const double* __restrict
                           float* __restrict__ p32, float* __restrict__ y32, int64_t n, double* __restrict__ part,
                           Scalars* sc) {
   double ff = 0, rr = 0;
-  float rz = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  float rz[1] = {0};
+  sum_pairs(n, rz, [&](int64_t i, float(&t)[1]) {
     const double fi = f[i];
     const double ri = w ? fi - w[i] : fi;
     const float rf = (float)ri;
@@ -612,9 +635,9 @@ __global__ void k_ru_init(const double* __restrict__ f, const double* __restrict
     const double m = mult[i];
     ff += m * fi * fi;
     rr += m * ri * ri;
-    rz += (float)m * rf * zf;
-  }
-  double v[3] = {ff, rr, (double)rz};
+    t[0] += (float)m * rf * zf;
+  });
+  double v[3] = {ff, rr, (double)rz[0]};
   grid_reduce<3>(v, part, sc, FinRUInit());
 }
 
@@ -675,21 +698,21 @@ __global__ void k_update_rr(float* __restrict__ r, const float* __restrict__ w, 
   dependent_start();
   if (sc->done) return;
   const float alpha = (float)sc->alpha;
-  float rr = 0.f;
+  float rr[1] = {0.f};
   const int64_t n4 = n >> 2, g0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, gs = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t i = g0; i < n4; i += gs) {
+  sum_pairs(n4, rr, [&](int64_t i, float(&t)[1]) {
     const float4 w4 = reinterpret_cast<const float4*>(w)[i], m4 = reinterpret_cast<const float4*>(mult)[i];
     float4 r4 = reinterpret_cast<float4*>(r)[i];
     r4.x -= alpha * w4.x; r4.y -= alpha * w4.y; r4.z -= alpha * w4.z; r4.w -= alpha * w4.w;
     reinterpret_cast<float4*>(r)[i] = r4;
-    rr += m4.x * r4.x * r4.x + m4.y * r4.y * r4.y + m4.z * r4.z * r4.z + m4.w * r4.w * r4.w;
-  }
+    t[0] += m4.x * r4.x * r4.x + m4.y * r4.y * r4.y + m4.z * r4.z * r4.z + m4.w * r4.w * r4.w;
+  });
   for (int64_t i = 4 * n4 + g0; i < n; i += gs) {
     const float ri = r[i] - alpha * w[i];
     r[i] = ri;
-    rr += mult[i] * ri * ri;
+    rr[0] += mult[i] * ri * ri;
   }
-  double v[2] = {0.0, (double)rr};
+  double v[2] = {0.0, (double)rr[0]};
   grid_reduce<2>(v, part, sc, FinUpd());
 }
 
@@ -771,9 +794,10 @@ __global__ void __launch_bounds__(256, 4)
     for (int i = 0; i < LX; ++i) rv.f[i] -= alpha * (((mb >> i) & 1u) ? 0.f : acc[i]);
     store(r + o, rv);
     if ((j > 0 || cy == 0) && (k > 0 || cz == 0)) {
+      float t = cx == 0 ? rv.f[0] * rv.f[0] : 0.f;  // a row's sum first: short chains of additions
 #pragma unroll
-      for (int i = 0; i < LX; ++i)
-        if (i > 0 || cx == 0) rr += rv.f[i] * rv.f[i];
+      for (int i = 1; i < LX; ++i) t += rv.f[i] * rv.f[i];
+      rr += t;
     }
   }
   double v[2] = {0.0, (double)rr};
@@ -806,16 +830,21 @@ __global__ void k_ru_resid(const double* __restrict__ f, const double* __restric
                            const double* __restrict__ mult, const float* __restrict__ multf, double* __restrict__ r,
                            float* __restrict__ r32, int64_t n, int mode, double* __restrict__ part, Scalars* sc) {
   double rr = 0;
-  float rz = 0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  float rz[1] = {0};
+  auto item = [&](int64_t i, float(&t)[1]) {
     const double ri = f[i] - w[i];
     const float rf = (float)ri;
     r[i] = ri;
     r32[i] = rf;
     rr = fma(mult[i] * ri, ri, rr);
-    if (RZ) rz += multf[i] * rf * (dinv[i] * rf);
+    if (RZ) t[0] += multf[i] * rf * (dinv[i] * rf);
+  };
+  if constexpr (RZ) {
+    sum_pairs(n, rz, item);
+  } else {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) item(i, rz);
   }
-  double v[2] = {rr, (double)rz};
+  double v[2] = {rr, (double)rz[0]};
   grid_reduce<2>(v, part, sc, FinRU{mode});
 }
 

@@ -849,9 +849,10 @@ __global__ void __launch_bounds__(256, 4)
       // no lower neighbour in any direction): the sum over unique nodes that
       // the mult-weighted sum over local copies equals, without the mult stream
       if ((j > 0 || cy == 0) && (k > 0 || cz == 0)) {
+        float t = cx == 0 ? rv[0] * acc[0] : 0.f;  // a row's sum first, as in k_update_box
 #pragma unroll
-        for (int i = 0; i < LX; ++i)
-          if (i > 0 || cx == 0) rz += rv[i] * acc[i];
+        for (int i = 1; i < LX; ++i) t += rv[i] * acc[i];
+        rz += t;
       }
     }
   }
