@@ -4,8 +4,11 @@
 // threads per SM, timed with CUDA events on the given stream.
 //
 // A measurement tool, not part of the drop-in: it is built into its own
-// library (lib/libntgb300_probe.so) that only bench.py --fp64-peak loads.
+// library (lib/libntgb300_probe.so) that only bench.py --fp64-peak and the test
+// of the library's reciprocal (csrc/rcp.cuh) load.
 #include <cuda_runtime.h>
+
+#include "../csrc/rcp.cuh"
 
 namespace {
 
@@ -23,7 +26,19 @@ __global__ void __launch_bounds__(256) k_fp64_fma(double* __restrict__ out, int 
   out[blockIdx.x * blockDim.x + threadIdx.x] = s;  // keeps the chains live
 }
 
+__global__ void k_rcp(const double* __restrict__ x, double* __restrict__ y, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    y[i] = ntg::rcp(x[i]);
+}
+
 }  // namespace
+
+// y[i] = the library's reciprocal of x[i] (device pointers); 0 or a CUDA error code
+extern "C" __attribute__((visibility("default"))) int ntgprobe_rcp(const double* x, double* y, long long n, void* stream) {
+  if (!x || !y || n <= 0) return -1;
+  k_rcp<<<1024, 256, 0, (cudaStream_t)stream>>>(x, y, n);
+  return (int)cudaGetLastError();
+}
 
 // Returns 0 and the FMA rate in TFLOP/s (an FMA counts 2), or a CUDA error
 // code.

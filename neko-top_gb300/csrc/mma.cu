@@ -14,13 +14,14 @@
 // totals come back in one small copy, the GPU stand-in for the reference's
 // MPI_Allreduce calls.  m <= 4 constraints.
 //
-// The FP64 pipe bounds it, mostly with the reciprocals (rcp below): a design
+// The FP64 pipe bounds it, mostly with the reciprocals (rcp.cuh): a design
 // update of 16.8M variables, m = 1, took 91.6 ms with the trial's residual and
 // the next Newton assembly in separate passes, each with divisions of its own,
 // and takes 56.0 with one (k_point).
 #include <cmath>
 #include <vector>
 
+#include "rcp.cuh"
 #include "reduce.cuh"
 
 namespace ntg {
@@ -32,17 +33,6 @@ constexpr int LANES = 2 * MMAX + MMAX * (MMAX + 1) / 2 + 2;  // sums + 1 max
 
 // the reference's default-kind (single precision) literals
 constexpr double C001 = (double)0.01f, C01 = (double)0.1f, C09 = (double)0.9f, C101 = (double)1.01f;
-
-// 1/x by the third-order iteration r (1 + e + e^2), e = 1 - x r (Householder),
-// from the hardware's approximation r0: e0 < 2^-19 leaves e0^3 < 2^-57, the
-// result within an ulp.  The FP64 pipe (2 operations per clock and SM) bounds
-// these kernels; this takes three of them, a division about ten.
-__device__ __forceinline__ double rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double e = fma(-x, r, 1.0);
-  return fma(fma(e, e, e), r, r);
-}
 
 // the larger of a >= 0 and |v| (NaN ignored, as fmax does) on the integer
 // pipes: an FP64 comparison takes a slot of the FP64 pipe
