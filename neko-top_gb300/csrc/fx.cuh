@@ -37,6 +37,7 @@
 #include <cmath>
 #include <memory>
 #include <mutex>
+#include <new>
 
 #include "common.cuh"
 
@@ -142,10 +143,13 @@ Mats<LX> plan_mats(const ntg_plan* p, double scale, bool weighted = false) {
   auto& c = p->fx->mats;
   for (auto& e : c)
     if (e.scale == scale && e.weighted == weighted) return *static_cast<const Mats<LX>*>(e.mats.get());
-  if (c.size() >= 6) c.erase(c.begin());
-  auto m = std::make_shared<Mats<LX>>(make_mats<LX>(p->D, weighted ? p->wq : nullptr, scale));
-  c.push_back({scale, weighted, m});
-  return *m;
+  const Mats<LX> m = make_mats<LX>(p->D, weighted ? p->wq : nullptr, scale);
+  try {
+    if (c.size() >= 6) c.erase(c.begin());
+    c.push_back({scale, weighted, std::make_shared<Mats<LX>>(m)});
+  } catch (const std::bad_alloc&) {  // not kept, then: no exception leaves the C entry points
+  }
+  return m;
 }
 
 // whether a constant factor may be folded into a matrix (its exponent offset must stay small)
