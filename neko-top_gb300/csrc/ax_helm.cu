@@ -20,41 +20,41 @@
 
 namespace ntg {
 
-template <typename T, int LX>
+template <int LX>
 struct DParam {
-  T d[LX * LX];
+  float d[LX * LX];
 };
 
-template <typename T, int LX>
+template <int LX>
 struct AxShape {
   static constexpr int LX2 = LX * LX, LX3 = LX * LX * LX;
   static constexpr int EPB_T = (256 / LX2) < 1 ? 1 : ((256 / LX2) > 8 ? 8 : 256 / LX2);
-  static constexpr int EPB_S = 49152 / (3 * LX3 * (int)sizeof(T));
+  static constexpr int EPB_S = 49152 / (3 * LX3 * (int)sizeof(float));
   static constexpr int EPB = EPB_T < EPB_S ? EPB_T : (EPB_S < 1 ? 1 : EPB_S);
   static constexpr int NW = LX2 * EPB;             // working threads
   static constexpr int NT = (NW + 31) / 32 * 32;   // launched threads
 };
 
-template <typename T, int LX, bool H1ARR, bool H2, bool DOT, bool DIR = false>
-__global__ void __launch_bounds__(AxShape<T, LX>::NT)
-    k_ax_helm(T* __restrict__ w, const T* __restrict__ u, const T* __restrict__ g11, const T* __restrict__ g12,
-              const T* __restrict__ g13, const T* __restrict__ g22, const T* __restrict__ g23,
-              const T* __restrict__ g33, const T* __restrict__ h1, T h1c, const T* __restrict__ hB, int64_t nelv,
-              const __grid_constant__ DParam<T, LX> Dp, double* __restrict__ part, Scalars* sc, AxDir dir) {
-  using S = AxShape<T, LX>;
+template <int LX, bool H1ARR, bool H2, bool DOT, bool DIR = false>
+__global__ void __launch_bounds__(AxShape<LX>::NT)
+    k_ax_helm(float* __restrict__ w, const float* __restrict__ u, const float* __restrict__ g11,
+              const float* __restrict__ g12, const float* __restrict__ g13, const float* __restrict__ g22,
+              const float* __restrict__ g23, const float* __restrict__ g33, const float* __restrict__ h1, float h1c,
+              const float* __restrict__ hB, int64_t nelv, const __grid_constant__ DParam<LX> Dp, double* __restrict__ part, Scalars* sc, AxDir dir) {
+  using S = AxShape<LX>;
   constexpr int LX2 = S::LX2, LX3 = S::LX3, EPB = S::EPB;
   dependent_start();
   if (DOT && sc->done) return;
-  const T alpha = DIR ? (T)sc->alpha : T(0), beta = DIR ? (T)sc->beta : T(0);
-  __shared__ T s_u[EPB][LX3];
-  __shared__ T s_r[EPB][LX3];
-  __shared__ T s_s[EPB][LX3];
+  const float alpha = DIR ? (float)sc->alpha : 0.f, beta = DIR ? (float)sc->beta : 0.f;
+  __shared__ float s_u[EPB][LX3];
+  __shared__ float s_r[EPB][LX3];
+  __shared__ float s_s[EPB][LX3];
   const int tid = threadIdx.x;
   const bool worker = tid < S::NW;
   const int le = worker ? tid / LX2 : 0;  // element slot in the block
   const int ij = worker ? tid - le * LX2 : 0;
   const int i = ij % LX, j = ij / LX;
-  T Dri[LX], Dsj[LX], DTi[LX], DTj[LX];
+  float Dri[LX], Dsj[LX], DTi[LX], DTj[LX];
 #pragma unroll
   for (int l = 0; l < LX; ++l) {
     Dri[l] = Dp.d[i * LX + l];
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
     DTi[l] = Dp.d[l * LX + i];
     DTj[l] = Dp.d[l * LX + j];
   }
-  T dot = 0;  // per-thread partial in the kernel's precision (FP64 math is scarce on GB300)
+  float dot = 0.f;  // per-thread partial in FP32 (FP64 math is scarce on GB300)
   const int64_t ngroups = (nelv + EPB - 1) / EPB;
   for (int64_t grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
     const int64_t e = grp * EPB + le;
@@ -71,24 +71,24 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
     // every stream's loads first: the bytes in flight bound this kernel.  With
     // the metric loads between the contractions the operator, gather-scatter and
     // preconditioner of 4641 elements of lx = 6 took 89 us, so 81
-    T ureg[LX], G[6][LX], hh[LX], zv[LX], yv[LX];
+    float ureg[LX], G[6][LX], hh[LX], zv[LX], yv[LX];
 #pragma unroll
     for (int k = 0; k < LX; ++k) {
       const int64_t q = base + k * LX2;
       if constexpr (DIR) {
-        ureg[k] = active && dir.mode != 1 ? dir.p[q] : T(0);
-        zv[k] = active ? dir.z[q] : T(0);
-        yv[k] = active && dir.mode == 0 ? dir.y[q] : T(0);
+        ureg[k] = active && dir.mode != 1 ? dir.p[q] : 0.f;
+        zv[k] = active ? dir.z[q] : 0.f;
+        yv[k] = active && dir.mode == 0 ? dir.y[q] : 0.f;
       } else {
-        ureg[k] = active ? u[q] : T(0);
+        ureg[k] = active ? u[q] : 0.f;
       }
-      G[0][k] = active ? g11[q] : T(0);
-      G[1][k] = active ? g12[q] : T(0);
-      G[2][k] = active ? g13[q] : T(0);
-      G[3][k] = active ? g22[q] : T(0);
-      G[4][k] = active ? g23[q] : T(0);
-      G[5][k] = active ? g33[q] : T(0);
-      if (H1ARR) hh[k] = active ? h1[q] : T(0);
+      G[0][k] = active ? g11[q] : 0.f;
+      G[1][k] = active ? g12[q] : 0.f;
+      G[2][k] = active ? g13[q] : 0.f;
+      G[3][k] = active ? g22[q] : 0.f;
+      G[4][k] = active ? g23[q] : 0.f;
+      G[5][k] = active ? g33[q] : 0.f;
+      if (H1ARR) hh[k] = active ? h1[q] : 0.f;
     }
     if constexpr (DIR) {
 #pragma unroll
@@ -103,20 +103,20 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
     for (int k = 0; k < LX; ++k)
       if (worker) s_u[le][ij + k * LX2] = ureg[k];
     __syncthreads();
-    T wt[LX];
+    float wt[LX];
 #pragma unroll
     for (int k = 0; k < LX; ++k) {
-      T ur = 0, us = 0, ut = 0;
+      float ur = 0.f, us = 0.f, ut = 0.f;
 #pragma unroll
       for (int l = 0; l < LX; ++l) {
         ur = fma(Dri[l], s_u[le][k * LX2 + j * LX + l], ur);
         us = fma(Dsj[l], s_u[le][k * LX2 + l * LX + i], us);
         ut = fma(Dp.d[k * LX + l], ureg[l], ut);
       }
-      const T h = H1ARR ? hh[k] : h1c;
-      const T wr = G[0][k] * ur + G[1][k] * us + G[2][k] * ut;
-      const T ws = G[1][k] * ur + G[3][k] * us + G[4][k] * ut;
-      const T wtt = G[2][k] * ur + G[4][k] * us + G[5][k] * ut;
+      const float h = H1ARR ? hh[k] : h1c;
+      const float wr = G[0][k] * ur + G[1][k] * us + G[2][k] * ut;
+      const float ws = G[1][k] * ur + G[3][k] * us + G[4][k] * ut;
+      const float wtt = G[2][k] * ur + G[4][k] * us + G[5][k] * ut;
       if (worker) {
         s_r[le][ij + k * LX2] = h * wr;
         s_s[le][ij + k * LX2] = h * ws;
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < LX; ++k) {
-      T acc = 0;
+      float acc = 0.f;
 #pragma unroll
       for (int l = 0; l < LX; ++l) {
         acc = fma(DTi[l], s_r[le][k * LX2 + j * LX + l], acc);
@@ -154,13 +154,13 @@ __global__ void __launch_bounds__(AxShape<T, LX>::NT)
 int ax_f32_tma_launch(ntg_plan* p, float* w, const float* u, const float* const* g, const float* h1, float h1c,
                       const float* hB, Scalars* sc, const AxDir* dir, cudaStream_t s);
 
-template <typename T, int LX>
-static int launch_lx(ntg_plan* p, T* w, const T* u, const T* const* g, const T* h1, T h1c, const T* hB,
-                     Scalars* sc, const AxDir* dir, cudaStream_t s) {
-  constexpr int EPB = AxShape<T, LX>::EPB;
-  constexpr int NT = AxShape<T, LX>::NT;
-  DParam<T, LX> Dp;
-  for (int q = 0; q < LX * LX; ++q) Dp.d[q] = (T)p->D[q];
+template <int LX>
+static int launch_lx(ntg_plan* p, float* w, const float* u, const float* const* g, const float* h1, float h1c,
+                     const float* hB, Scalars* sc, const AxDir* dir, cudaStream_t s) {
+  constexpr int EPB = AxShape<LX>::EPB;
+  constexpr int NT = AxShape<LX>::NT;
+  DParam<LX> Dp;
+  for (int q = 0; q < LX * LX; ++q) Dp.d[q] = (float)p->D[q];
   int64_t ngroups = (p->nelv + EPB - 1) / EPB;
   int64_t cap = sc ? kRedSlots : (int64_t)num_sms() * 32;
   int grid = (int)(ngroups < cap ? ngroups : cap);
@@ -168,7 +168,7 @@ static int launch_lx(ntg_plan* p, T* w, const T* u, const T* const* g, const T* 
   const AxDir d = dir ? *dir : AxDir{};
 #define NTG_AX_CASE(H1A, HH2, DT, DR)                                                                              \
   if (h1arr == H1A && h2 == HH2 && (sc != nullptr) == DT) {                                                     \
-    NTG_TRY((launch_dependent(p, k_ax_helm<T, LX, H1A, HH2, DT, DR>, grid, NT, 0, s, w, u, g[0], g[1], g[2],    \
+    NTG_TRY((launch_dependent(p, k_ax_helm<LX, H1A, HH2, DT, DR>, grid, NT, 0, s, w, u, g[0], g[1], g[2],    \
                               g[3], g[4], g[5], h1, h1c, hB, p->nelv, Dp, p->red_part, sc, d)));               \
   }
   if (dir) {
@@ -196,19 +196,18 @@ static int launch_lx(ntg_plan* p, T* w, const T* u, const T* const* g, const T* 
   return NTG_OK;
 }
 
-template <typename T>
-static int ax_dispatch(ntg_plan* p, T* w, const T* u, const T* const* g, const T* h1, T h1c, const T* hB,
-                       Scalars* sc, const AxDir* dir, cudaStream_t s) {
+static int ax_dispatch(ntg_plan* p, float* w, const float* u, const float* const* g, const float* h1, float h1c,
+                       const float* hB, Scalars* sc, const AxDir* dir, cudaStream_t s) {
   switch (p->lx) {
-    case 2: return launch_lx<T, 2>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 3: return launch_lx<T, 3>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 4: return launch_lx<T, 4>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 5: return launch_lx<T, 5>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 6: return launch_lx<T, 6>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 7: return launch_lx<T, 7>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 8: return launch_lx<T, 8>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 9: return launch_lx<T, 9>(p, w, u, g, h1, h1c, hB, sc, dir, s);
-    case 10: return launch_lx<T, 10>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 2: return launch_lx<2>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 3: return launch_lx<3>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 4: return launch_lx<4>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 5: return launch_lx<5>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 6: return launch_lx<6>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 7: return launch_lx<7>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 8: return launch_lx<8>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 9: return launch_lx<9>(p, w, u, g, h1, h1c, hB, sc, dir, s);
+    case 10: return launch_lx<10>(p, w, u, g, h1, h1c, hB, sc, dir, s);
     default: set_error("ax_helm: lx=%d not compiled", p->lx); return NTG_ERR_UNSUPPORTED;
   }
 }
@@ -221,7 +220,7 @@ int ax_launch_f32(ntg_plan* p, float* w, const float* u, Scalars* dot_scal, int,
   const float* hB = p->ifh2 ? p->hBf : nullptr;
   int st = NTG_ERR_UNSUPPORTED;
   if (p->lx == 8 && p->use_tma) st = ax_f32_tma_launch(p, w, u, g, h1, (float)p->h1c, hB, dot_scal, dir, s);
-  if (st == NTG_ERR_UNSUPPORTED) st = ax_dispatch<float>(p, w, u, g, h1, (float)p->h1c, hB, dot_scal, dir, s);
+  if (st == NTG_ERR_UNSUPPORTED) st = ax_dispatch(p, w, u, g, h1, (float)p->h1c, hB, dot_scal, dir, s);
   timer_stop(TM_AX32, s);
   return st;
 }

@@ -44,14 +44,12 @@ constexpr int NT = 256;
 template <int LX, int LXD>
 struct GLMat {
   double J[LXD * LX];  // J[A * LX + a] = l_a(xg_A)
-  double D[LXD * LXD]; // D[A * LXD + l] = l_l'(xg_A) on the GL points
-  double w[LXD];
 };
 
 template <int LX, int LXD>
 struct Smem {
   static constexpr int N3 = LXD * LXD * LXD, TA = LXD * LX * LX, TB = LXD * LXD * LX, G3 = LX * LX * LX;
-  static constexpr int DOUBLES = 2 * N3 + TA + TB + LXD * LX + LXD * LXD + LXD;
+  static constexpr int DOUBLES = 2 * N3 + TA + TB + LXD * LX;
   static constexpr size_t BYTES = sizeof(double) * DOUBLES;
 };
 
@@ -87,7 +85,7 @@ __device__ __forceinline__ void to_gl(double* dst, const double* src, double* tA
 // out[c][b][a] (+)= sign * sum J[C][c] J[B][b] J[A][a] src[C][B][A]; out in global memory
 template <int LX, int LXD>
 __device__ __forceinline__ void to_gll(double* __restrict__ out, const double* src, double* tA, double* tB,
-                                       const double* J, bool sub) {
+                                       const double* J) {
   for (int t = threadIdx.x; t < LX * LXD * LXD; t += NT) {
     const int BA = t % (LXD * LXD), c = t / (LXD * LXD);
     double acc = 0.0;
@@ -109,23 +107,9 @@ __device__ __forceinline__ void to_gll(double* __restrict__ out, const double* s
     double acc = 0.0;
 #pragma unroll
     for (int A = 0; A < LXD; ++A) acc = fma(J[A * LX + a], tA[cb * LXD + A], acc);
-    if (sub) out[t] -= acc;
-    else out[t] = acc;
+    out[t] = acc;
   }
   __syncthreads();
-}
-
-template <int LX, int LXD>
-__device__ __forceinline__ double* stage_mats(double* sm, const GLMat<LX, LXD>& M, double*& J, double*& D,
-                                              double*& w) {
-  using S = Smem<LX, LXD>;
-  J = sm + 2 * S::N3 + S::TA + S::TB;
-  D = J + LXD * LX;
-  w = D + LXD * LXD;
-  for (int t = threadIdx.x; t < LXD * LX; t += NT) J[t] = M.J[t];
-  for (int t = threadIdx.x; t < LXD * LXD; t += NT) D[t] = M.D[t];
-  for (int t = threadIdx.x; t < LXD; t += NT) w[t] = M.w[t];
-  return sm;
 }
 
 // out = to_gl(in) (DIR 0) or to_gll(in) (DIR 1) for `nf` fields (stride = field size)
@@ -135,11 +119,11 @@ __global__ void __launch_bounds__(NT) k_map(double* __restrict__ out, const doub
                                             const __grid_constant__ GLMat<LX, LXD> M) {
   using S = Smem<LX, LXD>;
   extern __shared__ double sm[];
-  double *J, *D, *w;
-  stage_mats<LX, LXD>(sm, M, J, D, w);
   double* tile = sm;
   double* tA = sm + 2 * S::N3;
   double* tB = tA + S::TA;
+  double* J = tB + S::TB;
+  for (int t = threadIdx.x; t < LXD * LX; t += NT) J[t] = M.J[t];
   constexpr int NIN = DIR == 0 ? S::G3 : S::N3;
   constexpr int NOUT = DIR == 0 ? S::N3 : S::G3;
   __syncthreads();
@@ -153,7 +137,7 @@ __global__ void __launch_bounds__(NT) k_map(double* __restrict__ out, const doub
         to_gl<LX, LXD>(tile + S::N3, tile, tA, tB, J);
         for (int t = threadIdx.x; t < S::N3; t += NT) dst[t] = tile[S::N3 + t];
       } else {
-        to_gll<LX, LXD>(dst, tile, tA, tB, J, false);
+        to_gll<LX, LXD>(dst, tile, tA, tB, J);
       }
       __syncthreads();
     }
@@ -250,7 +234,7 @@ __global__ void __launch_bounds__(AdvShape<LX, LXD>::NT, AdvShape<LX, LXD>::MINB
     // tiles 0-2: u, 3-5: Ub; adjoint: 6-8 fluxes, 9-11 a_d, then the result per
     // component; linear: 6-8 the result, 9-11 V_d of the undifferentiated field
     if constexpr (MODE == 0) {
-// a_d along its lines: the three fields' derivatives of one line each
+      // a_d along its lines: the three fields' derivatives of one line each
       // are weighted by u and summed in registers
       items(3 * G2, [&](double* T, int t, int64_t) {
         const int d = t / G2, b = TG::base(d, t - d * G2), st = TG::stride(d);
@@ -389,8 +373,6 @@ template <int LX, int LXD>
 GLMat<LX, LXD> glmat(const ntg_dealias* d) {
   GLMat<LX, LXD> M;
   for (int q = 0; q < LXD * LX; ++q) M.J[q] = d->J[q];
-  for (int q = 0; q < LXD * LXD; ++q) M.D[q] = d->Dg[q];
-  for (int q = 0; q < LXD; ++q) M.w[q] = d->wg[q];
   return M;
 }
 
