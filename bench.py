@@ -991,10 +991,10 @@ def run_mma(args, local):
 
 def fp64_ax_roof(use, n, ncoef, t, pk, kind):
     """The FP64 operator against HBM.  Its contractions run in fixed point on
-    the integer pipes, which bound it; on the FP64 pipe its 116 flop per local
-    DOF would take longer than it does."""
+    the integer pipes; the 11 products per local DOF around them still bound it
+    on the FP64 pipe, on which its 116 flop would take longer than it does."""
     gbs = (2 + 6 + ncoef) * 8 * n / t / 1e9
-    return {"kernel": f"k_ax_fx<8> (FP64 Ax: {use})", "bound": "integer pipes", "achieved": round(gbs, 1),
+    return {"kernel": f"k_ax_fx<8> (FP64 Ax: {use})", "bound": "fp64 pipe", "achieved": round(gbs, 1),
             "peak": pk["hbm_gbs"], "unit": "GB/s", "frac": round(gbs / pk["hbm_gbs"], 4), "peak_source": kind,
             "ratio_to_fp64_pipe_roof": round(116.0 * n / t / 1e12 / FP64_TFLOPS, 3)}
 

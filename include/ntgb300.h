@@ -457,7 +457,11 @@ int ntg_filter_apply(ntg_plan* plan, ntg_ksp* ksp, double* X_out_d, const double
 /* stream).  The operators are Neko's (operators.f90: opgrad, dudxyz, cdtp, */
 /* conv1, curl) as the reference calls them; ntg_metrics_set must come     */
 /* first (it derives the cofactors drdx..dtdz, 1/jac and 1/gs(B) from the   */
-/* coordinates, as coef_t's generate_dxyz does).                            */
+/* coordinates, as coef_t's generate_dxyz does).  Contractions, here and in  */
+/* ntg_ax_helm, run in 60-bit integers per line of nodes, or in FP64 where   */
+/* one value exceeds its line's others eightfold or the exponents are        */
+/* extreme: the error is some roundings (2^-53) of the terms of the result's */
+/* own sum.                                                                  */
 /* ---------------------------------------------------------------------- */
 int ntg_metrics_set(ntg_plan* plan, const double* x_d, const double* y_d, const double* z_d);
 /* du = du/dx_dir, strong (dir 0..2) */
@@ -557,7 +561,10 @@ int ntg_mma_create(ntg_mma** mma, int64_t n, int m, const double* x_d, double a0
 int ntg_mma_destroy(ntg_mma* mma);
 /* mma_t%update (mma.f90:297-324): x_d (device, n) is replaced by the new
    design; df0dx_d device n; fval host m; dfdx_d device, the reference's
-   dfdx(m, n) layout (entry (i, j) at i + m j).  Synchronises the stream. */
+   dfdx(m, n) layout (entry (i, j) at i + m j).  Synchronises the stream.
+   With values that are not finite no Newton step is taken: the new design
+   is the middle of the move limits.  An optimiser keeps 23 + 3 m doubles
+   per variable on the device. */
 int ntg_mma_update(ntg_mma* mma, int iter, double* x_d, const double* df0dx_d, const double* fval,
                    const double* dfdx_d);
 /* mma_t%KKT (mma.f90:355-393): max and 2-norm of the KKT residual at x */

@@ -1,9 +1,12 @@
 // The FP64 matrix-free Helmholtz operator with its contractions in fixed
 // point on the integer pipes (fx.cuh).  With every product on the FP64 pipe it
-// took 28 clocks per node and SM, 1.9 ms at 16.8M nodes of lx = 8; here the
-// metric products and the conversions leave that pipe 5.5 and the integer pipes
-// bound it: 0.38 ms, against 0.18 for its 72 B per node.  One element per block
-// at lx = 8: sixteen blocks per SM keep the phases of different elements apart.
+// took 28 clocks per node and SM, 1.9 ms at 16.8M nodes of lx = 8; here it has
+// the 11 operations of the metric products and the mass term, 5.5 clocks, and
+// still bounds it: 0.38 ms are 7.1 clocks, against 0.18 ms for its 72 B per node
+// (counters at 2.1M nodes: FP64 pipe 64%, integer and logic 40, wide
+// multiply-adds 13, load/store 12, 1.7 instructions a clock and SM).  One
+// element per block at lx = 8: up to sixteen blocks per SM keep the phases of
+// different elements apart.
 #include <cmath>
 
 #include "common.cuh"
@@ -16,6 +19,7 @@ template <int LX>
 struct FxAxShape {
   static constexpr int LX2 = LX * LX, LX3 = LX2 * LX;
   static constexpr int RS = LX | 1, TILE = LX2 * RS;  // odd row stride: rows and columns without bank conflicts
+  // elements per block: their lines fill the warps (98% at lx 3, 5 and 6, 96 at 7, 95 at 9, 94 at 10)
   static constexpr int EPB = LX == 8 ? 1 : LX <= 3 ? 14 : LX == 4 ? 4 : LX == 6 ? 7 : LX <= 7 ? 5 : 3;
   static constexpr int NW = LX2 * EPB, NT = (NW + 31) / 32 * 32;
   static constexpr int MINB = LX == 8 ? 16 : 896 / NT;

@@ -197,18 +197,23 @@ void timer_stop(int id, cudaStream_t s);
 // with dependent_wait() may be launched by launch_dependent() while its
 // predecessor still runs: it waits for the predecessor's end (which waited for
 // everything before it) before it touches memory.  (Exceptions, each with its
-// reason: the coarse solve's matrices and stop flag.)  dependent_start() also lets
-// the successor be scheduled.  k_fdm leaves that out (0.4% of a solve at 43M
-// nodes for the instruction alone; the coarse solve relies on it), and the FP64 operator takes no part: with
-// its successors waiting beside it an FP64 solve at 0.26M nodes went from 38.7
-// to 43.9 ms, without from 38.7 to 35.1.
+// reason: the coarse solve's matrices and stop flag.)  dependent_start() also
+// lets the successor be scheduled.  k_fdm leaves that out (0.4% of a solve at 43M
+// nodes for the instruction alone; the coarse solve relies on it), and the FP64
+// operator takes no part: with its successors waiting beside it an FP64 solve at
+// 0.26M nodes went from 38.7 to 43.9 ms, without from 38.7 to 35.1.
 //
 // The waiting blocks take room from the kernel that runs, so from some size on
 // they cost more than the launches they hide.  Measured with and without, one
 // FP32 operator and preconditioner at lx = 8: 28.6 and 45.1 us at 0.26M nodes,
 // 58 and 70 us at 1M; a mixed Poisson solve: 7.6 and 9.5 ms at 2.1M, 12.0 and
 // 14.0 ms at 4.2M; the sequence of Brinkman solves at 8.4M: 43.0 and 41.8 ms;
-// operator and preconditioner at 33M: 696 and 639 us.
+// operator and preconditioner at 33M: 696 and 639 us.  Mixed Brinkman solves of
+// other orders: lx = 6, 15.4 and 17.9 ms at 3.0M, 34.5 and 34.5 at 7.1M; lx = 4,
+// 19.1 and 19.5 ms at 4.1M, 39.8 and 37.8 at 9.0M.  FP64 CG, where only the
+// gather-scatter and the vector kernels are launched so, gains little above the
+// line: 274 and 278 ms at 9.0M, 188 and 191 at 8.0M of lx = 5 (below, 57.7 and
+// 60.3 at 2.1M); the residuals' gather-scatters 1 to 2% at most.
 constexpr int64_t kDependentNodes = 6000000;
 __device__ __forceinline__ void dependent_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dependent_start() {

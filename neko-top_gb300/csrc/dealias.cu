@@ -16,9 +16,12 @@
 // so the three cdtp of a component become one transposed derivative and the
 // linear term needs none.  The contractions run in fixed point (fx.cuh): the
 // adjoint term of 24^3 elements, lx = 8, takes 5.3 ms where FP64 sums took
-// 22.5, the linear one of 315 elements, lx = 6, 63 us where they took 201.  The
-// integer pipes bound it, at 1.3 instructions per clock with the 14 warps that
-// the tiles of LXD^3 64-bit values leave room for.
+// 22.5, the linear one of 315 elements, lx = 6, 63 us where they took 201.
+// Latency bounds it: the tiles of LXD^3 64-bit values leave room for 14 warps per
+// SM at lx = 8, with some 20 barriers per element, and these issue 1.3
+// instructions per clock and SM, 2,960 per GL point (counters at 4096 elements:
+// integer and logic pipe 31% of its rate, FP64 29, wide multiply-adds 12,
+// load/store 6).
 #include <cmath>
 
 #include "deriv.cuh"
@@ -171,6 +174,7 @@ template <int LX, int LXD>
 struct AdvShape {
   using TG = fx::Tile<LXD>;
   static constexpr int G2 = LXD * LXD, G3 = G2 * LXD, L2 = LX * LX, L3 = L2 * LX, RS = TG::RS, TS = TG::SIZE;
+  // elements per block: nearly whole warps (432 of 448 threads at lxd 6, 441 of 448 at 7)
   static constexpr int EPB = LXD == 6 ? 4 : LXD == 7 ? 3 : 1;
   static constexpr int NT = (EPB * 3 * G2 + 31) / 32 * 32;  // a thread per line of three fields or directions
   static constexpr int EL = 12 * TS + (3 * G2 + 1) / 2;     // doubles per element: tiles, line exponents

@@ -33,6 +33,7 @@ struct Shape {
 template <int LX, int TILES>
 struct FxShape {
   static constexpr int L2 = LX * LX, L3 = L2 * LX, TS = fx::Tile<LX>::SIZE;
+  // elements per block: their 3 L2 lines fill the warps (100% at lx 2 and 4, 98 at 3 and 5, 96 at 6)
   static constexpr int EPB = LX <= 2 ? 16 : LX == 3 ? 7 : LX == 4 ? 4 : LX == 5 ? 5 : LX == 6 ? 2 : 1;
   // lx = 7 and 8: two whole passes over the nodes (256 against 192 threads at lx = 8: 2.50 and 2.56 ms for the
   // residuals at 24^3 elements)
@@ -62,7 +63,9 @@ int fx_grid(const ntg_plan* p) {
 // three (derivatives, fx::deriv_line / flux_line) and barriers between.
 // What bounds them is the FP64 pipe (2 operations per clock and SM), which
 // only the metric products still use; the contractions run beside them on
-// the integer pipes.  NODES / LINES number the work items of a block's ne
+// the integer pipes (k_vel_res, 4096 elements of lx = 8: FP64 pipe 67% of its
+// rate, integer and logic 37, wide multiply-adds 13, 1.7 instructions a clock).
+// NODES / LINES number the work items of a block's ne
 // elements: item t -> element el of the block, node or line.
 #define NTG_FX_PROLOGUE(TILES)                                                                  \
   using S = FxShape<LX, TILES>;                                                                 \

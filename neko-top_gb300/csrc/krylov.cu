@@ -46,7 +46,7 @@ struct DiagMats {
 template <int LX>
 struct DiagShape {
   static constexpr int L2 = LX * LX, L3 = L2 * LX, TS = fx::Tile<LX>::SIZE;
-  static constexpr int EPB = LX <= 2 ? 16 : LX == 3 ? 7 : LX == 4 ? 4 : LX == 5 ? 5 : LX == 6 ? 2 : 1;
+  static constexpr int EPB = LX <= 2 ? 16 : LX == 3 ? 7 : LX == 4 ? 4 : LX == 5 ? 5 : LX == 6 ? 2 : 1;  // as in dv::FxShape
   static constexpr int NT = (EPB * 3 * L2 + 31) / 32 * 32;
   static constexpr size_t SMEM = sizeof(double) * EPB * 3 * TS;
 };
@@ -1413,8 +1413,8 @@ int ntg_ksp_solve(ntg_ksp* ksp, double* x_d, const double* f_d, ntg_monitor* mon
     // application and two dots decide.  For the reliable-update mixed CG
     // the operator is the FP32 one: its image of the guess becomes the
     // initial residual, which the first FP64 residual replacement of that
-    // solver recomputes exactly (the FP64 operator costs 20x the FP32 one
-    // on GB300's FP64 pipe); every other solver takes the FP64 operator.
+    // solver recomputes exactly (the FP64 operator takes four times as long
+    // as the FP32 one); every other solver takes the FP64 operator.
     ntg_plan* p = ksp->plan;
     cudaStream_t s = p->stream;
     double xx = 0.0;

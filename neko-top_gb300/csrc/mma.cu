@@ -10,14 +10,16 @@
 // the reference, where they are scalars per rank.  Each Newton step is
 // a direction kernel and one per line-search trial, which also assembles the
 // next Newton system; each reduction is deterministic (per-block
-// partials summed in block order by the last block) and its m + 2 .. m(m+5)/2
-// totals come back in one small copy, the GPU stand-in for the reference's
+// partials summed in block order by the last block) and its 2 (direction) or
+// m (m + 5) / 2 + 2 totals come back in one small copy, the GPU stand-in for the reference's
 // MPI_Allreduce calls.  m <= 4 constraints.
 //
 // The FP64 pipe bounds it, mostly with the reciprocals (rcp.cuh): a design
 // update of 16.8M variables, m = 1, took 91.6 ms with the trial's residual and
 // the next Newton assembly in separate passes, each with divisions of its own,
-// and takes 56.0 with one (k_point).
+// and takes 56.0 with one (k_point: 86% of the pipe's rate).  What a trial leaves
+// for the next direction takes memory: 23 + 3 m vectors of n in all, 2 + m more
+// than with separate passes.
 #include <cmath>
 #include <vector>
 
