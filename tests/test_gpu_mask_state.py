@@ -129,5 +129,5 @@ def test_first_solve_keeps_weights_of_one_precision(pkg, orc, dev, method, bytes
         return before - torch.cuda.mem_get_info()[0], c.n
 
     (a, n), (b, _) = allocated(True), allocated(False)
-    # the driver hands memory out in pieces of 2 MiB
+    # device memory is handed out in pieces of 2 MiB
     assert abs(a - b - bytes_per_node * n) <= 1 << 21
