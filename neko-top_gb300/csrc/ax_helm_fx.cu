@@ -28,6 +28,9 @@ struct FxAxShape {
 
 // FIELD: h1 is a field (the fluxes' guard, fx::flux_line); null otherwise.  The
 // pointer is tested all the same: products by h1s alone would be predicated.
+// 16.8M nodes of lx = 8: constant h1 368 us; a smooth field 484 (444 without the
+// guard), one that jumps between 1e-3 and 1 from node to node 660, where FP64
+// sums throughout took 1979.
 template <int LX, bool FIELD, bool DOT>
 __global__ void __launch_bounds__(FxAxShape<LX>::NT, FxAxShape<LX>::MINB)
     k_ax_fx(double* __restrict__ w, const double* __restrict__ u, const double* __restrict__ g11,
